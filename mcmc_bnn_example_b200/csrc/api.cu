@@ -13,25 +13,22 @@
 
 #include <algorithm>
 #include <limits>
+#include <mutex>
 #include <random>
 #include <string>
 #include <vector>
-
-#include <thrust/random.h>
 
 #include "../../include/mcmc_b200.h"
 #include "chain.cuh"
 #include "common.cuh"
 #include "philox.h"
+#include "refstream.cuh"
 
 using namespace mcmc_b200;
 
 #define API extern "C" __attribute__((visibility("default")))
 
 static thread_local std::string g_last_error;
-// the one-launch-per-iteration path for single-window contexts: opt-in (MCMC_B200_MULTISTEP=1) while
-// false, opt-out (MCMC_B200_NO_MULTISTEP=1) while true
-static constexpr bool MULTISTEP_DEFAULT = false;
 
 static int fail(int code, const std::string& msg) {
   g_last_error = msg;
@@ -97,6 +94,42 @@ constexpr int kNcclChar = 0;
 constexpr int kNcclSum = 0;
 }  // namespace
 
+constexpr int HB_FLOATS = 3076;  // P of the widest model, rounded up
+struct HostBlock {
+  double scalars[2];
+  int status, pad[3];
+  float w[HB_FLOATS], m[HB_FLOATS], g[HB_FLOATS];  // in: position, momentum, gradient
+  float w_out[HB_FLOATS], m_out[HB_FLOATS], g_out[HB_FLOATS];
+};
+
+// Page-locking takes milliseconds, so the blocks of destroyed contexts are kept for the next ones: at most
+// HB_CHUNK of them, one allocation, returned when the process ends.  Any thread may take and give.
+constexpr int HB_CHUNK = 16;
+static std::mutex g_hb_mutex;
+static HostBlock* g_hb_chunk = nullptr;
+static unsigned g_hb_used = 0;  // bit i: block i of the chunk is taken
+static HostBlock* host_block_take() {
+  std::lock_guard<std::mutex> lock(g_hb_mutex);
+  if (!g_hb_chunk) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(HostBlock) * HB_CHUNK, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    g_hb_chunk = static_cast<HostBlock*>(p);
+  }
+  for (int i = 0; i < HB_CHUNK; ++i)
+    if (!(g_hb_used >> i & 1u)) {
+      g_hb_used |= 1u << i;
+      return g_hb_chunk + i;
+    }
+  void* p = nullptr;  // more contexts than that at once: a block of its own
+  return cudaHostAlloc(&p, sizeof(HostBlock), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess
+             ? static_cast<HostBlock*>(p) : nullptr;
+}
+static void host_block_give(HostBlock* b) {
+  std::lock_guard<std::mutex> lock(g_hb_mutex);
+  if (b >= g_hb_chunk && b < g_hb_chunk + HB_CHUNK) g_hb_used &= ~(1u << (b - g_hb_chunk));
+  else cudaFreeHost(b);
+}
+
 struct mcmc_b200_ctx {
   mcmc_b200_config cfg;
   int device = 0, W = 0, P = 0, Pp = 0;
@@ -152,9 +185,16 @@ struct mcmc_b200_ctx {
   unsigned int *os_seq = nullptr, *os_done = nullptr;
   unsigned int os_poll_limit = 1u << 22;    // polls of about 0.1 us .. 1 us each
   long long launches = 0;
-  // all L leapfrog steps of an iteration in one cooperative launch (one window, TF32, H = 40)
-  bool multistep = false;
-  unsigned int* grid_bar = nullptr;
+  // whole iterations in one cooperative launch (resident.cuh): plans and message buffers of the chain launches
+  // and of the single-window explicit calls; null where the rows do not fit on the chip
+  bool res_ok = false, res_x_ok = false;
+  ResidentParams res, res_x;
+  int res_cluster = 1, res_x_cluster = 1;  // CTAs per cluster
+  // host block the kernels of the explicit host-pointer calls read and write directly (mapped, page-locked)
+  HostBlock* hb = nullptr;
+  // small device arrays are cut from zeroed slabs
+  char* slab = nullptr;
+  size_t slab_left = 0;
   float* stage = nullptr;  // upload staging for one window: [rows][D] then [rows]
   // forward-only pass over the stored samples: scratch that grows on demand and is kept (no allocation per call)
   float* fwd_x = nullptr;
@@ -167,14 +207,31 @@ struct mcmc_b200_ctx {
   std::vector<void*> allocs;
 };
 
+// Device memory of the context.  Small arrays share zeroed slabs: a context has some forty of them, and an
+// allocator call each (they synchronise the device) was most of the time to create one.
+constexpr size_t SLAB_BYTES = 1u << 20, SLAB_MAX = 16u << 10;
 static int dalloc(mcmc_b200_ctx* c, void** p, size_t bytes, bool zero = true) {
-  if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMalloc(p, bytes);
+  bytes = (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
+  const bool small = bytes <= SLAB_MAX;
+  if (small && bytes <= c->slab_left) {
+    *p = c->slab;
+    c->slab += bytes;
+    c->slab_left -= bytes;
+    return MCMC_B200_OK;
+  }
+  const size_t take = small ? SLAB_BYTES : bytes;
+  cudaError_t e = cudaMalloc(p, take);
   if (e != cudaSuccess) return fail(MCMC_B200_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   c->allocs.push_back(*p);
-  if (zero) {
-    e = cudaMemset(*p, 0, bytes);
+  if (zero || small) {
+    // waited for here: what fills the array next may be queued on another stream
+    e = cudaMemsetAsync(*p, 0, take, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, std::string("cudaMemset: ") + cudaGetErrorString(e));
+  }
+  if (small) {
+    c->slab = (char*)*p + bytes;
+    c->slab_left = take - bytes;
   }
   return MCMC_B200_OK;
 }
@@ -272,6 +329,78 @@ static int build_work_table(mcmc_b200_ctx* c, int windows, long long tiles_per_w
                             int chunks_per_window, int** d_seg_ptr, int4** d_segs, int** d_nslot,
                             int* n_ctas, int* max_slots);
 
+// How a window of `rows` rows is dealt to clusters when `windows` of them share the GPU (resident.cuh).  max_clusters[i]
+// = clusters of 1 << i CTAs that can be resident.  False when the rows do not fit.
+//   * one cluster per window, of the most CTAs (8, 4, 2, 1) that every window can have, if that holds the rows: the
+//     exchange then never leaves the cluster;
+//   * rows that one cluster of 8 cannot hold: as many clusters of 8 as every window can have (up to 16) while each
+//     CTA still has at least four 32-row units (below that the step is all exchange and more CTAs only add to it).
+static bool resident_plan(long long rows, int windows, const int max_clusters[4], int* cluster, int* clusters) {
+  const long long units = (rows + 31) / 32;
+  for (int i = 3; i >= 0; --i)
+    if (windows <= max_clusters[i] && units <= (long long)RES_UNITS << i) {
+      *cluster = 1 << i;
+      *clusters = 1;
+      return true;
+    }
+  const long long have = std::min<long long>(max_clusters[3] / windows, RES_MAX_CLUSTERS);
+  const long long need = (units + 8 * RES_UNITS - 1) / (8 * RES_UNITS);
+  if (need > have) return false;
+  *cluster = 8;
+  *clusters = (int)std::max(need, std::min(have, units / 32));
+  return true;
+}
+
+// 16-byte words of one rank and cluster through L2 (resident.cuh: STR)
+static size_t resident_words_stride(int P, int cluster) {
+  const size_t words = (size_t)(P + 5) / 3;
+  return ((words + cluster - 1) / cluster + 7) / 8 * 8;
+}
+
+// Plans the resident launches of a context and allocates their message buffers.  A fixed `slices` asks for bits
+// that do not depend on what shares the launch: such contexts keep one launch per step.
+static int resident_setup(mcmc_b200_ctx* c) {
+  const char* off = getenv("MCMC_B200_NO_MULTISTEP");
+  if ((off && off[0] == '1') || c->cfg.slices > 0 || c->cfg.precision != MCMC_B200_PREC_TF32 || c->cfg.H != 40)
+    return MCMC_B200_OK;
+  // (asked once per device: the queries cost as much as the rest of a small context)
+  static std::mutex mutex;
+  static int known[64][4];
+  static bool asked[64] = {};
+  int max_clusters[4];
+  {
+    std::lock_guard<std::mutex> lock(mutex);
+    const int d = c->device & 63;
+    if (!asked[d]) {
+      for (int i = 0; i < 4; ++i)
+        if (launch_resident_tf32(1 << i, nullptr, c->res, nullptr, &known[d][i]) != cudaSuccess) {
+          cudaGetLastError();
+          known[d][i] = 0;
+        }
+      asked[d] = true;
+    }
+    memcpy(max_clusters, known[d], sizeof max_clusters);
+  }
+  for (int k = 0; k < 2; ++k) {
+    ResidentParams& g = k ? c->res_x : c->res;
+    int& cluster = k ? c->res_x_cluster : c->res_cluster;
+    memset(&g, 0, sizeof g);
+    g.windows = k ? 1 : c->W;
+    if (!resident_plan(c->rows, g.windows, max_clusters, &cluster, &g.clusters)) continue;
+    g.n_rows = (int)c->rows;
+    g.rows_pad = (int)c->rows_pad;
+    g.Pp = c->Pp;
+    g.lik = make_lik(c->cfg);
+    g.prior = make_prior(c->cfg);
+    g.status = c->status;
+    int r = dalloc(c, (void**)&g.msg, (size_t)2 * g.windows * g.clusters * cluster * resident_words_stride(c->P, cluster) * 16);
+    if (r == MCMC_B200_OK) r = dalloc(c, (void**)&g.seq, (size_t)g.windows * 4);
+    if (r) return r;
+    (k ? c->res_x_ok : c->res_ok) = true;
+  }
+  return MCMC_B200_OK;
+}
+
 API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows, int64_t rows,
                          mcmc_b200_ctx** out) {
   if (!cfg || !out || n_windows < 1 || rows < 1) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
@@ -296,9 +425,10 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
     return fail(MCMC_B200_ERR_CUDA, "no CUDA device: this library has no CPU path");
   if (device < 0 || device >= ndev) return fail(MCMC_B200_ERR_INVALID, "device ordinal out of range");
   CK(cudaSetDevice(device));
-  cudaDeviceProp prop;
-  CK(cudaGetDeviceProperties(&prop, device));
-  if (prop.major != 10)
+  int cc_major = 0, sm_count = 0;  // (two attributes: the whole property record takes milliseconds)
+  CK(cudaDeviceGetAttribute(&cc_major, cudaDevAttrComputeCapabilityMajor, device));
+  CK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+  if (cc_major != 10)
     return fail(MCMC_B200_ERR_UNSUPPORTED, "kernels are built for sm_100a (B200) only");
 
   mcmc_b200_ctx* c = new mcmc_b200_ctx();
@@ -309,7 +439,7 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
   c->rows_pad = (rows + TF32_TILE - 1) / TF32_TILE * TF32_TILE;
   c->P = cfg->D * cfg->H + 2 * cfg->H + 1;
   c->Pp = (c->P + 3) / 4 * 4;
-  c->num_sms = prop.multiProcessorCount;
+  c->num_sms = sm_count;
   const bool tf32 = cfg->precision == MCMC_B200_PREC_TF32;
   c->tile_rows = tf32 ? TF32_TILE : fp32_tile_rows(cfg->H);
   c->ctas_per_sm = tf32 ? 1 : fp32_max_ctas_per_sm(cfg->H);
@@ -357,17 +487,6 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
   // every CTA of the next launch summing all of them in its prologue
   c->use_red = c->slices > 4;
   c->use_red_x = c->slices_x > 4;
-  {
-    // one window on the whole GPU: run the L steps of an iteration as ONE cooperative launch (the CTAs
-    // meet at a grid barrier after every step).  Needs every CTA resident, the sums in `red` (use_red) and
-    // the free partition (a fixed `slices` asks for placement-independent bits: keep one launch per step).
-    const char* off = getenv("MCMC_B200_NO_MULTISTEP");
-    const char* on = getenv("MCMC_B200_MULTISTEP");
-    const bool want = MULTISTEP_DEFAULT ? !(off && off[0] == '1') : (on && on[0] == '1');
-    c->multistep = tf32 && n_windows == 1 && cfg->slices == 0 && c->use_red && cfg->leapfrog_steps >= 2 &&
-                   want && c->tab_ctas > 0 && c->tab_ctas <= tf32_multistep_max_ctas(cfg->H) &&
-                   (c->P + c->tab_ctas - 1) / c->tab_ctas <= 12;
-  }
   const size_t W = n_windows, Pp = c->Pp, P = c->P;
   DA(c->xaug, W * c->rows_pad * KP * sizeof(float));
   for (int i = 0; i < 2; ++i) {
@@ -392,7 +511,6 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
   DA(c->n_accept, W * 4);
   DA(c->gwin, W * 8);
   DA(c->status, 4);
-  DA(c->grid_bar, 4);
   DA(c->xg, Pp * 4);
   DA(c->g_out, Pp * 4);
   DA(c->row_loss, (size_t)c->rows_pad * 4);
@@ -414,8 +532,23 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
     int r_ = make_tensor_map(c);
     if (r_ != MCMC_B200_OK) { mcmc_b200_destroy(c); return r_; }
   }
+  {
+    int r_ = resident_setup(c);
+    if (r_ != MCMC_B200_OK) { mcmc_b200_destroy(c); return r_; }
+  }
+  c->hb = host_block_take();
+  if (!c->hb) {
+    mcmc_b200_destroy(c);
+    return fail(MCMC_B200_ERR_NOMEM, "cudaHostAlloc failed");
+  }
+  memset(c->hb, 0, sizeof(HostBlock));
   std::vector<float> e(W, (float)cfg->eps0);
-  cudaMemcpy(c->eps, e.data(), W * 4, cudaMemcpyHostToDevice);
+  cudaError_t e_end = cudaMemcpyAsync(c->eps, e.data(), W * 4, cudaMemcpyHostToDevice, c->stream);
+  if (e_end == cudaSuccess) e_end = cudaStreamSynchronize(c->stream);
+  if (e_end != cudaSuccess) {
+    mcmc_b200_destroy(c);
+    return fail(MCMC_B200_ERR_CUDA, std::string("context set-up: ") + cudaGetErrorString(e_end));
+  }
   *out = c;
   return MCMC_B200_OK;
 }
@@ -546,6 +679,7 @@ API void mcmc_b200_destroy(mcmc_b200_ctx* c) {
     if (p) cudaIpcCloseMemHandle(p);
   if (c->comm && g_nccl.ok) g_nccl.CommDestroy(c->comm);
   for (void* p : c->allocs) cudaFree(p);
+  if (c->hb) host_block_give(c->hb);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -553,11 +687,17 @@ API void mcmc_b200_destroy(mcmc_b200_ctx* c) {
 API int mcmc_b200_num_params(const mcmc_b200_ctx* c) { return c ? c->P : -1; }
 API void* mcmc_b200_stream(mcmc_b200_ctx* c) { return c ? (void*)c->stream : nullptr; }
 
+static int finish_status(mcmc_b200_ctx* c);
 static int check_status(mcmc_b200_ctx* c) {
-  int st = 0;
-  CK(cudaMemcpyAsync(&st, c->status, 4, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(&c->hb->status, c->status, 4, cudaMemcpyDeviceToHost, c->stream));
+  return finish_status(c);
+}
+// waits for the context's stream and reports the status word that has arrived in the host block
+static int finish_status(mcmc_b200_ctx* c) {
   CK(cudaStreamSynchronize(c->stream));
+  const int st = c->hb->status;
   if (st != 0) {
+    c->hb->status = 0;
     cudaMemsetAsync(c->status, 0, 4, c->stream);
     char b[96];
     snprintf(b, sizeof b, "device-side wait ran out (code %d)", st);
@@ -714,7 +854,6 @@ static AcceptParams base_accept_params(mcmc_b200_ctx* c) {
 }
 
 // ---- the reference's random streams (main.h:207-216, :235-239): the libraries' own engines ----------
-constexpr uint64_t REF_DRAWS_PER_ITER = 962;  // 961 momenta + 1 accept draw per iteration (main.h:216,237)
 static float refstream_log_uniform(uint64_t seed) {
   // main.h:235-239: a fresh engine per draw, U(FLT_MIN, 1), log() evaluated in double and narrowed
   std::default_random_engine engine;
@@ -837,44 +976,30 @@ static int chain_grad(mcmc_b200_ctx* c, int mode, int s, cudaStream_t st) {
   return MCMC_B200_OK;
 }
 
-// All L gradient evaluations of one iteration in one cooperative launch (chain_grad's L launches folded
-// into one; same buffers, same rotation).
-static int chain_grad_multistep(mcmc_b200_ctx* c, cudaStream_t st) {
-  GradParams g = base_grad_params(c);
-  g.slices_in = g.slices_out = c->slices;
-  g.nslot_in = c->tab_nslot;
-  g.seg_ptr = c->tab_seg_ptr;
-  g.segs = c->tab_segs;
-  g.g_carried = c->g_cur;
-  g.eps = c->eps;
+// n_iter HMC iterations in cooperative launches that keep the rows on the chip.  A launch is kept to about a
+// tenth of a second so that other work on the GPU gets its turn.
+static int resident_chain(mcmc_b200_ctx* c, int n_iter, cudaStream_t st) {
+  ResidentParams g = c->res;
+  g.mode = RES_CHAIN;
   g.n_steps = c->cfg.leapfrog_steps;
-  g.n_slots = c->slices;    // one window: the CTAs that own tiles of it, one partial vector each
-  for (int i = 0; i < 2; ++i) {
-    g.w_buf[i] = c->wbuf[i];
-    g.m_buf[i] = c->mbuf[i];
-    g.partial_buf[i] = c->partial[i];
-    g.ll_buf[i] = c->llp[i];
+  g.a = base_accept_params(c);
+  fill_chain_accept(c, g.a, ACC_ITERATE, g.n_steps);
+  const int per_launch = std::max(1, 20000 / g.n_steps);
+  for (int done = 0; done < n_iter; done += g.n_iter) {
+    g.n_iter = std::min(per_launch, n_iter - done);
+    cudaError_t e = launch_resident_tf32(c->res_cluster, &c->tmap_mn, g, st, nullptr);
+    c->launches++;
+    if (e != cudaSuccess)
+      return fail(MCMC_B200_ERR_CUDA, std::string("resident chain launch: ") + cudaGetErrorString(e));
   }
-  g.red = c->red;
-  g.grid_bar = c->grid_bar;
-  CK(cudaMemsetAsync(c->grid_bar, 0, 4, st));
-  cudaError_t e = launch_grad_tf32_multistep(c->cfg.H, &c->tmap_mn, g, c->tab_ctas, st);
-  c->launches++;
-  if (e != cudaSuccess)
-    return fail(MCMC_B200_ERR_CUDA, std::string("multi-step gradient kernel launch: ") + cudaGetErrorString(e));
   return MCMC_B200_OK;
 }
 
 static int queue_iteration(mcmc_b200_ctx* c, cudaStream_t st) {
   const int L = c->cfg.leapfrog_steps;
-  if (c->multistep) {
-    int r = chain_grad_multistep(c, st);
+  for (int s = 0; s < L; ++s) {
+    int r = chain_grad(c, s == 0 ? MODE_FIRST : MODE_NEXT, s, st);
     if (r) return r;
-  } else {
-    for (int s = 0; s < L; ++s) {
-      int r = chain_grad(c, s == 0 ? MODE_FIRST : MODE_NEXT, s, st);
-      if (r) return r;
-    }
   }
   AcceptParams a = base_accept_params(c);
   fill_chain_accept(c, a, ACC_ITERATE, L);
@@ -938,6 +1063,11 @@ API int mcmc_b200_run_chain_async(mcmc_b200_ctx* c, int n_iter) {
     int r = refstream_fill(c, c->iters_done + n_iter);
     if (r) return r;
   }
+  if (c->res_ok && !c->comm && !c->oneshot) {
+    int r = resident_chain(c, n_iter, c->stream);
+    if (r == MCMC_B200_OK) c->iters_done += n_iter;
+    return r;
+  }
   // One HMC iteration (L gradient launches + the accept kernel) is captured
   // once and replayed: launch cost stays off the critical path.
   if (!c->graph_tried) {
@@ -958,7 +1088,7 @@ API int mcmc_b200_run_chain_async(mcmc_b200_ctx* c, int n_iter) {
     c->launches = launches_before;
   }
   const long long per_iter =
-      c->multistep ? 2 : (long long)c->cfg.leapfrog_steps * ((c->comm || c->use_red || c->oneshot) ? 2 : 1) + 1;
+      (long long)c->cfg.leapfrog_steps * ((c->comm || c->use_red || c->oneshot) ? 2 : 1) + 1;
   for (int i = 0; i < n_iter; ++i) {
     if (c->graph_exec) {
       CK(cudaGraphLaunch(c->graph_exec, c->stream));
@@ -1147,6 +1277,35 @@ API int mcmc_b200_checkpoint_load(mcmc_b200_ctx* c, const void* host_buf, uint64
 }
 
 // ---- explicit-state calls (one window) -------------------------------------
+// The same in one launch where the window's rows fit on the chip.  Pointers may be device memory or the mapped
+// host block.
+static int resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, const float* w0, const float* m0,
+                          const float* g0, float* w_last, float* m_last, float* g_out, float* zero_out,
+                          float* row_loss, float* prior_loss, double* scalars, cudaStream_t st, bool eval_only) {
+  ResidentParams g = c->res_x;
+  g.mode = eval_only ? RES_EVAL : RES_STEPS;
+  g.n_steps = L;
+  g.n_iter = 1;
+  g.data_window0 = data_window;
+  g.status_host = &c->hb->status;
+  g.w0 = w0;
+  g.m0 = m0;
+  g.g0 = g0;
+  g.eps_scalar = eps;
+  g.w_out = w_last;
+  g.m_out = m_last;
+  g.g_out = g_out;
+  g.zero_out = zero_out;
+  g.row_loss = row_loss;
+  g.prior_loss = prior_loss;
+  g.scalars = scalars;
+  cudaError_t e = launch_resident_tf32(c->res_x_cluster, &c->tmap_mn, g, st, nullptr);
+  c->launches++;
+  if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, std::string("resident launch: ") + cudaGetErrorString(e));
+  return MCMC_B200_OK;
+}
+static bool use_resident_x(const mcmc_b200_ctx* c) { return c->res_x_ok && !c->comm && !c->oneshot; }
+
 // L leapfrog steps from (w0, m0, g0) on device; results in xw/xm[L&1], g_out, scalars.
 static int explicit_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, const float* w0,
                           const float* m0, const float* g0, float* w_last, float* m_last,
@@ -1208,6 +1367,21 @@ API int mcmc_b200_potential_and_grad(mcmc_b200_ctx* c, int window, const float* 
   if (!c || !w || window < 0 || window >= c->W) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
   if (!c->window_set[window]) return fail(MCMC_B200_ERR_INVALID, "window has no data yet");
   CK(cudaSetDevice(c->device));
+  if (use_resident_x(c)) {
+    // parameters, gradient and sums go through the mapped host block: one launch and one wait, no copies
+    memcpy(c->hb->w, w, (size_t)c->P * 4);
+    int r = resident_steps(c, window, 1, 0.f, c->hb->w, nullptr, nullptr, nullptr, nullptr, c->hb->g_out, nullptr,
+                           row_loss ? c->row_loss : nullptr, nullptr, c->hb->scalars, c->stream, true);
+    if (r) return r;
+    if (row_loss)
+      CK(cudaMemcpyAsync(row_loss, c->row_loss, (size_t)c->rows * 4, cudaMemcpyDeviceToHost, c->stream));
+    r = finish_status(c);
+    if (r) return r;
+    if (grad) memcpy(grad, c->hb->g_out, (size_t)c->P * 4);
+    if (loglik) *loglik = c->hb->scalars[0];
+    if (logprior) *logprior = c->hb->scalars[1];
+    return MCMC_B200_OK;
+  }
   CK(cudaMemcpyAsync(c->xw[0], w, (size_t)c->P * 4, cudaMemcpyHostToDevice, c->stream));
   int r = explicit_steps(c, window, 1, 0.f, c->xw[0], c->xm[0], c->xg, nullptr, nullptr, c->g_out,
                          row_loss ? c->row_loss : nullptr, nullptr, c->stream, true);
@@ -1232,6 +1406,22 @@ API int mcmc_b200_leapfrog(mcmc_b200_ctx* c, int window, int L, float eps, const
   if (!c->window_set[window]) return fail(MCMC_B200_ERR_INVALID, "window has no data yet");
   CK(cudaSetDevice(c->device));
   const size_t n = (size_t)c->P * 4;
+  if (use_resident_x(c)) {
+    HostBlock* h = c->hb;
+    memcpy(h->w, w_prev, n);
+    memcpy(h->m, mom_prev, n);
+    memcpy(h->g, grad_prev, n);
+    int r = resident_steps(c, window, L, eps, h->w, h->m, h->g, h->w_out, h->m_out, h->g_out, nullptr, nullptr, nullptr,
+                           h->scalars, c->stream, false);
+    if (r == MCMC_B200_OK) r = finish_status(c);
+    if (r) return r;
+    if (w_next) memcpy(w_next, h->w_out, n);
+    if (mom_next) memcpy(mom_next, h->m_out, n);
+    if (grad_cur) memcpy(grad_cur, h->g_out, n);
+    if (loglik) *loglik = h->scalars[0];
+    if (logprior) *logprior = h->scalars[1];
+    return MCMC_B200_OK;
+  }
   CK(cudaMemcpyAsync(c->xw[0], w_prev, n, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->xm[0], mom_prev, n, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->xg, grad_prev, n, cudaMemcpyHostToDevice, c->stream));
@@ -1272,6 +1462,9 @@ API int mcmc_b200_mcmc_step(mcmc_b200_ctx* c, const float* x, const float* y, co
     c->window_set[0] = 1;
     repacked = true;
   }
+  if (use_resident_x(c))
+    return resident_steps(c, 0, L, eps, weights_prev, mom_prev, grad_prev, weights_next, mom_next, grad_cur, grad_next,
+                          loss_values, loss_values ? loss_values + c->rows : nullptr, c->scalars, st, false);
   int r = explicit_steps(c, 0, L, eps, weights_prev, mom_prev, grad_prev, weights_next, mom_next, grad_cur,
                          loss_values, loss_values ? loss_values + c->rows : nullptr, st, false, repacked);
   if (r) return r;
@@ -1419,7 +1612,6 @@ API int mcmc_b200_enable_row_sharding(mcmc_b200_ctx* c, const unsigned char id[1
   }
   c->rank = rank;
   c->nranks = nranks;
-  c->multistep = false;  // every step's sums cross GPUs: one launch + one all-reduce per step
   drop_graph(c);         // a graph captured before this call has neither the sums nor the all-reduce in it
   return MCMC_B200_OK;
 }
@@ -1472,7 +1664,6 @@ static int oneshot_setup(mcmc_b200_ctx* c, bool fake_peers) {
     CK(cudaStreamSynchronize(c->stream));
   }
   c->oneshot = true;
-  c->multistep = false;
   drop_graph(c);
   return MCMC_B200_OK;
 }

@@ -11,25 +11,14 @@
 //   * repack_kernel — [N][22] + [N] -> [N_pad][24] rows {x, 1, y}.
 //   * reduce_partials_kernel — row sharding: the vector that is all-reduced.
 //   * log_acpt_kernel — the drop-in accept ratio on caller buffers.
-#include <thrust/random.h>
-
 #include "common.cuh"
 #include "chain.cuh"
 #include "philox.h"
+#include "refstream.cuh"
 
 namespace mcmc_b200 {
 
 constexpr int ACC_THREADS = 256;
-
-// One momentum draw of the reference's stream (main.h:207-213): a fresh Thrust engine advanced by n,
-// one N(0,1) draw.  Thrust's own code does the work, as it does in the reference.
-__device__ __forceinline__ float refstream_normal(unsigned long long n) {
-  thrust::default_random_engine engine;
-  engine.discard(n);
-  thrust::normal_distribution<float> unit_normal(0.f, 1.f);
-  return unit_normal(engine);
-}
-constexpr unsigned long long REF_DRAWS_PER_ITER = 962;  // 961 momenta + 1 accept draw (main.h:216,237)
 
 __global__ void __launch_bounds__(ACC_THREADS) hmc_accept_kernel(const AcceptParams a) {
   __shared__ double dsc[32];

@@ -111,6 +111,37 @@ cudaError_t launch_log_acpt(const float* prev_loss, const float* new_loss, long 
                             const float* prev_mom, const float* new_mom, const float* grad_cur, int P,
                             float eps, float* out, cudaStream_t st);
 
+// One cooperative launch for whole iterations / trajectories / evaluations of windows that fit on the chip
+// (resident.cuh)
+enum ResidentMode : int {
+  RES_CHAIN = 0,  // n_iter HMC iterations of n_steps leapfrog steps from the chain state in `a`
+  RES_STEPS = 1,  // n_steps leapfrog steps from (w0, m0, g0)
+  RES_EVAL = 2    // log density and gradient at w0
+};
+constexpr int RES_UNITS = 16;          // 32-row units per CTA
+constexpr int RES_MAX_CLUSTERS = 16;   // clusters of one window
+struct ResidentParams {
+  int mode, n_steps, n_iter;
+  int windows, clusters;    // clusters per window
+  int data_window0, n_rows, rows_pad, Pp;
+  uint4* msg;               // [2][windows][ranks][clusters][words] cluster sums
+  unsigned int* seq;        // [windows] last sequence number used
+  LikParams lik;
+  PriorParams prior;
+  int* status;
+  int* status_host;         // optional: the same code for the host to read without a copy
+  // RES_STEPS / RES_EVAL (one window); all outputs but g_out and scalars are optional
+  const float *w0, *m0, *g0;
+  float eps_scalar;
+  float *w_out, *m_out, *g_out, *zero_out, *row_loss, *prior_loss;
+  double* scalars;          // [2] log-likelihood, log-prior
+  AcceptParams a;           // RES_CHAIN
+};
+// The launch, for clusters of `cluster` CTAs (1, 2, 4, 8); or, when max_clusters is given, only the number of such
+// clusters that can be resident at once
+cudaError_t launch_resident_tf32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
+                                 int* max_clusters);
+
 // gradient kernels
 cudaError_t launch_grad_fp32(int H, const GradParams& g, int slices, int windows, cudaStream_t st);
 int fp32_max_ctas_per_sm(int H);
@@ -120,9 +151,6 @@ int fp32_tile_rows(int H);
 // dataset that stages a row tile with the 32-byte-chunk swizzle
 cudaError_t launch_grad_tf32(int H, const void* tmap_mn, const GradParams& g, int ctas, cudaStream_t st);
 int tf32_supported(int H);
-int tf32_multistep_max_ctas(int H);
-cudaError_t launch_grad_tf32_multistep(int H, const void* tmap_mn, const GradParams& g, int ctas,
-                                       cudaStream_t st);
 cudaError_t launch_grad_tf32_wide(const void* tmap_mn, const GradParams& g, int ctas, cudaStream_t st);
 constexpr int TF32_TILE = 128;
 

@@ -121,42 +121,7 @@ __device__ __forceinline__ void store_e_pairs(const uint32_t* e_ptr, const uint6
   (store_e_pair<Js>(e_ptr, hp, dy2, ndy2, dw1p), ...);
 }
 
-// One CTA's share of the cross-CTA sum inside a multi-step launch: parameters
-// [blockIdx.x * per_cta, ...) summed over the n_slots partial vectors in a fixed order (one warp per
-// parameter: lane l adds slots l, l+32, ..., then a shuffle tree).  Called by the 12 compute warps.
-__device__ __forceinline__ void sum_partials_slice(const GradParams& g, const float* partial_out,
-                                                   const double* ll_out, int tid) {
-  const int nb = (int)gridDim.x;
-  const int per_cta = (g.P + nb - 1) / nb;  // <= 12 (one per compute warp)
-  const int q = tid >> 5, lane = tid & 31;
-  const int p = (int)blockIdx.x * per_cta + q;
-  if (q < per_cta && p < g.P) {
-    const float* src = partial_out + p;
-    float acc = 0.f;
-#pragma unroll 5
-    for (int sidx = lane; sidx < g.n_slots; sidx += 32) acc += __ldcg(src + (size_t)sidx * g.Pp);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) g.red[p] = (double)acc;
-  }
-  if (blockIdx.x == (unsigned)(nb - 1) && q == 11) {  // log-likelihood, and the padding of the sum vector
-    double l = 0.0;
-    for (int sidx = lane; sidx < g.n_slots; sidx += 32) l += __ldcg(ll_out + sidx);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if (lane == 0) {
-      g.red[g.Pp] = l;
-      for (int k = g.P; k < g.Pp; ++k) g.red[k] = 0.0;
-    }
-  }
-}
-
-// MULTI = several leapfrog steps of ONE window in one cooperative launch (GradParams::n_steps): after
-// every step the CTAs meet at a grid-wide barrier, each CTA sums a few parameters' partials over all
-// CTAs into GradParams::red, they meet again, and the next step's prologue reads the sums.  This is
-// the reference's persistent-kernel structure (mcmc_step_kernel + sync_and_swap,
-// mcmc_step_tc.h:597-677) with a bounded barrier and a fixed-order sum instead of atomics.
-template <int H, bool MULTI>
+template <int H>
 __global__ void __launch_bounds__(TF32_THREADS, 1)
 grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g) {
   using G = Tf32Geom<H>;
@@ -214,9 +179,6 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
   const uint32_t w0s_addr = smem_u32(w0s);
   const int seg0 = g.seg_ptr[blockIdx.x], seg1 = g.seg_ptr[blockIdx.x + 1];  // host-written table
   bool ok = true;
-  // (every CTA of a multi-step launch owns at least one segment: the host only uses it when all CTAs have tiles)
-  const int nseg = seg1 - seg0;
-  const int n_iters = MULTI ? g.n_steps * nseg : nseg;
   // everything above is private set-up; from here on the kernel reads what its predecessor wrote
   pdl_trigger();
   pdl_wait();
@@ -229,10 +191,7 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
     // the warpgroup this warp issues for, in a form the compiler can see is the same in every lane
     const int wg = __shfl_sync(0xffffffffu, warp - NWG * 4, 0);
     uint32_t c_issued = 0;  // tiles of this warpgroup whose MMAs have been issued (mbarrier phases follow it)
-    bool alive = true;
-    // a multi-step launch walks its segments once per step: ONE loop over (step, segment) pairs
-    for (int it = 0; it < n_iters; ++it) {
-      const int sg = MULTI ? seg0 + it % nseg : seg0 + it;
+    for (int sg = seg0; sg < seg1; ++sg) {
       const int4 seg = g.segs[sg];
       const int win = seg.x, t0 = seg.y, nt = seg.z - seg.y;
       const int grow0 = (g.data_window0 + win) * rows_pad;
@@ -294,11 +253,6 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
       }
       __syncthreads();  // S2
       __syncthreads();  // S3
-      if (MULTI && (it + 1) % nseg == 0) {
-        // the two grid-wide barriers of a step: this role only keeps the CTA barriers inside them
-        grid_barrier(g.grid_bar, 0u, false, alive, g.status, 0);
-        if (it + 1 < n_iters) grid_barrier(g.grid_bar, 0u, false, alive, g.status, 0);
-      }
     }
   } else {
     // =====================  compute warpgroups: one row per thread  =====================================
@@ -331,11 +285,8 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
     for (int j = 0; j < 3; ++j)
       x_off[j] = pin(xb_wg + (uint32_t)(wtid * 128 + ((j ^ (wtid & 3)) << 5) + ((wtid & 4) ? 16 : 0)));
     const int row_in_tile = (int)pin((uint32_t)wtid);
-    bool alive = true;
 
-    for (int it = 0; it < n_iters; ++it) {
-      const int sg = MULTI ? seg0 + it % nseg : seg0 + it;
-      const int step = MULTI ? it / nseg : 0;
+    for (int sg = seg0; sg < seg1; ++sg) {
       const int4 seg = g.segs[sg];
       const int win = seg.x, t0 = seg.y, t1 = seg.z, slot = seg.w;
       const int nt = t1 - t0;
@@ -345,16 +296,14 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
       // ---- segment prologue: start the first row tiles, fused leapfrog update, stage W0a ----
       if (wtid == 0) {
         for (int i = 0; i < NST && i < my_nt; ++i) {
-          const uint32_t n = n_done + i;
           mbar_expect_tx(&bar_tma[wg][i], G::TILE_BYTES);
           tma_load_2d(xb + (wg * NST + i) * G::TILE_BYTES, &tmap_mn, 0,
                       grow0 + (t0 + wg + i * NWG) * TF32_TILE, &bar_tma[wg][i]);
         }
       }
       // element (n = hidden unit, k) of the K-major B operand at n*128 + ((k/4) ^ (n%8))*16 + (k%4)*4
-      const StepIo io = MULTI ? step_io(g, step) : step_io(g);
       for (int p = tid; p < G::P; p += NCOMPUTE) {
-        const float w = leapfrog_param(g, io, win, p, slot == 0);
+        const float w = leapfrog_param(g, win, p, slot == 0);
         if (p < D * H + H) {
           const int k = p / H, n = p - k * H;
           *reinterpret_cast<float*>(w0s + n * 128 + (((k >> 2) ^ (n & 7)) << 4) + ((k & 3) << 2)) = w;
@@ -521,20 +470,7 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
         for (int j = 0; j < H; j += 2) unpack2(dw1p[j >> 1], v[j], v[j + 1]);
         const float s_lo = warp_column_sums(v, lane);
         constexpr int REST = H - 32;  // 8
-        float* u = v + 32;
-#pragma unroll
-        for (int off = REST / 2; off > 0; off >>= 1) {
-          const bool up = (lane & off) != 0;
-#pragma unroll
-          for (int i = 0; i < off; ++i) {
-            const float send = up ? u[i] : u[i + off];
-            const float keep = up ? u[i + off] : u[i];
-            u[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-          }
-        }
-        float s_hi = u[0];
-#pragma unroll
-        for (int off = REST; off < 32; off <<= 1) s_hi += __shfl_xor_sync(0xffffffffu, s_hi, off);
+        const float s_hi = warp_rest_sums<REST>(v + 32, lane);
         red_w1[warp][lane] = s_lo;
         if (lane < REST) red_w1[warp][32 + lane] = s_hi;
       }
@@ -550,7 +486,7 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
       __syncthreads();  // S2
 
       // ---- segment read-out: one partial gradient vector for (window, slot) ----
-      float* po = (MULTI ? ((step & 1) ? g.partial_buf[1] : g.partial_buf[0]) : g.partial_out) + ((size_t)win * g.slices_out + slot) * g.Pp;
+      float* po = g.partial_out + ((size_t)win * g.slices_out + slot) * g.Pp;
       if (warp < 4) {
         // Gt accumulator row i = 32 * group + feature lives in lane 32 * (i / 16) + i % 16 (M = 64): warp w
         // holds, in its lanes 0..15, features 16 * (w & 1) + lane of row group w >> 1, whose hidden
@@ -606,18 +542,10 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
           double l = 0.0;
           for (int w = 0; w < NWG * 4; ++w) { s += red_db1[w]; l += red_ll[w]; }
           po[D * H + 2 * H] = s;
-          (MULTI ? ((step & 1) ? g.ll_buf[1] : g.ll_buf[0]) : g.ll_out)[(size_t)win * g.slices_out + slot] = l;
+          g.ll_out[(size_t)win * g.slices_out + slot] = l;
         }
       }
       __syncthreads();  // S3: read-out done before the next segment restages W0a / reuses the scratch
-      if (MULTI && (it + 1) % nseg == 0) {
-        // ---- all partial vectors of this step are written: sum them, a few parameters per CTA ----
-        const unsigned int nb = gridDim.x;
-        grid_barrier(g.grid_bar, (2u * step + 1u) * nb, tid == 0, alive, g.status, 401);
-        sum_partials_slice(g, (step & 1) ? g.partial_buf[1] : g.partial_buf[0],
-                           (step & 1) ? g.ll_buf[1] : g.ll_buf[0], tid);
-        if (it + 1 < n_iters) grid_barrier(g.grid_bar, (2u * step + 2u) * nb, tid == 0, alive, g.status, 402);
-      }
     }
   }
 
@@ -640,50 +568,13 @@ static cudaError_t launch_tf32_t(const void* tmap_mn, const GradParams& g, int c
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !attr_done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(grad_tf32_kernel<H, false>,
+    cudaError_t e = cudaFuncSetAttribute(grad_tf32_kernel<H>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM);
     if (e != cudaSuccess) return e;
     attr_done[dev] = true;
   }
-  return launch_chain_kernel(grad_tf32_kernel<H, false>, dim3(ctas), dim3(TF32_THREADS), G::SMEM, st,
+  return launch_chain_kernel(grad_tf32_kernel<H>, dim3(ctas), dim3(TF32_THREADS), G::SMEM, st,
                              *reinterpret_cast<const CUtensorMap*>(tmap_mn), g);
-}
-
-// Several leapfrog steps of one window in one COOPERATIVE launch (every CTA resident: the grid barrier
-// inside relies on it).  Returns cudaErrorCooperativeLaunchTooLarge-like errors to the caller, which then
-// falls back to one launch per step.
-int tf32_multistep_max_ctas(int H) {
-  if (H != 40) return 0;
-  using G = Tf32Geom<40>;
-  int dev = 0, coop = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (!coop) return 0;
-  if (cudaFuncSetAttribute(grad_tf32_kernel<40, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)G::SMEM) != cudaSuccess)
-    return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grad_tf32_kernel<40, true>, TF32_THREADS,
-                                                    G::SMEM) != cudaSuccess)
-    return 0;
-  return per_sm * sms;
-}
-
-cudaError_t launch_grad_tf32_multistep(int H, const void* tmap_mn, const GradParams& g, int ctas,
-                                       cudaStream_t st) {
-  if (H != 40) return cudaErrorInvalidValue;
-  using G = Tf32Geom<40>;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(TF32_THREADS);
-  cfg.dynamicSmemBytes = G::SMEM;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, grad_tf32_kernel<40, true>, *reinterpret_cast<const CUtensorMap*>(tmap_mn), g);
 }
 
 cudaError_t launch_grad_tf32(int H, const void* tmap_mn, const GradParams& g, int ctas, cudaStream_t st) {

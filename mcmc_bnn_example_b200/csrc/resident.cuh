@@ -1,0 +1,496 @@
+// Whole HMC iterations, leapfrog trajectories and single evaluations of a window whose rows fit on the chip, as
+// ONE launch: rows, weights, momenta and gradients stay in shared memory, tensor memory and registers from the
+// first step to the last.
+//
+// Why.  With one launch per leapfrog step the step of a single 58368-row window takes 12.0 us (TF32) although its
+// arithmetic needs about 1 us: what counts are the launches, the re-reading and re-staging of the rows, the partial
+// vectors' trip through a second launch and the accept launch.  Here a step is one pass over rows that are already
+// where the tensor core reads them, plus an exchange of sums and weights between the CTAs of the window.
+//
+// Work split.  A window's rows are dealt in units of 32 (a warp's) to K clusters of C CTAs, at most 16 units per
+// CTA (four warpgroups of four warps), so that nothing is loaded after the first step.
+//
+// Exchange.  Parameters travel in words of three, 322 of them for 961 parameters; word i belongs to rank
+// i / wpm of every cluster, where C lanes work on it:
+//   1. every CTA sends its sums for a word to the owner in its cluster (st.async into the owner's shared memory,
+//      counted by the owner's mbarrier); lane l of the word reads rank l's, a shuffle tree adds them;
+//   2. K > 1: the owner stores the cluster's sums through L2 in a 16-byte word {3 sums, sequence number}, and the
+//      rank's threads read the words of all clusters, consecutive threads consecutive words (with every lane reading
+//      the words it adds, 15 clusters needed 2,970 cycles for this hop instead of 1,870: what counts is the number
+//      of L2 requests while everybody polls).  A word is written and read by single 16-byte accesses, which the memory model
+//      keeps whole, so there is no flag, no fence and no grid-wide barrier.  Words alternate between two buffers:
+//      a cluster sends step s + 2 only after it has read every word of step s + 1, which the others send after
+//      they have read every word of step s;
+//   3. every lane does the leapfrog update of its word's parameters (the same numbers in the same order in every
+//      lane and every cluster) and lane l sends the new weights to rank l of the cluster.
+// So a step costs two trips through the cluster's shared memory and, for windows of more than one cluster, one
+// through L2.  The step is a chain of short latencies, and a taken branch costs some 50 - 100 of them (a two-turn loop
+// over shared memory took 380 cycles where the straight code takes 60): its code is kept straight, with selects for
+// the threads that differ.  No buffer of the two cluster trips needs a second copy: weights of step s + 1 leave their
+// owners only after every rank's sums of step s have been read, sums of step s + 1 leave a rank only after it has
+// every weight of step s + 1.
+// (A first version without clusters exchanged everything through L2, owners spread over all CTAs: two
+// trips, each 2,500 - 5,500 cycles with 148 CTAs polling the same lines: 9.4 us per step.)  The accept decision is
+// taken by every warp that owns parameters, from the same shares in the same order.  No atomics; every wait is
+// bounded and ends in the status word.
+//
+// It replaces, for such windows, the reference's persistent kernel with an unbounded grid barrier
+// (mcmc_step_tc.h:597-677) and its per-iteration host work (main.h:204-283).
+#pragma once
+#include "chain.cuh"
+#include "common.cuh"
+#include "philox.h"
+#include "refstream.cuh"
+#include "tc05.cuh"
+
+namespace mcmc_b200 {
+
+constexpr int RES_NWG = 4;                     // warpgroups = resident tiles per CTA
+constexpr int RES_THREADS = RES_NWG * 128;
+constexpr int RES_BAR_E = 1, RES_BAR_T = 5, RES_BAR_X = 9;  // named barriers: + warpgroup, + warpgroup, the exchange
+constexpr uint32_t RES_POLLS = 1u << 20;       // bounded waits: polls of about 0.5 us
+
+// ---- words through L2: single 16-byte accesses ----------------------------------------------
+__device__ __forceinline__ void st_word16(uint4* p, uint32_t a, uint32_t b, uint32_t c, uint32_t seq) {
+  asm volatile(
+      "{\n\t.reg .b64 lo, hi;\n\t.reg .b128 v;\n\t"
+      "mov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\tmov.b128 v, {lo, hi};\n\t"
+      "st.relaxed.gpu.global.b128 [%0], v;\n\t}" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(seq)
+      : "memory");
+}
+__device__ __forceinline__ uint4 ld_word16(const uint4* p) {
+  uint4 r;
+  asm volatile(
+      "{\n\t.reg .b64 lo, hi;\n\t.reg .b128 v;\n\t"
+      "ld.relaxed.gpu.global.b128 v, [%4];\n\tmov.b128 {lo, hi}, v;\n\t"
+      "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
+      : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+      : "l"(p)
+      : "memory");
+  return r;
+}
+
+// ---- words through the cluster's shared memory ----------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// 16 bytes into another CTA's shared memory, counted by that CTA's mbarrier
+__device__ __forceinline__ void st_async16(uint32_t dst, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];" ::"r"(dst),
+               "r"(bar), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __noinline__ void res_timeout(const ResidentParams& g, int code) {
+  if (g.status) atomicExch(g.status, code);
+  if (g.status_host) *reinterpret_cast<volatile int*>(g.status_host) = code;
+}
+// mbarrier wait of the resident kernel: a bounded spin in line (each try_wait sleeps in hardware for a moment)
+__device__ __forceinline__ void res_wait(uint64_t* bar, uint32_t parity, const ResidentParams& g, int code, bool& ok) {
+  uint32_t n = 0;
+  while (!mbar_try_wait(bar, parity) && ok)
+    if (++n == RES_POLLS) { ok = false; res_timeout(g, code); }
+}
+
+// One momentum draw: N(0,1) of (window, iteration, parameter), or the reference's stream
+__device__ __forceinline__ float res_momentum(const AcceptParams& a, uint32_t gwin, int iter, int p) {
+  return a.ref_streams ? refstream_normal(a.seed + REF_DRAWS_PER_ITER * (unsigned long long)iter + p)
+                       : philox_normal(a.seed, gwin, (uint32_t)iter, STREAM_MOMENTUM, (uint32_t)p);
+}
+__device__ __forceinline__ double u2d(uint32_t lo, uint32_t hi) {
+  return __longlong_as_double((long long)(((unsigned long long)hi << 32) | lo));
+}
+__device__ __forceinline__ uint2 d2u(double d) {
+  const unsigned long long l = (unsigned long long)__double_as_longlong(d);
+  return make_uint2((uint32_t)l, (uint32_t)(l >> 32));
+}
+// sums over the LPW lanes of a word; every lane gets them
+template <int LPW>
+__device__ __forceinline__ void word_sum(float v[3]) {
+#pragma unroll
+  for (int o = LPW >> 1; o > 0; o >>= 1) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+  }
+}
+template <int LPW>
+__device__ __forceinline__ double word_sum(double v) {
+#pragma unroll
+  for (int o = LPW >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Tile = the precision's arithmetic for the CTA's rows (resident_tf32.cu):
+//   Tile::H, Tile::SMEM               hidden units, bytes of dynamic shared memory
+//   Tile(smem, g, win, u0, u1)       per-thread constants; rows 32 u0 .. 32 u1 of the window are this CTA's
+//   setup(tmap, g)                   loads the rows
+//   stage(v)                         word `threadIdx.x` of the weights (the first ResWords::N threads)
+//   step(g, row_loss, last, ok)      forward, loss, backward of this warpgroup's tile
+//   collects()                       the word whose sum this thread makes, or -1
+//   collect(last, v)                 after the CTA barrier that follows step: the CTA's sums for that word
+//   teardown()
+// The parameters of a word, in an order of their own: words 0 .. 306 are W0 and b0 (the last one two of them), the next
+// fourteen W1 and b1, the last word is the log-likelihood.
+template <int H>
+struct ResWords {
+  static constexpr int P = 22 * H + 2 * H + 1;
+  static constexpr int W0 = (23 * H + 2) / 3;           // words of W0 and b0
+  static constexpr int N = W0 + (H + 1 + 2) / 3 + 1;    // all words
+  static constexpr int PAD = 3 * W0 - 23 * H;           // empty places of word W0 - 1
+  __device__ static int param(int t, int q) { return t < W0 ? 3 * t + q : 3 * t + q - PAD; }
+  __device__ static bool valid(int t, int q) { return t < W0 ? 3 * t + q < 23 * H : 3 * t + q - PAD < P; }
+};
+
+template <class Tile, int C>
+__global__ void __launch_bounds__(RES_THREADS, 1)
+resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ ResidentParams g) {
+  using Words = ResWords<Tile::H>;
+  constexpr int P = Words::P, NWORDS = Words::N;
+  constexpr int WPM = (NWORDS + C - 1) / C;            // words per rank
+  constexpr int XWARPS = (WPM * C + 31) / 32;          // warps that own words
+  static_assert(WPM * C <= RES_THREADS && NWORDS <= RES_THREADS, "one thread per lane of a word");
+  constexpr int XT = XWARPS * 32;
+  constexpr bool MULTI = C == 8;                       // windows of several clusters use clusters of eight
+  constexpr int STR = (WPM + 7) / 8 * 8;               // a cluster's words start on a line
+  constexpr int NR = MULTI ? (WPM * RES_MAX_CLUSTERS + XT - 1) / XT : 1;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* base =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(16) uint4 part_in[C][WPM];           // sums of every rank for the words owned here
+  __shared__ __align__(16) uint4 w_in[NWORDS];              // weights
+  __shared__ __align__(16) uint4 h_in[2][C * XWARPS + 1];   // {kinetic, log-prior} shares; log-likelihood
+  __shared__ __align__(16) uint4 x_in[MULTI ? RES_MAX_CLUSTERS * WPM : 1];  // words of all clusters
+  __shared__ __align__(8) uint64_t bar_part, bar_w, bar_h;
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = C == 1 ? 0 : (int)cluster_rank();
+  const int K = g.clusters;
+  const int cl = (int)blockIdx.x / C;
+  const int win = cl / K, k = cl - win * K;
+  const int cta = k * C + rank, n_cta = K * C;
+  const int units = (g.n_rows + 31) / 32;
+  Tile c(base, g, win, (int)((long long)cta * units / n_cta), (int)((long long)(cta + 1) * units / n_cta));
+  if (tid == 0) {
+    mbar_init(&bar_part, 1);
+    mbar_init(&bar_w, 1);
+    mbar_init(&bar_h, 1);
+    mbar_fence_init();
+  }
+  c.setup(&tmap, g);  // (holds a CTA barrier)
+  const int my_words = min(WPM, NWORDS - rank * WPM);
+  const uint32_t part_bytes = (uint32_t)(my_words * C * 16), w_bytes = NWORDS * 16, h_bytes = (C * XWARPS + 1) * 16;
+  if (tid == 0) {
+    mbar_expect_tx(&bar_part, part_bytes);
+    mbar_expect_tx(&bar_w, w_bytes);
+    mbar_expect_tx(&bar_h, h_bytes);
+  }
+  if (C > 1) cluster_sync_all();  // every rank's barriers exist before anyone sends
+  else __syncthreads();
+
+  // ---- who does what in the exchange ----
+  const int wl = tid / C, l = tid % C;       // word of this rank, lane of the word
+  const int word = rank * WPM + wl;
+  const bool mine = wl < WPM && word < NWORDS;
+  const bool ll_word = word == NWORDS - 1;
+  const int out = max(c.collects(), 0);      // the word of which this thread sends the CTA's sums
+  const uint32_t part_dst = mapa(smem_u32(&part_in[rank][out % WPM]), out / WPM);
+  const uint32_t part_bar = mapa(smem_u32(&bar_part), out / WPM);
+  const uint32_t w_dst = mapa(smem_u32(&w_in[mine ? word : 0]), l), w_bar = mapa(smem_u32(&bar_w), l);
+  constexpr uint32_t H_BUF = (C * XWARPS + 1) * 16;
+  // words through L2: [2 buffers][windows][ranks][clusters][STR]
+  const size_t msg_buf = (size_t)g.windows * C * K * STR;
+  uint4* const msg = g.msg + ((size_t)win * C + rank) * K * STR;
+  uint32_t x_src[NR];
+  bool x_has[NR];
+#pragma unroll
+  for (int i = 0; i < NR; ++i) {
+    const int u = tid + i * XT;
+    x_has[i] = MULTI && tid < XT && u < my_words * K;
+    x_src[i] = (uint32_t)(u / my_words * STR + u % my_words);
+  }
+  const bool chain = g.mode == RES_CHAIN;
+  const AcceptParams& a = g.a;
+  uint32_t seq = __ldcg(g.seq + win);
+  bool ok = true;
+
+  // ---- state of the word's parameters, the same in each of its lanes ----
+  const size_t so = (size_t)win * g.Pp;
+  float eps = chain ? __ldcg(a.eps + win) : g.eps_scalar;
+  int iter = chain ? a.iter[win] : 0;
+  const uint32_t gwin = chain ? (uint32_t)a.gwin[win] : 0u;
+  double ll_cur = chain ? a.ll_cur[win] : 0.0, lp_cur = chain ? a.lp_cur[win] : 0.0;
+  int n_acc = 0;
+  float w_s[3] = {}, g_s[3] = {}, m_s[3] = {}, w[3] = {}, m[3] = {};
+  bool has[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const int p = Words::param(word, q);
+    has[q] = mine && Words::valid(word, q);
+    if (has[q]) {
+      w_s[q] = __ldcg((chain ? a.w_cur + so : g.w0) + p);
+      w[q] = w_s[q];
+      if (g.mode != RES_EVAL) {
+        g_s[q] = __ldcg((chain ? a.g_cur + so : g.g0) + p);
+        m_s[q] = __ldcg((chain ? a.m_start + so : g.m0) + p);
+        m[q] = fmaf(eps * 0.5f, g_s[q], m_s[q]);  // half kick, drift (mcmc_step_ffma.h:106-120)
+        w[q] = fmaf(eps, m[q], w[q]);
+      }
+    }
+  }
+  auto send_weights = [&]() {
+    if (mine) st_async16(w_dst, w_bar, __float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), 0u);
+  };
+  uint32_t n = 0;        // steps done in this launch: the mbarrier phases follow it
+  uint32_t n_traj = 0;
+  send_weights();
+
+  const int L = g.n_steps;
+  for (int it = 0; it < g.n_iter; ++it) {
+    for (int s = 0; s < L; ++s, ++n) {
+      const uint32_t ph = n & 1;
+      const bool last = s == L - 1;
+      ++seq;
+      // ---- weights of this step ----
+      res_wait(&bar_w, ph, g, 601, ok);
+      if (tid == 0) mbar_expect_tx(&bar_w, w_bytes);
+      c.stage(w_in[min(tid, NWORDS - 1)]);
+      // ---- this warpgroup's tile ----
+      c.step(g, last ? g.row_loss : nullptr, last, ok);
+      __syncthreads();
+      // ---- the CTA's sums to their owners ----
+      {
+        uint4 v;
+        if (c.collect(last, v)) st_async16(part_dst, part_bar, v.x, v.y, v.z, 0u);
+      }
+      if (warp >= XWARPS) continue;
+      float m_nx[3];
+      if (last && chain) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) m_nx[q] = has[q] ? res_momentum(a, gwin, iter + 1, Words::param(word, q)) : 0.f;
+      }
+      // ---- owners: the cluster's sum, then the window's ----
+      // (the log-likelihood is wanted at the end of a trajectory only)
+      const bool ll_warp = last && rank == C - 1 && warp == (NWORDS - 1 - (C - 1) * WPM) * C / 32;
+      res_wait(&bar_part, ph, g, 602, ok);
+      if (tid == 0) mbar_expect_tx(&bar_part, part_bytes);
+      const uint4 x = part_in[l][min(wl, WPM - 1)];
+      float v[3] = {__uint_as_float(x.x), __uint_as_float(x.y), __uint_as_float(x.z)};
+      word_sum<C>(v);
+      double ll = 0.0;
+      if (ll_warp) ll = word_sum<C>(ll_word ? u2d(x.x, x.y) : 0.0);
+      if (MULTI && K > 1) {
+        uint4* const mb = msg + (seq & 1) * msg_buf;
+        if (mine && l == 0) {
+          const uint2 d = d2u(ll);
+          st_word16(mb + k * STR + wl, ll_word ? d.x : __float_as_uint(v[0]), ll_word ? d.y : __float_as_uint(v[1]),
+                    __float_as_uint(v[2]), seq);
+        }
+        uint4 y[NR];
+#pragma unroll
+        for (int i = 0; i < NR; ++i) y[i] = x_has[i] ? ld_word16(mb + x_src[i]) : make_uint4(0u, 0u, 0u, seq);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+          uint32_t t = 0;
+          while (y[i].w != seq && ok) {
+#pragma unroll
+            for (int j = i; j < NR; ++j)  // (a word that has arrived is read once more: its value stays)
+              if (x_has[j]) y[j] = ld_word16(mb + x_src[j]);
+            if (++t == RES_POLLS) { ok = false; res_timeout(g, 603); }
+          }
+          if (x_has[i]) x_in[tid + i * XT] = y[i];
+        }
+        named_sync(RES_BAR_X, XT);
+        // lane l adds clusters l and l + 8
+        const int wi = min(wl, my_words - 1);
+        const uint4 y0 = x_in[min(l, K - 1) * my_words + wi], y1 = x_in[min(l + C, K - 1) * my_words + wi];
+        const bool one = l < K, two = l + C < K;
+        v[0] = (one ? __uint_as_float(y0.x) : 0.f) + (two ? __uint_as_float(y1.x) : 0.f);
+        v[1] = (one ? __uint_as_float(y0.y) : 0.f) + (two ? __uint_as_float(y1.y) : 0.f);
+        v[2] = (one ? __uint_as_float(y0.z) : 0.f) + (two ? __uint_as_float(y1.z) : 0.f);
+        word_sum<C>(v);
+        if (ll_warp)
+          ll = word_sum<C>(ll_word ? (one ? u2d(y0.x, y0.y) : 0.0) + (two ? u2d(y1.x, y1.y) : 0.0) : 0.0);
+      }
+      float gf[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) gf[q] = fmaf(w[q], g.prior.neg_inv_s2, v[q]);
+      if (!last) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          m[q] = fmaf(eps, gf[q], m[q]);
+          w[q] = fmaf(eps, m[q], w[q]);
+        }
+        send_weights();
+        continue;
+      }
+      // ---- end of the trajectory: this warp's share of the log-prior and of the kinetic difference ----
+      double lp = 0.0, dk = 0.0;
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (has[q] && l == 0) {
+          const float u = w[q] * g.prior.inv_s;
+          const float pl = fmaf(-0.5f * u, u, -g.prior.norm);
+          lp += (double)pl;
+          if (chain) {  // closing half kick (kernel_helpers.h:163-175)
+            const float mf = fmaf(eps * 0.5f, gf[q], m[q]);
+            dk += 0.5 * ((double)m_s[q] * (double)m_s[q] - (double)mf * (double)mf);
+          } else if (k == 0) {
+            const int p = Words::param(word, q);
+            g.g_out[p] = gf[q];
+            if (g.w_out) g.w_out[p] = w[q];
+            if (g.m_out) g.m_out[p] = m[q];
+            if (g.zero_out) g.zero_out[p] = 0.f;
+            if (g.prior_loss) g.prior_loss[p] = pl;
+          }
+        }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        lp += __shfl_xor_sync(0xffffffffu, lp, o);
+        dk += __shfl_xor_sync(0xffffffffu, dk, o);
+      }
+      const uint32_t hb = n_traj & 1;
+      if (lane < C) {
+        const uint2 x1 = d2u(dk), x2 = d2u(lp);
+        st_async16(mapa(smem_u32(&h_in[0][rank * XWARPS + warp]), lane) + hb * H_BUF, mapa(smem_u32(&bar_h), lane), x1.x,
+                   x1.y, x2.x, x2.y);
+      }
+      if (ll_warp && mine && ll_word) {
+        const uint2 x1 = d2u(ll);
+        st_async16(mapa(smem_u32(&h_in[0][C * XWARPS]), l) + hb * H_BUF, mapa(smem_u32(&bar_h), l), x1.x, x1.y, 0u, 0u);
+      }
+      res_wait(&bar_h, hb, g, 604, ok);
+      if (tid == 0) mbar_expect_tx(&bar_h, h_bytes);
+      ++n_traj;
+      dk = lp = 0.0;
+      for (int i = lane; i < C * XWARPS; i += 32) {
+        const uint4 x1 = h_in[hb][i];
+        dk += u2d(x1.x, x1.y);
+        lp += u2d(x1.z, x1.w);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        lp += __shfl_xor_sync(0xffffffffu, lp, o);
+        dk += __shfl_xor_sync(0xffffffffu, dk, o);
+      }
+      const double ll_new = u2d(h_in[hb][C * XWARPS].x, h_in[hb][C * XWARPS].y);
+      if (!chain) {
+        if (k == 0 && rank == 0 && tid == 0) {
+          g.scalars[0] = ll_new;
+          g.scalars[1] = lp;
+        }
+        continue;
+      }
+      const double la = (ll_new - ll_cur) + (lp - lp_cur) + dk;
+      const float la_f = (float)la;
+      const float log_u = a.ref_streams ? a.ref_log_u[iter % a.ref_cap]
+                                        : logf(philox_accept_uniform(a.seed, gwin, (uint32_t)iter));
+      const bool acc = log_u < la_f;  // main.h:242; a NaN ratio rejects
+      float eps_next = eps;
+      if (iter < a.adapt_steps) {  // main.h:266-276
+        const float lmr = fminf(la_f, 0.f);
+        eps_next = eps + eps * (lmr < a.log_target ? a.dec_adj : a.inc_adj);
+      }
+      if (k == 0 && rank == 0 && tid == 0 && iter < a.trace_iters) {
+        const size_t ti = (size_t)win * a.trace_iters + iter;
+        a.tr_log_u[ti] = log_u;
+        a.tr_log_acpt[ti] = la;
+        a.tr_accept[ti] = acc;
+        a.tr_eps[ti] = eps;
+      }
+      if (acc) {
+        ll_cur = ll_new;
+        lp_cur = lp;
+        ++n_acc;
+      }
+      eps = eps_next;
+      const int store = iter - a.burn_in;
+      ++iter;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        if (acc) {
+          w_s[q] = w[q];
+          g_s[q] = gf[q];
+        }
+        m_s[q] = m_nx[q];
+        // start of the next trajectory (main.h:207-218)
+        m[q] = fmaf(eps * 0.5f, g_s[q], m_s[q]);
+        w[q] = fmaf(eps, m[q], w_s[q]);
+      }
+      if (it + 1 < g.n_iter) send_weights();
+      if (k == 0 && l == 0) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          if (has[q]) {
+            const int p = Words::param(word, q);
+            if (store >= 0 && store < a.sample_capacity)
+              a.samples[((size_t)win * a.sample_capacity + store) * P + p] = w_s[q];
+            if (iter < a.trace_iters) a.tr_mom[((size_t)win * a.trace_iters + iter) * P + p] = m_s[q];
+          }
+      }
+    }
+  }
+  // ---- the state the next launch (of either kind) starts from ----
+  if (chain && k == 0 && l == 0) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      if (has[q]) {
+        const size_t p = so + Words::param(word, q);
+        a.w_cur[p] = w_s[q];
+        a.g_cur[p] = g_s[q];
+        a.w_start[p] = w_s[q];
+        a.m_start[p] = m_s[q];
+        a.m0[p] = m_s[q];
+      }
+  }
+  if (k == 0 && rank == 0 && tid == 0) {
+    if (chain) {
+      a.ll_cur[win] = ll_cur;
+      a.lp_cur[win] = lp_cur;
+      a.eps[win] = eps;
+      a.iter[win] = iter;
+      a.n_accept[win] += n_acc;
+    }
+    // (every cluster of the window has read the counter: this one has used words that carry later values)
+    g.seq[win] = seq;
+  }
+  c.teardown();
+  if (C > 1) cluster_sync_all();  // no rank leaves while another may still write to it
+}
+
+// ---- host side ----------------------------------------------------------------------------
+// Every CTA has to be resident (they wait for one another's words): a cooperative launch of clusters.
+template <typename K>
+static cudaError_t resident_launch(K kernel, int cluster, size_t smem, const void* tmap, const ResidentParams& g,
+                                   cudaStream_t st, int* max_clusters) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(max_clusters ? cluster : g.windows * g.clusters * cluster);
+  cfg.blockDim = dim3(RES_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeCooperative;
+  attr[1].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  if (max_clusters) {
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return e != cudaSuccess ? e : cudaOccupancyMaxActiveClusters(max_clusters, kernel, &cfg);
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, *reinterpret_cast<const CUtensorMap*>(tmap), g);
+}
+
+}  // namespace mcmc_b200

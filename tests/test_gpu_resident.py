@@ -1,0 +1,60 @@
+"""The one-launch path for windows whose rows fit on the chip, at the sizes where its partition changes: one row, the
+last row of a 32-row unit and of a CTA, one cluster full and one row more, the largest window and one row more (one
+launch per step again), and window counts that take clusters of 8, 4, 2 and 1 CTAs."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+P = 961
+TOL = {0: 1e-5, 1: 2e-3}
+
+
+@pytest.mark.parametrize("prec", [1])
+@pytest.mark.parametrize("W,rows", [(1, 1), (1, 33), (1, 4096), (1, 4097), (1, 61440), (1, 61441), (3, 9001), (15, 300),
+                                    (16, 2048), (40, 1000), (100, 511)])
+def test_resident_launch_matches_oracle_and_per_step_launches(built, monkeypatch, prec, W, rows):
+    m, O = built
+    n_iter, L = 4, 3
+    cfg = m.reference_config(precision=prec, leapfrog_steps=L, burn_in=1, adapt_steps=3, sample_capacity=n_iter,
+                             trace_iters=n_iter, seed=5, eps0=0.02)
+    data = [m.synth_window(31, g, rows) for g in range(min(W, 3))]
+    w = (0.15 * np.random.default_rng(rows).standard_normal(P)).astype(np.float32)
+    mom = np.random.default_rng(1).standard_normal(P).astype(np.float32)
+
+    def run():
+        ctx = m.Context(cfg, n_windows=W, rows=rows)
+        for i in range(W):
+            x, y, _ = data[i % len(data)]
+            ctx.set_window_data(i, x, y, global_window=i)
+        grad = ctx.potential_and_grad(W - 1, w, want_row_loss=True)
+        steps = ctx.leapfrog(W - 1, 4, 1e-3, w, mom, grad["grad"])
+        ctx.run_chain(1)
+        ctx.run_chain(n_iter - 1)
+        out = [(ctx.get_samples(i), ctx.get_trace(i), ctx.chain_info(i), ctx.get_state(i)) for i in (0, W - 1)]
+        n = ctx.launch_count()
+        ctx.close()
+        return grad, steps, out, n
+
+    grad, steps, chains, n_one = run()
+    monkeypatch.setenv("MCMC_B200_NO_MULTISTEP", "1")
+    grad_s, steps_s, chains_s, n_many = run()
+    assert (n_one < n_many) == (rows <= 61440)
+    x, y, _ = data[(W - 1) % len(data)]
+    ref = O.logp_grad(O.reference_model(tf32=bool(prec)), x, y, w, want_losses=True)
+    tol = TOL[prec]
+    for got in (grad, grad_s):
+        assert np.abs(got["grad"] - ref["grad"]).max() <= tol * np.abs(ref["grad"]).max()
+        assert abs(got["loglik"] - ref["loglik"]) <= tol * abs(ref["loglik"])
+        assert abs(got["logprior"] - ref["logprior"]) <= 1e-6 * abs(ref["logprior"])
+        assert np.allclose(got["row_loss"], ref["row_loss"], rtol=10 * tol, atol=10 * tol)
+    # the two paths add the same rows in another order
+    for k in ("w_next", "mom_next", "grad_cur"):
+        assert np.abs(steps[k] - steps_s[k]).max() <= 1e-4 * np.abs(steps_s[k]).max(), k
+    for (s1, t1, i1, g1), (s2, t2, i2, g2) in zip(chains, chains_s):
+        assert i1 == i2 and np.array_equal(t1["accepted"], t2["accepted"])
+        assert np.array_equal(t1["momenta"], t2["momenta"]) and np.array_equal(t1["log_u"], t2["log_u"])
+        assert np.array_equal(t1["eps"], t2["eps"])
+        assert np.allclose(t1["log_acpt"], t2["log_acpt"], rtol=1e-3, atol=1e-3)
+        assert np.abs(s1[:n_iter - 1] - s2[:n_iter - 1]).max() <= 1e-4 * max(1e-3, np.abs(s2[:n_iter - 1]).max())
+        assert abs(g1["loglik"] - g2["loglik"]) <= 1e-6 * abs(g2["loglik"])
