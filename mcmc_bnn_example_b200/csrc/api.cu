@@ -143,7 +143,7 @@ struct mcmc_b200_ctx {
   // dataset
   float* xaug = nullptr;
   std::vector<char> window_set;
-  CUtensorMap tmap_mn;
+  CUtensorMap tmap_mn = {};
   bool tmap_ok = false;
   // persistent (TF32) kernel work tables: chain launches and single-window launches
   int *tab_seg_ptr = nullptr, *tab_nslot = nullptr, *xtab_seg_ptr = nullptr, *xtab_nslot = nullptr;
@@ -329,22 +329,47 @@ static int build_work_table(mcmc_b200_ctx* c, int windows, long long tiles_per_w
                             int chunks_per_window, int** d_seg_ptr, int4** d_segs, int** d_nslot,
                             int* n_ctas, int* max_slots);
 
-// How a window of `rows` rows is dealt to clusters when `windows` of them share the GPU (resident.cuh).  max_clusters[i]
-// = clusters of 1 << i CTAs that can be resident.  False when the rows do not fit.
+static cudaError_t launch_resident(const mcmc_b200_ctx* c, int cluster, const ResidentParams& g, cudaStream_t st,
+                                   int* max_clusters = nullptr) {
+  return (c->cfg.precision == MCMC_B200_PREC_TF32 ? launch_resident_tf32 : launch_resident_fp32)(
+      cluster, &c->tmap_mn, g, st, max_clusters);
+}
+// Clusters of 1 << i CTAs that can be resident.  Asked once per device and kernel, and only when a plan wants to know:
+// the first question loads the kernel, which costs more than the rest of a small context.
+static int resident_max_clusters(const mcmc_b200_ctx* c, int i) {
+  static std::mutex mutex;
+  static int known[2][64][4];
+  static bool asked[2][64][4] = {};
+  const int k = c->cfg.precision == MCMC_B200_PREC_TF32, d = c->device & 63;
+  std::lock_guard<std::mutex> lock(mutex);
+  if (!asked[k][d][i]) {
+    if (launch_resident(c, 1 << i, c->res, nullptr, &known[k][d][i]) != cudaSuccess) {
+      cudaGetLastError();
+      known[k][d][i] = 0;
+    }
+    asked[k][d][i] = true;
+  }
+  return known[k][d][i];
+}
+
+// How a window of the context is dealt to clusters when `windows` of them share the GPU (resident.cuh).  False when
+// the rows do not fit.
 //   * one cluster per window, of the most CTAs (8, 4, 2, 1) that every window can have, if that holds the rows: the
 //     exchange then never leaves the cluster;
 //   * rows that one cluster of 8 cannot hold: as many clusters of 8 as every window can have (up to 16) while each
 //     CTA still has at least four 32-row units (below that the step is all exchange and more CTAs only add to it).
-static bool resident_plan(long long rows, int windows, const int max_clusters[4], int* cluster, int* clusters) {
-  const long long units = (rows + 31) / 32;
+static bool resident_plan(const mcmc_b200_ctx* c, int windows, int* cluster, int* clusters) {
+  const long long units = (c->rows + 31) / 32;
+  if ((long long)windows * ((units + RES_UNITS - 1) / RES_UNITS) > c->num_sms) return false;
   for (int i = 3; i >= 0; --i)
-    if (windows <= max_clusters[i] && units <= (long long)RES_UNITS << i) {
+    if (units <= (long long)RES_UNITS << i && (long long)windows << i <= c->num_sms && windows <= resident_max_clusters(c, i)) {
       *cluster = 1 << i;
       *clusters = 1;
       return true;
     }
-  const long long have = std::min<long long>(max_clusters[3] / windows, RES_MAX_CLUSTERS);
   const long long need = (units + 8 * RES_UNITS - 1) / (8 * RES_UNITS);
+  if (8 * need * windows > c->num_sms) return false;
+  const long long have = std::min<long long>(resident_max_clusters(c, 3) / windows, RES_MAX_CLUSTERS);
   if (need > have) return false;
   *cluster = 8;
   *clusters = (int)std::max(need, std::min(have, units / 32));
@@ -361,35 +386,18 @@ static size_t resident_words_stride(int P, int cluster) {
 // that do not depend on what shares the launch: such contexts keep one launch per step.
 static int resident_setup(mcmc_b200_ctx* c) {
   const char* off = getenv("MCMC_B200_NO_MULTISTEP");
-  if ((off && off[0] == '1') || c->cfg.slices > 0 || c->cfg.precision != MCMC_B200_PREC_TF32 || c->cfg.H != 40)
+  if ((off && off[0] == '1') || c->cfg.slices > 0 || c->cfg.H != 40)
     return MCMC_B200_OK;
-  // (asked once per device: the queries cost as much as the rest of a small context)
-  static std::mutex mutex;
-  static int known[64][4];
-  static bool asked[64] = {};
-  int max_clusters[4];
-  {
-    std::lock_guard<std::mutex> lock(mutex);
-    const int d = c->device & 63;
-    if (!asked[d]) {
-      for (int i = 0; i < 4; ++i)
-        if (launch_resident_tf32(1 << i, nullptr, c->res, nullptr, &known[d][i]) != cudaSuccess) {
-          cudaGetLastError();
-          known[d][i] = 0;
-        }
-      asked[d] = true;
-    }
-    memcpy(max_clusters, known[d], sizeof max_clusters);
-  }
   for (int k = 0; k < 2; ++k) {
     ResidentParams& g = k ? c->res_x : c->res;
     int& cluster = k ? c->res_x_cluster : c->res_cluster;
     memset(&g, 0, sizeof g);
     g.windows = k ? 1 : c->W;
-    if (!resident_plan(c->rows, g.windows, max_clusters, &cluster, &g.clusters)) continue;
+    if (!resident_plan(c, g.windows, &cluster, &g.clusters)) continue;
     g.n_rows = (int)c->rows;
     g.rows_pad = (int)c->rows_pad;
     g.Pp = c->Pp;
+    g.xaug = c->xaug;
     g.lik = make_lik(c->cfg);
     g.prior = make_prior(c->cfg);
     g.status = c->status;
@@ -984,10 +992,10 @@ static int resident_chain(mcmc_b200_ctx* c, int n_iter, cudaStream_t st) {
   g.n_steps = c->cfg.leapfrog_steps;
   g.a = base_accept_params(c);
   fill_chain_accept(c, g.a, ACC_ITERATE, g.n_steps);
-  const int per_launch = std::max(1, 20000 / g.n_steps);
+  const int per_launch = std::max(1, (c->cfg.precision == MCMC_B200_PREC_TF32 ? 20000 : 10000) / g.n_steps);
   for (int done = 0; done < n_iter; done += g.n_iter) {
     g.n_iter = std::min(per_launch, n_iter - done);
-    cudaError_t e = launch_resident_tf32(c->res_cluster, &c->tmap_mn, g, st, nullptr);
+    cudaError_t e = launch_resident(c, c->res_cluster, g, st);
     c->launches++;
     if (e != cudaSuccess)
       return fail(MCMC_B200_ERR_CUDA, std::string("resident chain launch: ") + cudaGetErrorString(e));
@@ -1299,7 +1307,7 @@ static int resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, c
   g.row_loss = row_loss;
   g.prior_loss = prior_loss;
   g.scalars = scalars;
-  cudaError_t e = launch_resident_tf32(c->res_x_cluster, &c->tmap_mn, g, st, nullptr);
+  cudaError_t e = launch_resident(c, c->res_x_cluster, g, st);
   c->launches++;
   if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, std::string("resident launch: ") + cudaGetErrorString(e));
   return MCMC_B200_OK;
@@ -1506,6 +1514,7 @@ static int fwd_reserve(mcmc_b200_ctx* c, T** buf, size_t* cap, size_t need) {
   *cap = need;
   return MCMC_B200_OK;
 }
+
 // sample chunks per row tile: enough CTAs for two waves of the GPU, at most one chunk per sample
 static int fwd_chunks(const mcmc_b200_ctx* c, long long n, int count) {
   const long long tiles = forward_row_tiles(n);

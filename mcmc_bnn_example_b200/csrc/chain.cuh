@@ -124,6 +124,7 @@ struct ResidentParams {
   int mode, n_steps, n_iter;
   int windows, clusters;    // clusters per window
   int data_window0, n_rows, rows_pad, Pp;
+  const float* xaug;        // [windows][rows_pad][KP] (FP32; TF32 goes through the tensor map)
   uint4* msg;               // [2][windows][ranks][clusters][words] cluster sums
   unsigned int* seq;        // [windows] last sequence number used
   LikParams lik;
@@ -140,6 +141,8 @@ struct ResidentParams {
 // The launch, for clusters of `cluster` CTAs (1, 2, 4, 8); or, when max_clusters is given, only the number of such
 // clusters that can be resident at once
 cudaError_t launch_resident_tf32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
+                                 int* max_clusters);
+cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters);
 
 // gradient kernels

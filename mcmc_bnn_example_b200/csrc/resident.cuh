@@ -91,7 +91,7 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-__device__ __noinline__ void res_timeout(const ResidentParams& g, int code) {
+static __device__ __noinline__ void res_timeout(const ResidentParams& g, int code) {
   if (g.status) atomicExch(g.status, code);
   if (g.status_host) *reinterpret_cast<volatile int*>(g.status_host) = code;
 }
@@ -130,10 +130,10 @@ __device__ __forceinline__ double word_sum(double v) {
   return v;
 }
 
-// Tile = the precision's arithmetic for the CTA's rows (resident_tf32.cu):
+// Tile = the precision's arithmetic for the CTA's rows (resident_tf32.cu, resident_fp32.cu):
 //   Tile::H, Tile::SMEM               hidden units, bytes of dynamic shared memory
 //   Tile(smem, g, win, u0, u1)       per-thread constants; rows 32 u0 .. 32 u1 of the window are this CTA's
-//   setup(tmap, g)                   loads the rows
+//   setup(tmap, g, win)              loads the rows
 //   stage(v)                         word `threadIdx.x` of the weights (the first ResWords::N threads)
 //   step(g, row_loss, last, ok)      forward, loss, backward of this warpgroup's tile
 //   collects()                       the word whose sum this thread makes, or -1
@@ -186,7 +186,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     mbar_init(&bar_h, 1);
     mbar_fence_init();
   }
-  c.setup(&tmap, g);  // (holds a CTA barrier)
+  c.setup(&tmap, g, win);  // (holds a CTA barrier)
   const int my_words = min(WPM, NWORDS - rank * WPM);
   const uint32_t part_bytes = (uint32_t)(my_words * C * 16), w_bytes = NWORDS * 16, h_bytes = (C * XWARPS + 1) * 16;
   if (tid == 0) {

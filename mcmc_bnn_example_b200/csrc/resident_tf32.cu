@@ -80,7 +80,7 @@ struct ResTf32 {
     stage_setup();
   }
 
-  __device__ __forceinline__ void setup(const CUtensorMap* tmap, const ResidentParams& g) {
+  __device__ __forceinline__ void setup(const CUtensorMap* tmap, const ResidentParams& g, int) {
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x;
     if (warp == 0) {

@@ -10,7 +10,7 @@ P = 961
 TOL = {0: 1e-5, 1: 2e-3}
 
 
-@pytest.mark.parametrize("prec", [1])
+@pytest.mark.parametrize("prec", [0, 1])
 @pytest.mark.parametrize("W,rows", [(1, 1), (1, 33), (1, 4096), (1, 4097), (1, 61440), (1, 61441), (3, 9001), (15, 300),
                                     (16, 2048), (40, 1000), (100, 511)])
 def test_resident_launch_matches_oracle_and_per_step_launches(built, monkeypatch, prec, W, rows):
