@@ -1515,21 +1515,13 @@ static int fwd_reserve(mcmc_b200_ctx* c, T** buf, size_t* cap, size_t need) {
   return MCMC_B200_OK;
 }
 
-// sample chunks per row tile: enough CTAs for two waves of the GPU, at most one chunk per sample
-static int fwd_chunks(const mcmc_b200_ctx* c, long long n, int count) {
-  const long long tiles = forward_row_tiles(n);
-  long long ch = (2LL * c->num_sms * 3 + tiles - 1) / tiles;
-  ch = std::max<long long>(1, std::min<long long>(std::min<long long>(ch, count), 64));
-  return (int)ch;
-}
-
 API int mcmc_b200_predict_mean(mcmc_b200_ctx* c, int window, const float* xs, int64_t n, int first,
                                int count, float* out) {
   if (!c || !xs || !out || n < 1 || window < 0 || window >= c->W || first < 0 || count < 1 ||
       !c->samples || first + count > c->cfg.sample_capacity)
     return fail(MCMC_B200_ERR_INVALID, "bad arguments or no sample storage");
   CK(cudaSetDevice(c->device));
-  const int chunks = fwd_chunks(c, n, count);
+  const int chunks = forward_chunks(c->num_sms, n, count);
   int r = fwd_reserve(c, &c->fwd_x, &c->fwd_x_cap, (size_t)n * c->cfg.D);
   if (r == MCMC_B200_OK) r = fwd_reserve(c, &c->fwd_out, &c->fwd_out_cap, (size_t)n);
   if (r == MCMC_B200_OK) r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)chunks * n);
@@ -1562,7 +1554,7 @@ API int mcmc_b200_final_loss(mcmc_b200_ctx* c, int window, int first, int count,
   CK(cudaSetDevice(c->device));
   // all samples against the window's rows in one launch (FP32 forward pass, no gradient)
   const int tiles = forward_row_tiles(c->rows);
-  const int chunks = fwd_chunks(c, c->rows, count);
+  const int chunks = forward_chunks(c->num_sms, c->rows, count);
   int r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)tiles * count + 2 * (size_t)count);
   if (r) return r;
   const float* xw = c->xaug + (size_t)window * c->rows_pad * KP;
