@@ -97,7 +97,9 @@ constexpr int kNcclSum = 0;
 constexpr int HB_FLOATS = 3076;  // P of the widest model, rounded up
 struct HostBlock {
   double scalars[2];
-  int status, pad[3];
+  int status;
+  float log_acpt;  // out: the drop-in accept ratio
+  int pad[2];
   float w[HB_FLOATS], m[HB_FLOATS], g[HB_FLOATS];  // in: position, momentum, gradient
   float w_out[HB_FLOATS], m_out[HB_FLOATS], g_out[HB_FLOATS];
 };
@@ -167,7 +169,6 @@ struct mcmc_b200_ctx {
   int iters_done = 0;
   // explicit-state scratch (one window)
   float *xw[2] = {}, *xm[2] = {}, *xg = nullptr, *xpartial[2] = {}, *g_out = nullptr, *row_loss = nullptr;
-  float* scalar_f = nullptr;
   double *xllp[2] = {}, *xred = nullptr, *scalars = nullptr;
   // bound dataset of the drop-in mcmc_step
   const float *bound_x = nullptr, *bound_y = nullptr;
@@ -523,7 +524,6 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
   DA(c->g_out, Pp * 4);
   DA(c->row_loss, (size_t)c->rows_pad * 4);
   DA(c->scalars, 4 * 8);
-  DA(c->scalar_f, 16);
   if (cfg->sample_capacity > 0) {
     int r_ = dalloc(c, (void**)&c->samples, W * (size_t)cfg->sample_capacity * P * 4, false);
     if (r_ != MCMC_B200_OK) { mcmc_b200_destroy(c); return r_; }
@@ -1495,11 +1495,11 @@ API int mcmc_b200_log_acpt(mcmc_b200_ctx* c, const float* prev_loss, const float
   CK(cudaSetDevice(c->device));
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = launch_log_acpt(prev_loss, new_loss, n_loss, prev_mom, new_mom, grad_cur, c->P, eps,
-                                  c->scalar_f, st);
+                                  &c->hb->log_acpt, st);
   c->launches++;
   if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
-  CK(cudaMemcpyAsync(out, c->scalar_f, 4, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  *out = c->hb->log_acpt;
   return MCMC_B200_OK;
 }
 
