@@ -8,9 +8,8 @@
 //     whatever precision the chain was sampled in;
 //   * a CTA owns 512 rows (4 per thread, held in registers for the whole launch) and walks through its
 //     chunk of the samples; a sample's 961 parameters are staged in shared memory once per CTA, the next one's while
-//     this one is worked on, and read as 16-byte broadcasts: 16 multiplications per load;
-//   * features go in pairs, two multiplications to an instruction (sums over the even and over the odd features, added
-//     at the end): with single ones the instruction slots were the limit, not the FMA pipe;
+//     this one is worked on, and read as 16-byte broadcasts: 16 multiplications per load
+//     (packed FMAs on pairs of features were no faster: with three different operands they issue every third cycle);
 //   * PREDICT: per-row sums over the chunk's samples -> partial[chunk][row]; LOSS: per-sample sums over the
 //     CTA's rows -> partial[tile][sample].  A second small launch adds the partials in a fixed order (and, for
 //     LOSS, the log-prior of every sample).  Doubles, no atomics: bit-reproducible.
@@ -27,7 +26,7 @@ template <int H, bool LOSS>
 __global__ void __launch_bounds__(FWD_THREADS, FWD_CTAS_PER_SM) forward_samples_kernel(const ForwardParams a) {
   constexpr int D = 22, P = D * H + 2 * H + 1;
   constexpr int SW = (P + 3) / 4 * 4;
-  // one sample: W0[k / 2][j][k % 2], b0, W1, b1
+  // one sample: W0[k][j], b0, W1, b1
   extern __shared__ __align__(16) float sw_raw[];
   __shared__ double red[FWD_THREADS / 32];
   const int tid = threadIdx.x;
@@ -37,14 +36,13 @@ __global__ void __launch_bounds__(FWD_THREADS, FWD_CTAS_PER_SM) forward_samples_
   auto stage = [&](int s) {
     float* dst = sw_raw + (s & 1) * SW;
     for (int p = tid; p < P; p += FWD_THREADS) {
-      const int k = p / H, j = p - k * H;
-      const uint32_t d = smem_u32(dst + (p < D * H ? (k >> 1) * (2 * H) + 2 * j + (k & 1) : p));
+      const uint32_t d = smem_u32(dst + p);
       asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(a.samples + (size_t)s * P + p) : "memory");
     }
   };
   if (s0 < s1) stage(s0);
   // rows tid, tid + 128, ...: consecutive threads read consecutive rows
-  uint64_t x[FWD_RPT][D / 2];
+  float x[FWD_RPT][D];
   float y[FWD_RPT];
   bool valid[FWD_RPT];
 #pragma unroll
@@ -53,7 +51,7 @@ __global__ void __launch_bounds__(FWD_THREADS, FWD_CTAS_PER_SM) forward_samples_
     valid[r] = row < a.n;
     const float* xr = a.x + row * a.x_stride;
 #pragma unroll
-    for (int k = 0; k < D / 2; ++k) x[r][k] = valid[r] ? pack2(xr[2 * k], xr[2 * k + 1]) : 0ull;
+    for (int k = 0; k < D; ++k) x[r][k] = valid[r] ? xr[k] : 0.f;
     y[r] = (LOSS && valid[r]) ? a.y[row * a.y_stride] : 0.f;
   }
   double acc[FWD_RPT];
@@ -70,43 +68,33 @@ __global__ void __launch_bounds__(FWD_THREADS, FWD_CTAS_PER_SM) forward_samples_
     for (int r = 0; r < FWD_RPT; ++r) pred[r] = sw[D * H + 2 * H];
 #pragma unroll 1
     for (int j0 = 0; j0 < H; j0 += 4) {
-      uint64_t z[FWD_RPT][4];
+      float z[FWD_RPT][4];
       const float4 b = *reinterpret_cast<const float4*>(sw + D * H + j0);
 #pragma unroll
       for (int r = 0; r < FWD_RPT; ++r) {
-        z[r][0] = pack2(b.x, 0.f);
-        z[r][1] = pack2(b.y, 0.f);
-        z[r][2] = pack2(b.z, 0.f);
-        z[r][3] = pack2(b.w, 0.f);
+        z[r][0] = b.x;
+        z[r][1] = b.y;
+        z[r][2] = b.z;
+        z[r][3] = b.w;
       }
 #pragma unroll
-      for (int k = 0; k < D / 2; ++k) {
-        const ulonglong2 w01 = *reinterpret_cast<const ulonglong2*>(sw + k * (2 * H) + 2 * j0);
-        const ulonglong2 w23 = *reinterpret_cast<const ulonglong2*>(sw + k * (2 * H) + 2 * j0 + 4);
+      for (int k = 0; k < D; ++k) {
+        const float4 w = *reinterpret_cast<const float4*>(sw + k * H + j0);
 #pragma unroll
         for (int r = 0; r < FWD_RPT; ++r) {
-          z[r][0] = fma2(x[r][k], w01.x, z[r][0]);
-          z[r][1] = fma2(x[r][k], w01.y, z[r][1]);
-          z[r][2] = fma2(x[r][k], w23.x, z[r][2]);
-          z[r][3] = fma2(x[r][k], w23.y, z[r][3]);
+          z[r][0] = fmaf(x[r][k], w.x, z[r][0]);
+          z[r][1] = fmaf(x[r][k], w.y, z[r][1]);
+          z[r][2] = fmaf(x[r][k], w.z, z[r][2]);
+          z[r][3] = fmaf(x[r][k], w.w, z[r][3]);
         }
       }
       const float4 w1 = *reinterpret_cast<const float4*>(sw + D * H + H + j0);
 #pragma unroll
       for (int r = 0; r < FWD_RPT; ++r) {
-        float h[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float even, odd;
-          unpack2(z[r][q], even, odd);
-          h[q] = even + odd;
-        }
-        tanh_ref2(h[0], h[1]);
-        tanh_ref2(h[2], h[3]);
-        pred[r] = fmaf(w1.x, h[0], pred[r]);
-        pred[r] = fmaf(w1.y, h[1], pred[r]);
-        pred[r] = fmaf(w1.z, h[2], pred[r]);
-        pred[r] = fmaf(w1.w, h[3], pred[r]);
+        pred[r] = fmaf(w1.x, tanh_ref(z[r][0]), pred[r]);
+        pred[r] = fmaf(w1.y, tanh_ref(z[r][1]), pred[r]);
+        pred[r] = fmaf(w1.z, tanh_ref(z[r][2]), pred[r]);
+        pred[r] = fmaf(w1.w, tanh_ref(z[r][3]), pred[r]);
       }
     }
     if (LOSS) {
