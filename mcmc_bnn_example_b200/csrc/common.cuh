@@ -81,14 +81,13 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 // ---- reference tanh (kernel_helpers.h:32-44): 2*sigmoid(2x)-1 on ex2/rcp
 // approximations, identity below the cut-off -------------------------------
-constexpr float TANH_IDENTITY = 0.0048176045529544353485f;
 __device__ __forceinline__ float tanh_ref(float x) {
   float e, d, s;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -2.88539008177792681472f));
   asm("add.ftz.f32 %0, %1, %2;" : "=f"(d) : "f"(1.f), "f"(e));
   // (ftz: d >= 1, and a result that would be denormal comes out as -1 either way)
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(d));
-  return fabsf(x) < TANH_IDENTITY ? x : fmaf(s, 2.f, -1.f);
+  return fabsf(x) < 0.0048176045529544353485f ? x : fmaf(s, 2.f, -1.f);
 }
 // one MUFU op; absolute error about 5e-4, inside the TF32 mode's tolerance
 __device__ __forceinline__ float tanh_fast(float x) {
@@ -248,30 +247,10 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
-}
-
-// tanh_ref of two values: the same operations, the multiplications and additions packed
-__device__ __forceinline__ void tanh_ref2(float& a, float& b) {
-  float x, y;
-  unpack2(mul2(pack2(a, b), pack2(-2.88539008177792681472f, -2.88539008177792681472f)), x, y);
-  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(x));
-  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(y));
-  const uint64_t one = pack2(1.f, 1.f);
-  unpack2(add2(one, pack2(x, y)), x, y);
-  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(x));
-  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(y));
-  unpack2(fma2(pack2(x, y), pack2(2.f, 2.f), pack2(-1.f, -1.f)), x, y);
-  a = fabsf(a) < TANH_IDENTITY ? a : x;
-  b = fabsf(b) < TANH_IDENTITY ? b : y;
 }
 
 // ---- programmatic dependent launch -----------------------------------------

@@ -6,8 +6,10 @@
 // Layouts.  What bounds the multiplications is feeding them: a 16-byte load of a whole warp takes four passes over
 // shared memory, but two when lanes i and i ^ 1 (or i and i ^ 2) read the same address, measured; the same address in
 // lanes 8 apart does not help.  So lane bits 0 and 1 go to different operands in both products:
-//   * forward: a lane owns RPT rows x HPL hidden units.  Features go in pairs, one packed FMA for two of them (sums
-//     over the even and the odd features, added at the end): rows are read as they lie, weights are staged in pairs.
+//   * forward: a lane owns HALF rows x HPL hidden units at a time.  Features go in pairs, one packed FMA for two of them
+//     (sums over the even and the odd features, added at the end): rows are read as they lie, weights are staged in
+//     pairs.  Packed FMAs with three different operands issue every third cycle, so they save issue slots and not FMA
+//     time; single ones took the same time for 40 units and 10 % more for 128.
 //     Row group = lane bits 0, 2 (bit 0 for 128 units), unit group = the other bits.
 //   * backward: a lane owns 12 features x HPL units of every second row (every row for 128 units): feature half =
 //     bit 0, unit group = the next bits.  W1's factor of dL/dz is left to whoever reads the sums out.
@@ -101,10 +103,7 @@ struct Fp32Warp {
         float a, b, c, d;
         unpack2(z[i][j], a, b);
         unpack2(z[i + 1][j], c, d);
-        a += b;
-        c += d;
-        tanh_ref2(a, c);
-        hp[i / 2][j] = pack2(a, c);
+        hp[i / 2][j] = pack2(tanh_ref(a + b), tanh_ref(c + d));
       }
   }
 
@@ -139,14 +138,15 @@ struct Fp32Warp {
     __syncwarp();
     uint64_t dy[2];
     lds2x64(dys + rg * HALF, dy[0], dy[1]);
-    const uint64_t one = pack2(1.f, 1.f), sign = 0x8000000080000000ull;
+    const uint64_t minus1 = pack2(-1.f, -1.f), sign = 0x8000000080000000ull;
+    const uint64_t ndy[2] = {dy[0] ^ sign, dy[1] ^ sign};
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       float e[2][HPL];
 #pragma unroll
       for (int j = 0; j < HPL; ++j) {
         dw1[j] = fma2(dy[i], hp[i][j], dw1[j]);
-        const uint64_t d = mul2(fma2(hp[i][j] ^ sign, hp[i][j], one), dy[i]);  // tanh_t::bwd
+        const uint64_t d = mul2(fma2(hp[i][j], hp[i][j], minus1), ndy[i]);  // tanh_t::bwd
         unpack2(d, e[0][j], e[1][j]);
       }
 #pragma unroll
@@ -168,7 +168,7 @@ struct Fp32Warp {
                                         const LikParams& lik, int rows_left, float* dys, float* es, uint64_t* dw1,
                                         float& dy_sum, float& loss) const {
     float y_own = 0.f, pred_own = 0.f;
-#pragma unroll 1
+#pragma unroll(H == 40 ? 2 : 1)
     for (int hf = 0; hf < 2; ++hf) {
       uint64_t hp[2][HPL];
       hidden(xb, wp, b0, hf, hp);

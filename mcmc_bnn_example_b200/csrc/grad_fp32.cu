@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(Fp32Geom<H>::NT, MINB) grad_fp32_kernel(const 
       const int row = r0 + lanes.loss_row();
       if (g.row_loss && row < g.n_rows) g.row_loss[(long long)win * g.row_loss_stride + row] = loss;
     }
-    lanes.template backward<4>(xb, es, acc);
+    lanes.template backward<8>(xb, es, acc);
     __syncwarp();  // rows and dL/dz have been read: the next copy and the next block may overwrite them
   }
 
