@@ -1,6 +1,6 @@
 // Tile arithmetic of the resident kernel in FP32 mode (resident.cuh has the launch structure, fp32_tile.cuh what a warp
 // does with its 32 rows): every warp owns one 32-row unit for the whole launch.
-// One launch per step took 29.5 us a step for a 58368-row window, this takes 13.2 (2000 steps, one B200); a log density
+// One launch per step took 29.5 us a step for a 58368-row window, this takes 12.8 (2000 steps, one B200); a log density
 // and gradient of 1000 rows from host pointers takes 34 us instead of 64.
 // What bounds a step: the FMA pipe (about 1,900 multiplications per row, 3,500 cycles each for forward and backward at
 // 512 rows per CTA) and the tanh pass (two MUFU operations each, 2,560 cycles), which overlap as far as the warps of a
