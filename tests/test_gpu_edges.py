@@ -1,0 +1,63 @@
+"""Sizes where the accept ratio's cluster, the prediction kernel's row tiles and sample chunks, and the FP32 kernel's row
+blocks change their partition."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 1023, 8193, 65536, 65537, 200001])
+def test_log_acpt_matches_a_double_sum(built, n):
+    import torch
+    m, _ = built
+    ctx = m.Context(m.baseline_config(precision=m.PREC_FP32, sample_capacity=0), 1, 64)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    prev, new = (torch.randn(n, device="cuda", generator=g) for _ in range(2))
+    m0, m1, grad = (torch.randn(ctx.P, device="cuda", generator=g) for _ in range(3))
+    torch.cuda.synchronize()
+    got = ctx.log_acpt(prev.data_ptr(), new.data_ptr(), n, m0.data_ptr(), m1.data_ptr(), grad.data_ptr(), 0.01)
+    ctx.close()
+    mf = m1.double() + 0.005 * grad.double()
+    kin = 0.5 * (m0.double() ** 2 - mf ** 2)
+    want = float((new.double() - prev.double()).sum() + kin.sum())
+    # the kicked momenta are floats (and so is the step size): 2^-23 of each square; the result is rounded once
+    assert abs(got - want) <= 2.0 ** -22 * float((mf ** 2).sum()) + 2.0 ** -23 * abs(want)
+
+
+@pytest.mark.parametrize("H", [40, 128])
+@pytest.mark.parametrize("rows,count", [(1, 1), (511, 3), (513, 65), (20000, 2)])
+def test_predict_mean_matches_double_arithmetic(built, H, rows, count):
+    m, _ = built
+    ctx = m.Context(m.baseline_config(H=H, precision=m.PREC_FP32, leapfrog_steps=3, sample_capacity=count), 1, 128)
+    x, y, _ = m.synth_window(1, 0, 128)
+    ctx.set_window_data(0, x, y)
+    ctx.run_chain(count)
+    s = ctx.get_samples(0).astype(np.float64)
+    xs = np.random.default_rng(rows).standard_normal((rows, 22)).astype(np.float32)
+    got = ctx.predict_mean(0, xs)
+    ctx.close()
+    want = np.zeros(rows)
+    for p in s:
+        w0, b0, w1, b1 = np.split(p, [22 * H, 23 * H, 24 * H])
+        want += np.tanh(xs.astype(np.float64) @ w0.reshape(22, H) + b0) @ w1 + b1[0]
+    want /= count
+    # 22 products and a tanh of ex2 / rcp approximations (a few 1e-7 each) in each of H units with |w1| of order one
+    scale = np.abs(s[:, 23 * H:24 * H]).sum(axis=1).max()
+    assert np.abs(got - want).max() <= 1e-5 * max(scale, 1.0)
+
+
+@pytest.mark.parametrize("H", [40, 128])
+@pytest.mark.parametrize("rows", [1, 15, 17, 127, 129, 3000])
+def test_fp32_row_blocks_match_the_oracle(built, monkeypatch, H, rows):
+    m, O = built
+    monkeypatch.setenv("MCMC_B200_NO_MULTISTEP", "1")
+    x, y, _ = m.synth_window(3, 0, rows)
+    ctx = m.Context(m.reference_config(H=H, precision=m.PREC_FP32, sample_capacity=0), 1, rows)
+    ctx.set_window_data(0, x, y)
+    w = (0.15 * np.random.default_rng(rows).standard_normal(ctx.P)).astype(np.float32)
+    got = ctx.potential_and_grad(0, w, want_row_loss=True)
+    ctx.close()
+    ref = O.logp_grad(O.reference_model(H=H), x, y, w, want_losses=True)
+    assert np.abs(got["grad"] - ref["grad"]).max() <= 1e-5 * np.abs(ref["grad"]).max()
+    assert abs(got["loglik"] - ref["loglik"]) <= 1e-5 * abs(ref["loglik"])
+    assert np.allclose(got["row_loss"], ref["row_loss"], rtol=1e-4, atol=1e-4)
