@@ -390,6 +390,17 @@ int mcmc_b200_chain_geometry(mcmc_b200_ctx* ctx, int* slices, int* ctas_per_sm, 
  * works.  The status word is cleared on the way out: the context stays usable.
  */
 int mcmc_b200_selftest_wait_timeout(mcmc_b200_ctx* ctx, int limit_us);
+/*
+ * The same for the launches that keep a window's rows on the chip.  Runs one
+ * launch (an iteration of the chain if it has started, else an evaluation; its
+ * results go nowhere) in which the wait `code` runs out after limit_us
+ * microseconds (40 .. 10000; 64 times that for the first wait of a launch),
+ * and returns what the context then reports.  The chain stays where it was.
+ *   603  words of another cluster of the window: one cluster is left out of
+ *        the launch.  Needs a one-window context whose rows (more than 4096)
+ *        several clusters hold.
+ */
+int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* ctx, int code, int limit_us);
 
 #ifdef __cplusplus
 }

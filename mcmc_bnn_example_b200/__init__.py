@@ -42,7 +42,7 @@ EXPORTS = [
     "mcmc_b200_launch_count", "mcmc_b200_chain_geometry", "mcmc_b200_potential_and_grad_static",
     "mcmc_b200_checkpoint_size", "mcmc_b200_checkpoint_save", "mcmc_b200_checkpoint_load",
     "mcmc_b200_read_table", "mcmc_b200_plan_work_table", "mcmc_b200_rebind_data",
-    "mcmc_b200_selftest_wait_timeout", "mcmc_b200_philox_device", "mcmc_b200_refstream_momentum_device",
+    "mcmc_b200_selftest_wait_timeout", "mcmc_b200_selftest_resident_wait", "mcmc_b200_philox_device", "mcmc_b200_refstream_momentum_device",
     "mcmc_b200_refstream_engine", "mcmc_b200_refstream_engine0", "mcmc_b200_refstream_log_uniform",
     "mcmc_b200_microbench_l2_read", "mcmc_b200_microbench_mufu", "mcmc_b200_enable_oneshot_allreduce",
     "mcmc_b200_time_allreduce", "mcmc_b200_selftest_oneshot_timeout",
@@ -410,6 +410,11 @@ class Context:
         """Runs a bounded device-side wait into its limit; returns the status code the context reports
         (4 = MCMC_B200_ERR_TIMEOUT when the time-out route works) and its message."""
         code = lib().mcmc_b200_selftest_wait_timeout(self._h, int(limit_us))
+        return code, lib().mcmc_b200_last_error().decode()
+
+    def selftest_resident_wait(self, code, limit_us=1000):
+        """Runs the wait `code` of an on-chip launch into its limit; returns what the context reports."""
+        code = lib().mcmc_b200_selftest_resident_wait(self._h, int(code), int(limit_us))
         return code, lib().mcmc_b200_last_error().decode()
 
     def philox_device(self, ctr, key, n):

@@ -383,6 +383,10 @@ static size_t resident_words_stride(int P, int cluster) {
   return ((words + cluster - 1) / cluster + 7) / 8 * 8;
 }
 
+static size_t resident_msg_bytes(const mcmc_b200_ctx* c, const ResidentParams& g, int cluster) {
+  return (size_t)2 * g.windows * g.clusters * cluster * resident_words_stride(c->P, cluster) * 16;
+}
+
 // Plans the resident launches of a context and allocates their message buffers.  A fixed `slices` asks for bits
 // that do not depend on what shares the launch: such contexts keep one launch per step.
 static int resident_setup(mcmc_b200_ctx* c) {
@@ -402,7 +406,8 @@ static int resident_setup(mcmc_b200_ctx* c) {
     g.lik = make_lik(c->cfg);
     g.prior = make_prior(c->cfg);
     g.status = c->status;
-    int r = dalloc(c, (void**)&g.msg, (size_t)2 * g.windows * g.clusters * cluster * resident_words_stride(c->P, cluster) * 16);
+    g.wait_ticks = RES_WAIT_TICKS;
+    int r = dalloc(c, (void**)&g.msg, resident_msg_bytes(c, g, cluster));
     if (r == MCMC_B200_OK) r = dalloc(c, (void**)&g.seq, (size_t)g.windows * 4);
     if (r) return r;
     (k ? c->res_x_ok : c->res_ok) = true;
@@ -705,8 +710,18 @@ static int finish_status(mcmc_b200_ctx* c) {
   CK(cudaStreamSynchronize(c->stream));
   const int st = c->hb->status;
   if (st != 0) {
+    // resident launches have done nothing since the report (resident.cuh): none of their words is awaited any more.
+    // (Some may be queued on a caller's stream.)
+    cudaDeviceSynchronize();
     c->hb->status = 0;
+    for (int k = 0; k < 2; ++k)
+      if (k ? c->res_x_ok : c->res_ok) {
+        const ResidentParams& g = k ? c->res_x : c->res;
+        cudaMemsetAsync(g.msg, 0, resident_msg_bytes(c, g, k ? c->res_x_cluster : c->res_cluster), c->stream);
+        cudaMemsetAsync(g.seq, 0, (size_t)g.windows * 4, c->stream);
+      }
     cudaMemsetAsync(c->status, 0, 4, c->stream);
+    cudaStreamSynchronize(c->stream);
     char b[96];
     snprintf(b, sizeof b, "device-side wait ran out (code %d)", st);
     return fail(MCMC_B200_ERR_TIMEOUT, b);
@@ -1313,6 +1328,26 @@ static int resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, c
   return MCMC_B200_OK;
 }
 static bool use_resident_x(const mcmc_b200_ctx* c) { return c->res_x_ok && !c->comm && !c->oneshot; }
+
+API int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* c, int code, int limit_us) {
+  if (!c || limit_us < 40 || limit_us > 10000 || code != 603) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
+  if (c->W != 1 || !c->window_set[0] || !use_resident_x(c) || c->res_x.clusters < 2)
+    return fail(MCMC_B200_ERR_INVALID, "needs one window with data whose rows several clusters hold on the chip");
+  CK(cudaSetDevice(c->device));
+  int r = refstream_fill(c, c->iters_done + 1);
+  if (r) return r;
+  ResidentParams& g = c->bootstrapped ? c->res : c->res_x;
+  g.missing = 1;
+  g.wait_ticks = (unsigned int)limit_us / 33;
+  if (c->bootstrapped) r = resident_chain(c, 1, c->stream);
+  else
+    r = resident_steps(c, 0, 1, 0.f, c->xw[0], nullptr, nullptr, nullptr, nullptr, c->g_out, nullptr, nullptr, nullptr,
+                       c->scalars, c->stream, true);
+  g.missing = 0;
+  g.wait_ticks = RES_WAIT_TICKS;
+  if (r) return r;
+  return check_status(c);
+}
 
 // L leapfrog steps from (w0, m0, g0) on device; results in xw/xm[L&1], g_out, scalars.
 static int explicit_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, const float* w0,

@@ -121,6 +121,7 @@ enum ResidentMode : int {
 };
 constexpr int RES_UNITS = 16;          // 32-row units per CTA
 constexpr int RES_MAX_CLUSTERS = 16;   // clusters of one window
+constexpr unsigned int RES_WAIT_TICKS = 15000;  // about half a second
 struct ResidentParams {
   int mode, n_steps, n_iter;
   int windows, clusters;    // clusters per window
@@ -132,6 +133,8 @@ struct ResidentParams {
   PriorParams prior;
   int* status;
   int* status_host;         // optional: the same code for the host to read without a copy
+  unsigned int wait_ticks;  // limit of the waits, in 2^16 cycles
+  int missing;              // self-test: clusters of the last window that do not start
   // RES_STEPS / RES_EVAL (one window); all outputs but g_out and scalars are optional
   const float *w0, *m0, *g0;
   float eps_scalar;

@@ -31,8 +31,20 @@
 // every weight of step s + 1.
 // (A first version without clusters exchanged everything through L2, owners spread over all CTAs: two
 // trips, each 2,500 - 5,500 cycles with 148 CTAs polling the same lines: 9.4 us per step.)  The accept decision is
-// taken by every warp that owns parameters, from the same shares in the same order.  No atomics; every wait is
-// bounded and ends in the status word.
+// taken by every warp that owns parameters, from the same shares in the same order.  No atomics.
+//
+// Waits that run out.  Every wait is bounded.  The words of another cluster (603) are the only ones that may really
+// stay out: the CTAs of a cluster start together, what they send one another arrives, copies and MMAs end.  When they
+// do, the CTA goes on with the step's exchange, whose sums then mean nothing, and says so in the fourth element of every
+// weight it sends (at the end of a trajectory: in its shares of the log-prior).  So all ranks of the cluster learn of
+// it at the same point, where everything sent has been received; they leave between two barriers of the next step with
+// nothing in flight, and neither samples nor state are stored.  The other clusters' words then stay out too.
+// For waits inside the cluster to run out something must be broken; a CTA then leaves by itself, does not arm its
+// barriers again, waits once more for its copies and MMAs, and for 100 us after the cluster has stopped sending.
+// Launches that start while the status word is set do nothing: the host takes the report, clears the words and
+// the counter, and only then do sequence numbers start anew (old words could otherwise pass for new ones).
+// Limits: `wait_ticks` for words of another cluster, 64 times that for the first ones of a launch (until then some of
+// its CTAs may be waiting for SMs that another stream's kernel holds), four times as long inside a cluster.
 //
 // It replaces, for such windows, the reference's persistent kernel with an unbounded grid barrier
 // (mcmc_step_tc.h:597-677) and its per-iteration host work (main.h:204-283).
@@ -48,7 +60,7 @@ namespace mcmc_b200 {
 constexpr int RES_NWG = 4;                     // warpgroups = resident tiles per CTA
 constexpr int RES_THREADS = RES_NWG * 128;
 constexpr int RES_BAR_E = 1, RES_BAR_T = 5, RES_BAR_X = 9;  // named barriers: + warpgroup, + warpgroup, the exchange
-constexpr uint32_t RES_POLLS = 1u << 20;       // bounded waits: polls of about 0.5 us
+constexpr uint32_t RES_DEAD_LO = 0x4c4f5354u, RES_DEAD_HI = 0x7ff8dead;  // a log-prior share that no sum makes
 
 // ---- words through L2: single 16-byte accesses ----------------------------------------------
 __device__ __forceinline__ void st_word16(uint4* p, uint32_t a, uint32_t b, uint32_t c, uint32_t seq) {
@@ -95,11 +107,19 @@ static __device__ __noinline__ void res_timeout(const ResidentParams& g, int cod
   if (g.status) atomicExch(g.status, code);
   if (g.status_host) *reinterpret_cast<volatile int*>(g.status_host) = code;
 }
+__device__ __forceinline__ uint32_t res_ticks() { return (uint32_t)(clock64() >> 16); }  // of 33 us at 1.965 GHz
 // mbarrier wait of the resident kernel: a bounded spin in line (each try_wait sleeps in hardware for a moment)
-__device__ __forceinline__ void res_wait(uint64_t* bar, uint32_t parity, const ResidentParams& g, int code, bool& ok) {
-  uint32_t n = 0;
-  while (!mbar_try_wait(bar, parity) && ok)
-    if (++n == RES_POLLS) { ok = false; res_timeout(g, code); }
+__device__ __forceinline__ void res_wait(uint64_t* bar, uint32_t parity, const ResidentParams& g, uint32_t limit, int code,
+                                         bool& ok) {
+  if (mbar_try_wait(bar, parity)) return;
+  const uint32_t t0 = res_ticks();
+  while (ok && !mbar_try_wait(bar, parity))
+    if (res_ticks() - t0 > limit) { ok = false; res_timeout(g, code); }
+}
+// for a copy or MMAs that a wait has run out on already, before their memory is given back
+__device__ __forceinline__ void res_drain(uint64_t* bar, uint32_t parity, const ResidentParams& g) {
+  const uint32_t t0 = res_ticks();
+  while (!mbar_try_wait(bar, parity) && res_ticks() - t0 <= g.wait_ticks) {}
 }
 
 // One momentum draw: N(0,1) of (window, iteration, parameter), or the reference's stream
@@ -133,12 +153,12 @@ __device__ __forceinline__ double word_sum(double v) {
 // Tile = the precision's arithmetic for the CTA's rows (resident_tf32.cu, resident_fp32.cu):
 //   Tile::H, Tile::SMEM               hidden units, bytes of dynamic shared memory
 //   Tile(smem, g, win, u0, u1)       per-thread constants; rows 32 u0 .. 32 u1 of the window are this CTA's
-//   setup(tmap, g, win)              loads the rows
+//   setup(tmap, g, win)              loads the rows; false when they did not arrive
 //   stage(v)                         word `threadIdx.x` of the weights (the first ResWords::N threads)
 //   step(g, row_loss, last, ok)      forward, loss, backward of this warpgroup's tile
 //   collects()                       the word whose sum this thread makes, or -1
 //   collect(last, v)                 after the CTA barrier that follows step: the CTA's sums for that word
-//   teardown()
+//   teardown(g, dead)                gives memory back; dead: after one more wait for MMAs
 // The parameters of a word, in an order of their own: words 0 .. 306 are W0 and b0 (the last one two of them), the next
 // fourteen W1 and b1, the last word is the log-likelihood.
 template <int H>
@@ -171,6 +191,8 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   __shared__ __align__(16) uint4 h_in[2][C * XWARPS + 1];   // {kinetic, log-prior} shares; log-likelihood
   __shared__ __align__(16) uint4 x_in[MULTI ? RES_MAX_CLUSTERS * WPM : 1];  // words of all clusters
   __shared__ __align__(8) uint64_t bar_part, bar_w, bar_h;
+  __shared__ int dead_;  // a wait has run out, here or in another CTA of the cluster
+  volatile int& dead = dead_;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = C == 1 ? 0 : (int)cluster_rank();
@@ -185,8 +207,13 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     mbar_init(&bar_w, 1);
     mbar_init(&bar_h, 1);
     mbar_fence_init();
+    dead = 0;
   }
-  c.setup(&tmap, g, win);  // (holds a CTA barrier)
+  // (a status that is set already: see above)
+  const int pending = __ldcg(g.status);
+  if (!c.setup(&tmap, g, win) || pending != 0) dead = 1;  // (setup holds a CTA barrier)
+  bool ok = true;     // no wait of this thread inside the cluster has run out
+  bool lost = false;  // the launch has given up
   const int my_words = min(WPM, NWORDS - rank * WPM);
   const uint32_t part_bytes = (uint32_t)(my_words * C * 16), w_bytes = NWORDS * 16, h_bytes = (C * XWARPS + 1) * 16;
   if (tid == 0) {
@@ -221,7 +248,8 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   const bool chain = g.mode == RES_CHAIN;
   const AcceptParams& a = g.a;
   uint32_t seq = __ldcg(g.seq + win);
-  bool ok = true;
+  // limits of the waits that may last until the last CTA of the launch has started, and of the others
+  auto limit = [&](uint32_t n) { return g.wait_ticks << (n < 2 ? 8 : 2); };
 
   // ---- state of the word's parameters, the same in each of its lanes ----
   const size_t so = (size_t)win * g.Pp;
@@ -247,12 +275,12 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       }
     }
   }
-  auto send_weights = [&]() {
-    if (mine) st_async16(w_dst, w_bar, __float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), 0u);
+  auto send_weights = [&](bool bad) {
+    if (mine) st_async16(w_dst, w_bar, __float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), bad);
   };
   uint32_t n = 0;        // steps done in this launch: the mbarrier phases follow it
   uint32_t n_traj = 0;
-  send_weights();
+  send_weights(dead != 0);
 
   const int L = g.n_steps;
   for (int it = 0; it < g.n_iter; ++it) {
@@ -261,12 +289,22 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       const bool last = s == L - 1;
       ++seq;
       // ---- weights of this step ----
-      res_wait(&bar_w, ph, g, 601, ok);
-      if (tid == 0) mbar_expect_tx(&bar_w, w_bytes);
-      c.stage(w_in[min(tid, NWORDS - 1)]);
+      res_wait(&bar_w, ph, g, limit(n), 601, ok);
+      if (tid == 0 && ok) mbar_expect_tx(&bar_w, w_bytes);
+      {
+        const uint4 v = w_in[min(tid, NWORDS - 1)];
+        if (!ok || v.w != 0u) dead = 1;
+        c.stage(v);  // (ends in a CTA barrier)
+      }
       // ---- this warpgroup's tile ----
       c.step(g, last ? g.row_loss : nullptr, last, ok);
+      const bool leave = dead != 0;  // the same in every thread: nobody writes it between the step's two barriers
       __syncthreads();
+      if (leave) {
+        lost = true;
+        it = g.n_iter;
+        break;
+      }
       // ---- the CTA's sums to their owners ----
       {
         uint4 v;
@@ -281,12 +319,13 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       // ---- owners: the cluster's sum, then the window's ----
       // (the log-likelihood is wanted at the end of a trajectory only)
       const bool ll_warp = last && rank == C - 1 && warp == (NWORDS - 1 - (C - 1) * WPM) * C / 32;
-      res_wait(&bar_part, ph, g, 602, ok);
-      if (tid == 0) mbar_expect_tx(&bar_part, part_bytes);
+      res_wait(&bar_part, ph, g, limit(n), 602, ok);
+      if (tid == 0 && ok) mbar_expect_tx(&bar_part, part_bytes);
       const uint4 x = part_in[l][min(wl, WPM - 1)];
       float v[3] = {__uint_as_float(x.x), __uint_as_float(x.y), __uint_as_float(x.z)};
       word_sum<C>(v);
       double ll = 0.0;
+      bool bad = !ok;
       if (ll_warp) ll = word_sum<C>(ll_word ? u2d(x.x, x.y) : 0.0);
       if (MULTI && K > 1) {
         uint4* const mb = msg + (seq & 1) * msg_buf;
@@ -298,18 +337,24 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         uint4 y[NR];
 #pragma unroll
         for (int i = 0; i < NR; ++i) y[i] = x_has[i] ? ld_word16(mb + x_src[i]) : make_uint4(0u, 0u, 0u, seq);
+        const uint32_t t0 = res_ticks();
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
-          uint32_t t = 0;
-          while (y[i].w != seq && ok) {
+          while (y[i].w != seq) {
 #pragma unroll
             for (int j = i; j < NR; ++j)  // (a word that has arrived is read once more: its value stays)
               if (x_has[j]) y[j] = ld_word16(mb + x_src[j]);
-            if (++t == RES_POLLS) { ok = false; res_timeout(g, 603); }
+            if (res_ticks() - t0 > g.wait_ticks << (n == 0 ? 6 : 0)) {
+              dead = 1;
+              res_timeout(g, 603);
+              break;
+            }
           }
           if (x_has[i]) x_in[tid + i * XT] = y[i];
         }
+        if (!ok) dead = 1;
         named_sync(RES_BAR_X, XT);
+        bad = dead != 0;
         // lane l adds clusters l and l + 8
         const int wi = min(wl, my_words - 1);
         const uint4 y0 = x_in[min(l, K - 1) * my_words + wi], y1 = x_in[min(l + C, K - 1) * my_words + wi];
@@ -330,7 +375,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
           m[q] = fmaf(eps, gf[q], m[q]);
           w[q] = fmaf(eps, m[q], w[q]);
         }
-        send_weights();
+        send_weights(bad);
         continue;
       }
       // ---- end of the trajectory: this warp's share of the log-prior and of the kinetic difference ----
@@ -344,7 +389,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
           if (chain) {  // closing half kick (kernel_helpers.h:163-175)
             const float mf = fmaf(eps * 0.5f, gf[q], m[q]);
             dk += 0.5 * ((double)m_s[q] * (double)m_s[q] - (double)mf * (double)mf);
-          } else if (k == 0) {
+          } else if (k == 0 && !bad) {
             const int p = Words::param(word, q);
             g.g_out[p] = gf[q];
             if (g.w_out) g.w_out[p] = w[q];
@@ -359,8 +404,9 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         dk += __shfl_xor_sync(0xffffffffu, dk, o);
       }
       const uint32_t hb = n_traj & 1;
+      bad = __any_sync(0xffffffffu, bad);
       if (lane < C) {
-        const uint2 x1 = d2u(dk), x2 = d2u(lp);
+        const uint2 x1 = d2u(dk), x2 = bad ? make_uint2(RES_DEAD_LO, RES_DEAD_HI) : d2u(lp);
         st_async16(mapa(smem_u32(&h_in[0][rank * XWARPS + warp]), lane) + hb * H_BUF, mapa(smem_u32(&bar_h), lane), x1.x,
                    x1.y, x2.x, x2.y);
       }
@@ -368,21 +414,28 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         const uint2 x1 = d2u(ll);
         st_async16(mapa(smem_u32(&h_in[0][C * XWARPS]), l) + hb * H_BUF, mapa(smem_u32(&bar_h), l), x1.x, x1.y, 0u, 0u);
       }
-      res_wait(&bar_h, hb, g, 604, ok);
-      if (tid == 0) mbar_expect_tx(&bar_h, h_bytes);
+      res_wait(&bar_h, hb, g, limit(n), 604, ok);
+      if (tid == 0 && ok) mbar_expect_tx(&bar_h, h_bytes);
       ++n_traj;
       dk = lp = 0.0;
+      bad = !ok;
       for (int i = lane; i < C * XWARPS; i += 32) {
         const uint4 x1 = h_in[hb][i];
         dk += u2d(x1.x, x1.y);
         lp += u2d(x1.z, x1.w);
+        bad |= x1.z == RES_DEAD_LO && x1.w == RES_DEAD_HI;
       }
+      lost = __any_sync(0xffffffffu, bad);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         lp += __shfl_xor_sync(0xffffffffu, lp, o);
         dk += __shfl_xor_sync(0xffffffffu, dk, o);
       }
       const double ll_new = u2d(h_in[hb][C * XWARPS].x, h_in[hb][C * XWARPS].y);
+      if (lost) {
+        if (it + 1 < g.n_iter) send_weights(true);
+        continue;
+      }
       if (!chain) {
         if (k == 0 && rank == 0 && tid == 0) {
           g.scalars[0] = ll_new;
@@ -426,7 +479,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         m[q] = fmaf(eps * 0.5f, g_s[q], m_s[q]);
         w[q] = fmaf(eps, m[q], w_s[q]);
       }
-      if (it + 1 < g.n_iter) send_weights();
+      if (it + 1 < g.n_iter) send_weights(false);
       if (k == 0 && l == 0) {
 #pragma unroll
         for (int q = 0; q < 3; ++q)
@@ -439,8 +492,8 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       }
     }
   }
-  // ---- the state the next launch (of either kind) starts from ----
-  if (chain && k == 0 && l == 0) {
+  // ---- the state the next launch (of either kind) starts from; of a launch that gave up: the one it started from ----
+  if (chain && !lost && k == 0 && l == 0) {
 #pragma unroll
     for (int q = 0; q < 3; ++q)
       if (has[q]) {
@@ -453,7 +506,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       }
   }
   if (k == 0 && rank == 0 && tid == 0) {
-    if (chain) {
+    if (chain && !lost) {
       a.ll_cur[win] = ll_cur;
       a.lp_cur[win] = lp_cur;
       a.eps[win] = eps;
@@ -463,8 +516,10 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     // (every cluster of the window has read the counter: this one has used words that carry later values)
     g.seq[win] = seq;
   }
-  c.teardown();
+  if (!ok) dead = 1;
+  c.teardown(g, dead);
   if (C > 1) cluster_sync_all();  // no rank leaves while another may still write to it
+  if (dead) __nanosleep(100000);
 }
 
 // ---- host side ----------------------------------------------------------------------------
@@ -473,7 +528,7 @@ template <typename K>
 static cudaError_t resident_launch(K kernel, int cluster, size_t smem, const void* tmap, const ResidentParams& g,
                                    cudaStream_t st, int* max_clusters) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(max_clusters ? cluster : g.windows * g.clusters * cluster);
+  cfg.gridDim = dim3(max_clusters ? cluster : (g.windows * g.clusters - g.missing) * cluster);
   cfg.blockDim = dim3(RES_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;

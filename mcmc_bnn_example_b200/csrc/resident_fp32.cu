@@ -52,7 +52,8 @@ struct ResFp32 {
     }
   }
 
-  __device__ __forceinline__ void setup(const CUtensorMap*, const ResidentParams& g, int win) {
+  __device__ __forceinline__ bool setup(const CUtensorMap*, const ResidentParams& g, int win) {
+    bool ok = true;
     const int tid = threadIdx.x;
     uint64_t* bar = reinterpret_cast<uint64_t*>(base + BAR);
     if (tid == 0) {
@@ -65,15 +66,16 @@ struct ResFp32 {
     for (int i = tid; i < DUMMY - RW1; i += RES_THREADS) base[RW1 + i] = 0.f;
     __syncthreads();
     if (n_units > 0) {
-      bool ok = true;
       const uint32_t bytes = (uint32_t)n_units * 32 * KP * 4;
       if (tid == 0) {
         mbar_expect_tx(bar, bytes);
         bulk_g2s(base + XB, g.xaug + ((size_t)(g.data_window0 + win) * g.rows_pad + row0) * KP, bytes, bar);
       }
-      res_wait(bar, 0, g, 611, ok);
+      res_wait(bar, 0, g, g.wait_ticks << 2, 611, ok);
+      if (!ok) res_drain(bar, 0, g);
     }
     __syncthreads();
+    return ok;
   }
 
   // word `threadIdx.x` of the weights
@@ -179,7 +181,7 @@ struct ResFp32 {
     v = make_uint4(__float_as_uint(o[0]), __float_as_uint(o[1]), __float_as_uint(o[2]), 0u);
     return (int)threadIdx.x < Words::W0;
   }
-  __device__ __forceinline__ void teardown() {}
+  __device__ __forceinline__ void teardown(const ResidentParams&, const volatile int&) {}
 };
 
 cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,

@@ -80,7 +80,7 @@ struct ResTf32 {
     stage_setup();
   }
 
-  __device__ __forceinline__ void setup(const CUtensorMap* tmap, const ResidentParams& g, int) {
+  __device__ __forceinline__ bool setup(const CUtensorMap* tmap, const ResidentParams& g, int) {
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x;
     if (warp == 0) {
@@ -132,6 +132,7 @@ struct ResTf32 {
     __syncthreads();
     if (tid < RES_THREADS / 4) reinterpret_cast<float4*>(base + GP)[tid] = zero;
     fence_proxy_async_smem();
+    return true;
   }
 
   // word `threadIdx.x` of the weights: where its three values go (addresses found once, words of W1 twice, the second
@@ -188,7 +189,7 @@ struct ResTf32 {
     uint64_t w1p[5];
 #pragma unroll
     for (int n = 0; n < 5; ++n) w1p[n] = *reinterpret_cast<const uint64_t*>(w1 + 8 * n + 2 * (lane & 3));
-    res_wait(bar(wg, 1), par, g, 612, ok);
+    res_wait(bar(wg, 1), par, g, g.wait_ticks << 2, 612, ok);
     tc_fence_after();
     float dy_row = 0.f, loss = 0.f;
     if (wg > 0) named_sync(RES_BAR_T + wg, 256);  // the warpgroup before this one has had its turn
@@ -310,7 +311,7 @@ struct ResTf32 {
     if (nt == RES_NWG && warp == 0)
       for (int w = 1; w < nt; ++w) issue_backward(w, nt, 160);
     // ---- the first warpgroup reads the accumulator out ----
-    res_wait(bar_bwd(), ph, g, 613, ok);
+    res_wait(bar_bwd(), ph, g, g.wait_ticks << 2, 613, ok);
     tc_fence_after();
     // accumulator row i = 32 * group + feature lives in lane 32 * (i / 16) + i % 16 (M = 64)
     {
@@ -414,9 +415,13 @@ struct ResTf32 {
     return t < Words::W0;
   }
 
-  __device__ __forceinline__ void teardown() {
+  __device__ __forceinline__ void teardown(const ResidentParams& g, const volatile int& dead) {
     tc_fence_before();
     __syncthreads();
+    if (warp == 0 && dead) {
+      for (int w = 0; 4 * w < n_units; ++w) res_drain(bar(w, 1), par ^ 1, g);
+      if (n_units > 0) res_drain(bar_bwd(), par ^ 1, g);
+    }
     if (warp == 0)
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS)
                    : "memory");

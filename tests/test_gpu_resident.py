@@ -58,3 +58,36 @@ def test_resident_launch_matches_oracle_and_per_step_launches(built, monkeypatch
         assert np.allclose(t1["log_acpt"], t2["log_acpt"], rtol=1e-3, atol=1e-3)
         assert np.abs(s1[:n_iter - 1] - s2[:n_iter - 1]).max() <= 1e-4 * max(1e-3, np.abs(s2[:n_iter - 1]).max())
         assert abs(g1["loglik"] - g2["loglik"]) <= 1e-6 * abs(g2["loglik"])
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_a_wait_that_runs_out_reports_and_leaves_the_chain_where_it_was(built, prec):
+    """One cluster of the window is left out of a launch, so that the others' waits for its words run out: by themselves,
+    with a status, and without a step of the chain."""
+    m, _ = built
+    rows = 9001
+    x, y, _ = m.synth_window(8, 0, rows)
+    w = (0.1 * np.random.default_rng(2).standard_normal(P)).astype(np.float32)
+
+    def run(disturbed):
+        ctx = m.Context(m.reference_config(precision=prec, leapfrog_steps=3, burn_in=0, sample_capacity=8, seed=3), 1, rows)
+        ctx.set_window_data(0, x, y)
+        if disturbed:
+            code, msg = ctx.selftest_resident_wait(603)
+            assert code == 4 and "603" in msg, (code, msg)
+        out = [ctx.potential_and_grad(0, w)["grad"]]
+        ctx.run_chain(4)
+        if disturbed:
+            before = ctx.get_state(0), ctx.chain_info(0)
+            code, msg = ctx.selftest_resident_wait(603)
+            assert code == 4 and "603" in msg, (code, msg)
+            after = ctx.get_state(0), ctx.chain_info(0)
+            assert before[1] == after[1] and all(np.array_equal(before[0][k], after[0][k]) for k in before[0])
+            ctx.synchronize()  # reported once
+        ctx.run_chain(4)
+        out += [ctx.get_samples(0), ctx.potential_and_grad(0, w)["grad"]]
+        ctx.close()
+        return out
+
+    for a, b in zip(run(True), run(False)):
+        assert np.array_equal(a, b)
