@@ -399,6 +399,9 @@ int mcmc_b200_selftest_wait_timeout(mcmc_b200_ctx* ctx, int limit_us);
  *   603  words of another cluster of the window: one cluster is left out of
  *        the launch.  Needs a one-window context whose rows (more than 4096)
  *        several clusters hold.
+ *   611  the load of the rows.  An evaluation (mcmc_b200_potential_and_grad).
+ *   901  a wait of an earlier launch that nobody has asked about yet, before
+ *        an evaluation, which then has to report it.
  */
 int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* ctx, int code, int limit_us);
 

@@ -1330,10 +1330,25 @@ static int resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, c
 static bool use_resident_x(const mcmc_b200_ctx* c) { return c->res_x_ok && !c->comm && !c->oneshot; }
 
 API int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* c, int code, int limit_us) {
-  if (!c || limit_us < 40 || limit_us > 10000 || code != 603) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
-  if (c->W != 1 || !c->window_set[0] || !use_resident_x(c) || c->res_x.clusters < 2)
-    return fail(MCMC_B200_ERR_INVALID, "needs one window with data whose rows several clusters hold on the chip");
+  if (!c || limit_us < 40 || limit_us > 10000 || (code != 603 && code != 611 && code != 901))
+    return fail(MCMC_B200_ERR_INVALID, "bad arguments");
+  if (c->W != 1 || !c->window_set[0] || !use_resident_x(c) || (code == 603 && c->res_x.clusters < 2))
+    return fail(MCMC_B200_ERR_INVALID, "needs one window with data whose rows (603: more than 4096) fit on the chip");
   CK(cudaSetDevice(c->device));
+  if (code == 901) {
+    cudaError_t e = launch_wait_probe(c->status, (unsigned int)(limit_us / 20), c->stream);
+    c->launches++;
+    if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
+  }
+  if (code == 611 || code == 901) {
+    c->res_x.test_code = code;
+    c->res_x.wait_ticks = (unsigned int)limit_us / 33;
+    const std::vector<float> w(c->P, 0.f);
+    const int r = mcmc_b200_potential_and_grad(c, 0, w.data(), nullptr, nullptr, nullptr, nullptr);
+    c->res_x.test_code = 0;
+    c->res_x.wait_ticks = RES_WAIT_TICKS;
+    return r;
+  }
   int r = refstream_fill(c, c->iters_done + 1);
   if (r) return r;
   ResidentParams& g = c->bootstrapped ? c->res : c->res_x;
@@ -1534,6 +1549,8 @@ API int mcmc_b200_log_acpt(mcmc_b200_ctx* c, const float* prev_loss, const float
   c->launches++;
   if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
   CK(cudaStreamSynchronize(st));
+  // (the losses may come from a trajectory that has given up)
+  if (*reinterpret_cast<volatile int*>(&c->hb->status) != 0) return finish_status(c);
   *out = c->hb->log_acpt;
   return MCMC_B200_OK;
 }

@@ -132,9 +132,10 @@ struct ResidentParams {
   LikParams lik;
   PriorParams prior;
   int* status;
-  int* status_host;         // optional: the same code for the host to read without a copy
+  int* status_host;         // optional: the same code for the host to read without a copy; also one that was set before
   unsigned int wait_ticks;  // limit of the waits, in 2^16 cycles
   int missing;              // self-test: clusters of the last window that do not start
+  int test_code;            // self-test: 611 adds a wait for rows that nothing ends
   // RES_STEPS / RES_EVAL (one window); all outputs but g_out and scalars are optional
   const float *w0, *m0, *g0;
   float eps_scalar;

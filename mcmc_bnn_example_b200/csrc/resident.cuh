@@ -211,6 +211,8 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   }
   // (a status that is set already: see above)
   const int pending = __ldcg(g.status);
+  if (pending != 0 && g.status_host && blockIdx.x == 0 && tid == 0)
+    *reinterpret_cast<volatile int*>(g.status_host) = pending;
   if (!c.setup(&tmap, g, win) || pending != 0) dead = 1;  // (setup holds a CTA barrier)
   bool ok = true;     // no wait of this thread inside the cluster has run out
   bool lost = false;  // the launch has given up

@@ -73,6 +73,7 @@ struct ResFp32 {
       }
       res_wait(bar, 0, g, g.wait_ticks << 2, 611, ok);
       if (!ok) res_drain(bar, 0, g);
+      if (g.test_code == 611) res_wait(bar, 1, g, g.wait_ticks << 2, 611, ok);  // (nothing ends this phase)
     }
     __syncthreads();
     return ok;

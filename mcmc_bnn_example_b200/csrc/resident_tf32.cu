@@ -104,14 +104,16 @@ struct ResTf32 {
     tc_fence_after();
     tmem = tmem_slot;
     y = 0.f;
+    bool ok = true;
     if (tile_active) {
-      bool ok = true;
       unsigned char* xt = base + XB + wg * TILE_BYTES;
       if (wtid == 0) {
         mbar_expect_tx(bar(wg, 0), TILE_BYTES);
         tma_load_2d(xt, tmap, 0, row0, bar(wg, 0));
       }
-      mbar_wait_q(bar(wg, 0), 0, g.status, 611, ok);
+      res_wait(bar(wg, 0), 0, g, g.wait_ticks << 2, 611, ok);
+      if (!ok) res_drain(bar(wg, 0), 0, g);
+      if (g.test_code == 611) res_wait(bar(wg, 0), 1, g, g.wait_ticks << 2, 611, ok);  // (nothing ends this phase)
       // this thread's row: 32-byte chunk j of row r sits at position j ^ (r % 4); once per launch, so bank
       // conflicts do not matter here.  Rows of other CTAs or windows in the tile are zeroed.
       const uint32_t xr = smem_u32(xt) + wtid * 128;
@@ -132,7 +134,7 @@ struct ResTf32 {
     __syncthreads();
     if (tid < RES_THREADS / 4) reinterpret_cast<float4*>(base + GP)[tid] = zero;
     fence_proxy_async_smem();
-    return true;
+    return ok;
   }
 
   // word `threadIdx.x` of the weights: where its three values go (addresses found once, words of W1 twice, the second

@@ -91,3 +91,19 @@ def test_a_wait_that_runs_out_reports_and_leaves_the_chain_where_it_was(built, p
 
     for a, b in zip(run(True), run(False)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("code", [611, 901])
+def test_evaluations_report_rows_that_do_not_arrive_and_earlier_time_outs(built, prec, code):
+    m, _ = built
+    x, y, _ = m.synth_window(8, 0, 700)
+    w = (0.1 * np.random.default_rng(2).standard_normal(P)).astype(np.float32)
+    ctx = m.Context(m.baseline_config(precision=prec), 1, 700)
+    ctx.set_window_data(0, x, y)
+    before = ctx.potential_and_grad(0, w)
+    got, msg = ctx.selftest_resident_wait(code)
+    assert got == 4 and str(code) in msg, (got, msg)
+    after = ctx.potential_and_grad(0, w)
+    assert np.array_equal(before["grad"], after["grad"]) and before["loglik"] == after["loglik"]
+    ctx.close()
