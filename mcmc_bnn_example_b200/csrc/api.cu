@@ -999,15 +999,18 @@ static int chain_grad(mcmc_b200_ctx* c, int mode, int s, cudaStream_t st) {
   return MCMC_B200_OK;
 }
 
-// n_iter HMC iterations in cooperative launches that keep the rows on the chip.  A launch is kept to about a
-// tenth of a second so that other work on the GPU gets its turn.
+// Leapfrog steps of one resident launch: about a tenth of a second, so that other work on the GPU gets its turn.
+// Longer trajectories take one launch per step.
+static int resident_max_steps(const mcmc_b200_ctx* c) { return c->cfg.precision == MCMC_B200_PREC_TF32 ? 20000 : 10000; }
+
+// n_iter HMC iterations in cooperative launches that keep the rows on the chip
 static int resident_chain(mcmc_b200_ctx* c, int n_iter, cudaStream_t st) {
   ResidentParams g = c->res;
   g.mode = RES_CHAIN;
   g.n_steps = c->cfg.leapfrog_steps;
   g.a = base_accept_params(c);
   fill_chain_accept(c, g.a, ACC_ITERATE, g.n_steps);
-  const int per_launch = std::max(1, (c->cfg.precision == MCMC_B200_PREC_TF32 ? 20000 : 10000) / g.n_steps);
+  const int per_launch = resident_max_steps(c) / g.n_steps;
   for (int done = 0; done < n_iter; done += g.n_iter) {
     g.n_iter = std::min(per_launch, n_iter - done);
     cudaError_t e = launch_resident(c, c->res_cluster, g, st);
@@ -1086,7 +1089,7 @@ API int mcmc_b200_run_chain_async(mcmc_b200_ctx* c, int n_iter) {
     int r = refstream_fill(c, c->iters_done + n_iter);
     if (r) return r;
   }
-  if (c->res_ok && !c->comm && !c->oneshot) {
+  if (c->res_ok && !c->comm && !c->oneshot && c->cfg.leapfrog_steps <= resident_max_steps(c)) {
     int r = resident_chain(c, n_iter, c->stream);
     if (r == MCMC_B200_OK) c->iters_done += n_iter;
     return r;
@@ -1327,12 +1330,14 @@ static int resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, c
   if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, std::string("resident launch: ") + cudaGetErrorString(e));
   return MCMC_B200_OK;
 }
-static bool use_resident_x(const mcmc_b200_ctx* c) { return c->res_x_ok && !c->comm && !c->oneshot; }
+static bool use_resident_x(const mcmc_b200_ctx* c, int L) {
+  return c->res_x_ok && !c->comm && !c->oneshot && L <= resident_max_steps(c);
+}
 
 API int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* c, int code, int limit_us) {
   if (!c || limit_us < 40 || limit_us > 10000 || (code != 603 && code != 611 && code != 901))
     return fail(MCMC_B200_ERR_INVALID, "bad arguments");
-  if (c->W != 1 || !c->window_set[0] || !use_resident_x(c) || (code == 603 && c->res_x.clusters < 2))
+  if (c->W != 1 || !c->window_set[0] || !use_resident_x(c, 1) || (code == 603 && c->res_x.clusters < 2))
     return fail(MCMC_B200_ERR_INVALID, "needs one window with data whose rows (603: more than 4096) fit on the chip");
   CK(cudaSetDevice(c->device));
   if (code == 901) {
@@ -1425,7 +1430,7 @@ API int mcmc_b200_potential_and_grad(mcmc_b200_ctx* c, int window, const float* 
   if (!c || !w || window < 0 || window >= c->W) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
   if (!c->window_set[window]) return fail(MCMC_B200_ERR_INVALID, "window has no data yet");
   CK(cudaSetDevice(c->device));
-  if (use_resident_x(c)) {
+  if (use_resident_x(c, 1)) {
     // parameters, gradient and sums go through the mapped host block: one launch and one wait, no copies
     memcpy(c->hb->w, w, (size_t)c->P * 4);
     int r = resident_steps(c, window, 1, 0.f, c->hb->w, nullptr, nullptr, nullptr, nullptr, c->hb->g_out, nullptr,
@@ -1464,7 +1469,7 @@ API int mcmc_b200_leapfrog(mcmc_b200_ctx* c, int window, int L, float eps, const
   if (!c->window_set[window]) return fail(MCMC_B200_ERR_INVALID, "window has no data yet");
   CK(cudaSetDevice(c->device));
   const size_t n = (size_t)c->P * 4;
-  if (use_resident_x(c)) {
+  if (use_resident_x(c, L)) {
     HostBlock* h = c->hb;
     memcpy(h->w, w_prev, n);
     memcpy(h->m, mom_prev, n);
@@ -1520,7 +1525,7 @@ API int mcmc_b200_mcmc_step(mcmc_b200_ctx* c, const float* x, const float* y, co
     c->window_set[0] = 1;
     repacked = true;
   }
-  if (use_resident_x(c))
+  if (use_resident_x(c, L))
     return resident_steps(c, 0, L, eps, weights_prev, mom_prev, grad_prev, weights_next, mom_next, grad_cur, grad_next,
                           loss_values, loss_values ? loss_values + c->rows : nullptr, c->scalars, st, false);
   int r = explicit_steps(c, 0, L, eps, weights_prev, mom_prev, grad_prev, weights_next, mom_next, grad_cur,

@@ -107,3 +107,20 @@ def test_evaluations_report_rows_that_do_not_arrive_and_earlier_time_outs(built,
     after = ctx.potential_and_grad(0, w)
     assert np.array_equal(before["grad"], after["grad"]) and before["loglik"] == after["loglik"]
     ctx.close()
+
+
+@pytest.mark.parametrize("prec,most", [(0, 10000), (1, 20000)])
+def test_trajectories_above_a_launch_of_a_tenth_of_a_second_take_one_launch_per_step(built, prec, most):
+    m, _ = built
+    x, y, _ = m.synth_window(8, 0, 64)
+    w = (0.1 * np.random.default_rng(2).standard_normal(P)).astype(np.float32)
+    for L, per_step in ((most, False), (most + 1, True)):
+        ctx = m.Context(m.reference_config(precision=prec, leapfrog_steps=L, burn_in=0, adapt_steps=0, sample_capacity=1,
+                                           eps0=1e-6), 1, 64)
+        ctx.set_window_data(0, x, y)
+        ctx.launch_count(reset=True)
+        out = ctx.leapfrog(0, L, 1e-6, w, w, w)
+        assert (ctx.launch_count(reset=True) > L) == per_step and np.isfinite(out["w_next"]).all()
+        ctx.run_chain(1)
+        assert (ctx.launch_count() > L) == per_step and ctx.chain_info(0)["iterations"] == 1
+        ctx.close()
