@@ -404,6 +404,9 @@ int mcmc_b200_selftest_wait_timeout(mcmc_b200_ctx* ctx, int limit_us);
  *        an evaluation, which then has to report it.
  */
 int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* ctx, int code, int limit_us);
+/* The next `launches` launches of that kind are answered as too large for the
+ * GPU, without a launch: the calls then take one launch per leapfrog step. */
+int mcmc_b200_selftest_refuse_resident(mcmc_b200_ctx* ctx, int launches);
 
 #ifdef __cplusplus
 }

@@ -191,6 +191,7 @@ struct mcmc_b200_ctx {
   bool res_ok = false, res_x_ok = false;
   ResidentParams res, res_x;
   int res_cluster = 1, res_x_cluster = 1;  // CTAs per cluster
+  int refuse = 0;  // self-test: the next such launches that are answered as too large
   // host block the kernels of the explicit host-pointer calls read and write directly (mapped, page-locked)
   HostBlock* hb = nullptr;
   // small device arrays are cut from zeroed slabs
@@ -330,14 +331,18 @@ static int build_work_table(mcmc_b200_ctx* c, int windows, long long tiles_per_w
                             int chunks_per_window, int** d_seg_ptr, int4** d_segs, int** d_nslot,
                             int* n_ctas, int* max_slots);
 
-static cudaError_t launch_resident(const mcmc_b200_ctx* c, int cluster, const ResidentParams& g, cudaStream_t st,
+static cudaError_t launch_resident(mcmc_b200_ctx* c, int cluster, const ResidentParams& g, cudaStream_t st,
                                    int* max_clusters = nullptr) {
+  if (!max_clusters && c->refuse > 0) {
+    --c->refuse;
+    return cudaErrorCooperativeLaunchTooLarge;
+  }
   return (c->cfg.precision == MCMC_B200_PREC_TF32 ? launch_resident_tf32 : launch_resident_fp32)(
       cluster, &c->tmap_mn, g, st, max_clusters);
 }
 // Clusters of 1 << i CTAs that can be resident.  Asked once per device and kernel, and only when a plan wants to know:
 // the first question loads the kernel, which costs more than the rest of a small context.
-static int resident_max_clusters(const mcmc_b200_ctx* c, int i) {
+static int resident_max_clusters(mcmc_b200_ctx* c, int i) {
   static std::mutex mutex;
   static int known[2][64][4];
   static bool asked[2][64][4] = {};
@@ -359,7 +364,7 @@ static int resident_max_clusters(const mcmc_b200_ctx* c, int i) {
 //     exchange then never leaves the cluster;
 //   * rows that one cluster of 8 cannot hold: as many clusters of 8 as every window can have (up to 16) while each
 //     CTA still has at least four 32-row units (below that the step is all exchange and more CTAs only add to it).
-static bool resident_plan(const mcmc_b200_ctx* c, int windows, int* cluster, int* clusters) {
+static bool resident_plan(mcmc_b200_ctx* c, int windows, int* cluster, int* clusters) {
   const long long units = (c->rows + 31) / 32;
   if ((long long)windows * ((units + RES_UNITS - 1) / RES_UNITS) > c->num_sms) return false;
   for (int i = 3; i >= 0; --i)
@@ -1003,7 +1008,9 @@ static int chain_grad(mcmc_b200_ctx* c, int mode, int s, cudaStream_t st) {
 // Longer trajectories take one launch per step.
 static int resident_max_steps(const mcmc_b200_ctx* c) { return c->cfg.precision == MCMC_B200_PREC_TF32 ? 20000 : 10000; }
 
-// n_iter HMC iterations in cooperative launches that keep the rows on the chip
+// Up to n_iter HMC iterations in cooperative launches that keep the rows on the chip; returns how many were queued.  A
+// launch that is refused (not all of its CTAs fit into what the stream or the process may use) has done nothing: the
+// caller goes on with one launch per step, and an error of another kind shows up there again.
 static int resident_chain(mcmc_b200_ctx* c, int n_iter, cudaStream_t st) {
   ResidentParams g = c->res;
   g.mode = RES_CHAIN;
@@ -1011,14 +1018,16 @@ static int resident_chain(mcmc_b200_ctx* c, int n_iter, cudaStream_t st) {
   g.a = base_accept_params(c);
   fill_chain_accept(c, g.a, ACC_ITERATE, g.n_steps);
   const int per_launch = resident_max_steps(c) / g.n_steps;
-  for (int done = 0; done < n_iter; done += g.n_iter) {
+  int done = 0;
+  for (; done < n_iter; done += g.n_iter) {
     g.n_iter = std::min(per_launch, n_iter - done);
-    cudaError_t e = launch_resident(c, c->res_cluster, g, st);
+    if (launch_resident(c, c->res_cluster, g, st) != cudaSuccess) {
+      cudaGetLastError();
+      break;
+    }
     c->launches++;
-    if (e != cudaSuccess)
-      return fail(MCMC_B200_ERR_CUDA, std::string("resident chain launch: ") + cudaGetErrorString(e));
   }
-  return MCMC_B200_OK;
+  return done;
 }
 
 static int queue_iteration(mcmc_b200_ctx* c, cudaStream_t st) {
@@ -1090,9 +1099,10 @@ API int mcmc_b200_run_chain_async(mcmc_b200_ctx* c, int n_iter) {
     if (r) return r;
   }
   if (c->res_ok && !c->comm && !c->oneshot && c->cfg.leapfrog_steps <= resident_max_steps(c)) {
-    int r = resident_chain(c, n_iter, c->stream);
-    if (r == MCMC_B200_OK) c->iters_done += n_iter;
-    return r;
+    const int done = resident_chain(c, n_iter, c->stream);
+    c->iters_done += done;
+    n_iter -= done;
+    if (n_iter == 0) return MCMC_B200_OK;
   }
   // One HMC iteration (L gradient launches + the accept kernel) is captured
   // once and replayed: launch cost stays off the critical path.
@@ -1303,9 +1313,9 @@ API int mcmc_b200_checkpoint_load(mcmc_b200_ctx* c, const void* host_buf, uint64
 }
 
 // ---- explicit-state calls (one window) -------------------------------------
-// The same in one launch where the window's rows fit on the chip.  Pointers may be device memory or the mapped
-// host block.
-static int resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, const float* w0, const float* m0,
+// explicit_steps in one launch where the window's rows fit on the chip.  Pointers may be device memory or the mapped
+// host block.  False: the launch was refused and nothing has been done (see resident_chain).
+static bool resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, const float* w0, const float* m0,
                           const float* g0, float* w_last, float* m_last, float* g_out, float* zero_out,
                           float* row_loss, float* prior_loss, double* scalars, cudaStream_t st, bool eval_only) {
   ResidentParams g = c->res_x;
@@ -1325,10 +1335,12 @@ static int resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, c
   g.row_loss = row_loss;
   g.prior_loss = prior_loss;
   g.scalars = scalars;
-  cudaError_t e = launch_resident(c, c->res_x_cluster, g, st);
+  if (launch_resident(c, c->res_x_cluster, g, st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
   c->launches++;
-  if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, std::string("resident launch: ") + cudaGetErrorString(e));
-  return MCMC_B200_OK;
+  return true;
 }
 static bool use_resident_x(const mcmc_b200_ctx* c, int L) {
   return c->res_x_ok && !c->comm && !c->oneshot && L <= resident_max_steps(c);
@@ -1359,14 +1371,19 @@ API int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* c, int code, int limit_u
   ResidentParams& g = c->bootstrapped ? c->res : c->res_x;
   g.missing = 1;
   g.wait_ticks = (unsigned int)limit_us / 33;
-  if (c->bootstrapped) r = resident_chain(c, 1, c->stream);
-  else
-    r = resident_steps(c, 0, 1, 0.f, c->xw[0], nullptr, nullptr, nullptr, nullptr, c->g_out, nullptr, nullptr, nullptr,
-                       c->scalars, c->stream, true);
+  const bool done = c->bootstrapped ? resident_chain(c, 1, c->stream) == 1
+                                    : resident_steps(c, 0, 1, 0.f, c->xw[0], nullptr, nullptr, nullptr, nullptr, c->g_out,
+                                                     nullptr, nullptr, nullptr, c->scalars, c->stream, true);
   g.missing = 0;
   g.wait_ticks = RES_WAIT_TICKS;
-  if (r) return r;
+  if (!done) return fail(MCMC_B200_ERR_CUDA, "the launch was refused");
   return check_status(c);
+}
+
+API int mcmc_b200_selftest_refuse_resident(mcmc_b200_ctx* c, int launches) {
+  if (!c || launches < 0) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
+  c->refuse = launches;
+  return MCMC_B200_OK;
 }
 
 // L leapfrog steps from (w0, m0, g0) on device; results in xw/xm[L&1], g_out, scalars.
@@ -1430,15 +1447,14 @@ API int mcmc_b200_potential_and_grad(mcmc_b200_ctx* c, int window, const float* 
   if (!c || !w || window < 0 || window >= c->W) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
   if (!c->window_set[window]) return fail(MCMC_B200_ERR_INVALID, "window has no data yet");
   CK(cudaSetDevice(c->device));
-  if (use_resident_x(c, 1)) {
-    // parameters, gradient and sums go through the mapped host block: one launch and one wait, no copies
-    memcpy(c->hb->w, w, (size_t)c->P * 4);
-    int r = resident_steps(c, window, 1, 0.f, c->hb->w, nullptr, nullptr, nullptr, nullptr, c->hb->g_out, nullptr,
-                           row_loss ? c->row_loss : nullptr, nullptr, c->hb->scalars, c->stream, true);
-    if (r) return r;
+  // parameters, gradient and sums go through the mapped host block: one launch and one wait, no copies
+  if (use_resident_x(c, 1) &&
+      (memcpy(c->hb->w, w, (size_t)c->P * 4),
+       resident_steps(c, window, 1, 0.f, c->hb->w, nullptr, nullptr, nullptr, nullptr, c->hb->g_out, nullptr,
+                      row_loss ? c->row_loss : nullptr, nullptr, c->hb->scalars, c->stream, true))) {
     if (row_loss)
       CK(cudaMemcpyAsync(row_loss, c->row_loss, (size_t)c->rows * 4, cudaMemcpyDeviceToHost, c->stream));
-    r = finish_status(c);
+    int r = finish_status(c);
     if (r) return r;
     if (grad) memcpy(grad, c->hb->g_out, (size_t)c->P * 4);
     if (loglik) *loglik = c->hb->scalars[0];
@@ -1469,14 +1485,12 @@ API int mcmc_b200_leapfrog(mcmc_b200_ctx* c, int window, int L, float eps, const
   if (!c->window_set[window]) return fail(MCMC_B200_ERR_INVALID, "window has no data yet");
   CK(cudaSetDevice(c->device));
   const size_t n = (size_t)c->P * 4;
-  if (use_resident_x(c, L)) {
-    HostBlock* h = c->hb;
-    memcpy(h->w, w_prev, n);
-    memcpy(h->m, mom_prev, n);
-    memcpy(h->g, grad_prev, n);
-    int r = resident_steps(c, window, L, eps, h->w, h->m, h->g, h->w_out, h->m_out, h->g_out, nullptr, nullptr, nullptr,
-                           h->scalars, c->stream, false);
-    if (r == MCMC_B200_OK) r = finish_status(c);
+  HostBlock* h = c->hb;
+  if (use_resident_x(c, L) &&
+      (memcpy(h->w, w_prev, n), memcpy(h->m, mom_prev, n), memcpy(h->g, grad_prev, n),
+       resident_steps(c, window, L, eps, h->w, h->m, h->g, h->w_out, h->m_out, h->g_out, nullptr, nullptr, nullptr,
+                      h->scalars, c->stream, false))) {
+    int r = finish_status(c);
     if (r) return r;
     if (w_next) memcpy(w_next, h->w_out, n);
     if (mom_next) memcpy(mom_next, h->m_out, n);
@@ -1525,9 +1539,10 @@ API int mcmc_b200_mcmc_step(mcmc_b200_ctx* c, const float* x, const float* y, co
     c->window_set[0] = 1;
     repacked = true;
   }
-  if (use_resident_x(c, L))
-    return resident_steps(c, 0, L, eps, weights_prev, mom_prev, grad_prev, weights_next, mom_next, grad_cur, grad_next,
-                          loss_values, loss_values ? loss_values + c->rows : nullptr, c->scalars, st, false);
+  if (use_resident_x(c, L) &&
+      resident_steps(c, 0, L, eps, weights_prev, mom_prev, grad_prev, weights_next, mom_next, grad_cur, grad_next,
+                     loss_values, loss_values ? loss_values + c->rows : nullptr, c->scalars, st, false))
+    return MCMC_B200_OK;
   int r = explicit_steps(c, 0, L, eps, weights_prev, mom_prev, grad_prev, weights_next, mom_next, grad_cur,
                          loss_values, loss_values ? loss_values + c->rows : nullptr, st, false, repacked);
   if (r) return r;

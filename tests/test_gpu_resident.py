@@ -124,3 +124,49 @@ def test_trajectories_above_a_launch_of_a_tenth_of_a_second_take_one_launch_per_
         ctx.run_chain(1)
         assert (ctx.launch_count() > L) == per_step and ctx.chain_info(0)["iterations"] == 1
         ctx.close()
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_a_refused_launch_becomes_one_launch_per_step(built, monkeypatch, prec):
+    """The driver's answer to a launch that does not fit is made on the host."""
+    import torch
+    m, _ = built
+    rows, L = 5000, 3
+    x, y, _ = m.synth_window(8, 0, rows)
+    w = (0.1 * np.random.default_rng(2).standard_normal(P)).astype(np.float32)
+    xd, yd, wd = (torch.from_numpy(v).cuda() for v in (x, y, w))
+
+    def run(refuse):
+        ctx = m.Context(m.reference_config(precision=prec, leapfrog_steps=L, burn_in=0, sample_capacity=6), 1, rows)
+        ctx.set_window_data(0, x, y)
+        out = []
+        if refuse:
+            ctx.selftest_refuse_resident(1)
+        out.append(ctx.potential_and_grad(0, w, want_row_loss=True)["row_loss"])
+        if refuse:
+            ctx.selftest_refuse_resident(1)
+        out.append(ctx.leapfrog(0, L, 1e-3, w, w, w)["w_next"])
+        if refuse:
+            ctx.selftest_refuse_resident(1)
+        ctx.run_chain(6)
+        out.append(ctx.get_samples(0))
+        b = [torch.full((P,), 7.0, device="cuda") for _ in range(4)]
+        loss = torch.zeros(rows + P, device="cuda")
+        torch.cuda.synchronize()
+        if refuse:
+            ctx.selftest_refuse_resident(1)
+        ctx.mcmc_step(xd.data_ptr(), yd.data_ptr(), wd.data_ptr(), b[0].data_ptr(), wd.data_ptr(), b[1].data_ptr(),
+                      wd.data_ptr(), b[2].data_ptr(), b[3].data_ptr(), loss.data_ptr(), L, 1e-3)
+        ctx.synchronize()
+        out += [v.cpu().numpy() for v in b] + [loss.cpu().numpy()]
+        n = ctx.launch_count()
+        ctx.close()
+        return out, n
+
+    monkeypatch.delenv("MCMC_B200_NO_MULTISTEP", raising=False)
+    refused, n_refused = run(True)
+    monkeypatch.setenv("MCMC_B200_NO_MULTISTEP", "1")
+    per_step, n_per_step = run(False)
+    assert n_refused == n_per_step
+    for a, b in zip(refused, per_step):
+        assert np.array_equal(a, b)
