@@ -377,6 +377,16 @@ int64_t mcmc_b200_launch_count(mcmc_b200_ctx* ctx, int reset);
 /* How the context's chain launches are cut: partial-gradient slots per window,
  * resident CTAs per SM of the gradient kernel, rows per tile.  Any may be null. */
 int mcmc_b200_chain_geometry(mcmc_b200_ctx* ctx, int* slices, int* ctas_per_sm, int* tile_rows);
+/* How a window whose rows stay on the chip is dealt out, in the launches of the
+ * chain or of the explicit calls: CTAs per cluster and clusters per window, or
+ * 0 and 0 where there is one launch per leapfrog step. */
+int mcmc_b200_resident_plan(mcmc_b200_ctx* ctx, int explicit_calls, int* ctas_per_cluster, int* clusters);
+/* The same as host arithmetic (no context, no GPU): available[i] = clusters of
+ * 1 << i CTAs that the GPU holds at once.  What a B200 holds beyond 148, 74, 33
+ * and 15 is not used: the order of the sums, and with it every bit of a chain,
+ * then follows from windows and rows alone. */
+int mcmc_b200_plan_resident(int windows, int64_t rows, int num_sms, const int32_t available[4],
+                            int32_t* ctas_per_cluster, int32_t* clusters);
 
 /*
  * Self-test of the device-side time-out route.  Every wait inside the kernels

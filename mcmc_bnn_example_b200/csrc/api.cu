@@ -187,8 +187,9 @@ struct mcmc_b200_ctx {
   unsigned int os_poll_limit = 1u << 22;    // polls of about 0.1 us .. 1 us each
   long long launches = 0;
   // whole iterations in one cooperative launch (resident.cuh): plans and message buffers of the chain launches
-  // and of the single-window explicit calls; null where the rows do not fit on the chip
-  bool res_ok = false, res_x_ok = false;
+  // and of the single-window explicit calls, for contexts that may have such launches at all (res_try); a plan is made
+  // when the first call wants it
+  bool res_try = false, res_asked = false, res_x_asked = false, res_ok = false, res_x_ok = false;
   ResidentParams res, res_x;
   int res_cluster = 1, res_x_cluster = 1;  // CTAs per cluster
   int refuse = 0;  // self-test: the next such launches that are answered as too large
@@ -341,7 +342,7 @@ static cudaError_t launch_resident(mcmc_b200_ctx* c, int cluster, const Resident
       cluster, &c->tmap_mn, g, st, max_clusters);
 }
 // Clusters of 1 << i CTAs that can be resident.  Asked once per device and kernel, and only when a plan wants to know:
-// the first question loads the kernel, which costs more than the rest of a small context.
+// the first question loads the kernel, which costs milliseconds.
 static int resident_max_clusters(mcmc_b200_ctx* c, int i) {
   static std::mutex mutex;
   static int known[2][64][4];
@@ -358,24 +359,32 @@ static int resident_max_clusters(mcmc_b200_ctx* c, int i) {
   return known[k][d][i];
 }
 
-// How a window of the context is dealt to clusters when `windows` of them share the GPU (resident.cuh).  False when
-// the rows do not fit.
+// What a plan counts on at most: the clusters of 1, 2, 4 and 8 CTAs that every B200 measured holds at once.  So a plan
+// follows from windows and rows alone, and a chain has the same bits on every GPU that holds as many.
+constexpr int RES_CLUSTERS[4] = {148, 74, 33, 15};
+
+// How a window is dealt to clusters when `windows` of them share the GPU (resident.cuh); available(i): clusters of 1 << i
+// CTAs that can be resident.  False when the rows do not fit.
 //   * one cluster per window, of the most CTAs (8, 4, 2, 1) that every window can have, if that holds the rows: the
 //     exchange then never leaves the cluster;
 //   * rows that one cluster of 8 cannot hold: as many clusters of 8 as every window can have (up to 16) while each
 //     CTA still has at least four 32-row units (below that the step is all exchange and more CTAs only add to it).
-static bool resident_plan(mcmc_b200_ctx* c, int windows, int* cluster, int* clusters) {
-  const long long units = (c->rows + 31) / 32;
-  if ((long long)windows * ((units + RES_UNITS - 1) / RES_UNITS) > c->num_sms) return false;
+// Against one launch per step (one B200, 1 to 148 windows of 100 to 61440 rows that fit): 1.1 (FP32, one window of 4096
+// rows: 11.8 and 12.9 us a step) to 3.2 times as fast, so every window that fits goes this way.
+template <typename F>
+static bool resident_plan(long long rows, int windows, int num_sms, F available, int* cluster, int* clusters) {
+  const long long units = (rows + 31) / 32;
+  auto count = [&](int i) { return std::min(RES_CLUSTERS[i], available(i)); };
+  if ((long long)windows * ((units + RES_UNITS - 1) / RES_UNITS) > num_sms) return false;
   for (int i = 3; i >= 0; --i)
-    if (units <= (long long)RES_UNITS << i && (long long)windows << i <= c->num_sms && windows <= resident_max_clusters(c, i)) {
+    if (units <= (long long)RES_UNITS << i && windows <= RES_CLUSTERS[i] && windows <= count(i)) {
       *cluster = 1 << i;
       *clusters = 1;
       return true;
     }
   const long long need = (units + 8 * RES_UNITS - 1) / (8 * RES_UNITS);
-  if (8 * need * windows > c->num_sms) return false;
-  const long long have = std::min<long long>(resident_max_clusters(c, 3) / windows, RES_MAX_CLUSTERS);
+  if (need * windows > RES_CLUSTERS[3]) return false;
+  const long long have = std::min<long long>(count(3) / windows, RES_MAX_CLUSTERS);
   if (need > have) return false;
   *cluster = 8;
   *clusters = (int)std::max(need, std::min(have, units / 32));
@@ -388,22 +397,25 @@ static size_t resident_words_stride(int P, int cluster) {
   return ((words + cluster - 1) / cluster + 7) / 8 * 8;
 }
 
-static size_t resident_msg_bytes(const mcmc_b200_ctx* c, const ResidentParams& g, int cluster) {
-  return (size_t)2 * g.windows * g.clusters * cluster * resident_words_stride(c->P, cluster) * 16;
+// enough for any plan of the context: only windows of several clusters of eight send such words
+static size_t resident_msg_bytes(const mcmc_b200_ctx* c, int windows) {
+  const int clusters = std::min(RES_CLUSTERS[3] / windows, RES_MAX_CLUSTERS);
+  if (clusters < 2 || c->rows <= 8 * RES_UNITS * 32) return 0;
+  return (size_t)2 * windows * clusters * 8 * resident_words_stride(c->P, 8) * 16;
 }
 
-// Plans the resident launches of a context and allocates their message buffers.  A fixed `slices` asks for bits
+// Prepares the resident launches of a context and allocates their message buffers.  A fixed `slices` asks for bits
 // that do not depend on what shares the launch: such contexts keep one launch per step.
 static int resident_setup(mcmc_b200_ctx* c) {
   const char* off = getenv("MCMC_B200_NO_MULTISTEP");
   if ((off && off[0] == '1') || c->cfg.slices > 0 || c->cfg.H != 40)
     return MCMC_B200_OK;
+  c->res_try = true;
   for (int k = 0; k < 2; ++k) {
     ResidentParams& g = k ? c->res_x : c->res;
-    int& cluster = k ? c->res_x_cluster : c->res_cluster;
     memset(&g, 0, sizeof g);
     g.windows = k ? 1 : c->W;
-    if (!resident_plan(c, g.windows, &cluster, &g.clusters)) continue;
+    if (g.windows > RES_CLUSTERS[0]) continue;
     g.n_rows = (int)c->rows;
     g.rows_pad = (int)c->rows_pad;
     g.Pp = c->Pp;
@@ -412,11 +424,48 @@ static int resident_setup(mcmc_b200_ctx* c) {
     g.prior = make_prior(c->cfg);
     g.status = c->status;
     g.wait_ticks = RES_WAIT_TICKS;
-    int r = dalloc(c, (void**)&g.msg, resident_msg_bytes(c, g, cluster));
-    if (r == MCMC_B200_OK) r = dalloc(c, (void**)&g.seq, (size_t)g.windows * 4);
+    int r = dalloc(c, (void**)&g.seq, (size_t)g.windows * 4);
+    const size_t bytes = resident_msg_bytes(c, g.windows);
+    if (r == MCMC_B200_OK && bytes > 0) r = dalloc(c, (void**)&g.msg, bytes);
     if (r) return r;
-    (k ? c->res_x_ok : c->res_ok) = true;
   }
+  return MCMC_B200_OK;
+}
+
+// Leapfrog steps of one resident launch: about a tenth of a second, so that other work on the GPU gets its turn.
+// Longer trajectories take one launch per step.
+static int resident_max_steps(const mcmc_b200_ctx* c) { return c->cfg.precision == MCMC_B200_PREC_TF32 ? 20000 : 10000; }
+
+// Whether trajectories of L steps are resident launches: those of the chain, or of the explicit calls (x)
+static bool use_resident(mcmc_b200_ctx* c, bool x, int L) {
+  if (!c->res_try || c->comm || c->oneshot || L > resident_max_steps(c)) return false;
+  bool &asked = x ? c->res_x_asked : c->res_asked, &ok = x ? c->res_x_ok : c->res_ok;
+  if (!asked) {
+    ResidentParams& g = x ? c->res_x : c->res;
+    ok = resident_plan(c->rows, g.windows, c->num_sms, [&](int i) { return resident_max_clusters(c, i); },
+                       x ? &c->res_x_cluster : &c->res_cluster, &g.clusters);
+    asked = true;
+  }
+  return ok;
+}
+
+API int mcmc_b200_resident_plan(mcmc_b200_ctx* c, int explicit_calls, int* ctas_per_cluster, int* clusters) {
+  if (!c || !ctas_per_cluster || !clusters) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
+  CK(cudaSetDevice(c->device));
+  const bool x = explicit_calls != 0, on = use_resident(c, x, x ? 1 : c->cfg.leapfrog_steps);
+  *ctas_per_cluster = !on ? 0 : x ? c->res_x_cluster : c->res_cluster;
+  *clusters = !on ? 0 : x ? c->res_x.clusters : c->res.clusters;
+  return MCMC_B200_OK;
+}
+
+API int mcmc_b200_plan_resident(int windows, int64_t rows, int num_sms, const int32_t available[4],
+                                int32_t* ctas_per_cluster, int32_t* clusters) {
+  if (windows < 1 || rows < 1 || num_sms < 1 || !available || !ctas_per_cluster || !clusters)
+    return fail(MCMC_B200_ERR_INVALID, "bad arguments");
+  int C = 0, K = 0;
+  if (!resident_plan(rows, windows, num_sms, [&](int i) { return available[i]; }, &C, &K)) C = K = 0;
+  *ctas_per_cluster = C;
+  *clusters = K;
   return MCMC_B200_OK;
 }
 
@@ -722,7 +771,7 @@ static int finish_status(mcmc_b200_ctx* c) {
     for (int k = 0; k < 2; ++k)
       if (k ? c->res_x_ok : c->res_ok) {
         const ResidentParams& g = k ? c->res_x : c->res;
-        cudaMemsetAsync(g.msg, 0, resident_msg_bytes(c, g, k ? c->res_x_cluster : c->res_cluster), c->stream);
+        if (g.msg) cudaMemsetAsync(g.msg, 0, resident_msg_bytes(c, g.windows), c->stream);
         cudaMemsetAsync(g.seq, 0, (size_t)g.windows * 4, c->stream);
       }
     cudaMemsetAsync(c->status, 0, 4, c->stream);
@@ -1004,10 +1053,6 @@ static int chain_grad(mcmc_b200_ctx* c, int mode, int s, cudaStream_t st) {
   return MCMC_B200_OK;
 }
 
-// Leapfrog steps of one resident launch: about a tenth of a second, so that other work on the GPU gets its turn.
-// Longer trajectories take one launch per step.
-static int resident_max_steps(const mcmc_b200_ctx* c) { return c->cfg.precision == MCMC_B200_PREC_TF32 ? 20000 : 10000; }
-
 // Up to n_iter HMC iterations in cooperative launches that keep the rows on the chip; returns how many were queued.  A
 // launch that is refused (not all of its CTAs fit into what the stream or the process may use) has done nothing: the
 // caller goes on with one launch per step, and an error of another kind shows up there again.
@@ -1098,7 +1143,7 @@ API int mcmc_b200_run_chain_async(mcmc_b200_ctx* c, int n_iter) {
     int r = refstream_fill(c, c->iters_done + n_iter);
     if (r) return r;
   }
-  if (c->res_ok && !c->comm && !c->oneshot && c->cfg.leapfrog_steps <= resident_max_steps(c)) {
+  if (use_resident(c, false, c->cfg.leapfrog_steps)) {
     const int done = resident_chain(c, n_iter, c->stream);
     c->iters_done += done;
     n_iter -= done;
@@ -1342,16 +1387,13 @@ static bool resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, 
   c->launches++;
   return true;
 }
-static bool use_resident_x(const mcmc_b200_ctx* c, int L) {
-  return c->res_x_ok && !c->comm && !c->oneshot && L <= resident_max_steps(c);
-}
 
 API int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* c, int code, int limit_us) {
   if (!c || limit_us < 40 || limit_us > 10000 || (code != 603 && code != 611 && code != 901))
     return fail(MCMC_B200_ERR_INVALID, "bad arguments");
-  if (c->W != 1 || !c->window_set[0] || !use_resident_x(c, 1) || (code == 603 && c->res_x.clusters < 2))
-    return fail(MCMC_B200_ERR_INVALID, "needs one window with data whose rows (603: more than 4096) fit on the chip");
   CK(cudaSetDevice(c->device));
+  if (c->W != 1 || !c->window_set[0] || !use_resident(c, true, 1) || (code == 603 && c->res_x.clusters < 2))
+    return fail(MCMC_B200_ERR_INVALID, "needs one window with data whose rows (603: more than 4096) fit on the chip");
   if (code == 901) {
     cudaError_t e = launch_wait_probe(c->status, (unsigned int)(limit_us / 20), c->stream);
     c->launches++;
@@ -1368,10 +1410,11 @@ API int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* c, int code, int limit_u
   }
   int r = refstream_fill(c, c->iters_done + 1);
   if (r) return r;
-  ResidentParams& g = c->bootstrapped ? c->res : c->res_x;
+  const bool chain = c->bootstrapped && use_resident(c, false, c->cfg.leapfrog_steps);
+  ResidentParams& g = chain ? c->res : c->res_x;
   g.missing = 1;
   g.wait_ticks = (unsigned int)limit_us / 33;
-  const bool done = c->bootstrapped ? resident_chain(c, 1, c->stream) == 1
+  const bool done = chain ? resident_chain(c, 1, c->stream) == 1
                                     : resident_steps(c, 0, 1, 0.f, c->xw[0], nullptr, nullptr, nullptr, nullptr, c->g_out,
                                                      nullptr, nullptr, nullptr, c->scalars, c->stream, true);
   g.missing = 0;
@@ -1448,7 +1491,7 @@ API int mcmc_b200_potential_and_grad(mcmc_b200_ctx* c, int window, const float* 
   if (!c->window_set[window]) return fail(MCMC_B200_ERR_INVALID, "window has no data yet");
   CK(cudaSetDevice(c->device));
   // parameters, gradient and sums go through the mapped host block: one launch and one wait, no copies
-  if (use_resident_x(c, 1) &&
+  if (use_resident(c, true, 1) &&
       (memcpy(c->hb->w, w, (size_t)c->P * 4),
        resident_steps(c, window, 1, 0.f, c->hb->w, nullptr, nullptr, nullptr, nullptr, c->hb->g_out, nullptr,
                       row_loss ? c->row_loss : nullptr, nullptr, c->hb->scalars, c->stream, true))) {
@@ -1486,7 +1529,7 @@ API int mcmc_b200_leapfrog(mcmc_b200_ctx* c, int window, int L, float eps, const
   CK(cudaSetDevice(c->device));
   const size_t n = (size_t)c->P * 4;
   HostBlock* h = c->hb;
-  if (use_resident_x(c, L) &&
+  if (use_resident(c, true, L) &&
       (memcpy(h->w, w_prev, n), memcpy(h->m, mom_prev, n), memcpy(h->g, grad_prev, n),
        resident_steps(c, window, L, eps, h->w, h->m, h->g, h->w_out, h->m_out, h->g_out, nullptr, nullptr, nullptr,
                       h->scalars, c->stream, false))) {
@@ -1539,7 +1582,7 @@ API int mcmc_b200_mcmc_step(mcmc_b200_ctx* c, const float* x, const float* y, co
     c->window_set[0] = 1;
     repacked = true;
   }
-  if (use_resident_x(c, L) &&
+  if (use_resident(c, true, L) &&
       resident_steps(c, 0, L, eps, weights_prev, mom_prev, grad_prev, weights_next, mom_next, grad_cur, grad_next,
                      loss_values, loss_values ? loss_values + c->rows : nullptr, c->scalars, st, false))
     return MCMC_B200_OK;

@@ -185,3 +185,33 @@ def test_reference_stream_engines_are_the_published_generators():
         u = (x - 1) / 2147483646.0
         lu = L.mcmc_b200_refstream_log_uniform(seed)
         assert abs(lu - np.log(max(u, 1.2e-38))) <= 2e-6 * max(1.0, abs(lu)), (seed, lu, np.log(u))
+
+
+def test_resident_plan_follows_from_windows_and_rows_alone():
+    """Every row has a place (16 units of 32 rows to a CTA), all clusters fit, and clusters beyond those that a plan counts on
+    change nothing, while a GPU that holds fewer gets a plan that fits it, or none."""
+    import ctypes as C
+    import mcmc_bnn_example_b200 as m
+    m.build()
+
+    def plan(windows, rows, available, sms=148):
+        a, b = C.c_int32(), C.c_int32()
+        assert m.lib().mcmc_b200_plan_resident(windows, C.c_int64(rows), sms, (C.c_int32 * 4)(*available), C.byref(a),
+                                               C.byref(b)) == 0
+        return a.value, b.value
+
+    counted = (148, 74, 33, 15)
+    for windows in (1, 2, 3, 5, 7, 8, 15, 16, 33, 34, 36, 74, 75, 100, 148, 149, 200):
+        for rows in (1, 32, 33, 500, 512, 513, 1024, 1025, 2048, 4096, 4097, 9001, 30000, 58368, 61440, 61441, 1 << 20):
+            for have in (counted, (148, 74, 36, 18), (148, 72, 32, 14), (132, 66, 32, 16), (148, 74, 33, 1), (148, 0, 0, 0)):
+                c, k = plan(windows, rows, have)
+                if c == 0:
+                    continue
+                i = {1: 0, 2: 1, 4: 2, 8: 3}[c]
+                assert 1 <= k <= 16 and (k == 1 or c == 8) and windows * k <= have[i]
+                assert c * k * 512 >= rows
+                if all(a >= b for a, b in zip(have, counted)):
+                    assert (c, k) == plan(windows, rows, counted)
+    assert plan(1, 58368, counted) == (8, 15) and plan(1, 58368, (148, 74, 33, 14)) == (0, 0)
+    assert plan(1, 61441, (148, 74, 37, 18)) == (0, 0) and plan(1, 1000, counted) == (8, 1)
+    assert plan(33, 1000, counted) == (4, 1) and plan(36, 1000, counted) == (2, 1) and plan(100, 511, counted) == (1, 1)

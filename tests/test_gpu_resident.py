@@ -1,6 +1,7 @@
 """The one-launch path for windows whose rows fit on the chip, at the sizes where its partition changes: one row, the
-last row of a 32-row unit and of a CTA, one cluster full and one row more, the largest window and one row more (one
-launch per step again), and window counts that take clusters of 8, 4, 2 and 1 CTAs."""
+last row of a 32-row unit and of a CTA, one cluster full and one row more, the largest window (on a GPU that holds 15
+clusters of eight CTAs) and one row more (one launch per step again), and window counts that take clusters of 8, 4, 2 and 1
+CTAs."""
 import numpy as np
 import pytest
 
@@ -32,14 +33,19 @@ def test_resident_launch_matches_oracle_and_per_step_launches(built, monkeypatch
         ctx.run_chain(1)
         ctx.run_chain(n_iter - 1)
         out = [(ctx.get_samples(i), ctx.get_trace(i), ctx.chain_info(i), ctx.get_state(i)) for i in (0, W - 1)]
-        n = ctx.launch_count()
+        n = ctx.launch_count(), ctx.resident_plan(), ctx.resident_plan(explicit_calls=True)
         ctx.close()
         return grad, steps, out, n
 
-    grad, steps, chains, n_one = run()
+    grad, steps, chains, (n_one, plan, plan_x) = run()
     monkeypatch.setenv("MCMC_B200_NO_MULTISTEP", "1")
-    grad_s, steps_s, chains_s, n_many = run()
-    assert (n_one < n_many) == (rows <= 61440)
+    grad_s, steps_s, chains_s, (n_many, none, none_x) = run()
+    assert none == none_x == (0, 0)
+    assert (n_one < n_many) == (plan[0] > 0 or plan_x[0] > 0)
+    for c, k in (plan, plan_x):
+        assert c * k * 512 >= rows or c == 0
+    assert rows <= 61440 or plan_x == (0, 0)
+    assert rows > 4096 or plan_x == (8, 1)
     x, y, _ = data[(W - 1) % len(data)]
     ref = O.logp_grad(O.reference_model(tf32=bool(prec)), x, y, w, want_losses=True)
     tol = TOL[prec]
