@@ -224,7 +224,10 @@ static int dalloc(mcmc_b200_ctx* c, void** p, size_t bytes, bool zero = true) {
   }
   const size_t take = small ? SLAB_BYTES : bytes;
   cudaError_t e = cudaMalloc(p, take);
-  if (e != cudaSuccess) return fail(MCMC_B200_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // (not the error of the next launch)
+    return fail(MCMC_B200_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  }
   c->allocs.push_back(*p);
   if (zero || small) {
     // waited for here: what fills the array next may be queued on another stream
@@ -1636,10 +1639,18 @@ API int mcmc_b200_predict_mean(mcmc_b200_ctx* c, int window, const float* xs, in
       !c->samples || first + count > c->cfg.sample_capacity)
     return fail(MCMC_B200_ERR_INVALID, "bad arguments or no sample storage");
   CK(cudaSetDevice(c->device));
-  const int chunks = forward_chunks(c->num_sms, n, count);
+  // a chunk's sums are 8 bytes a row beside the row's own 92: at most five chunks or 64 MB (5,000 samples of 10 M rows
+  // would take eight for less than one per cent), and one where there is no memory for more
+  const int most = (int)std::max<int64_t>(5, std::min<int64_t>(FWD_MAX_CHUNKS, (64 << 20) / (8 * n)));
+  int chunks = forward_chunks(c->num_sms, n, count, most);
   int r = fwd_reserve(c, &c->fwd_x, &c->fwd_x_cap, (size_t)n * c->cfg.D);
   if (r == MCMC_B200_OK) r = fwd_reserve(c, &c->fwd_out, &c->fwd_out_cap, (size_t)n);
-  if (r == MCMC_B200_OK) r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)chunks * n);
+  if (r) return r;
+  r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)chunks * n);
+  if (r == MCMC_B200_ERR_NOMEM && chunks > 1) {
+    chunks = 1;
+    r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)n);
+  }
   if (r) return r;
   CK(cudaMemcpyAsync(c->fwd_x, xs, (size_t)n * c->cfg.D * 4, cudaMemcpyHostToDevice, c->stream));
   ForwardParams a;
@@ -1669,7 +1680,7 @@ API int mcmc_b200_final_loss(mcmc_b200_ctx* c, int window, int first, int count,
   CK(cudaSetDevice(c->device));
   // all samples against the window's rows in one launch (FP32 forward pass, no gradient)
   const int tiles = forward_row_tiles(c->rows);
-  const int chunks = forward_chunks(c->num_sms, c->rows, count);
+  const int chunks = forward_chunks(c->num_sms, c->rows, count, FWD_MAX_CHUNKS);
   int r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)tiles * count + 2 * (size_t)count);
   if (r) return r;
   const float* xw = c->xaug + (size_t)window * c->rows_pad * KP;

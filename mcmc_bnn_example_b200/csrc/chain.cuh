@@ -98,7 +98,8 @@ struct ForwardParams {
   double* partial;         // PREDICT: [chunks][n]   LOSS: [row tiles][count]
 };
 int forward_row_tiles(long long n);
-int forward_chunks(int num_sms, long long n, int count);
+constexpr int FWD_MAX_CHUNKS = 64;
+int forward_chunks(int num_sms, long long n, int count, int most);
 cudaError_t launch_forward_samples(int H, const ForwardParams& a, int chunks, bool loss, cudaStream_t st);
 cudaError_t launch_forward_finish_predict(const double* partial, int chunks, long long n, int count, float* out,
                                           cudaStream_t st);

@@ -161,14 +161,14 @@ __global__ void __launch_bounds__(128) forward_finish_loss(const double* partial
 
 int forward_row_tiles(long long n) { return (int)((n + FWD_ROWS - 1) / FWD_ROWS); }
 
-// Sample chunks per row tile, at most 64 and one per sample.  All CTAs take the same time, so what counts is how many
+// Sample chunks per row tile, at most `most` and one per sample.  All CTAs take the same time, so what counts is how many
 // rounds of the GPU they make and how many samples the longest one has; a CTA's start (its rows, its first sample)
 // costs about two samples.  58368 rows x 800 samples: 8 chunks would be 2.07 rounds, paid as three.
-int forward_chunks(int num_sms, long long n, int count) {
+int forward_chunks(int num_sms, long long n, int count, int most) {
   const long long tiles = forward_row_tiles(n), slots = (long long)num_sms * FWD_CTAS_PER_SM;
   long long best = 0;
   int ch = 1;
-  for (int k = 1; k <= std::min(count, 64); ++k) {
+  for (int k = 1; k <= std::min(count, most); ++k) {
     const long long cost = (tiles * k + slots - 1) / slots * ((count + k - 1) / k + 2);
     if (k == 1 || cost < best) {
       best = cost;

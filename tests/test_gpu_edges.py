@@ -46,6 +46,30 @@ def test_predict_mean_matches_double_arithmetic(built, H, rows, count):
     assert np.abs(got - want).max() <= 1e-5 * max(scale, 1.0)
 
 
+def test_predict_mean_takes_one_chunk_where_memory_is_short(built):
+    """Two million rows would like five chunks of samples, whose sums (80 MB) do not fit beside the rows: one chunk's do."""
+    import torch
+    m, _ = built
+    n, count = 2000000, 800
+    ctx = m.Context(m.baseline_config(precision=m.PREC_FP32, leapfrog_steps=1, sample_capacity=count), 1, 128)
+    x, y, _ = m.synth_window(1, 0, 128)
+    ctx.set_window_data(0, x, y)
+    ctx.run_chain(count)
+    xs = np.random.default_rng(0).standard_normal((n, 22)).astype(np.float32)
+    few = ctx.predict_mean(0, xs[:1000])
+    torch.cuda.empty_cache()
+    room = n * 4 * 23 + n * 8 + (40 << 20)
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+    try:
+        got = ctx.predict_mean(0, xs)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+        ctx.close()
+    # doubles added in another order, rounded to floats
+    assert np.allclose(got[:1000], few, rtol=3e-7, atol=1e-12)
+
+
 @pytest.mark.parametrize("H", [40, 128])
 @pytest.mark.parametrize("rows", [1, 15, 17, 127, 129, 3000])
 def test_fp32_row_blocks_match_the_oracle(built, monkeypatch, H, rows):
