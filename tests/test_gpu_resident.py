@@ -176,3 +176,140 @@ def test_a_refused_launch_becomes_one_launch_per_step(built, monkeypatch, prec):
     assert n_refused == n_per_step
     for a, b in zip(refused, per_step):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_reference_random_streams_on_the_chip(built, monkeypatch, prec):
+    m, _ = built
+    rows, n_iter = 5000, 6
+    x, y, _ = m.synth_window(8, 0, rows)
+
+    def run():
+        cfg = m.reference_config(precision=prec, leapfrog_steps=3, burn_in=1, adapt_steps=4, sample_capacity=n_iter,
+                                 trace_iters=n_iter, seed=11, eps0=0.02, rng_streams=m.RNG_REFERENCE)
+        ctx = m.Context(cfg, 1, rows)
+        ctx.set_window_data(0, x, y)
+        plan = ctx.resident_plan()
+        ctx.run_chain(2)          # (the host's accept draws are extended between launches)
+        ctx.run_chain(n_iter - 2)
+        out = ctx.get_samples(0)[:n_iter - 1], ctx.get_trace(0), ctx.chain_info(0)
+        ctx.close()
+        return plan, out
+
+    plan, (s1, t1, i1) = run()
+    monkeypatch.setenv("MCMC_B200_NO_MULTISTEP", "1")
+    none, (s2, t2, i2) = run()
+    assert plan != (0, 0) and none == (0, 0)
+    assert i1 == i2 and np.array_equal(t1["momenta"], t2["momenta"]) and np.array_equal(t1["log_u"], t2["log_u"])
+    assert np.array_equal(t1["accepted"], t2["accepted"]) and np.array_equal(t1["eps"], t2["eps"])
+    assert np.abs(s1 - s2).max() <= 1e-4 * max(1e-3, np.abs(s2).max())
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_a_diverging_trajectory_rejects_and_the_chain_stays(built, monkeypatch, prec):
+    """Steps so long that weights become infinite and NaN: what travels with the weights then is no report of a wait."""
+    m, _ = built
+    rows = 5000
+    x, y, _ = m.synth_window(8, 0, rows)
+
+    def run(eps0):
+        ctx = m.Context(m.baseline_config(precision=prec, leapfrog_steps=8, sample_capacity=4, trace_iters=4, eps0=eps0), 1, rows)
+        ctx.set_window_data(0, x, y)
+        ctx.run_chain(4)
+        out = ctx.get_samples(0), ctx.get_trace(0)["accepted"], ctx.chain_info(0), ctx.get_state(0)
+        ctx.close()
+        return out
+
+    for eps0 in (1e19, 1e30):
+        monkeypatch.delenv("MCMC_B200_NO_MULTISTEP", raising=False)
+        s1, a1, i1, g1 = run(eps0)
+        monkeypatch.setenv("MCMC_B200_NO_MULTISTEP", "1")
+        s2, a2, i2, g2 = run(eps0)
+        assert not a1.any() and not a2.any() and i1 == i2
+        assert not s1.any() and not s2.any()   # the chain's start, w = 0
+        # (the start's gradient is the bootstrap launch's in both)
+        assert np.array_equal(g1["grad"], g2["grad"]) and g1["loglik"] == g2["loglik"]
+
+
+def _step_args(m, torch, ctx, x, y, in_place):
+    P_ = ctx.P
+    g = torch.Generator(device="cuda").manual_seed(4)
+    w, mom, grad = (0.1 * torch.randn(P_, device="cuda", generator=g) for _ in range(3))
+    out = [w, mom, grad] if in_place else [torch.zeros(P_, device="cuda") for _ in range(3)]
+    zero, loss = torch.ones(P_, device="cuda"), torch.zeros(x.shape[0] + P_, device="cuda")
+    torch.cuda.synchronize()
+    keep = (w, mom, grad, zero, loss)
+    p = [t.data_ptr() for t in (x, y, w, out[0], mom, out[1], grad, out[2], zero, loss)]
+    return p, out + [zero, loss], keep
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_mcmc_step_in_place_and_replayed_from_a_graph(built, prec):
+    import torch
+    m, _ = built
+    rows, L = 9001, 4
+    ctx = m.Context(m.reference_config(precision=prec, sample_capacity=0), 1, rows)
+    x, y = (torch.from_numpy(v).cuda() for v in m.synth_window(8, 0, rows)[:2])
+    res = {}
+    for in_place in (False, True):
+        p, out, keep = _step_args(m, torch, ctx, x, y, in_place)
+        ctx.mcmc_step(*p, L, 1e-3)
+        ctx.synchronize()
+        res[in_place] = [v.cpu().numpy() for v in out]
+    assert not res[False][3].any()     # grad_next
+    for a, b in zip(res[False], res[True]):
+        assert np.array_equal(a, b)
+    # captured once, replayed three times
+    p, out, keep = _step_args(m, torch, ctx, x, y, False)
+    s = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        ctx.mcmc_step(*p, L, 1e-3, stream=s.cuda_stream)
+    for _ in range(3):
+        for v in out:
+            v.fill_(5.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(out, res[False]):
+            assert np.array_equal(a.cpu().numpy(), b)
+    del graph
+    ctx.close()
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_two_contexts_at_once(built, prec):
+    """Two chains of 120 CTAs each, from two threads on their own streams: neither launch may hold SMs while it waits for
+    the other's."""
+    import threading
+    m, _ = built
+    rows, n = 58368, 40
+    data = m.synth_window(8, 0, rows)[:2]
+
+    def make():
+        ctx = m.Context(m.reference_config(precision=prec, leapfrog_steps=5, burn_in=0, adapt_steps=0, sample_capacity=n,
+                                           seed=1), 1, rows)
+        ctx.set_window_data(0, *data)
+        return ctx
+
+    alone = make()
+    alone.run_chain(n)
+    want = alone.get_samples(0)
+    alone.close()
+    both, errors = [make(), make()], []
+
+    def work(ctx):
+        try:
+            for _ in range(n // 2):
+                ctx.run_chain(2)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(c,)) for c in both]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for c in both:
+        assert np.array_equal(c.get_samples(0), want)
+        c.close()
