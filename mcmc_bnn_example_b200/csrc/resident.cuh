@@ -525,7 +525,8 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
 }
 
 // ---- host side ----------------------------------------------------------------------------
-// Every CTA has to be resident (they wait for one another's words): a cooperative launch of clusters.
+// CTAs that wait for one another's words have to be resident together.  The hardware sees to that within a cluster; for
+// windows of several clusters the launch is cooperative.
 template <typename K>
 static cudaError_t resident_launch(K kernel, int cluster, size_t smem, const void* tmap, const ResidentParams& g,
                                    cudaStream_t st, int* max_clusters) {
@@ -541,7 +542,7 @@ static cudaError_t resident_launch(K kernel, int cluster, size_t smem, const voi
   attr[1].id = cudaLaunchAttributeCooperative;
   attr[1].val.cooperative = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = g.clusters > 1 ? 2 : 1;
   if (max_clusters) {
     cfg.numAttrs = 1;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
