@@ -104,6 +104,34 @@ struct HostBlock {
   float w_out[HB_FLOATS], m_out[HB_FLOATS], g_out[HB_FLOATS];
 };
 
+// Page-locking takes milliseconds, so the blocks of destroyed contexts are kept for the next ones: at most
+// HB_CHUNK of them, one allocation, returned when the process ends.  Any thread may take and give.
+constexpr int HB_CHUNK = 16;
+static std::mutex g_hb_mutex;
+static HostBlock* g_hb_chunk = nullptr;
+static unsigned g_hb_used = 0;  // bit i: block i of the chunk is taken
+static HostBlock* host_block_take() {
+  std::lock_guard<std::mutex> lock(g_hb_mutex);
+  if (!g_hb_chunk) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(HostBlock) * HB_CHUNK, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    g_hb_chunk = static_cast<HostBlock*>(p);
+  }
+  for (int i = 0; i < HB_CHUNK; ++i)
+    if (!(g_hb_used >> i & 1u)) {
+      g_hb_used |= 1u << i;
+      return g_hb_chunk + i;
+    }
+  void* p = nullptr;  // more contexts than that at once: a block of its own
+  return cudaHostAlloc(&p, sizeof(HostBlock), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess
+             ? static_cast<HostBlock*>(p) : nullptr;
+}
+static void host_block_give(HostBlock* b) {
+  std::lock_guard<std::mutex> lock(g_hb_mutex);
+  if (b >= g_hb_chunk && b < g_hb_chunk + HB_CHUNK) g_hb_used &= ~(1u << (b - g_hb_chunk));
+  else cudaFreeHost(b);
+}
+
 struct mcmc_b200_ctx {
   mcmc_b200_config cfg;
   int device = 0, W = 0, P = 0, Pp = 0;
@@ -578,10 +606,8 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
     int r_ = resident_setup(c);
     if (r_ != MCMC_B200_OK) { mcmc_b200_destroy(c); return r_; }
   }
-  // (74 KB: the driver cuts blocks of this size from what it has page-locked, 2 us; from 1 MB on it takes milliseconds)
-  if (cudaHostAlloc((void**)&c->hb, sizeof(HostBlock), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
-    cudaGetLastError();
-    c->hb = nullptr;
+  c->hb = host_block_take();
+  if (!c->hb) {
     mcmc_b200_destroy(c);
     return fail(MCMC_B200_ERR_NOMEM, "cudaHostAlloc failed");
   }
@@ -723,7 +749,7 @@ API void mcmc_b200_destroy(mcmc_b200_ctx* c) {
     if (p) cudaIpcCloseMemHandle(p);
   if (c->comm && g_nccl.ok) g_nccl.CommDestroy(c->comm);
   for (void* p : c->allocs) cudaFree(p);
-  if (c->hb) cudaFreeHost(c->hb);
+  if (c->hb) host_block_give(c->hb);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
