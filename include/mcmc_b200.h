@@ -66,7 +66,8 @@ typedef struct mcmc_b200_config {
   int32_t trace_iters;     /* first K iterations whose draws and energies are recorded */
   int32_t slices;          /* pieces each window is cut into per launch; 0 = chosen from the SM count
                               (fastest).  A fixed value makes a window's results bit-identical
-                              however many windows share the context or the GPU. */
+                              however many windows share the context or the GPU; such contexts
+                              take one launch per leapfrog step. */
   int32_t rng_streams;     /* MCMC_B200_RNG_*: which random streams drive the chain */
 } mcmc_b200_config;
 
@@ -219,7 +220,9 @@ int mcmc_b200_read_table(const char* path, int64_t rows, int total_cols, int ski
  * gradient and energies, step size, counters, stored samples and trace.  The
  * dataset is NOT part of it: upload every window's data (same global window
  * ids) before loading.  Because every random draw is a pure function of
- * (seed, global window, iteration), a resumed chain continues bit-identically.
+ * (seed, global window, iteration), a resumed chain continues bit-identically
+ * where its sums are added in the same order: in a context of the same windows
+ * and rows with the same mcmc_b200_resident_plan, or with a fixed `slices`.
  *   size : bytes a save needs for this context
  *   save : synchronises the context, writes the blob to host_buf
  *   load : checks the header against this context's configuration, restores

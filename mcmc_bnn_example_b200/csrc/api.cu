@@ -372,6 +372,9 @@ constexpr int RES_CLUSTERS[4] = {148, 74, 33, 15};
 //     exchange then never leaves the cluster;
 //   * rows that one cluster of 8 cannot hold: as many clusters of 8 as every window can have (up to 16) while each
 //     CTA still has at least four 32-row units (below that the step is all exchange and more CTAs only add to it).
+// us a step by clusters, TF32: 4096 rows 4.2 (1), 4.2 (8); 6000 rows 4.2 (3), 4.3 (5, taken), 4.6 (15); 16384 rows 5.4 (4),
+// 4.5 (8), 4.8 (15, taken).  FP32, whose work per row is larger, would take more of them: 4096 rows 11.6 (1, taken), 6.9
+// (4); 6000 rows 8.3 (5, taken), 6.9 (8); 10000 rows 8.4 (9, taken), 7.1 (10); 16384 rows 8.7 (15, taken).
 // Against one launch per step (one B200, 1 to 148 windows of 100 to 61440 rows that fit): 1.1 (FP32, one window of 4096
 // rows: 11.8 and 12.9 us a step) to 3.2 times as fast, so every window that fits goes this way.
 template <typename F>
@@ -1247,7 +1250,8 @@ API int mcmc_b200_get_trace(mcmc_b200_ctx* c, int window, int first, int count, 
 // ---- checkpoint / resume ------------------------------------------------------
 // The reference keeps its samples in device memory and loses them, with the chain state, when the
 // process ends (main.h:183,277-283,295).  Every random draw here is a pure function of (seed, global
-// window, iteration), so a chain resumed from a checkpoint continues bit-identically.
+// window, iteration), so a chain resumed from a checkpoint continues bit-identically where sums are added in the same
+// order (same windows, rows and resident plan, or a fixed `slices`).
 namespace {
 struct CkptHeader {
   char magic[8];          // "MCB2CKPT"

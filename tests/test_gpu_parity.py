@@ -448,9 +448,9 @@ def test_full_size_additivity_over_row_blocks(built, prec, shape):
 
 
 def test_multistep_launch_matches_per_step_launches(built, monkeypatch):
-    """One window in TF32 mode runs the L leapfrog steps of an iteration as ONE cooperative launch (grid
-    barrier + cross-CTA sum inside the kernel).  The same chain with one launch per step must agree: same
-    accept decisions, states equal up to the order of the cross-CTA sums."""
+    """One window whose rows fit on the chip runs whole iterations in one launch (clusters of CTAs that exchange
+    sums and weights).  The same chain with one launch per step must agree: same accept decisions, states equal up to
+    the order of the cross-CTA sums."""
     m, O = built
     rows, n_iter = 58368, 12
     x, y, _ = m.synth_window(41, 0, rows)
@@ -467,13 +467,11 @@ def test_multistep_launch_matches_per_step_launches(built, monkeypatch):
         ctx.close()
         return out
 
-    monkeypatch.setenv("MCMC_B200_MULTISTEP", "1")
     monkeypatch.delenv("MCMC_B200_NO_MULTISTEP", raising=False)
     s_multi, t_multi, i_multi, l_multi = run()
-    monkeypatch.delenv("MCMC_B200_MULTISTEP")
     monkeypatch.setenv("MCMC_B200_NO_MULTISTEP", "1")
     s_step, t_step, i_step, l_step = run()
-    assert l_multi < l_step  # 2 launches per iteration instead of 21
+    assert l_multi < l_step  # one launch for all iterations instead of 21 (bootstrap aside) for each
     assert i_multi == i_step
     assert np.array_equal(t_multi["accepted"], t_step["accepted"])
     assert 0 < t_multi["accepted"].sum()
