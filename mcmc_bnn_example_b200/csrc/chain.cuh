@@ -143,6 +143,7 @@ struct ResidentParams {
   float *w_out, *m_out, *g_out, *zero_out, *row_loss, *prior_loss;
   double* scalars;          // [2] log-likelihood, log-prior
   AcceptParams a;           // RES_CHAIN
+  float w_val[964];         // RES_EVAL without w0: the parameters themselves
 };
 // The launch, for clusters of `cluster` CTAs (1, 2, 4, 8); or, when max_clusters is given, only the number of such
 // clusters that can be resident at once

@@ -209,6 +209,38 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     mbar_fence_init();
     dead = 0;
   }
+  // ---- what this thread owns ----
+  const int wl = tid / C, l = tid % C;       // word of this rank, lane of the word
+  const int word = rank * WPM + wl;
+  const bool mine = wl < WPM && word < NWORDS;
+  const bool ll_word = word == NWORDS - 1;
+  const bool chain = g.mode == RES_CHAIN;
+  const AcceptParams& a = g.a;
+  uint32_t seq = __ldcg(g.seq + win);
+  // ---- state of the word's parameters, the same in each of its lanes: read first, so that it arrives beside the rows ----
+  const size_t so = (size_t)win * g.Pp;
+  float eps = chain ? __ldcg(a.eps + win) : g.eps_scalar;
+  int iter = chain ? a.iter[win] : 0;
+  const uint32_t gwin = chain ? (uint32_t)a.gwin[win] : 0u;
+  double ll_cur = chain ? a.ll_cur[win] : 0.0, lp_cur = chain ? a.lp_cur[win] : 0.0;
+  int n_acc = 0;
+  float w_s[3] = {}, g_s[3] = {}, m_s[3] = {}, w[3] = {}, m[3] = {};
+  bool has[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const int p = Words::param(word, q);
+    has[q] = mine && Words::valid(word, q);
+    if (has[q]) {
+      w_s[q] = chain ? __ldcg(a.w_cur + so + p) : g.w0 ? __ldcg(g.w0 + p) : g.w_val[p];
+      w[q] = w_s[q];
+      if (g.mode != RES_EVAL) {
+        g_s[q] = __ldcg((chain ? a.g_cur + so : g.g0) + p);
+        m_s[q] = __ldcg((chain ? a.m_start + so : g.m0) + p);
+        m[q] = fmaf(eps * 0.5f, g_s[q], m_s[q]);  // half kick, drift (mcmc_step_ffma.h:106-120)
+        w[q] = fmaf(eps, m[q], w[q]);
+      }
+    }
+  }
   // (a status that is set already: see above)
   const int pending = __ldcg(g.status);
   if (pending != 0 && g.status_host && blockIdx.x == 0 && tid == 0)
@@ -226,11 +258,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   if (C > 1) cluster_sync_all();  // every rank's barriers exist before anyone sends
   else __syncthreads();
 
-  // ---- who does what in the exchange ----
-  const int wl = tid / C, l = tid % C;       // word of this rank, lane of the word
-  const int word = rank * WPM + wl;
-  const bool mine = wl < WPM && word < NWORDS;
-  const bool ll_word = word == NWORDS - 1;
+  // ---- where this thread sends ----
   const int out = max(c.collects(), 0);      // the word of which this thread sends the CTA's sums
   const uint32_t part_dst = mapa(smem_u32(&part_in[rank][out % WPM]), out / WPM);
   const uint32_t part_bar = mapa(smem_u32(&bar_part), out / WPM);
@@ -247,36 +275,9 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     x_has[i] = MULTI && tid < XT && u < my_words * K;
     x_src[i] = (uint32_t)(u / my_words * STR + u % my_words);
   }
-  const bool chain = g.mode == RES_CHAIN;
-  const AcceptParams& a = g.a;
-  uint32_t seq = __ldcg(g.seq + win);
   // limits of the waits that may last until the last CTA of the launch has started, and of the others
   auto limit = [&](uint32_t n) { return g.wait_ticks << (n < 2 ? 8 : 2); };
 
-  // ---- state of the word's parameters, the same in each of its lanes ----
-  const size_t so = (size_t)win * g.Pp;
-  float eps = chain ? __ldcg(a.eps + win) : g.eps_scalar;
-  int iter = chain ? a.iter[win] : 0;
-  const uint32_t gwin = chain ? (uint32_t)a.gwin[win] : 0u;
-  double ll_cur = chain ? a.ll_cur[win] : 0.0, lp_cur = chain ? a.lp_cur[win] : 0.0;
-  int n_acc = 0;
-  float w_s[3] = {}, g_s[3] = {}, m_s[3] = {}, w[3] = {}, m[3] = {};
-  bool has[3];
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const int p = Words::param(word, q);
-    has[q] = mine && Words::valid(word, q);
-    if (has[q]) {
-      w_s[q] = __ldcg((chain ? a.w_cur + so : g.w0) + p);
-      w[q] = w_s[q];
-      if (g.mode != RES_EVAL) {
-        g_s[q] = __ldcg((chain ? a.g_cur + so : g.g0) + p);
-        m_s[q] = __ldcg((chain ? a.m_start + so : g.m0) + p);
-        m[q] = fmaf(eps * 0.5f, g_s[q], m_s[q]);  // half kick, drift (mcmc_step_ffma.h:106-120)
-        w[q] = fmaf(eps, m[q], w[q]);
-      }
-    }
-  }
   auto send_weights = [&](bool bad) {
     if (mine) st_async16(w_dst, w_bar, __float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), bad);
   };
