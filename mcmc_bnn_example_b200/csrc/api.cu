@@ -145,8 +145,7 @@ struct mcmc_b200_ctx {
   // dataset
   float* xaug = nullptr;
   std::vector<char> window_set;
-  CUtensorMap tmap_mn = {};
-  bool tmap_ok = false;
+  CUtensorMap tmaps[2] = {};  // 32-byte-chunk swizzle; 128 units: and 16-byte-chunk swizzle
   // persistent (TF32) kernel work tables: chain launches and single-window launches
   int *tab_seg_ptr = nullptr, *tab_nslot = nullptr, *xtab_seg_ptr = nullptr, *xtab_nslot = nullptr;
   int4 *tab_segs = nullptr, *xtab_segs = nullptr;
@@ -314,18 +313,20 @@ static int make_tensor_map(mcmc_b200_ctx* c) {
   // arrive as zeros without being read.
   cuuint64_t gdim[2] = {(cuuint64_t)KP, (cuuint64_t)((long long)c->W * c->rows_pad)};
   cuuint64_t gstride[1] = {(cuuint64_t)(KP * sizeof(float))};
-  cuuint32_t box[2] = {32, (cuuint32_t)TF32_TILE};
+  cuuint32_t box[2] = {32, (cuuint32_t)(c->cfg.H == 128 ? WIDE_TILE : TF32_TILE)};
   cuuint32_t estr[2] = {1, 1};
-  // 32-byte-chunk swizzle: the layout the tensor core wants for MN-major TF32 operands
-  CUresult r = ((EncodeFn)fn)(&c->tmap_mn, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, c->xaug, gdim, gstride, box,
-                              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    char b[96];
-    snprintf(b, sizeof b, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-    return fail(MCMC_B200_ERR_CUDA, b);
+  // 32-byte-chunk swizzle: the layout the tensor core wants for MN-major TF32 operands; 16-byte-chunk: K-major ones
+  const CUtensorMapSwizzle swizzle[2] = {CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_SWIZZLE_128B};
+  for (int k = 0; k < (c->cfg.H == 128 ? 2 : 1); ++k) {
+    CUresult r = ((EncodeFn)fn)(&c->tmaps[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, c->xaug, gdim, gstride, box, estr,
+                                CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle[k], CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+      char b[96];
+      snprintf(b, sizeof b, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+      return fail(MCMC_B200_ERR_CUDA, b);
+    }
   }
-  c->tmap_ok = true;
   return MCMC_B200_OK;
 }
 
@@ -342,7 +343,7 @@ static cudaError_t launch_resident(mcmc_b200_ctx* c, int cluster, const Resident
     return cudaErrorCooperativeLaunchTooLarge;
   }
   return (c->cfg.precision == MCMC_B200_PREC_TF32 ? launch_resident_tf32 : launch_resident_fp32)(
-      cluster, &c->tmap_mn, g, st, max_clusters);
+      cluster, c->tmaps, g, st, max_clusters);
 }
 // Clusters of 1 << i CTAs that can be resident.  Asked once per device and kernel, and only when a plan wants to know:
 // the first question loads the kernel, which costs milliseconds.
@@ -878,7 +879,7 @@ static int launch_grad(mcmc_b200_ctx* c, GradParams g, bool single, cudaStream_t
     g.nslot_in = single ? c->xtab_nslot : c->tab_nslot;
     g.seg_ptr = single ? c->xtab_seg_ptr : c->tab_seg_ptr;
     g.segs = single ? c->xtab_segs : c->tab_segs;
-    e = launch_grad_tf32(c->cfg.H, &c->tmap_mn, g, single ? c->xtab_ctas : c->tab_ctas, st);
+    e = launch_grad_tf32(c->cfg.H, c->tmaps, g, single ? c->xtab_ctas : c->tab_ctas, st);
   } else {
     e = launch_grad_fp32(c->cfg.H, g, slots, single ? 1 : c->W, st);
   }

@@ -157,11 +157,12 @@ cudaError_t launch_grad_fp32(int H, const GradParams& g, int slices, int windows
 int fp32_max_ctas_per_sm(int H);
 int fp32_tile_rows(int H);
 
-// TF32 (tcgen05) path: persistent, one CTA per SM; `tmap_mn` is a CUtensorMap over the repacked
-// dataset that stages a row tile with the 32-byte-chunk swizzle
-cudaError_t launch_grad_tf32(int H, const void* tmap_mn, const GradParams& g, int ctas, cudaStream_t st);
+// TF32 (tcgen05) path: persistent, one CTA per SM; `tmaps` are CUtensorMaps over the repacked dataset: one that stages a
+// row tile with the 32-byte-chunk swizzle and, for 128 units, a second with the 16-byte-chunk swizzle
+cudaError_t launch_grad_tf32(int H, const void* tmaps, const GradParams& g, int ctas, cudaStream_t st);
 int tf32_supported(int H);
-cudaError_t launch_grad_tf32_wide(const void* tmap_mn, const GradParams& g, int ctas, cudaStream_t st);
+cudaError_t launch_grad_tf32_wide(const void* tmaps, const GradParams& g, int ctas, cudaStream_t st);
 constexpr int TF32_TILE = 128;
+constexpr int WIDE_TILE = 64;  // rows of a tile of the 128-unit kernel
 
 }  // namespace mcmc_b200

@@ -577,9 +577,9 @@ static cudaError_t launch_tf32_t(const void* tmap_mn, const GradParams& g, int c
                              *reinterpret_cast<const CUtensorMap*>(tmap_mn), g);
 }
 
-cudaError_t launch_grad_tf32(int H, const void* tmap_mn, const GradParams& g, int ctas, cudaStream_t st) {
-  if (H == 40) return launch_tf32_t<40>(tmap_mn, g, ctas, st);
-  if (H == 128) return launch_grad_tf32_wide(tmap_mn, g, ctas, st);  // grad_tf32_wide.cu
+cudaError_t launch_grad_tf32(int H, const void* tmaps, const GradParams& g, int ctas, cudaStream_t st) {
+  if (H == 40) return launch_tf32_t<40>(tmaps, g, ctas, st);
+  if (H == 128) return launch_grad_tf32_wide(tmaps, g, ctas, st);  // grad_tf32_wide.cu
   return cudaErrorInvalidValue;
 }
 

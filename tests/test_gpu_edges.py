@@ -85,3 +85,34 @@ def test_fp32_row_blocks_match_the_oracle(built, monkeypatch, H, rows):
     assert np.abs(got["grad"] - ref["grad"]).max() <= 1e-5 * np.abs(ref["grad"]).max()
     assert abs(got["loglik"] - ref["loglik"]) <= 1e-5 * abs(ref["loglik"])
     assert np.allclose(got["row_loss"], ref["row_loss"], rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("rows,W", [(1, 2), (64, 2), (65, 300), (129, 2), (250, 2), (449, 150), (900, 2), (1665, 2)])
+def test_wide_tf32_tiles_of_one_cta_match_the_oracle(built, rows, W):
+    """The whole window on one CTA (`slices=1`), in one to twenty-six tiles of 64 rows: fewer than there are warpgroups,
+    buffers or row stages, all of them once, and several rounds.  More windows than SMs: CTAs with several segments."""
+    m, O = built
+    H = 128
+    cfg = m.reference_config(H=H, precision=m.PREC_TF32, slices=1, sample_capacity=2, leapfrog_steps=2, burn_in=0, adapt_steps=0)
+    ctx = m.Context(cfg, W, rows)
+    data = [m.synth_window(3, g, rows, H=H)[:2] for g in range(2)]
+    for g in range(W):
+        ctx.set_window_data(g, *data[g % 2])
+    w = (0.1 * np.random.default_rng(rows).standard_normal(ctx.P)).astype(np.float32)
+    for g in (0, W - 1):
+        x, y = data[g % 2]
+        got = ctx.potential_and_grad(g, w, want_row_loss=True)
+        ref = O.logp_grad(O.reference_model(tf32=True, H=H), x, y, w, want_losses=True)
+        assert np.abs(got["grad"] - ref["grad"]).max() <= 2e-3 * np.abs(ref["grad"]).max()
+        assert abs(got["loglik"] - ref["loglik"]) <= 2e-3 * abs(ref["loglik"])
+        assert np.allclose(got["row_loss"], ref["row_loss"], rtol=2e-2, atol=2e-2)
+    ctx.run_chain(2)
+    both = ctx.get_samples(W - 1), ctx.get_state(W - 1)
+    ctx.close()
+    # the last window alone: the same bits wherever its chunk runs
+    ctx = m.Context(cfg, 1, rows)
+    ctx.set_window_data(0, *data[(W - 1) % 2], global_window=W - 1)
+    ctx.run_chain(2)
+    assert np.array_equal(ctx.get_samples(0), both[0])
+    assert all(np.array_equal(ctx.get_state(0)[k], both[1][k]) for k in both[1])
+    ctx.close()
