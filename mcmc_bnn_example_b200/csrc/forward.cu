@@ -8,8 +8,11 @@
 //     whatever precision the chain was sampled in;
 //   * a CTA owns 512 rows (4 per thread, held in registers for the whole launch) and walks through its
 //     chunk of the samples; a sample's 961 parameters are staged in shared memory once per CTA, the next one's while
-//     this one is worked on, and read as 16-byte broadcasts: 16 multiplications per load
-//     (packed FMAs on pairs of features were no faster: with three different operands they issue every third cycle);
+//     this one is worked on, and read as 16-byte broadcasts: 16 multiplications per load.  Two units to a packed FMA, the
+//     row's feature as one value for both: that issues every 2.3 cycles of a scheduler where one with three different
+//     pairs takes 2.8 and two single ones 2.1 to 2.3 and twice the issue slots, which the tanh needs (58368 rows x 800
+//     samples: 2.28 ms instead of 2.48 a call, 128 units 6.42 instead of 7.15; with single FMAs and the tanh of four units
+//     between the multiplications of the next four it was 2.66);
 //   * PREDICT: per-row sums over the chunk's samples -> partial[chunk][row]; LOSS: per-sample sums over the
 //     CTA's rows -> partial[tile][sample].  A second small launch adds the partials in a fixed order (and, for
 //     LOSS, the log-prior of every sample).  Doubles, no atomics: bit-reproducible.
@@ -68,25 +71,27 @@ __global__ void __launch_bounds__(FWD_THREADS, FWD_CTAS_PER_SM) forward_samples_
     for (int r = 0; r < FWD_RPT; ++r) pred[r] = sw[D * H + 2 * H];
 #pragma unroll 1
     for (int j0 = 0; j0 < H; j0 += 4) {
-      float z[FWD_RPT][4];
-      const float4 b = *reinterpret_cast<const float4*>(sw + D * H + j0);
+      uint64_t zp[FWD_RPT][2];
+      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(sw + D * H + j0);
 #pragma unroll
       for (int r = 0; r < FWD_RPT; ++r) {
-        z[r][0] = b.x;
-        z[r][1] = b.y;
-        z[r][2] = b.z;
-        z[r][3] = b.w;
+        zp[r][0] = b.x;
+        zp[r][1] = b.y;
       }
 #pragma unroll
       for (int k = 0; k < D; ++k) {
-        const float4 w = *reinterpret_cast<const float4*>(sw + k * H + j0);
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(sw + k * H + j0);
 #pragma unroll
         for (int r = 0; r < FWD_RPT; ++r) {
-          z[r][0] = fmaf(x[r][k], w.x, z[r][0]);
-          z[r][1] = fmaf(x[r][k], w.y, z[r][1]);
-          z[r][2] = fmaf(x[r][k], w.z, z[r][2]);
-          z[r][3] = fmaf(x[r][k], w.w, z[r][3]);
+          zp[r][0] = fma2(w.x, pack2(x[r][k], x[r][k]), zp[r][0]);
+          zp[r][1] = fma2(w.y, pack2(x[r][k], x[r][k]), zp[r][1]);
         }
+      }
+      float z[FWD_RPT][4];
+#pragma unroll
+      for (int r = 0; r < FWD_RPT; ++r) {
+        unpack2(zp[r][0], z[r][0], z[r][1]);
+        unpack2(zp[r][1], z[r][2], z[r][3]);
       }
       const float4 w1 = *reinterpret_cast<const float4*>(sw + D * H + H + j0);
 #pragma unroll
