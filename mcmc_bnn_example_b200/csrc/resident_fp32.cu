@@ -1,7 +1,7 @@
 // Tile arithmetic of the resident kernel in FP32 mode (resident.cuh has the launch structure, fp32_tile.cuh what a warp
 // does with its 32 rows): every warp owns one 32-row unit for the whole launch.
-// One launch per step took 29.5 us a step for a 58368-row window, this takes 12.8 (2000 steps, one B200); a log density
-// and gradient of 1000 rows from host pointers takes 34 us instead of 64.
+// One launch per step took 29.5 us a step for a 58368-row window, this takes 12.5 (2000 steps, one B200); a log density
+// and gradient of 1000 rows from host pointers takes 30 us instead of 64.
 // What bounds a step: the FMA pipe (about 1,900 multiplications per row, 3,500 cycles each for forward and backward at
 // 512 rows per CTA) and the tanh pass (two MUFU operations each, 2,560 cycles), which overlap as far as the warps of a
 // scheduler are in different phases; then the exchange.
@@ -28,6 +28,12 @@ struct ResFp32 {
                        DUMMY = RLL + NWARPS * 2, BAR = DUMMY + 4;
   static constexpr size_t SMEM = 1024 + (BAR + 4) * 4;
   static_assert(WP % 4 == 0 && DYS % 4 == 0 && RLL % 2 == 0 && BAR % 2 == 0, "vector alignment");
+
+  // The four warps of a scheduler get the weights at the same moment.  In step with one another they would all multiply,
+  // then all wait for their tanh (646 cycles of the MUFU pipe each), and so on; so each starts this many cycles after the
+  // one before it, about the multiplications of half a block.  58368 rows, us a step: 12.91 (0), 12.61 (300), 12.46 (500
+  // to 700), 12.57 (1000), 12.69 (1300).  Windows with one unit to a scheduler have nothing to wait for.
+  static constexpr uint32_t TURN = 600;
 
   Warp lanes;
   float* base;
@@ -89,6 +95,10 @@ struct ResFp32 {
 
   __device__ __forceinline__ void step(const ResidentParams& g, float* row_loss, bool last, bool&) {
     if (!active) return;
+    {
+      const uint32_t t0 = (uint32_t)clock64();
+      while ((uint32_t)clock64() - t0 < (uint32_t)(warp >> 2) * TURN) {}
+    }
     const float* xb = base + XB + warp * 32 * KP;
     float* es = base + ES + warp * Warp::ES;
     uint64_t dw1[Warp::HPL] = {};
