@@ -372,14 +372,16 @@ constexpr int RES_CLUSTERS[4] = {148, 74, 33, 15};
 //   * one cluster per window, of the most CTAs (8, 4, 2, 1) that every window can have, if that holds the rows: the
 //     exchange then never leaves the cluster;
 //   * rows that one cluster of 8 cannot hold: as many clusters of 8 as every window can have (up to 16) while each
-//     CTA still has at least four 32-row units (below that the step is all exchange and more CTAs only add to it).
-// us a step by clusters, TF32: 4096 rows 4.2 (1), 4.2 (8); 6000 rows 4.2 (3), 4.3 (5, taken), 4.6 (15); 16384 rows 5.4 (4),
-// 4.5 (8), 4.8 (15, taken).  FP32, whose work per row is larger, would take more of them: 4096 rows 11.6 (1, taken), 6.9
-// (4); 6000 rows 8.3 (5, taken), 6.9 (8); 10000 rows 8.4 (9, taken), 7.1 (10); 16384 rows 8.7 (15, taken).
+//     CTA still has at least four 32-row units (below that the step is all exchange and more CTAs only add to it).  FP32:
+//     as many as leave it at most four, since a fifth unit costs its scheduler a second round.
+// us a step by clusters, TF32: 4096 rows 4.2 (1), 4.2 (8); 4097 rows 3.9 (4, taken), 4.0 (5); 6000 rows 4.2 (3), 4.1 (5, taken),
+// 4.1 (6), 4.6 (15); 16384 rows 5.4 (4), 4.5 (8), 4.8 (15, taken).  FP32: 4097 rows 7.65 (4), 6.6 (5, taken); 6000 rows 8.1 (5),
+// 6.7 (6, taken), 6.9 (8); 10000 rows 8.2 (9), 6.9 (10, taken); 13000 rows 8.3 (12), 7.1 (13, taken); three windows of 5000
+// rows 8.1 (4), 6.8 (5, taken); 16384 rows 8.4 (15, taken); 4096 rows 10.8 (1, taken), 6.9 (4).
 // Against one launch per step (one B200, 1 to 148 windows of 100 to 61440 rows that fit): 1.1 (FP32, one window of 4096
 // rows: 11.8 and 12.9 us a step) to 3.2 times as fast, so every window that fits goes this way.
 template <typename F>
-static bool resident_plan(long long rows, int windows, int num_sms, F available, int* cluster, int* clusters) {
+static bool resident_plan(long long rows, int windows, int num_sms, bool fp32, F available, int* cluster, int* clusters) {
   const long long units = (rows + 31) / 32;
   auto count = [&](int i) { return std::min(RES_CLUSTERS[i], available(i)); };
   if ((long long)windows * ((units + RES_UNITS - 1) / RES_UNITS) > num_sms) return false;
@@ -394,7 +396,7 @@ static bool resident_plan(long long rows, int windows, int num_sms, F available,
   const long long have = std::min<long long>(count(3) / windows, RES_MAX_CLUSTERS);
   if (need > have) return false;
   *cluster = 8;
-  *clusters = (int)std::max(need, std::min(have, units / 32));
+  *clusters = (int)std::max(need, std::min(have, (units + (fp32 ? 31 : 0)) / 32));
   return true;
 }
 
@@ -449,7 +451,7 @@ static bool use_resident(mcmc_b200_ctx* c, bool x, int L) {
   bool &asked = x ? c->res_x_asked : c->res_asked, &ok = x ? c->res_x_ok : c->res_ok;
   if (!asked) {
     ResidentParams& g = x ? c->res_x : c->res;
-    ok = resident_plan(c->rows, g.windows, c->num_sms, [&](int i) { return resident_max_clusters(c, i); },
+    ok = resident_plan(c->rows, g.windows, c->num_sms, c->cfg.precision == MCMC_B200_PREC_FP32, [&](int i) { return resident_max_clusters(c, i); },
                        x ? &c->res_x_cluster : &c->res_cluster, &g.clusters);
     asked = true;
   }
@@ -470,7 +472,7 @@ API int mcmc_b200_plan_resident(int windows, int64_t rows, int num_sms, const in
   if (windows < 1 || rows < 1 || num_sms < 1 || !available || !ctas_per_cluster || !clusters)
     return fail(MCMC_B200_ERR_INVALID, "bad arguments");
   int C = 0, K = 0;
-  if (!resident_plan(rows, windows, num_sms, [&](int i) { return available[i]; }, &C, &K)) C = K = 0;
+  if (!resident_plan(rows, windows, num_sms, false, [&](int i) { return available[i]; }, &C, &K)) C = K = 0;
   *ctas_per_cluster = C;
   *clusters = K;
   return MCMC_B200_OK;

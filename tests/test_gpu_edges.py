@@ -116,3 +116,20 @@ def test_wide_tf32_tiles_of_one_cta_match_the_oracle(built, rows, W):
     assert np.array_equal(ctx.get_samples(0), both[0])
     assert all(np.array_equal(ctx.get_state(0)[k], both[1][k]) for k in both[1])
     ctx.close()
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("rows,fp32,tf32", [(4097, 5, 4), (5120, 5, 5), (5121, 6, 5), (15360, 15, 15), (15361, 15, 15)])
+def test_clusters_of_a_window_leave_fp32_ctas_four_units(built, prec, rows, fp32, tf32):
+    m, O = built
+    x, y, _ = m.synth_window(3, 0, rows)
+    ctx = m.Context(m.reference_config(precision=prec, sample_capacity=0), 1, rows)
+    assert ctx.resident_plan() == ctx.resident_plan(explicit_calls=True) == (8, tf32 if prec else fp32)
+    ctx.set_window_data(0, x, y)
+    w = (0.15 * np.random.default_rng(rows).standard_normal(ctx.P)).astype(np.float32)
+    got = ctx.potential_and_grad(0, w)
+    ctx.close()
+    ref = O.logp_grad(O.reference_model(tf32=bool(prec)), x, y, w)
+    tol = 2e-3 if prec else 1e-5
+    assert np.abs(got["grad"] - ref["grad"]).max() <= tol * np.abs(ref["grad"]).max()
+    assert abs(got["loglik"] - ref["loglik"]) <= tol * abs(ref["loglik"])
