@@ -76,9 +76,14 @@ __global__ void __launch_bounds__(Fp32Geom<H>::NT, MINB) grad_fp32_kernel(const 
   pdl_wait();
   if (lane == 0 && t0 < t1 && !early_rows) fetch(t0);
   // fused leapfrog update; parameters land in the layout the lanes read
-  for (int p = tid; p < Warp::P; p += NT) {
-    const float w = leapfrog_param(g, win, p, slice == 0);
-    wp[p < D * H ? Warp::w_off(p / H, p % H) : p + (Warp::WP - D * H)] = w;
+  {
+    float w[(Warp::P + NT - 1) / NT];
+    leapfrog_params(g, step_io(g), win, tid, NT, Warp::P, slice == 0, w);
+#pragma unroll
+    for (int i = 0; i < (Warp::P + NT - 1) / NT; ++i) {
+      const int p = tid + i * NT;
+      if (p < Warp::P) wp[p < D * H ? Warp::w_off(p / H, p % H) : p + (Warp::WP - D * H)] = w[i];
+    }
   }
   __syncthreads();
 

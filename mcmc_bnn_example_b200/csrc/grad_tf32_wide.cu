@@ -243,14 +243,17 @@ grad_tf32_wide_kernel(const __grid_constant__ CUtensorMap tmap_mn, const __grid_
       {
         const StepIo io = step_io(g);
         float w[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) w[k] = leapfrog_param(g, io, win, (8 * wg + k) * H + hid, slot == 0);
+        leapfrog_params(g, io, win, 8 * wg * H + hid, H, G::P, slot == 0, w);
         if (wg == NWG - 1) {
           w1s[hid] = w[7];
           w[7] = 0.f;
         }
         tc_st8(tmem + G::W_COL0 + 8 * wg + lane_off, make_float4(w[0], w[1], w[2], w[3]), make_float4(w[4], w[5], w[6], w[7]));
-        if (tid == 0) b1s = leapfrog_param(g, io, win, D * H + 2 * H, slot == 0);
+        if (tid == 0) {
+          float b[1];
+          leapfrog_params(g, io, win, D * H + 2 * H, 1, G::P, slot == 0, b);
+          b1s = b[0];
+        }
         tc_wait_st();
         tc_fence_before();
       }
