@@ -18,7 +18,7 @@
 
 namespace mcmc_b200 {
 
-constexpr int ACC_THREADS = 256;
+constexpr int ACC_THREADS = 1024;  // (256: 2 to 13 us more an iteration; the loads of a thread's parameters wait for one another)
 
 __global__ void __launch_bounds__(ACC_THREADS) hmc_accept_kernel(const AcceptParams a) {
   __shared__ double dsc[32];
@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(ACC_THREADS) hmc_accept_kernel(const AcceptPar
     for (int s = 0; s < ns; ++s) ll_new += a.ll_partial[(size_t)win * a.slices + s];
   }
 
-  constexpr int MAXPT = 16;  // parameters per thread (P <= 4096)
+  constexpr int MAXPT = 4;  // parameters per thread (P <= 4096)
   float wv[MAXPT], gv[MAXPT];
   double lp_loc = 0.0, dk_loc = 0.0;
   int n = 0;
@@ -228,33 +228,42 @@ cudaError_t launch_repack(const float* x, const float* y, float* out, long long 
 // Used (a) when many CTAs touch one window (few windows per GPU): one small launch sums the
 // slots once instead of every CTA of the next launch summing all of them in its prologue, and
 // (b) for row sharding, where the result is what is all-reduced.  Fixed order: deterministic.
-constexpr int RED_PARAMS = 32, RED_GROUPS = 32;  // every load of a thread is in flight at once
-__global__ void __launch_bounds__(RED_PARAMS* RED_GROUPS)
+// Slots s, s + 32, ... are added first, then the 32 sums in order: the same whatever the launch's shape.
+constexpr int RED_PARAMS = 32, RED_GROUPS = 32;
+template <int ROWS>  // of 32 threads; each makes RED_GROUPS / ROWS of the sums, every load of a thread in flight at once
+__global__ void __launch_bounds__(RED_PARAMS* ROWS)
 reduce_partials_kernel(const float* __restrict__ partial, const double* __restrict__ ll_partial, int slices,
                        const int* __restrict__ nslot, int P, int Pp, double* __restrict__ red) {
   __shared__ float sg[RED_GROUPS][RED_PARAMS];
   __shared__ double sl[RED_GROUPS];
   const int win = blockIdx.y;
   const int ns = nslot ? nslot[win] : slices;
-  const int pi = threadIdx.x % RED_PARAMS, gi = threadIdx.x / RED_PARAMS;
+  const int pi = threadIdx.x % RED_PARAMS, ti = threadIdx.x / RED_PARAMS;
   const int p = blockIdx.x * RED_PARAMS + pi;
   double* r = red + (size_t)win * (Pp + 4);
   pdl_trigger();
   pdl_wait();
-  float g = 0.f;
+  const float* src = partial + (size_t)win * slices * Pp + p;
+  float g[RED_GROUPS / ROWS];
+#pragma unroll
+  for (int k = 0; k < RED_GROUPS / ROWS; ++k) g[k] = 0.f;
   if (p < P) {
-    const float* src = partial + (size_t)win * slices * Pp + p;
-#pragma unroll 8
-    for (int s = gi; s < ns; s += RED_GROUPS) g += src[(size_t)s * Pp];
+#pragma unroll(8 / (RED_GROUPS / ROWS))
+    for (int s0 = ti; s0 < ns; s0 += RED_GROUPS)
+#pragma unroll
+      for (int k = 0; k < RED_GROUPS / ROWS; ++k)
+        if (s0 + k * ROWS < ns) g[k] += src[(size_t)(s0 + k * ROWS) * Pp];
   }
-  sg[gi][pi] = g;
-  if (blockIdx.x == 0 && pi == 0) {
+#pragma unroll
+  for (int k = 0; k < RED_GROUPS / ROWS; ++k) sg[ti + k * ROWS][pi] = g[k];
+  if (blockIdx.x == 0 && pi < RED_GROUPS / ROWS) {
+    const int gi = ti + pi * ROWS;
     double l = 0.0;
     for (int s = gi; s < ns; s += RED_GROUPS) l += ll_partial[(size_t)win * slices + s];
     sl[gi] = l;
   }
   __syncthreads();
-  if (gi == 0) {
+  if (ti == 0) {
     if (p < P) {
       float t = sg[0][pi];
 #pragma unroll
@@ -273,11 +282,18 @@ reduce_partials_kernel(const float* __restrict__ partial, const double* __restri
   }
 }
 
+// A CTA of 1,024 threads per 32 parameters is the shortest while the GPU holds all of them (two to each of 148 SMs); beyond
+// that they come in waves, and CTAs of 256 are faster.  us a leapfrog iteration of ten steps, 1,024 and 256 threads: 25
+// TF32 windows 486, 457; 50 FP32 windows of 5,000 rows 403, 359; 8 windows of 128 units 273, 250; 4 FP32 windows 360, 365.
 cudaError_t launch_reduce_partials(const float* partial, const double* ll_partial, int slices,
                                    const int* nslot, int P, int Pp, double* red, int windows,
                                    cudaStream_t st) {
-  dim3 grid((Pp + RED_PARAMS - 1) / RED_PARAMS, windows);
-  return launch_chain_kernel(reduce_partials_kernel, grid, dim3(RED_PARAMS * RED_GROUPS), 0, st, partial,
+  constexpr int SMALL = 8;
+  const dim3 grid((Pp + RED_PARAMS - 1) / RED_PARAMS, windows);
+  if ((long long)grid.x * windows > 2 * 148)
+    return launch_chain_kernel(reduce_partials_kernel<SMALL>, grid, dim3(RED_PARAMS * SMALL), 0, st, partial, ll_partial,
+                               slices, nslot, P, Pp, red);
+  return launch_chain_kernel(reduce_partials_kernel<RED_GROUPS>, grid, dim3(RED_PARAMS * RED_GROUPS), 0, st, partial,
                              ll_partial, slices, nslot, P, Pp, red);
 }
 
