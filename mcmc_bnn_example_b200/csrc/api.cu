@@ -345,6 +345,13 @@ static cudaError_t launch_resident(mcmc_b200_ctx* c, int cluster, const Resident
   return (c->cfg.precision == MCMC_B200_PREC_TF32 ? launch_resident_tf32 : launch_resident_fp32)(
       cluster, c->tmaps, g, st, max_clusters);
 }
+static cudaError_t launch_resident_eval(mcmc_b200_ctx* c, const ResidentEvalParams& g, cudaStream_t st) {
+  if (c->refuse > 0) {
+    --c->refuse;
+    return cudaErrorCooperativeLaunchTooLarge;
+  }
+  return (c->cfg.precision == MCMC_B200_PREC_TF32 ? launch_resident_eval_tf32 : launch_resident_eval_fp32)(c->tmaps, g, st);
+}
 // Clusters of 1 << i CTAs that can be resident.  Asked once per device and kernel, and only when a plan wants to know:
 // the first question loads the kernel, which costs milliseconds.
 static int resident_max_clusters(mcmc_b200_ctx* c, int i) {
@@ -1381,7 +1388,6 @@ static bool resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, 
   g.data_window0 = data_window;
   g.status_host = &c->hb->status;
   g.w0 = w0;
-  if (w_host) memcpy(g.w_val, w_host, (size_t)c->P * 4);
   g.m0 = m0;
   g.g0 = g0;
   g.eps_scalar = eps;
@@ -1392,7 +1398,20 @@ static bool resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, 
   g.row_loss = row_loss;
   g.prior_loss = prior_loss;
   g.scalars = scalars;
-  if (launch_resident(c, c->res_x_cluster, g, st) != cudaSuccess) {
+  cudaError_t e;
+  if (w_host && c->res_x_cluster == 8) {
+    ResidentEvalParams v;
+    static_cast<ResidentParams&>(v) = g;
+    memcpy(v.w_val, w_host, (size_t)c->P * 4);
+    e = launch_resident_eval(c, v, st);
+  } else {
+    if (w_host) {
+      memcpy(c->hb->w, w_host, (size_t)c->P * 4);
+      g.w0 = c->hb->w;
+    }
+    e = launch_resident(c, c->res_x_cluster, g, st);
+  }
+  if (e != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

@@ -143,7 +143,11 @@ struct ResidentParams {
   float *w_out, *m_out, *g_out, *zero_out, *row_loss, *prior_loss;
   double* scalars;          // [2] log-likelihood, log-prior
   AcceptParams a;           // RES_CHAIN
-  float w_val[964];         // RES_EVAL without w0: the parameters themselves
+};
+// RES_EVAL with the parameters themselves in place of w0 (a type of its own: 3.8 KB more in every launch of a trajectory
+// cost 0.7 us)
+struct ResidentEvalParams : ResidentParams {
+  float w_val[964];
 };
 // The launch, for clusters of `cluster` CTAs (1, 2, 4, 8); or, when max_clusters is given, only the number of such
 // clusters that can be resident at once
@@ -151,6 +155,9 @@ cudaError_t launch_resident_tf32(int cluster, const void* tmap, const ResidentPa
                                  int* max_clusters);
 cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters);
+// ... of an evaluation with its parameters, for clusters of eight
+cudaError_t launch_resident_eval_tf32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st);
+cudaError_t launch_resident_eval_fp32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st);
 
 // gradient kernels
 cudaError_t launch_grad_fp32(int H, const GradParams& g, int slices, int windows, cudaStream_t st);

@@ -171,9 +171,12 @@ struct ResWords {
   __device__ static bool valid(int t, int q) { return t < W0 ? 3 * t + q < 23 * H : 3 * t + q - PAD < P; }
 };
 
-template <class Tile, int C>
+__device__ __forceinline__ float res_w0(const ResidentParams& g, int p) { return __ldcg(g.w0 + p); }
+__device__ __forceinline__ float res_w0(const ResidentEvalParams& g, int p) { return g.w_val[p]; }
+
+template <class Tile, int C, class Params>
 __global__ void __launch_bounds__(RES_THREADS, 1)
-resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ ResidentParams g) {
+resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ Params g) {
   using Words = ResWords<Tile::H>;
   constexpr int P = Words::P, NWORDS = Words::N;
   constexpr int WPM = (NWORDS + C - 1) / C;            // words per rank
@@ -231,7 +234,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     const int p = Words::param(word, q);
     has[q] = mine && Words::valid(word, q);
     if (has[q]) {
-      w_s[q] = chain ? __ldcg(a.w_cur + so + p) : g.w0 ? __ldcg(g.w0 + p) : g.w_val[p];
+      w_s[q] = chain ? __ldcg(a.w_cur + so + p) : res_w0(g, p);
       w[q] = w_s[q];
       if (g.mode != RES_EVAL) {
         g_s[q] = __ldcg((chain ? a.g_cur + so : g.g0) + p);
@@ -528,8 +531,8 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
 // ---- host side ----------------------------------------------------------------------------
 // CTAs that wait for one another's words have to be resident together.  The hardware sees to that within a cluster; for
 // windows of several clusters the launch is cooperative.
-template <typename K>
-static cudaError_t resident_launch(K kernel, int cluster, size_t smem, const void* tmap, const ResidentParams& g,
+template <typename K, typename Params>
+static cudaError_t resident_launch(K kernel, int cluster, size_t smem, const void* tmap, const Params& g,
                                    cudaStream_t st, int* max_clusters) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(max_clusters ? cluster : (g.windows * g.clusters - g.missing) * cluster);
@@ -550,6 +553,20 @@ static cudaError_t resident_launch(K kernel, int cluster, size_t smem, const voi
     return e != cudaSuccess ? e : cudaOccupancyMaxActiveClusters(max_clusters, kernel, &cfg);
   }
   return cudaLaunchKernelEx(&cfg, kernel, *reinterpret_cast<const CUtensorMap*>(tmap), g);
+}
+
+template <class Tile>
+static cudaError_t resident_launch_eval(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
+  static bool attr_done[64] = {};
+  auto kernel = resident_kernel<Tile, 8, ResidentEvalParams>;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !attr_done[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::SMEM);
+    if (e != cudaSuccess) return e;
+    if (dev < 64) attr_done[dev] = true;
+  }
+  return resident_launch(kernel, 8, Tile::SMEM, tmap, g, st, nullptr);
 }
 
 }  // namespace mcmc_b200

@@ -433,12 +433,16 @@ struct ResTf32 {
 cudaError_t launch_resident_tf32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters) {
   switch (cluster) {
-    case 1: return resident_launch(resident_kernel<ResTf32, 1>, 1, ResTf32::SMEM, tmap, g, st, max_clusters);
-    case 2: return resident_launch(resident_kernel<ResTf32, 2>, 2, ResTf32::SMEM, tmap, g, st, max_clusters);
-    case 4: return resident_launch(resident_kernel<ResTf32, 4>, 4, ResTf32::SMEM, tmap, g, st, max_clusters);
-    case 8: return resident_launch(resident_kernel<ResTf32, 8>, 8, ResTf32::SMEM, tmap, g, st, max_clusters);
+    case 1: return resident_launch(resident_kernel<ResTf32, 1, ResidentParams>, 1, ResTf32::SMEM, tmap, g, st, max_clusters);
+    case 2: return resident_launch(resident_kernel<ResTf32, 2, ResidentParams>, 2, ResTf32::SMEM, tmap, g, st, max_clusters);
+    case 4: return resident_launch(resident_kernel<ResTf32, 4, ResidentParams>, 4, ResTf32::SMEM, tmap, g, st, max_clusters);
+    case 8: return resident_launch(resident_kernel<ResTf32, 8, ResidentParams>, 8, ResTf32::SMEM, tmap, g, st, max_clusters);
   }
   return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_resident_eval_tf32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
+  return resident_launch_eval<ResTf32>(tmap, g, st);
 }
 
 }  // namespace mcmc_b200
