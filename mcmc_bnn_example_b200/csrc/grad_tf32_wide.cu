@@ -15,10 +15,10 @@
 //             MN-major operands of 32-bit types, and not valid for K-major ones, hence two copies).
 // Why.  With a row per thread (h written back to tensor memory between two passes, E of a tile 64 KB through shared memory,
 // W1 read as broadcasts, 128 dW1 sums per thread) the pipe that serves shared memory carried 2,400 wavefronts per 128 rows
-// and such a tile took 2,800 cycles; here it carries about 900 and the tile takes 2,130.  20 gradients of 8 x 1,048,576
-// rows: 12.4 ms before, 10.4 now for a first pass, 10.8 under the power cap.
-// What bounds it: no pipe.  Issue slots and MUFU (128 x 128 tanh are 1,024 cycles) are 49 % busy, the shared-memory pipe 29 %,
-// the tensor pipe 21 %; three warps a scheduler do not hide the latencies of their tiles.  Four warpgroups (7 buffers, one
+// and such a tile took 2,800 cycles; here it carries about 900 and the tile takes 1,910.  20 gradients of 8 x 1,048,576
+// rows: 12.4 ms before, 10.0 now for a first pass, 10.6 under the power cap.
+// What bounds it: no pipe.  Issue slots are 52 %, MUFU (128 x 128 tanh are 1,024 cycles) 54 % busy, the shared-memory pipe 38 %,
+// the tensor pipe 23 %; three warps a scheduler do not hide the latencies of their tiles.  Four warpgroups (7 buffers, one
 // accumulator, 112 registers) were slower, 12.0 ms, as was E in smaller pieces (16 instead of 32 columns a store: 12.6).
 // The reference has no kernel of this shape: its sizes are compile-time
 // constants for 40 hidden units (global_params.h:55-58).
