@@ -458,8 +458,8 @@ static bool use_resident(mcmc_b200_ctx* c, bool x, int L) {
   bool &asked = x ? c->res_x_asked : c->res_asked, &ok = x ? c->res_x_ok : c->res_ok;
   if (!asked) {
     ResidentParams& g = x ? c->res_x : c->res;
-    ok = resident_plan(c->rows, g.windows, c->num_sms, c->cfg.precision == MCMC_B200_PREC_FP32, [&](int i) { return resident_max_clusters(c, i); },
-                       x ? &c->res_x_cluster : &c->res_cluster, &g.clusters);
+    ok = resident_plan(c->rows, g.windows, c->num_sms, c->cfg.precision == MCMC_B200_PREC_FP32,
+                       [&](int i) { return resident_max_clusters(c, i); }, x ? &c->res_x_cluster : &c->res_cluster, &g.clusters);
     asked = true;
   }
   return ok;
@@ -1376,7 +1376,8 @@ API int mcmc_b200_checkpoint_load(mcmc_b200_ctx* c, const void* host_buf, uint64
 
 // ---- explicit-state calls (one window) -------------------------------------
 // explicit_steps in one launch where the window's rows fit on the chip.  Pointers may be device memory or the mapped
-// host block; the parameters of an evaluation may come from the host by value (w_host).  False: the launch was refused and nothing has been done (see resident_chain).
+// host block; the parameters of an evaluation may come from the host by value (w_host).  False: the launch was refused and
+// nothing has been done (see resident_chain).
 static bool resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, const float* w0, const float* m0,
                           const float* g0, float* w_last, float* m_last, float* g_out, float* zero_out,
                           float* row_loss, float* prior_loss, double* scalars, cudaStream_t st, bool eval_only,

@@ -302,19 +302,17 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
         }
       }
       // element (n = hidden unit, k) of the K-major B operand at n*128 + ((k/4) ^ (n%8))*16 + (k%4)*4
-      constexpr int NPAR = (G::P + NCOMPUTE - 1) / NCOMPUTE;
-      float wv[NPAR];
-      leapfrog_params(g, step_io(g), win, tid, NCOMPUTE, G::P, slot == 0, wv);
-#pragma unroll
-      for (int i = 0; i < NPAR; ++i) {
-        const int p = tid + i * NCOMPUTE;
+      // (one after the other: all three of a thread's at once cost a register spilled in the tile loop, 200 windows 0.8 %)
+      for (int p = tid; p < G::P; p += NCOMPUTE) {
+        float w[1];
+        leapfrog_params(g, step_io(g), win, p, NCOMPUTE, G::P, slot == 0, w);
         if (p < D * H + H) {
           const int k = p / H, n = p - k * H;
-          *reinterpret_cast<float*>(w0s + n * 128 + (((k >> 2) ^ (n & 7)) << 4) + ((k & 3) << 2)) = wv[i];
+          *reinterpret_cast<float*>(w0s + n * 128 + (((k >> 2) ^ (n & 7)) << 4) + ((k & 3) << 2)) = w[0];
         } else if (p < D * H + 2 * H) {
-          w1s[p - (D * H + H)] = wv[i];
-        } else if (p < G::P) {
-          b1s = wv[i];
+          w1s[p - (D * H + H)] = w[0];
+        } else {
+          b1s = w[0];
         }
       }
       fence_proxy_async_smem();
