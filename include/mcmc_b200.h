@@ -384,11 +384,15 @@ int mcmc_b200_chain_geometry(mcmc_b200_ctx* ctx, int* slices, int* ctas_per_sm, 
  * chain or of the explicit calls: CTAs per cluster and clusters per window, or
  * 0 and 0 where there is one launch per leapfrog step. */
 int mcmc_b200_resident_plan(mcmc_b200_ctx* ctx, int explicit_calls, int* ctas_per_cluster, int* clusters);
-/* The same as host arithmetic (no context, no GPU): available[i] = clusters of
- * 1 << i CTAs that the GPU holds at once.  What a B200 holds beyond 148, 74, 33
- * and 15 is not used: the order of the sums, and with it every bit of a chain,
- * then follows from windows and rows alone.  (TF32; an FP32 window of more than
- * 4096 rows takes one cluster more where that leaves no CTA a fifth 32-row unit.) */
+/* The same as host arithmetic (no context, no GPU), for MCMC_B200_PREC_FP32 or
+ * MCMC_B200_PREC_TF32: available[i] = clusters of 1 << i CTAs that the GPU holds
+ * at once.  What a B200 holds beyond 148, 74, 33 and 15 is not used: the order of
+ * the sums, and with it every bit of a chain, then follows from precision, windows
+ * and rows alone.  (An FP32 window of more than 4096 rows takes one cluster more
+ * than a TF32 one where that leaves no CTA a fifth 32-row unit.) */
+int mcmc_b200_plan_resident_for(int precision, int windows, int64_t rows, int num_sms, const int32_t available[4],
+                                int32_t* ctas_per_cluster, int32_t* clusters);
+/* mcmc_b200_plan_resident_for(MCMC_B200_PREC_TF32, ...) */
 int mcmc_b200_plan_resident(int windows, int64_t rows, int num_sms, const int32_t available[4],
                             int32_t* ctas_per_cluster, int32_t* clusters);
 

@@ -42,7 +42,7 @@ EXPORTS = [
     "mcmc_b200_launch_count", "mcmc_b200_chain_geometry", "mcmc_b200_potential_and_grad_static",
     "mcmc_b200_checkpoint_size", "mcmc_b200_checkpoint_save", "mcmc_b200_checkpoint_load",
     "mcmc_b200_read_table", "mcmc_b200_plan_work_table", "mcmc_b200_rebind_data",
-    "mcmc_b200_selftest_wait_timeout", "mcmc_b200_resident_plan", "mcmc_b200_plan_resident", "mcmc_b200_selftest_resident_wait", "mcmc_b200_selftest_refuse_resident",
+    "mcmc_b200_selftest_wait_timeout", "mcmc_b200_resident_plan", "mcmc_b200_plan_resident", "mcmc_b200_plan_resident_for", "mcmc_b200_selftest_resident_wait", "mcmc_b200_selftest_refuse_resident",
     "mcmc_b200_philox_device", "mcmc_b200_refstream_momentum_device",
     "mcmc_b200_refstream_engine", "mcmc_b200_refstream_engine0", "mcmc_b200_refstream_log_uniform",
     "mcmc_b200_microbench_l2_read", "mcmc_b200_microbench_mufu", "mcmc_b200_enable_oneshot_allreduce",

@@ -371,7 +371,7 @@ static int resident_max_clusters(mcmc_b200_ctx* c, int i) {
 }
 
 // What a plan counts on at most: the clusters of 1, 2, 4 and 8 CTAs that every B200 measured holds at once.  So a plan
-// follows from windows and rows alone, and a chain has the same bits on every GPU that holds as many.
+// follows from precision, windows and rows alone, and a chain has the same bits on every GPU that holds as many.
 constexpr int RES_CLUSTERS[4] = {148, 74, 33, 15};
 
 // How a window is dealt to clusters when `windows` of them share the GPU (resident.cuh); available(i): clusters of 1 << i
@@ -474,15 +474,21 @@ API int mcmc_b200_resident_plan(mcmc_b200_ctx* c, int explicit_calls, int* ctas_
   return MCMC_B200_OK;
 }
 
-API int mcmc_b200_plan_resident(int windows, int64_t rows, int num_sms, const int32_t available[4],
-                                int32_t* ctas_per_cluster, int32_t* clusters) {
-  if (windows < 1 || rows < 1 || num_sms < 1 || !available || !ctas_per_cluster || !clusters)
+API int mcmc_b200_plan_resident_for(int precision, int windows, int64_t rows, int num_sms, const int32_t available[4],
+                                    int32_t* ctas_per_cluster, int32_t* clusters) {
+  if ((precision != MCMC_B200_PREC_FP32 && precision != MCMC_B200_PREC_TF32) || windows < 1 || rows < 1 || num_sms < 1 ||
+      !available || !ctas_per_cluster || !clusters)
     return fail(MCMC_B200_ERR_INVALID, "bad arguments");
   int C = 0, K = 0;
-  if (!resident_plan(rows, windows, num_sms, false, [&](int i) { return available[i]; }, &C, &K)) C = K = 0;
+  if (!resident_plan(rows, windows, num_sms, precision == MCMC_B200_PREC_FP32, [&](int i) { return available[i]; }, &C, &K))
+    C = K = 0;
   *ctas_per_cluster = C;
   *clusters = K;
   return MCMC_B200_OK;
+}
+API int mcmc_b200_plan_resident(int windows, int64_t rows, int num_sms, const int32_t available[4],
+                                int32_t* ctas_per_cluster, int32_t* clusters) {
+  return mcmc_b200_plan_resident_for(MCMC_B200_PREC_TF32, windows, rows, num_sms, available, ctas_per_cluster, clusters);
 }
 
 API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows, int64_t rows,

@@ -215,3 +215,42 @@ def test_resident_plan_follows_from_windows_and_rows_alone():
     assert plan(1, 58368, counted) == (8, 15) and plan(1, 58368, (148, 74, 33, 14)) == (0, 0)
     assert plan(1, 61441, (148, 74, 37, 18)) == (0, 0) and plan(1, 1000, counted) == (8, 1)
     assert plan(33, 1000, counted) == (4, 1) and plan(36, 1000, counted) == (2, 1) and plan(100, 511, counted) == (1, 1)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_resident_plan_of_either_precision(prec):
+    """The sweep of the test above in both precisions.  TF32 is what the entry point without a precision answers; an FP32
+    window of several clusters leaves no CTA more than four 32-row units unless it has all the clusters that it can have."""
+    import ctypes as C
+    import mcmc_bnn_example_b200 as m
+    m.build()
+
+    def plan(windows, rows, available, sms=148, first=(prec,), fn="mcmc_b200_plan_resident_for"):
+        a, b = C.c_int32(), C.c_int32()
+        assert getattr(m.lib(), fn)(*first, windows, C.c_int64(rows), sms, (C.c_int32 * 4)(*available), C.byref(a),
+                                    C.byref(b)) == 0
+        return a.value, b.value
+
+    counted = (148, 74, 33, 15)
+    for windows in (1, 2, 3, 5, 7, 8, 15, 16, 33, 34, 36, 74, 75, 100, 148, 149, 200):
+        for rows in (1, 32, 512, 513, 1025, 2048, 4096, 4097, 5000, 5120, 5121, 6000, 9001, 15360, 15361, 30000, 61440, 61441):
+            for have in (counted, (148, 74, 36, 18), (148, 72, 32, 14), (132, 66, 32, 16), (148, 74, 33, 1), (148, 0, 0, 0)):
+                c, k = plan(windows, rows, have)
+                if prec == m.PREC_TF32:
+                    assert (c, k) == plan(windows, rows, have, first=(), fn="mcmc_b200_plan_resident")
+                if c == 0:
+                    continue
+                i = {1: 0, 2: 1, 4: 2, 8: 3}[c]
+                assert 1 <= k <= 16 and (k == 1 or c == 8) and windows * k <= have[i]
+                assert c * k * 512 >= rows
+                if all(a >= b for a, b in zip(have, counted)):
+                    assert (c, k) == plan(windows, rows, counted)
+                if prec == m.PREC_FP32 and rows > 4096:
+                    assert -(-rows // 32) <= 8 * k * 4 or k == min(have[3], 15) // windows
+    # one window, and three that share fifteen clusters: five each at most
+    want = {(1, 4097): (5, 4), (1, 5120): (5, 5), (1, 5121): (6, 5), (3, 5000): (5, 4), (3, 5121): (5, 5), (3, 20480): (5, 5)}
+    for (windows, rows), k in want.items():
+        assert plan(windows, rows, counted) == (8, k[prec]), (windows, rows)
+    a, b = C.c_int32(), C.c_int32()
+    bad = m.lib().mcmc_b200_plan_resident_for(2, 1, C.c_int64(1000), 148, (C.c_int32 * 4)(*counted), C.byref(a), C.byref(b))
+    assert bad != 0
