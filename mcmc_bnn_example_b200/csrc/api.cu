@@ -1382,7 +1382,7 @@ API int mcmc_b200_checkpoint_load(mcmc_b200_ctx* c, const void* host_buf, uint64
 
 // ---- explicit-state calls (one window) -------------------------------------
 // explicit_steps in one launch where the window's rows fit on the chip.  Pointers may be device memory or the mapped
-// host block; the parameters of an evaluation may come from the host by value (w_host).  False: the launch was refused and
+// host block; the parameters of an evaluation come from the host by value (w_host).  False: the launch was refused and
 // nothing has been done (see resident_chain).
 static bool resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, const float* w0, const float* m0,
                           const float* g0, float* w_last, float* m_last, float* g_out, float* zero_out,
@@ -1405,18 +1405,14 @@ static bool resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, 
   g.row_loss = row_loss;
   g.prior_loss = prior_loss;
   g.scalars = scalars;
-  cudaError_t e;
-  if (w_host && c->res_x_cluster == 8) {
+  cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
+  if (!w_host) {
+    e = launch_resident(c, c->res_x_cluster, g, st);
+  } else if (c->res_x_cluster == 8) {  // one window has clusters of eight on every GPU that holds one of them
     ResidentEvalParams v;
     static_cast<ResidentParams&>(v) = g;
     memcpy(v.w_val, w_host, (size_t)c->P * 4);
     e = launch_resident_eval(c, v, st);
-  } else {
-    if (w_host) {
-      memcpy(c->hb->w, w_host, (size_t)c->P * 4);
-      g.w0 = c->hb->w;
-    }
-    e = launch_resident(c, c->res_x_cluster, g, st);
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -1437,10 +1433,10 @@ API int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* c, int code, int limit_u
     c->launches++;
     if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
   }
+  const std::vector<float> w(c->P, 0.f);
   if (code == 611 || code == 901) {
     c->res_x.test_code = code;
     c->res_x.wait_ticks = (unsigned int)limit_us / 33;
-    const std::vector<float> w(c->P, 0.f);
     const int r = mcmc_b200_potential_and_grad(c, 0, w.data(), nullptr, nullptr, nullptr, nullptr);
     c->res_x.test_code = 0;
     c->res_x.wait_ticks = RES_WAIT_TICKS;
@@ -1453,8 +1449,8 @@ API int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* c, int code, int limit_u
   g.missing = 1;
   g.wait_ticks = (unsigned int)limit_us / 33;
   const bool done = chain ? resident_chain(c, 1, c->stream) == 1
-                                    : resident_steps(c, 0, 1, 0.f, c->xw[0], nullptr, nullptr, nullptr, nullptr, c->g_out,
-                                                     nullptr, nullptr, nullptr, c->scalars, c->stream, true);
+                          : resident_steps(c, 0, 1, 0.f, nullptr, nullptr, nullptr, nullptr, nullptr, c->hb->g_out,
+                                           nullptr, nullptr, nullptr, c->hb->scalars, c->stream, true, w.data());
   g.missing = 0;
   g.wait_ticks = RES_WAIT_TICKS;
   if (!done) return fail(MCMC_B200_ERR_CUDA, "the launch was refused");
