@@ -1064,7 +1064,7 @@ static int chain_grad(mcmc_b200_ctx* c, int mode, int s, cudaStream_t st) {
   if (c->oneshot) return oneshot_allreduce(c, c->partial[s & 1], c->llp[s & 1], st);
   if (red) {
     cudaError_t e = launch_reduce_partials(c->partial[s & 1], c->llp[s & 1], c->slices, c->tab_nslot, c->P,
-                                           c->Pp, c->red, c->W, st);
+                                           c->Pp, c->red, c->W, c->num_sms, st);
     c->launches++;
     if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
     if (c->comm) {
@@ -1493,7 +1493,7 @@ static int explicit_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, c
     if (r) return r;
     if (red) {
       cudaError_t e = launch_reduce_partials(c->xpartial[s & 1], c->xllp[s & 1], S, c->xtab_nslot, c->P, c->Pp,
-                                             c->xred, 1, st);
+                                             c->xred, 1, c->num_sms, st);
       c->launches++;
       if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
       if (c->comm) {
@@ -1869,7 +1869,7 @@ API int mcmc_b200_time_allreduce(mcmc_b200_ctx* c, int reps, float* us_per_call)
   auto once = [&]() -> int {
     if (c->oneshot) return oneshot_allreduce(c, c->partial[0], c->llp[0], c->stream);
     cudaError_t e = launch_reduce_partials(c->partial[0], c->llp[0], c->slices, c->tab_nslot, c->P, c->Pp, c->red,
-                                           c->W, c->stream);
+                                           c->W, c->num_sms, c->stream);
     c->launches++;
     if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
     return allreduce(c, c->red, (size_t)c->W * (c->Pp + 4), c->stream);

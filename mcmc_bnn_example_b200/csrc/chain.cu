@@ -282,15 +282,15 @@ reduce_partials_kernel(const float* __restrict__ partial, const double* __restri
   }
 }
 
-// A CTA of 1,024 threads per 32 parameters is the shortest while the GPU holds all of them (two to each of 148 SMs); beyond
+// A CTA of 1,024 threads per 32 parameters is the shortest while the GPU holds all of them (two to an SM); beyond
 // that they come in waves, and CTAs of 256 are faster.  us a leapfrog iteration of ten steps, 1,024 and 256 threads: 25
 // TF32 windows 486, 457; 50 FP32 windows of 5,000 rows 403, 359; 8 windows of 128 units 273, 250; 4 FP32 windows 360, 365.
 cudaError_t launch_reduce_partials(const float* partial, const double* ll_partial, int slices,
                                    const int* nslot, int P, int Pp, double* red, int windows,
-                                   cudaStream_t st) {
+                                   int num_sms, cudaStream_t st) {
   constexpr int SMALL = 8;
   const dim3 grid((Pp + RED_PARAMS - 1) / RED_PARAMS, windows);
-  if ((long long)grid.x * windows > 2 * 148)
+  if ((long long)grid.x * windows > 2 * num_sms)
     return launch_chain_kernel(reduce_partials_kernel<SMALL>, grid, dim3(RED_PARAMS * SMALL), 0, st, partial, ll_partial,
                                slices, nslot, P, Pp, red);
   return launch_chain_kernel(reduce_partials_kernel<RED_GROUPS>, grid, dim3(RED_PARAMS * RED_GROUPS), 0, st, partial,

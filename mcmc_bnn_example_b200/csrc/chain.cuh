@@ -62,7 +62,7 @@ cudaError_t launch_repack(const float* x, const float* y, float* out, long long 
                           long long rows_pad, int D, cudaStream_t st);
 cudaError_t launch_reduce_partials(const float* partial, const double* ll_partial, int slices,
                                    const int* nslot, int P, int Pp, double* red, int windows,
-                                   cudaStream_t st);
+                                   int num_sms, cudaStream_t st);
 // One-shot all-reduce over peer memory for row sharding (chain.cu): what every rank's launch needs
 constexpr int ONESHOT_SLICE = 32;   // parameters per CTA
 constexpr int ONESHOT_MAX_RANKS = 16;
