@@ -133,3 +133,28 @@ def test_clusters_of_a_window_leave_fp32_ctas_four_units(built, prec, rows, fp32
     tol = 2e-3 if prec else 1e-5
     assert np.abs(got["grad"] - ref["grad"]).max() <= tol * np.abs(ref["grad"]).max()
     assert abs(got["loglik"] - ref["loglik"]) <= tol * abs(ref["loglik"])
+
+
+@pytest.mark.parametrize("prec,H,W", [(0, 40, 11), (1, 40, 11), (0, 128, 4), (1, 128, 4)])
+@pytest.mark.parametrize("slices", [5, 13, 37])
+def test_partial_sums_have_the_same_bits_in_large_and_small_ctas(built, prec, H, W, slices):
+    """A batch whose partial sums are added in CTAs of 256 threads (more than two to an SM) and its last window alone, in CTAs
+    of 1,024: slot counts below the eight rows of threads of the small ones, between them and 32, and above 32."""
+    m, _ = built
+    rows = 128 * slices + 77
+    cfg = m.reference_config(H=H, precision=prec, slices=slices, sample_capacity=2, leapfrog_steps=3, burn_in=0, adapt_steps=0)
+    data = [m.synth_window(3, g, rows, H=H)[:2] for g in range(2)]
+
+    def run(first, last):
+        ctx = m.Context(cfg, last - first, rows)
+        for g in range(first, last):
+            ctx.set_window_data(g - first, *data[g % 2], global_window=g)
+        ctx.run_chain(2)
+        out = ctx.get_samples(last - first - 1), ctx.get_state(last - first - 1), ctx.geometry()["slices"]
+        ctx.close()
+        return out
+
+    (s1, g1, n1), (s2, g2, n2) = run(0, W), run(W - 1, W)
+    assert n1 == n2 == slices
+    assert s1.any() and np.array_equal(s1, s2)
+    assert all(np.array_equal(g1[k], g2[k]) for k in g1)
