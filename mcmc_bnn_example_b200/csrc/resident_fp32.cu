@@ -95,7 +95,7 @@ struct ResFp32 {
 
   __device__ __forceinline__ void step(const ResidentParams& g, float* row_loss, bool last, bool&) {
     if (!active) return;
-    {
+    if (warp >= 4) {  // (a scheduler's first warp waits for nothing: looking at the clock cost it 0.02 to 0.04 us a step)
       const uint32_t t0 = (uint32_t)clock64();
       while ((uint32_t)clock64() - t0 < (uint32_t)(warp >> 2) * TURN) {}
     }
