@@ -127,44 +127,30 @@ __device__ __forceinline__ void lik_terms(const LikParams& lk, float y, float pr
 // All of a thread's loads come before its stores: one parameter after the other, a store between the loads of two of them
 // kept the second's from being issued early, and eight of them were eight trips to L2 in a row (FP32, 16 windows of 40013
 // rows: 82 us a step instead of 79; 128 units TF32, 8 x 1,048,576 rows: 541 instead of 530).
-// The launch's vectors are taken out of the parameters first.  With each of them read from there where it is used, the
-// 128-unit TF32 kernel took 2.5 % longer (11.75 instead of 11.46 ms for 20 gradients of 8 x 1,048,576 rows; same
-// registers and spills), the other kernels the same.
-struct StepIo {
-  const float* w_in;
-  const float* m_in;
-  float* w_out;
-  float* m_out;
-  const double* red_in;
-  int mode;
-};
-__device__ __forceinline__ StepIo step_io(const GradParams& g) {
-  return StepIo{g.w_in, g.m_in, g.w_out, g.m_out, g.red_in, g.mode};
-}
 template <int N>
-__device__ __forceinline__ void leapfrog_params(const GradParams& g, const StepIo& io, int win, int p0, int step, int limit,
-                                                bool store, float (&w)[N]) {
+__device__ __forceinline__ void leapfrog_params(const GradParams& g, int win, int p0, int step, int limit, bool store,
+                                                float (&w)[N]) {
   const size_t o = (size_t)win * g.Pp + p0;
   const float eps = g.eps ? g.eps[win] : g.eps_scalar;
   float grad[N], m[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     w[i] = grad[i] = m[i] = 0.f;
-    if (p0 + i * step < limit) w[i] = __ldcg(io.w_in + o + i * step);
+    if (p0 + i * step < limit) w[i] = __ldcg(g.w_in + o + i * step);
   }
-  if (io.mode == MODE_EVAL) return;
+  if (g.mode == MODE_EVAL) return;
   float kick;
 #pragma unroll
   for (int i = 0; i < N; ++i)
-    if (p0 + i * step < limit) m[i] = __ldcg(io.m_in + o + i * step);
-  if (io.mode == MODE_FIRST) {
+    if (p0 + i * step < limit) m[i] = __ldcg(g.m_in + o + i * step);
+  if (g.mode == MODE_FIRST) {
 #pragma unroll
     for (int i = 0; i < N; ++i)
       if (p0 + i * step < limit) grad[i] = __ldcg(g.g_carried + o + i * step);
     kick = 0.5f;
   } else {
-    if (io.red_in) {
-      const double* r = io.red_in + (size_t)win * (g.Pp + 4) + p0;
+    if (g.red_in) {
+      const double* r = g.red_in + (size_t)win * (g.Pp + 4) + p0;
 #pragma unroll
       for (int i = 0; i < N; ++i)
         if (p0 + i * step < limit) grad[i] = (float)__ldcg(r + i * step);
@@ -189,8 +175,8 @@ __device__ __forceinline__ void leapfrog_params(const GradParams& g, const StepI
 #pragma unroll
     for (int i = 0; i < N; ++i)
       if (p0 + i * step < limit) {
-        io.w_out[o + i * step] = w[i];
-        io.m_out[o + i * step] = m[i];
+        g.w_out[o + i * step] = w[i];
+        g.m_out[o + i * step] = m[i];
       }
   }
 }

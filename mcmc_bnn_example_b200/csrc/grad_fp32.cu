@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(Fp32Geom<H>::NT, MINB) grad_fp32_kernel(const 
   // fused leapfrog update; parameters land in the layout the lanes read
   {
     float w[(Warp::P + NT - 1) / NT];
-    leapfrog_params(g, step_io(g), win, tid, NT, Warp::P, slice == 0, w);
+    leapfrog_params(g, win, tid, NT, Warp::P, slice == 0, w);
 #pragma unroll
     for (int i = 0; i < (Warp::P + NT - 1) / NT; ++i) {
       const int p = tid + i * NT;

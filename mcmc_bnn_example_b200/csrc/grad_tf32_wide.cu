@@ -241,9 +241,8 @@ grad_tf32_wide_kernel(const __grid_constant__ CUtensorMap tmap_mn, const __grid_
       // ---- segment prologue: fused leapfrog update of features 8 wg .. 8 wg + 7 of the thread's unit (22 is the
       // bias, 23 is y, whose weight is zero; in its place W1) ----
       {
-        const StepIo io = step_io(g);
         float w[8];
-        leapfrog_params(g, io, win, 8 * wg * H + hid, H, G::P, slot == 0, w);
+        leapfrog_params(g, win, 8 * wg * H + hid, H, G::P, slot == 0, w);
         if (wg == NWG - 1) {
           w1s[hid] = w[7];
           w[7] = 0.f;
@@ -251,7 +250,7 @@ grad_tf32_wide_kernel(const __grid_constant__ CUtensorMap tmap_mn, const __grid_
         tc_st8(tmem + G::W_COL0 + 8 * wg + lane_off, make_float4(w[0], w[1], w[2], w[3]), make_float4(w[4], w[5], w[6], w[7]));
         if (tid == 0) {
           float b[1];
-          leapfrog_params(g, io, win, D * H + 2 * H, 1, G::P, slot == 0, b);
+          leapfrog_params(g, win, D * H + 2 * H, 1, G::P, slot == 0, b);
           b1s = b[0];
         }
         tc_wait_st();
