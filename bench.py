@@ -40,9 +40,10 @@ ALG_BYTES_PER_ROW = 92          # 22 features + y, FP32: what one gradient must 
 MIN_TIMED_S = 2.0               # the K-step region is repeated until this much has been timed
 METRIC = "hmc_samples_per_sec_all_windows"
 UNIT = "samples/s"
-# DRAM traffic of the gradient kernel per row, from the ncu capture summarised in
-# profiles/grad_tf32_kernel_w32.md (dram read + write bytes of one launch / rows of that launch)
-NCU_DRAM_BYTES_PER_ROW = 99.0
+# Gradient kernel by precision and hidden width, and its DRAM traffic per row from the ncu captures summarised in
+# profiles/ (dram read + write bytes of one launch / rows of that launch)
+GRAD_KERNELS = {("tf32", 40): ("grad_tf32_kernel", 99.0), ("tf32", 128): ("grad_tf32_wide_kernel", 97.0),
+                ("fp32", 40): ("grad_fp32_kernel", 99.0), ("fp32", 128): ("grad_fp32_kernel", 97.0)}
 
 
 def measured_peaks():
@@ -585,10 +586,10 @@ def main():
         "roofline": {
             "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_source": peak_src,
-            "kernel": "grad_tf32_kernel" if args.precision == "tf32" else "grad_fp32_kernel",
+            "kernel": GRAD_KERNELS[args.precision, HID][0],
             "algorithmic_bytes_per_launch": ALG_BYTES_PER_ROW * rows_per_launch,
             "avg_launch_ms": grad_ms,
-            "traffic": NCU_DRAM_BYTES_PER_ROW * rows_per_launch,
+            "traffic": GRAD_KERNELS[args.precision, HID][1] * rows_per_launch,
         },
     }
     if args.precision == "tf32":

@@ -384,7 +384,8 @@ constexpr int RES_CLUSTERS[4] = {148, 74, 33, 15};
 // us a step by clusters, TF32: 4096 rows 4.2 (1), 4.2 (8); 4097 rows 3.9 (4, taken), 4.0 (5); 6000 rows 4.2 (3), 4.1 (5, taken),
 // 4.1 (6), 4.6 (15); 16384 rows 5.4 (4), 4.5 (8), 4.8 (15, taken).  FP32: 4097 rows 7.65 (4), 6.6 (5, taken); 6000 rows 8.1 (5),
 // 6.7 (6, taken), 6.9 (8); 10000 rows 8.2 (9), 6.9 (10, taken); 13000 rows 8.3 (12), 7.1 (13, taken); three windows of 5000
-// rows 8.1 (4), 6.8 (5, taken); 16384 rows 8.4 (15, taken); 4096 rows 10.8 (1, taken), 6.9 (4).
+// rows 8.1 (4), 6.8 (5, taken); 16384 rows 8.4 (15, taken); 4096 rows 10.8 (1, taken), 6.9 (4).  So the rule is not the best
+// one for a TF32 window of 16384 rows (8 and 15 clusters both give a CTA two 128-row tiles) nor for an FP32 one of 4096.
 // Against one launch per step (one B200, 1 to 148 windows of 100 to 61440 rows that fit): 1.1 (FP32, one window of 4096
 // rows: 11.8 and 12.9 us a step) to 3.2 times as fast, so every window that fits goes this way.
 template <typename F>

@@ -2,9 +2,9 @@
 // does with its 32 rows): every warp owns one 32-row unit for the whole launch.
 // One launch per step took 29.5 us a step for a 58368-row window, this takes 12.5 (2000 steps, one B200); a log density
 // and gradient of 1000 rows from host pointers takes 30 us instead of 64.
-// What bounds a step: the FMA pipe (about 1,900 multiplications per row, 3,500 cycles each for forward and backward at
-// 512 rows per CTA) and the tanh pass (two MUFU operations each, 2,560 cycles), which overlap as far as the warps of a
-// scheduler are in different phases; then the exchange.
+// What bounds a step: no pipe (at 512 rows a CTA the one that serves shared memory is 71 % busy, issue slots 58 %, FMA 52 %).
+// A block takes a scheduler 3,600 cycles, of which its multiplications keep the FMA pipe busy for 2,240: they, the tanh and the
+// multiplications after it overlap as far as the warps of a scheduler are in different phases.  Then the exchange.
 #include <cuda.h>
 #include "fp32_tile.cuh"
 #include "resident.cuh"
@@ -32,7 +32,9 @@ struct ResFp32 {
   // The four warps of a scheduler get the weights at the same moment.  In step with one another they would all multiply,
   // then all wait for their tanh (646 cycles of the MUFU pipe each), and so on; so each starts this many cycles after the
   // one before it, about the multiplications of half a block.  58368 rows, us a step: 12.91 (0), 12.61 (300), 12.46 (500
-  // to 700), 12.57 (1000), 12.69 (1300).  Windows with one unit to a scheduler have nothing to wait for.
+  // to 700), 12.57 (1000), 12.69 (1300).  Two to four units to a scheduler, 0 and 600: 1100 rows 7.10, 6.98; 2048 rows 7.61,
+  // 7.43; 3000 rows 9.60, 9.22; 4096 rows 11.75, 11.14; single evaluations 0 to 0.6 less.  A scheduler's first unit never
+  // waits.
   static constexpr uint32_t TURN = 600;
 
   Warp lanes;

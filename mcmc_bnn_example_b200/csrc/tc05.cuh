@@ -42,8 +42,8 @@ __device__ __forceinline__ void tc_mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem,
 // One lane of a converged warp, for the *_if forms below.  They are executed by the whole warp under a predicate, not
 // inside a branch on the lane: the operands then stay in uniform registers.  Inside a branch every MMA first moves
 // its descriptors there, and eight MMAs take a warp 810 cycles from issue to completion instead of 585 (32: 2,130
-// instead of 1,530).  For the kernels whose control warps issue a whole tile ahead this does not pay: the wide kernel
-// ran 7 % slower with it (its MMAs then come in bursts that hold up the compute warps' shared-memory accesses).
+// instead of 1,530).  The streaming kernels, whose control warps issue a whole tile ahead of the compute warps, issue from one
+// lane.
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
