@@ -99,7 +99,8 @@ struct HostBlock {
   double scalars[2];
   int status;
   float log_acpt;  // out: the drop-in accept ratio
-  int pad[2];
+  int fwd_status;  // a wait of a forward pass that ran out
+  int pad[1];
   float w[HB_FLOATS], m[HB_FLOATS], g[HB_FLOATS];  // in: position, momentum, gradient
   float w_out[HB_FLOATS], m_out[HB_FLOATS], g_out[HB_FLOATS];
 };
@@ -1666,42 +1667,57 @@ static int fwd_reserve(mcmc_b200_ctx* c, T** buf, size_t* cap, size_t need) {
   return MCMC_B200_OK;
 }
 
+// waits for a forward pass; a wait of its kernel that ran out is reported through the mapped host block
+static int forward_finish(mcmc_b200_ctx* c) {
+  CK(cudaStreamSynchronize(c->stream));
+  const int code = *reinterpret_cast<volatile int*>(&c->hb->fwd_status);
+  if (code == 0) return MCMC_B200_OK;
+  c->hb->fwd_status = 0;
+  char b[96];
+  snprintf(b, sizeof b, "device-side wait ran out (code %d)", code);
+  return fail(MCMC_B200_ERR_TIMEOUT, b);
+}
+
 API int mcmc_b200_predict_mean(mcmc_b200_ctx* c, int window, const float* xs, int64_t n, int first,
                                int count, float* out) {
   if (!c || !xs || !out || n < 1 || window < 0 || window >= c->W || first < 0 || count < 1 ||
       !c->samples || first + count > c->cfg.sample_capacity)
     return fail(MCMC_B200_ERR_INVALID, "bad arguments or no sample storage");
   CK(cudaSetDevice(c->device));
-  // a chunk's sums are 8 bytes a row beside the row's own 92: at most five chunks or 64 MB (5,000 samples of 10 M rows
-  // would take eight for less than one per cent), and one where there is no memory for more
-  const int most = (int)std::max<int64_t>(5, std::min<int64_t>(FWD_MAX_CHUNKS, (64 << 20) / (8 * n)));
-  int chunks = forward_chunks(c->num_sms, n, count, most);
-  int r = fwd_reserve(c, &c->fwd_x, &c->fwd_x_cap, (size_t)n * c->cfg.D);
-  if (r == MCMC_B200_OK) r = fwd_reserve(c, &c->fwd_out, &c->fwd_out_cap, (size_t)n);
-  if (r) return r;
-  r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)chunks * n);
-  if (r == MCMC_B200_ERR_NOMEM && chunks > 1) {
-    chunks = 1;
-    r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)n);
-  }
-  if (r) return r;
-  CK(cudaMemcpyAsync(c->fwd_x, xs, (size_t)n * c->cfg.D * 4, cudaMemcpyHostToDevice, c->stream));
+  const bool split = c->cfg.H == SPLIT_H;
   ForwardParams a;
   memset(&a, 0, sizeof a);
-  a.x = c->fwd_x;
   a.x_stride = c->cfg.D;
   a.n = n;
   a.samples = c->samples + ((size_t)window * c->cfg.sample_capacity + first) * c->P;
   a.count = count;
   a.lik = make_lik(c->cfg);
+  a.status = &c->hb->fwd_status;
+  // 128 units: a chunk's sums are 8 bytes a row beside the row's own 92: at most five chunks or 64 MB (5,000 samples of 10 M
+  // rows would take eight for less than one per cent), and one where there is no memory for more
+  const int most = (int)std::max<int64_t>(5, std::min<int64_t>(FWD_MAX_CHUNKS, (64 << 20) / (8 * n)));
+  int chunks = split ? forward_split_slots(c->num_sms, a) : forward_chunks(c->num_sms, n, count, most);
+  int r = fwd_reserve(c, &c->fwd_x, &c->fwd_x_cap, (size_t)n * c->cfg.D);
+  if (r == MCMC_B200_OK) r = fwd_reserve(c, &c->fwd_out, &c->fwd_out_cap, (size_t)n);
+  if (r) return r;
+  r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)chunks * n);
+  if (r == MCMC_B200_ERR_NOMEM && chunks > 1) {
+    chunks = a.whole = 1;
+    r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)n);
+  }
+  if (r) return r;
+  CK(cudaMemcpyAsync(c->fwd_x, xs, (size_t)n * c->cfg.D * 4, cudaMemcpyHostToDevice, c->stream));
+  a.x = c->fwd_x;
   a.partial = c->fwd_partial;
-  cudaError_t e = launch_forward_samples(c->cfg.H, a, chunks, false, c->stream);
-  if (e == cudaSuccess) e = launch_forward_finish_predict(c->fwd_partial, chunks, n, count, c->fwd_out, c->stream);
+  cudaError_t e = split ? launch_forward_split(a, c->num_sms, false, c->stream)
+                        : launch_forward_samples(c->cfg.H, a, chunks, false, c->stream);
+  if (e == cudaSuccess)
+    e = split ? launch_forward_split_finish(a, c->num_sms, c->fwd_out, c->stream)
+              : launch_forward_finish_predict(c->fwd_partial, chunks, n, count, c->fwd_out, c->stream);
   c->launches += 2;
   if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
   CK(cudaMemcpyAsync(out, c->fwd_out, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  return MCMC_B200_OK;
+  return forward_finish(c);
 }
 
 API int mcmc_b200_final_loss(mcmc_b200_ctx* c, int window, int first, int count, double* mean_loglik,
@@ -1712,7 +1728,7 @@ API int mcmc_b200_final_loss(mcmc_b200_ctx* c, int window, int first, int count,
   if (!c->window_set[window]) return fail(MCMC_B200_ERR_INVALID, "window has no data yet");
   CK(cudaSetDevice(c->device));
   // all samples against the window's rows in one launch (FP32 forward pass, no gradient)
-  const int tiles = forward_row_tiles(c->rows);
+  const int tiles = forward_row_tiles(c->cfg.H, c->rows);
   const int chunks = forward_chunks(c->num_sms, c->rows, count, FWD_MAX_CHUNKS);
   int r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)tiles * count + 2 * (size_t)count);
   if (r) return r;
@@ -1731,14 +1747,17 @@ API int mcmc_b200_final_loss(mcmc_b200_ctx* c, int window, int first, int count,
   a.partial = c->fwd_partial;
   double* d_ll = c->fwd_partial + (size_t)tiles * count;
   double* d_lp = d_ll + count;
-  cudaError_t e = launch_forward_samples(c->cfg.H, a, chunks, true, c->stream);
+  a.status = &c->hb->fwd_status;
+  cudaError_t e = c->cfg.H == SPLIT_H ? launch_forward_split(a, c->num_sms, true, c->stream)
+                                      : launch_forward_samples(c->cfg.H, a, chunks, true, c->stream);
   if (e == cudaSuccess)
     e = launch_forward_finish_loss(c->fwd_partial, tiles, count, smp, c->P, make_prior(c->cfg), d_ll, d_lp, c->stream);
   c->launches += 2;
   if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
   std::vector<double> h(2 * (size_t)count);
   CK(cudaMemcpyAsync(h.data(), d_ll, h.size() * 8, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  r = forward_finish(c);
+  if (r) return r;
   double sa = 0, sb = 0;
   for (int s = 0; s < count; ++s) { sa += h[s]; sb += h[count + s]; }  // main.h:100-113: running means
   if (mean_loglik) *mean_loglik = sa / count;

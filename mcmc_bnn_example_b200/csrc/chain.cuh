@@ -96,8 +96,17 @@ struct ForwardParams {
   int count;
   LikParams lik;
   double* partial;         // PREDICT: [chunks][n]   LOSS: [row tiles][count]
+  int whole;               // 40 units: every CTA takes whole row tiles, so that a row has one sum
+  int* status;             // 40 units: where a bounded wait that runs out leaves its code
 };
-int forward_row_tiles(long long n);
+// 40 units (SPLIT_H): four 128-row tiles to a CTA (forward_split_kernel)
+constexpr int SPLIT_H = 40;
+constexpr int FWS_ROWS = 512;
+__host__ __device__ inline long long forward_split_tiles(long long n) { return (n + FWS_ROWS - 1) / FWS_ROWS; }
+int forward_split_slots(int num_sms, const ForwardParams& a);
+cudaError_t launch_forward_split(const ForwardParams& a, int num_sms, bool loss, cudaStream_t st);
+cudaError_t launch_forward_split_finish(const ForwardParams& a, int num_sms, float* out, cudaStream_t st);
+int forward_row_tiles(int H, long long n);
 constexpr int FWD_MAX_CHUNKS = 64;
 int forward_chunks(int num_sms, long long n, int count, int most);
 cudaError_t launch_forward_samples(int H, const ForwardParams& a, int chunks, bool loss, cudaStream_t st);

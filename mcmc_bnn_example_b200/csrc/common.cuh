@@ -79,6 +79,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// Dynamic shared memory from its first 1024-byte boundary on.  The offset is added to the array itself: a pointer rounded up as an
+// integer loses its address space, and every access through it becomes a generic one.
+__device__ __forceinline__ unsigned char* smem_align1024(unsigned char* raw) {
+  return raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
+}
+
 // ---- reference tanh (kernel_helpers.h:32-44): 2*sigmoid(2x)-1 on ex2/rcp
 // approximations, identity below the cut-off -------------------------------
 __device__ __forceinline__ float tanh_ref(float x) {
@@ -281,6 +287,24 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
+}
+
+// tanh_ref of two values, its arithmetic packed
+__device__ __forceinline__ uint64_t tanh_ref2(uint64_t x) {
+  float x0, x1, e0, e1, d0, d1, s0, s1, t0, t1;
+  uint64_t m, d, t;
+  unpack2(x, x0, x1);
+  m = mul2(x, pack2(-2.88539008177792681472f, -2.88539008177792681472f));
+  unpack2(m, e0, e1);
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e0));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e1));
+  d = add2(pack2(1.f, 1.f), pack2(e0, e1));
+  unpack2(d, d0, d1);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s0) : "f"(d0));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s1) : "f"(d1));
+  t = fma2(pack2(s0, s1), pack2(2.f, 2.f), pack2(-1.f, -1.f));
+  unpack2(t, t0, t1);
+  return pack2(fabsf(x0) < 0.0048176045529544353485f ? x0 : t0, fabsf(x1) < 0.0048176045529544353485f ? x1 : t1);
 }
 
 // ---- programmatic dependent launch -----------------------------------------

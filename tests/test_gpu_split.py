@@ -1,0 +1,96 @@
+"""The FP32 product of rows and weights on the tensor core (csrc/split_mma.cuh): its error against 64 bits, values that take
+plain FFMA, and the sizes where the kernels that use it change their partition."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+H, D = 40, 22
+
+
+def _with_samples(ctx, samples):
+    """Puts `samples` in the place of the stored ones (through a checkpoint)."""
+    blob = bytearray(ctx.checkpoint().tobytes())
+    old = ctx.get_samples(0).tobytes()
+    at = blob.rfind(old)
+    assert at >= 0
+    blob[at:at + len(old)] = np.ascontiguousarray(samples, np.float32).tobytes()
+    ctx.restore(bytes(blob))
+
+
+def _sampler(m, count):
+    ctx = m.Context(m.baseline_config(precision=m.PREC_FP32, leapfrog_steps=3, sample_capacity=count), 1, 128)
+    ctx.set_window_data(0, *m.synth_window(1, 0, 128)[:2])
+    ctx.run_chain(count)
+    return ctx
+
+
+def _forward(p, x):
+    w0, b0, w1, b1 = np.split(np.asarray(p, np.float64), [D * H, D * H + H, D * H + 2 * H])
+    return np.tanh(x.astype(np.float64) @ w0.reshape(D, H) + b0) @ w1 + b1[0]
+
+
+@pytest.mark.parametrize("scaled", [False, True])
+@pytest.mark.parametrize("unit", [0, 17, 39])
+def test_product_has_the_error_of_an_fp32_sum(built, unit, scaled):
+    """One unit passed through (its tanh is the identity below 0.0048): the prediction is the product itself.  With the products
+    that are left out the error is 4.4e-8 in the mean square over units and up to 6.3e-8 for one, simulated; that of a chain of
+    FP32 additions 6.9e-8 and 7.8e-8.  What a truncated sum would leave in every row alike (7e-8) must not be there: 1e-9 is,
+    up to 1e-8 for one unit."""
+    m, _ = built
+    rng = np.random.default_rng(unit)
+    ctx = _sampler(m, 1)
+    col = 10.0 ** rng.uniform(-3, 3, D) if scaled else np.ones(D)   # features of very different scales
+    p = np.zeros(ctx.P)
+    p[:D * H] = (1e-4 / col[:, None] * rng.standard_normal((D, H))).ravel()
+    p[D * H:D * H + H] = 1e-4 * rng.standard_normal(H)
+    p[D * H + H + unit] = 1.0
+    p = p.astype(np.float32)
+    _with_samples(ctx, p)
+    x = (col * rng.standard_normal((40000, D))).astype(np.float32)
+    got = ctx.predict_mean(0, x).astype(np.float64)
+    ctx.close()
+    want = x.astype(np.float64) @ p[:D * H].astype(np.float64).reshape(D, H)[:, unit] + float(p[D * H + unit])
+    assert np.abs(want).max() < 0.0048
+    err, rms = got - want, np.sqrt((want ** 2).mean())
+    assert np.sqrt((err ** 2).mean()) < 7e-8 * rms
+    assert np.abs(err).max() < 5e-7 * rms
+    assert abs((err * np.sign(want)).mean()) < 2e-8 * np.abs(want).mean()
+
+
+HARD = [np.inf, -np.inf, np.nan, 3e38, 2.0 ** 60, 2.0 ** 59, -1e-40]
+
+
+@pytest.mark.parametrize("value", HARD)
+def test_predictions_of_values_that_cannot_be_split(built, value):
+    m, _ = built
+    ctx = _sampler(m, 3)
+    rng = np.random.default_rng(3)
+    s = (0.2 * rng.standard_normal((3, ctx.P))).astype(np.float32)
+    x = rng.standard_normal((700, D)).astype(np.float32)
+    xe, se = x.copy(), s.copy()
+    xe[5, 3], xe[-1, 0] = value, -value
+    se[1, 7], se[2, D * H + 3] = value, -value
+    with np.errstate(all="ignore"):
+        want = [np.mean([_forward(p, xx) for p in ss], axis=0) for ss, xx in ((s, xe), (se, x))]
+    for ss, xx, ref in zip((s, se), (xe, x), want):
+        _with_samples(ctx, ss)
+        got = ctx.predict_mean(0, xx)
+        assert np.array_equal(np.isnan(got), np.isnan(ref))
+        ok = np.isfinite(ref)
+        assert np.abs(got[ok] - ref[ok]).max(initial=0) <= 1e-5 * np.abs(s[:, D * H + H:-1]).sum(axis=1).max()
+    ctx.close()
+
+
+@pytest.mark.parametrize("rows,count", [(1, 149), (512, 1), (513, 3), (1537, 97), (76289, 2), (300000, 1)])
+def test_prediction_tiles_and_their_ranges(built, rows, count):
+    """Row tiles of 512 with a row more or less, one tile shared by every CTA, more tiles than CTAs."""
+    m, _ = built
+    ctx = _sampler(m, count)
+    s = (0.2 * np.random.default_rng(rows).standard_normal((count, ctx.P))).astype(np.float32)
+    _with_samples(ctx, s)
+    x = np.random.default_rng(count).standard_normal((rows, D)).astype(np.float32)
+    got = ctx.predict_mean(0, x)
+    ctx.close()
+    want = sum(_forward(p, x) for p in s) / count
+    # a tanh of ex2 / rcp approximations (a few 1e-7) in each unit
+    assert np.abs(got - want).max() <= 1e-6 * max(1.0, np.abs(s[:, D * H + H:-1]).sum(axis=1).max())
