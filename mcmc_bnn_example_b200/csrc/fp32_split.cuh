@@ -1,0 +1,217 @@
+// FP32 arithmetic of a warp's 32 rows for 40 hidden units, behind the forward product on the tensor core (split_mma.cuh):
+// z out of tensor memory, output layer, loss, dL/dz through the warp's own shared memory, backward by FFMA.  No warp waits
+// for another inside it.
+//
+// Layouts.  z is read in the 16-lane quad shape: quad q = lane / 4 holds rows q, q + 8, q + 16, q + 24, its lane c units
+// 8 n + 2 c and the next one (n < 5).  A row's output is then a sum over four lanes, dW1 ten sums per lane.  dL/dz goes to
+// es[row][unit], eight bytes a store, free of bank conflicts (rows are 40 floats apart: 8 q + 2 c).
+// Backward: a lane owns 12 features x 5 units of every second row.  What bounds it is feeding the multiplications: a 16-byte load
+// of a whole warp takes four passes over shared memory, but two when neighbouring lanes read the same address; so the
+// feature half is lane bit 0, and the unit group the next three bits: units 4 b .. 4 b + 3 and 32 + b.  Features go in pairs through
+// packed FMAs (their common factor, dL/dz, is one value for both: 2.3 cycles a packed FMA instead of 2.8).
+// W1's factor of dL/dz is left to whoever reads the sums out.
+#pragma once
+#include "split_mma.cuh"
+
+namespace mcmc_b200 {
+
+struct SplitWarp {
+  static constexpr int H = SPLIT_H, D = SPLIT_D, P = D * H + 2 * H + 1;
+  static constexpr int ROWS = 32, ES = ROWS * H;
+  static constexpr int KPT = 12, UPT = 5;   // backward: features and units per lane
+
+  int lane, q, c;          // forward
+  int bcg, kh, rsub;       // backward
+  __device__ __forceinline__ SplitWarp() {
+    lane = threadIdx.x & 31;
+    q = lane >> 2;
+    c = lane & 3;
+    kh = lane & 1;
+    bcg = (lane >> 1) & 7;
+    rsub = lane >> 4;
+  }
+  __device__ __forceinline__ int own() const { return q + 8 * c; }  // the row whose dL/dpred this lane computes
+
+  static __device__ __forceinline__ uint64_t lds64(const float* p) { return *reinterpret_cast<const uint64_t*>(p); }
+
+  // z of rows and units as the quads hold them, from tensor memory (z_t with the warp's lanes)
+  __device__ __forceinline__ void load(uint32_t z_t, uint64_t (&z)[4][5]) const {
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const uint32_t t = z_t + ((uint32_t)(hf * 16) << 16);
+      float s1[20], s0[20];
+      tc_ld_quad32(t, s1);
+      tc_ld_quad8(t + 32, s1 + 16);
+      tc_ld_quad32(t + SPLIT_S0, s0);
+      tc_ld_quad8(t + SPLIT_S0 + 32, s0 + 16);
+      tc_wait_ld();
+#pragma unroll
+      for (int n = 0; n < 5; ++n)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          z[2 * hf + i][n] = add2(pack2(s0[4 * n + 2 * i], s0[4 * n + 2 * i + 1]), pack2(s1[4 * n + 2 * i], s1[4 * n + 2 * i + 1]));
+    }
+  }
+  // the same by FFMA, for values that split_wide finds: the lane's row, through es.  A weight is
+  // the sum of its parts (split_store_weight).  Even and odd features apart, added at the end
+  static __device__ __noinline__ void plain(const float* xb, const unsigned char* b, float* es) {
+    const int lane = threadIdx.x & 31;
+    const float* x = xb + lane * KP;
+#pragma unroll 1
+    for (int j = 0; j < H; ++j) {
+      float even = 0.f, odd = 0.f;
+#pragma unroll 1
+      for (int i = 0; i <= D; ++i) {
+        const int k = i == 0 ? D : i - 1;  // the bias first
+        const float* p = reinterpret_cast<const float*>(b + split_b_off(j, k & ~3)) + (k & 3);
+        const float w = p[0] + (p[SPLIT_B_PART / 4] + p[2 * (SPLIT_B_PART / 4)]);
+        if (i == 0) even = w;
+        else if (k & 1) odd = fmaf(x[k], w, odd);
+        else even = fmaf(x[k], w, even);
+      }
+      es[lane * H + j] = even + odd;
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ void load_plain(const float* es, uint64_t (&z)[4][5]) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int n = 0; n < 5; ++n) z[i][n] = lds64(es + (q + 8 * i) * H + 8 * n + 2 * c);
+  }
+
+  // Everything up to dL/dz: h in place of z, dL/dz without W1's factor to es, the lane's rows added to dw (units 8 n + 2 c, + 1).
+  // `valid`, y, dy and pred are those of the lane's own row.
+  // turn(i): called when the tanh of the i-th of a quad's four rows are under way, turn(4) at the end
+  template <class Turn>
+  __device__ __forceinline__ void block(uint64_t (&h)[4][5], const float* w1, const LikParams& lik, float y, bool valid,
+                                        float* es, uint64_t (&dw)[5], float& dy, float& pred, Turn turn) const {
+    float pr[4];
+    {
+      uint64_t w1p[5];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) w1p[n] = lds64(w1 + 8 * n + 2 * c);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint64_t acc = 0ull;
+#pragma unroll
+        for (int n = 0; n < 5; ++n) {
+          h[i][n] = tanh_ref2(h[i][n]);
+          acc = fma2(w1p[n], h[i][n], acc);
+        }
+        float a, b;
+        unpack2(acc, a, b);
+        pr[i] = a + b;
+        turn(i);
+      }
+    }
+    // the quad's four lanes add up; lane c keeps row q + 8 c
+    const bool b1 = (lane & 2) != 0, b0 = (lane & 1) != 0;
+    const float s0 = b1 ? pr[0] : pr[2], s1 = b1 ? pr[1] : pr[3];
+    const float k0 = (b1 ? pr[2] : pr[0]) + __shfl_xor_sync(0xffffffffu, s0, 2);
+    const float k1 = (b1 ? pr[3] : pr[1]) + __shfl_xor_sync(0xffffffffu, s1, 2);
+    const float s = b0 ? k0 : k1;
+    pred = (b0 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, s, 1) + w1[H];
+    dy = valid ? lik_grad(lik, y, pred) : 0.f;
+    // every lane of the quad needs the four dL/dpred
+    float d[4];
+    {
+      const float o1 = __shfl_xor_sync(0xffffffffu, dy, 1);
+      const float a0 = b0 ? o1 : dy, a1 = b0 ? dy : o1;
+      const float c0 = __shfl_xor_sync(0xffffffffu, a0, 2), c1 = __shfl_xor_sync(0xffffffffu, a1, 2);
+      d[0] = b1 ? c0 : a0;
+      d[1] = b1 ? c1 : a1;
+      d[2] = b1 ? a0 : c0;
+      d[3] = b1 ? a1 : c1;
+    }
+    const uint64_t minus1 = pack2(-1.f, -1.f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint64_t d2 = pack2(d[i], d[i]), nd2 = pack2(-d[i], -d[i]);
+      float* p = es + (q + 8 * i) * H + 2 * c;
+#pragma unroll
+      for (int n = 0; n < 5; ++n) {
+        dw[n] = fma2(d2, h[i][n], dw[n]);
+        *reinterpret_cast<uint64_t*>(p + 8 * n) = mul2(fma2(h[i][n], h[i][n], minus1), nd2);  // tanh_t::bwd
+      }
+    }
+    turn(4);
+    __syncwarp();
+  }
+
+  // Sums of dw over the eight quads to out[unit]
+  __device__ __forceinline__ void store_dw1(const uint64_t (&dw)[5], float* out) const {
+    float v[10];
+#pragma unroll
+    for (int n = 0; n < 5; ++n) unpack2(dw[n], v[2 * n], v[2 * n + 1]);
+    const bool q2 = (lane & 16) != 0, q1 = (lane & 8) != 0;
+#pragma unroll
+    for (int n = 0; n < 5; ++n) {  // lanes with bit 4 keep the odd units, the others the even ones
+      const float send = q2 ? v[2 * n] : v[2 * n + 1];
+      v[n] = (q2 ? v[2 * n + 1] : v[2 * n]) + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+    {  // bit 3: n = 3, 4 or n = 0, 1, 2
+      const float s0 = q1 ? v[0] : v[3], s1 = q1 ? v[1] : v[4], s2 = v[2];
+      const float r0 = __shfl_xor_sync(0xffffffffu, s0, 8), r1 = __shfl_xor_sync(0xffffffffu, s1, 8);
+      const float r2 = __shfl_xor_sync(0xffffffffu, s2, 8);
+      v[0] = (q1 ? v[3] : v[0]) + r0;
+      v[1] = (q1 ? v[4] : v[1]) + r1;
+      v[2] = v[2] + r2;
+    }
+#pragma unroll
+    for (int n = 0; n < 3; ++n) v[n] += __shfl_xor_sync(0xffffffffu, v[n], 4);
+    float* o = out + 2 * c + (q2 ? 1 : 0);
+    if ((lane & 4) == 0) {
+      o[q1 ? 24 : 0] = v[0];
+      o[q1 ? 32 : 8] = v[1];
+      if (!q1) o[16] = v[2];
+    }
+  }
+
+  // Sums of acc over the two row subsets, lanes 16 apart: the lower lane keeps features 0 - 5 of its twelve, the upper one 6 - 11.
+  // out: where feature 12 kh + 6 rsub of unit 0 goes, features H apart
+  __device__ __forceinline__ void store_dw0(const uint64_t (*acc)[UPT], float* out) const {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      float o[2][UPT];
+#pragma unroll
+      for (int j = 0; j < UPT; ++j) {
+        const uint64_t send = rsub ? acc[k][j] : acc[k + 3][j], keep = rsub ? acc[k + 3][j] : acc[k][j];
+        unpack2(add2(keep, __shfl_xor_sync(0xffffffffu, send, 16)), o[0][j], o[1][j]);
+      }
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        float* p = out + (2 * k + f) * H;
+        *reinterpret_cast<float4*>(p + 4 * bcg) = make_float4(o[f][0], o[f][1], o[f][2], o[f][3]);
+        p[32 + bcg] = o[f][4];
+      }
+    }
+  }
+
+  // acc[k][u] += features 12 kh + 2 k, + 1 of the rows x dL/dz (feature 22 is the constant 1: db0; 23 is y, unused)
+  template <int UNROLL>
+  __device__ __forceinline__ void backward(const float* xb, const float* es, uint64_t (*acc)[UPT]) const {
+#pragma unroll UNROLL
+    for (int s = 0; s < ROWS / 2; ++s) {
+      const int row = 2 * s + rsub;
+      const float* xr = xb + row * KP + kh * KPT;
+      uint64_t x[KPT / 2];
+#pragma unroll
+      for (int k = 0; k < KPT / 4; ++k) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(xr + 4 * k);
+        x[2 * k] = v.x;
+        x[2 * k + 1] = v.y;
+      }
+      const float4 e4 = *reinterpret_cast<const float4*>(es + row * H + 4 * bcg);
+      const float e[UPT] = {e4.x, e4.y, e4.z, e4.w, es[row * H + 32 + bcg]};
+#pragma unroll
+      for (int u = 0; u < UPT; ++u) {
+        const uint64_t e2 = pack2(e[u], e[u]);
+#pragma unroll
+        for (int k = 0; k < KPT / 2; ++k) acc[k][u] = fma2(x[k], e2, acc[k][u]);
+      }
+    }
+  }
+};
+
+}  // namespace mcmc_b200

@@ -187,8 +187,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   constexpr int STR = (WPM + 7) / 8 * 8;               // a cluster's words start on a line
   constexpr int NR = MULTI ? (WPM * RES_MAX_CLUSTERS + XT - 1) / XT : 1;
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* base =
-      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* base = smem_align1024(smem_raw);
   __shared__ __align__(16) uint4 part_in[C][WPM];           // sums of every rank for the words owned here
   __shared__ __align__(16) uint4 w_in[NWORDS];              // weights
   __shared__ __align__(16) uint4 h_in[2][C * XWARPS + 1];   // {kinetic, log-prior} shares; log-likelihood

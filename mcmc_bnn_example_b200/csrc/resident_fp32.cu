@@ -1,20 +1,28 @@
-// Tile arithmetic of the resident kernel in FP32 mode (resident.cuh has the launch structure, fp32_tile.cuh what a warp
-// does with its 32 rows): every warp owns one 32-row unit for the whole launch.
-// One launch per step took 29.5 us a step for a 58368-row window, this takes 12.5 (2000 steps, one B200); a log density
-// and gradient of 1000 rows from host pointers takes 30 us instead of 64.
-// What bounds a step: no pipe (at 512 rows a CTA the one that serves shared memory is 71 % busy, issue slots 58 %, FMA 52 %).
-// A block takes a scheduler 3,600 cycles, of which its multiplications keep the FMA pipe busy for 2,240: they, the tanh and the
-// multiplications after it overlap as far as the warps of a scheduler are in different phases.  Then the exchange.
+// Tile arithmetic of the resident kernel in FP32 mode (resident.cuh has the launch structure, split_mma.cuh the forward product on
+// the tensor core, fp32_split.cuh what a warp does with its 32 rows behind it): every warp owns one 32-row unit for the
+// whole launch, its rows in three parts in tensor memory and once more, whole, in shared memory for the backward pass.
+// One launch per step took 29.5 us a step for a 58368-row window, this took 12.25 with the forward product on the FMA pipe and
+// takes 9.5 now (one B200); 4096 rows 10.45 and 7.8, 1000 rows 5.2 and 4.4.  What changed, us a step of 58368 rows: the product on
+// the tensor core 9.84, shared memory through its own address space and packed tanh 9.5 to 10.2, sums collected four warps a
+// turn 9.55 to 9.65, the schedulers' warps taking turns at the tanh 9.45 to 9.5.
+// What bounds a step (clock reads, 58368 rows, 18,600 cycles): weights arrive and are cut up 0 - 650; first z 1,450 (18 MMAs);
+// tanh and dL/dz of a scheduler's four warps one after the other, backward passes beside them, until about 11,500; sums
+// to their owners 13,000; then the exchange (resident.cuh), 5,500, of which 3,000 are the trip between clusters.  In the tile
+// the FMA pipe is busy for about half of the time: 480 packed FMAs a warp that issue every third cycle with three
+// different operand pairs, and 160 moves that make pairs of one value.
+// Tried and slower: sums of a scheduler's four warps passed on from one to the next (the chain is serial: 10.1); every feature
+// twice in shared memory, which spares the moves (bank conflicts: 10.3); single FMAs in the backward pass (10.0); the turn at the
+// tanh handed over after the stores of dL/dz (9.66).
 #include <cuda.h>
-#include "fp32_tile.cuh"
+#include "fp32_split.cuh"
 #include "resident.cuh"
 
 namespace mcmc_b200 {
 
 struct ResFp32 {
-  static constexpr int H = 40, D = 22;
+  static constexpr int H = SPLIT_H, D = SPLIT_D;
   using Words = ResWords<H>;
-  using Warp = Fp32Warp<H>;
+  using Warp = SplitWarp;
   static constexpr int NWARPS = RES_NWG * 4;
   static_assert(Warp::ROWS == 32 && NWARPS == RES_UNITS, "a warp owns one 32-row unit");
   // a warp's sums of dW0 and db0, after the shuffle over its two row subsets a lane's 6 features x 5 units: eight
@@ -23,135 +31,184 @@ struct ResFp32 {
   static_assert(4 * GSTR <= Warp::ES, "sums fit where dL/dz was");
   static constexpr int RS = H + 4;   // dW1 and db1 of a warp's rows
   // float offsets
-  static constexpr int XB = 0, ES = XB + RES_UNITS * 32 * KP, WP = ES + NWARPS * Warp::ES, B0 = WP + Warp::WP,
-                       W1 = B0 + H, RW1 = W1 + RS, DYS = RW1 + NWARPS * RS, RLL = DYS + NWARPS * 32,
-                       DUMMY = RLL + NWARPS * 2, BAR = DUMMY + 4;
-  static constexpr size_t SMEM = 1024 + (BAR + 4) * 4;
-  static_assert(WP % 4 == 0 && DYS % 4 == 0 && RLL % 2 == 0 && BAR % 2 == 0, "vector alignment");
+  static constexpr int WB = 0, XB = WB + SPLIT_B_BYTES / 4, ES = XB + RES_UNITS * 32 * KP, W1 = ES + NWARPS * Warp::ES,
+                       RW1 = W1 + RS, RLL = RW1 + NWARPS * RS, DUMMY = RLL + NWARPS * 2, BAR = DUMMY + 4;
+  // barriers: rows landed; per tile, forward done; per accumulator buffer, read
+  static constexpr int NBARS = 1 + RES_NWG + 2;
+  static constexpr size_t SMEM = 1024 + (BAR + 2 * NBARS) * 4;
+  static_assert(XB % 4 == 0 && W1 % 4 == 0 && RW1 % 4 == 0 && RLL % 2 == 0 && BAR % 2 == 0, "vector alignment");
+  // tensor memory: the rows' parts for the whole launch; two accumulator buffers that the four tiles take in turn
+  static constexpr int ZBUF = 2, Z_COL0 = RES_NWG * SPLIT_A_COLS, TMEM_COLS = 512;
+  static_assert(Z_COL0 + ZBUF * SPLIT_Z_COLS <= TMEM_COLS, "tensor memory budget");
 
-  // The four warps of a scheduler get the weights at the same moment.  In step with one another they would all multiply,
-  // then all wait for their tanh (646 cycles of the MUFU pipe each), and so on; so each starts this many cycles after the
-  // one before it, about the multiplications of half a block.  58368 rows, us a step: 12.91 (0), 12.61 (300), 12.46 (500
-  // to 700), 12.57 (1000), 12.69 (1300).  Two to four units to a scheduler, 0 and 600: 1100 rows 7.10, 6.98; 2048 rows 7.61,
-  // 7.43; 3000 rows 9.60, 9.22; 4096 rows 11.75, 11.14; single evaluations 0 to 0.6 less.  A scheduler's first unit never
-  // waits.
-  static constexpr uint32_t TURN = 600;
+  // named barriers: a warp's turn is over (those of the last four are not needed)
+  static constexpr int BAR_LO = 1, BAR_HI = 10;
+  static_assert(BAR_LO + 8 <= RES_BAR_X && BAR_HI > RES_BAR_X && BAR_HI + 4 <= 16, "barrier numbers");
+  __device__ __forceinline__ static int bar_turn(int w) { return w < 8 ? BAR_LO + w : BAR_HI + w - 8; }
 
   Warp lanes;
   float* base;
-  int warp, n_units;
+  int warp, wg, n_units;
   int row0;          // this warp's first row in the window
-  bool active;
-  uint32_t s_dst[3];
+  bool active, plain_x, plain;
+  uint32_t s_dst[3], tmem, par;
+
+  __device__ __forceinline__ uint64_t* bar_rows() const { return reinterpret_cast<uint64_t*>(base + BAR); }
+  __device__ __forceinline__ uint64_t* bar_fwd(int w) const { return bar_rows() + 1 + w; }
+  __device__ __forceinline__ uint64_t* bar_read(int b) const { return bar_rows() + 1 + RES_NWG + b; }
 
   __device__ __forceinline__ ResFp32(unsigned char* b, const ResidentParams& g, int, int u0, int u1)
       : base(reinterpret_cast<float*>(b)) {
     warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    wg = warp >> 2;
     n_units = u1 - u0;
     active = warp < n_units;
     row0 = (u0 + warp) * 32;
+    par = 0;
+    plain_x = plain = false;
     const int t = threadIdx.x;
     for (int q = 0; q < 3; ++q) {
       const int p = Words::param(t, q);
-      float* dst = base + DUMMY;
-      if (t < Words::N - 1 && Words::valid(t, q))
-        dst = base + (p < D * H ? WP + Warp::w_off(p / H, p % H) : p < D * H + H ? B0 + p - D * H : W1 + p - (D * H + H));
-      s_dst[q] = smem_u32(dst);
+      // (threads and places of a word without a parameter write where feature 28 of unit 0 would be: nobody reads there)
+      s_dst[q] = smem_u32(b) + split_b_off(0, 28);
+      if (t >= Words::N - 1 || !Words::valid(t, q)) continue;
+      if (p < D * H + H) s_dst[q] = smem_u32(b) + split_b_off(p % H, p / H & ~3) + (p / H & 3) * 4;
+      else s_dst[q] = smem_u32(base + W1 + p - (D * H + H));
     }
   }
 
   __device__ __forceinline__ bool setup(const CUtensorMap*, const ResidentParams& g, int win) {
+    __shared__ uint32_t tmem_slot;
     bool ok = true;
     const int tid = threadIdx.x;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(base + BAR);
+    if (warp == 0) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                   "r"((uint32_t)TMEM_COLS)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
     if (tid == 0) {
-      mbar_init(bar, 1);
+      mbar_init(bar_rows(), 1);
+      for (int w = 0; w < RES_NWG; ++w) mbar_init(bar_fwd(w), 1);
+      for (int b = 0; b < ZBUF; ++b) mbar_init(bar_read(b), 4);
       mbar_fence_init();
     }
-    // sums that nothing writes stay zero: those of warps without rows
-    for (int i = tid; i < (WP - ES) / 4; i += RES_THREADS)
+    // sums that nothing writes stay zero: those of warps without rows; and what the last MMAs read behind the weights
+    for (int i = tid; i < (W1 - ES) / 4; i += RES_THREADS)
       reinterpret_cast<float4*>(base + ES)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = tid; i < (XB - WB) / 4; i += RES_THREADS)
+      reinterpret_cast<float4*>(base + WB)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int i = tid; i < DUMMY - RW1; i += RES_THREADS) base[RW1 + i] = 0.f;
+    tc_fence_before();
     __syncthreads();
+    tc_fence_after();
+    tmem = tmem_slot;
+    bool wide = false;
     if (n_units > 0) {
       const uint32_t bytes = (uint32_t)n_units * 32 * KP * 4;
       if (tid == 0) {
-        mbar_expect_tx(bar, bytes);
-        bulk_g2s(base + XB, g.xaug + ((size_t)(g.data_window0 + win) * g.rows_pad + row0) * KP, bytes, bar);
+        mbar_expect_tx(bar_rows(), bytes);
+        bulk_g2s(base + XB, g.xaug + ((size_t)(g.data_window0 + win) * g.rows_pad + row0) * KP, bytes, bar_rows());
       }
-      res_wait(bar, 0, g, g.wait_ticks << 2, 611, ok);
-      if (!ok) res_drain(bar, 0, g);
-      if (g.test_code == 611) res_wait(bar, 1, g, g.wait_ticks << 2, 611, ok);  // (nothing ends this phase)
+      res_wait(bar_rows(), 0, g, g.wait_ticks << 2, 611, ok);
+      if (!ok) res_drain(bar_rows(), 0, g);
+      if (g.test_code == 611) res_wait(bar_rows(), 1, g, g.wait_ticks << 2, 611, ok);  // (nothing ends this phase)
+      if (4 * wg < n_units) {  // the tile's rows to tensor memory, zeros for warps without rows
+        const float* x = base + XB + tid * KP;
+        const uint32_t a_t = tmem + wg * SPLIT_A_COLS + ((uint32_t)((warp & 3) * 32) << 16);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          float v[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            v[k] = active && 8 * j + k <= D ? x[8 * j + k] : 0.f;
+            wide |= split_wide(v[k]);
+          }
+          split_store_row(a_t, j, v);
+        }
+        tc_wait_st();
+        tc_fence_before();
+      }
     }
-    __syncthreads();
+    plain_x = __syncthreads_or(wide) != 0;
     return ok;
   }
 
   // word `threadIdx.x` of the weights
   __device__ __forceinline__ void stage(const uint4& v) {
     const uint32_t x[3] = {v.x, v.y, v.z};
+    bool wide = plain_x;
+    if ((int)threadIdx.x < Words::W0) {
 #pragma unroll
-    for (int q = 0; q < 3; ++q) asm volatile("st.shared.b32 [%0], %1;" ::"r"(s_dst[q]), "r"(x[q]) : "memory");
-    __syncthreads();
+      for (int q = 0; q < 3; ++q) wide |= split_store_weight(s_dst[q], __uint_as_float(x[q]));
+    } else {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) asm volatile("st.shared.b32 [%0], %1;" ::"r"(s_dst[q]), "r"(x[q]) : "memory");
+    }
+    fence_proxy_async_smem();
+    plain = __syncthreads_or(wide) != 0;
   }
 
-  __device__ __forceinline__ void step(const ResidentParams& g, float* row_loss, bool last, bool&) {
-    if (!active) return;
-    if (warp >= 4) {  // (a scheduler's first warp waits for nothing: looking at the clock cost it 0.02 to 0.04 us a step)
-      const uint32_t t0 = (uint32_t)clock64();
-      while ((uint32_t)clock64() - t0 < (uint32_t)(warp >> 2) * TURN) {}
+  __device__ __forceinline__ void step(const ResidentParams& g, float* row_loss, bool last, bool& ok) {
+    const int nt = (n_units + 3) / 4;
+    const uint32_t ph = par;
+    par ^= 1;
+    if (warp == NWARPS - 1) {
+      // the MMAs of all tiles, by the warp whose own rows come last; a buffer's second tile when its first has been read
+      const uint32_t on = elect_one(), tm = __shfl_sync(0xffffffffu, tmem, 0);
+      for (int w = 0; w < nt; ++w) {
+        if (w >= ZBUF) res_wait(bar_read(w % ZBUF), ph, g, g.wait_ticks << 2, 613, ok);
+        tc_fence_after();
+        split_issue(tm + Z_COL0 + w % ZBUF * SPLIT_Z_COLS, tm + w * SPLIT_A_COLS, smem_u32(base + WB), on);
+        tc_commit_if(bar_fwd(w), on);
+      }
     }
+    if (!active) return;
     const float* xb = base + XB + warp * 32 * KP;
     float* es = base + ES + warp * Warp::ES;
-    uint64_t dw1[Warp::HPL] = {};
-    float dy = 0.f, loss;
     const int left = g.n_rows - row0;
+    uint64_t h[4][5];
+    res_wait(bar_fwd(wg), ph, g, g.wait_ticks << 2, 612, ok);
+    tc_fence_after();
+    lanes.load(tmem + Z_COL0 + wg % ZBUF * SPLIT_Z_COLS + ((uint32_t)((warp & 3) * 32) << 16), h);
+    tc_fence_before();
+    if (wg + ZBUF < nt) {  // another tile takes the buffer (so this one is full: all its warps come here)
+      __syncwarp();
+      if (lanes.lane == 0) mbar_arrive(bar_read(wg % ZBUF));
+    }
+    if (plain) {
+      Warp::plain(xb, reinterpret_cast<const unsigned char*>(base + WB), es);
+      lanes.load_plain(es, h);
+    }
+    uint64_t dw1[5] = {};
+    float dy, pred;
+    const int own = lanes.own();
+    const bool valid = own < left;
+    const float y = xb[own * KP + COL_Y];
+    // The four warps of a scheduler take turns at the tanh, which MUFU bounds: side by side they would all end it late, and only
+    // then begin to multiply.  4096 rows 8.63 us a step without turns, 7.8 with them; 58368 rows 10.2 and 9.45
+    if (warp >= 4) named_sync(bar_turn(warp - 4), 64);
+    lanes.block(h, base + W1, g.lik, y, valid, es, dw1, dy, pred, [&](int i) {
+      if (i == 3 && warp + 4 < n_units) named_arrive(bar_turn(warp), 64);
+    });
     if (last) {
-      lanes.block<true>(xb, base + WP, base + B0, base + W1, base[W1 + H], g.lik, left, base + DYS + warp * 32, es, dw1,
-                        dy, loss);
-      const int r = lanes.loss_row();
-      if (row_loss && r < left) row_loss[row0 + r] = loss;
+      const float loss = valid ? lik_loss(g.lik, y, pred) : 0.f;
+      store_row_loss(row_loss, row0 + own, loss, valid);
       double ld = (double)loss;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) ld += __shfl_xor_sync(0xffffffffu, ld, o);
       if (lanes.lane == 0) reinterpret_cast<double*>(base + RLL)[warp] = ld;
-    } else {
-      lanes.block<false>(xb, base + WP, base + B0, base + W1, base[W1 + H], g.lik, left, base + DYS + warp * 32, es, dw1,
-                         dy, loss);
     }
-    uint64_t acc[Warp::KPT / 2][Warp::HPL];
-#pragma unroll
-    for (int k = 0; k < Warp::KPT / 2; ++k)
-#pragma unroll
-      for (int j = 0; j < Warp::HPL; ++j) acc[k][j] = 0ull;
-    lanes.backward<2>(xb, es, acc);
-    // dW1 over the four row groups (lane bits 0 and 2), db1 over the rows
     float* rw1 = base + RW1 + warp * RS;
+    lanes.store_dw1(dw1, rw1);
 #pragma unroll
-    for (int j = 0; j < Warp::HPL; ++j) {
-      float a, b;
-      unpack2(dw1[j], a, b);
-      a += b;
-      a += __shfl_xor_sync(0xffffffffu, a, 1);
-      a += __shfl_xor_sync(0xffffffffu, a, 4);
-      if (lanes.rg == 0) rw1[lanes.cg * Warp::HPL + j] = a;
-    }
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) dy += __shfl_xor_sync(0xffffffffu, dy, o);
+    for (int o = 16; o > 0; o >>= 1) dy += __shfl_xor_sync(0xffffffffu, dy, o);
     if (lanes.lane == 0) rw1[H] = dy;
+    uint64_t acc[Warp::KPT / 2][Warp::UPT] = {};
+    lanes.backward<2>(xb, es, acc);
     // dW0: lanes 16 apart have the two row subsets; the lower one keeps features 0 - 5 of the twelve, the upper 6 - 11
     __syncwarp();  // dL/dz has been read by every lane
-    float* gp = es + (2 * lanes.kh + lanes.rsub) * GSTR + lanes.bcg * Warp::HPL;
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int j = 0; j < Warp::HPL; ++j) {
-        float s0, s1, k0, k1;
-        unpack2(lanes.rsub ? acc[k][j] : acc[k + 3][j], s0, s1);
-        unpack2(lanes.rsub ? acc[k + 3][j] : acc[k][j], k0, k1);
-        gp[2 * k * H + j] = k0 + __shfl_xor_sync(0xffffffffu, s0, 16);
-        gp[(2 * k + 1) * H + j] = k1 + __shfl_xor_sync(0xffffffffu, s1, 16);
-      }
+    lanes.store_dw0(acc, es + (2 * lanes.kh + lanes.rsub) * GSTR);
   }
 
   // Words of W0 and b0 go to the threads of the same number; those of W1 and b1 and the log-likelihood to the last warp
@@ -162,15 +219,14 @@ struct ResFp32 {
     return (int)threadIdx.x < Words::W0 ? (int)threadIdx.x : -1;
   }
   __device__ __forceinline__ bool collect(bool last, uint4& v) const {
-    float s[3][2] = {};
+    float s[3] = {};
     if (warp == LAST) {
       const float* r = base + RW1 + 3 * min(lanes.lane, NW1 - 1);
-#pragma unroll
+#pragma unroll 4
       for (int w = 0; w < NWARPS; ++w)
 #pragma unroll
-        for (int q = 0; q < 3; ++q) s[q][w & 1] += r[w * RS + q];
-      v = make_uint4(__float_as_uint(s[0][0] + s[0][1]), __float_as_uint(s[1][0] + s[1][1]),
-                     __float_as_uint(s[2][0] + s[2][1]), 0u);
+        for (int q = 0; q < 3; ++q) s[q] += r[w * RS + q];
+      v = make_uint4(__float_as_uint(s[0]), __float_as_uint(s[1]), __float_as_uint(s[2]), 0u);
       if (last && lanes.lane == NW1) {
         const double* d = reinterpret_cast<const double*>(base + RLL);
         double t[2] = {};
@@ -184,17 +240,30 @@ struct ResFp32 {
     }
     const int t = min((int)threadIdx.x, Words::W0 - 1);
     const float* gp = base + ES + 3 * t + 8 * (3 * t / GROUP);
+    // (four warps to a turn, and no turn for tiles without rows: fetching the straight code for sixteen took 1,100 of a step's cycles)
+#pragma unroll 1
+    for (int w0 = 0; w0 < n_units; w0 += 4) {
 #pragma unroll
-    for (int w = 0; w < NWARPS; ++w)
+      for (int w = 0; w < 4; ++w)
 #pragma unroll
-      for (int q = 0; q < 3; ++q) s[q][w & 1] += gp[w * Warp::ES + q];
+        for (int q = 0; q < 3; ++q) s[q] += gp[w * Warp::ES + q];
+      gp += 4 * Warp::ES;
+    }
     float o[3];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) o[q] = base[W1 + (3 * t + q) % H] * (s[q][0] + s[q][1]);
+    for (int q = 0; q < 3; ++q) o[q] = base[W1 + (3 * t + q) % H] * s[q];
     v = make_uint4(__float_as_uint(o[0]), __float_as_uint(o[1]), __float_as_uint(o[2]), 0u);
     return (int)threadIdx.x < Words::W0;
   }
-  __device__ __forceinline__ void teardown(const ResidentParams&, const volatile int&) {}
+  __device__ __forceinline__ void teardown(const ResidentParams& g, const volatile int& dead) {
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0 && dead)
+      for (int w = 0; 4 * w < n_units; ++w) res_drain(bar_fwd(w), par ^ 1, g);
+    if (warp == 0)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS)
+                   : "memory");
+  }
 };
 
 cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,

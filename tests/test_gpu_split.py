@@ -81,6 +81,39 @@ def test_predictions_of_values_that_cannot_be_split(built, value):
     ctx.close()
 
 
+@pytest.mark.parametrize("streaming", [False, True])
+@pytest.mark.parametrize("value", HARD)
+def test_gradients_of_values_that_cannot_be_split(built, monkeypatch, value, streaming):
+    m, _ = built
+    if streaming:
+        monkeypatch.setenv("MCMC_B200_NO_MULTISTEP", "1")
+    rows = 768   # (whole tiles: a padding row's zeros make NaN of an infinite weight, in every FP32 kernel there has been)
+    rng = np.random.default_rng(4)
+    x = rng.standard_normal((rows, D)).astype(np.float32)
+    y = rng.standard_normal(rows).astype(np.float32)
+    w = (0.2 * rng.standard_normal(D * H + 2 * H + 1)).astype(np.float32)
+    xe, we = x.copy(), w.copy()
+    xe[5, 3], xe[-1, 0] = value, -value
+    we[7] = value
+    ctx = m.Context(m.baseline_config(precision=m.PREC_FP32, sample_capacity=0), 1, rows)
+    for xx, ww in ((xe, w), (x, we)):
+        ctx.set_window_data(0, xx, y)
+        got = ctx.potential_and_grad(0, ww, want_row_loss=True)
+        with np.errstate(all="ignore"):
+            w0, b0, w1, b1 = np.split(ww.astype(np.float64), [D * H, D * H + H, D * H + 2 * H])
+            xd = xx.astype(np.float64)
+            h = np.tanh(xd @ w0.reshape(D, H) + b0)
+            dy = y - (h @ w1 + b1[0])
+            e = dy[:, None] * (1 - h * h) * w1
+            grad = np.concatenate([(xd.T @ e).ravel(), e.sum(0), h.T @ dy, [dy.sum()]]) - ww.astype(np.float64)
+            loss = -0.5 * dy * dy - 0.5 * np.log(2 * np.pi)
+        for g, r in ((got["row_loss"], loss), (got["grad"], grad)):
+            assert np.array_equal(np.isnan(g), np.isnan(r))
+            ok = np.isfinite(r) & (np.abs(r) < 1e30)
+            assert np.abs(g[ok] - r[ok]).max(initial=0) <= 2e-5 * np.abs(r[ok]).max(initial=1)
+    ctx.close()
+
+
 @pytest.mark.parametrize("rows,count", [(1, 149), (512, 1), (513, 3), (1537, 97), (76289, 2), (300000, 1)])
 def test_prediction_tiles_and_their_ranges(built, rows, count):
     """Row tiles of 512 with a row more or less, one tile shared by every CTA, more tiles than CTAs."""
