@@ -304,7 +304,7 @@ int mcmc_b200_log_acpt(mcmc_b200_ctx* ctx, const float* prev_loss, const float* 
  * model: an application that has given all GPU memory to its own arena, or a
  * latency-critical loop where cudaMalloc/cudaFree would synchronise the device
  * and stall every stream.  No context is needed: the scratch (repacked dataset,
- * per-CTA gradient partials) is a fixed ~7.7 MB array inside the library image,
+ * per-CTA gradient partials) is a fixed ~6.9 MB array inside the library image,
  * held by every GPU that loads the library until the process exits.
  *   limits : rows <= 65536, D = 22, H = 40, cfg->precision = FP32 (others are refused)
  *   x [rows][22], y [rows], w [P] : DEVICE pointers (inputs)

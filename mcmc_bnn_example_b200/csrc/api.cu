@@ -147,7 +147,8 @@ struct mcmc_b200_ctx {
   float* xaug = nullptr;
   std::vector<char> window_set;
   CUtensorMap tmaps[2] = {};  // 32-byte-chunk swizzle; 128 units: and 16-byte-chunk swizzle
-  // persistent (TF32) kernel work tables: chain launches and single-window launches
+  // persistent kernels (TF32; FP32 with 40 units) have work tables: chain launches and single-window launches
+  bool table = false;
   int *tab_seg_ptr = nullptr, *tab_nslot = nullptr, *xtab_seg_ptr = nullptr, *xtab_nslot = nullptr;
   int4 *tab_segs = nullptr, *xtab_segs = nullptr;
   int tab_ctas = 0, xtab_ctas = 0;
@@ -334,7 +335,7 @@ static int make_tensor_map(mcmc_b200_ctx* c) {
 // Cuts the flattened (window, tile) list of a launch into one contiguous range per CTA and each
 // range into per-window segments; slot = the segment's index among its window's segments.
 static int build_work_table(mcmc_b200_ctx* c, int windows, long long tiles_per_window, int max_ctas,
-                            int chunks_per_window, int** d_seg_ptr, int4** d_segs, int** d_nslot,
+                            int chunks_per_window, double seg_cost, int** d_seg_ptr, int4** d_segs, int** d_nslot,
                             int* n_ctas, int* max_slots);
 
 static cudaError_t launch_resident(mcmc_b200_ctx* c, int cluster, const ResidentParams& g, cudaStream_t st,
@@ -493,6 +494,14 @@ API int mcmc_b200_plan_resident(int windows, int64_t rows, int num_sms, const in
   return mcmc_b200_plan_resident_for(MCMC_B200_PREC_TF32, windows, rows, num_sms, available, ctas_per_cluster, clusters);
 }
 
+// What a segment costs besides its tiles, in tiles.
+// TF32 (a tile is 0.53 us): 25-window step 0.5135 ms (8) -> 0.5063 (11) -> 0.5035 (14), flat up to 24; 13 windows 0.284 -> 0.282;
+// 50, 100 and 200 windows unchanged within 0.5 %
+// FP32, 40 units (a tile is 1.4 us): 200 windows of 2000 rows 45.1 us a step (3), 46.6 (5, 8, 12); 100 of 10000 rows 89.5, 90.1,
+// 93.4, 97.7; 25 of 58368 rows 123.0 (3, 5), 125.1
+constexpr double TF32_SEG_COST = 14.0, FP32_SEG_COST = 3.0;
+constexpr int FP32_START = 3;  // 128 units, FP32: a CTA
+
 API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows, int64_t rows,
                          mcmc_b200_ctx** out) {
   if (!cfg || !out || n_windows < 1 || rows < 1) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
@@ -534,44 +543,54 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
   c->num_sms = sm_count;
   const bool tf32 = cfg->precision == MCMC_B200_PREC_TF32;
   c->tile_rows = tf32 ? TF32_TILE : fp32_tile_rows(cfg->H);
-  c->ctas_per_sm = tf32 ? 1 : fp32_max_ctas_per_sm(cfg->H);
-  if (c->ctas_per_sm < 1) c->ctas_per_sm = 1;
   const long long n_tiles = c->rows_pad / c->tile_rows;
   c->window_set.assign(n_windows, 0);
   c->h_gwin.assign(n_windows, 0);
   cudaError_t es = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (es != cudaSuccess) { delete c; return fail(MCMC_B200_ERR_CUDA, "cudaStreamCreate failed"); }
-  if (tf32) {
-    // persistent kernel: by default every CTA gets an equal share of the launch's tiles, so where a
+  // FP32 with 40 units: the kernel with the tensor core's product costs 6 us a segment, whatever its rows, and has one CTA to an SM.
+  // For small windows of which there are more than SMs the one without, three CTAs to an SM, is faster: us a step 200 windows
+  // of 50 rows 9.6 (with the tensor core 13.6), 600 of 512 rows 46.0 (50.5), 200 of 700 rows 23.2 (24.2), but 600 of
+  // 700 rows 63.9 (61.2), 600 of 1500 rows 118 (97), 2000 of 1000 rows 219 (228).  So it is where there is a CTA for every tile
+  // and little to do in it (fp32_few_tiles).  Not with fixed `slices`: bits must not depend on the number of windows.
+  const bool small_windows = n_windows > sm_count && n_tiles <= (n_windows > 6 * sm_count ? 8 : 5);
+  c->table = tf32 || (cfg->H == SPLIT_H && (cfg->slices > 0 || !(small_windows || fp32_few_tiles(n_windows * n_tiles))));
+  c->ctas_per_sm = c->table ? 1 : std::max(1, fp32_max_ctas_per_sm(cfg->H));
+  if (c->table) {
+    // persistent kernels: by default every CTA gets an equal share of the launch's tiles, so where a
     // window is cut depends on how many windows share the launch.  cfg.slices > 0 instead cuts every
     // window into that many fixed chunks (whole chunks per CTA): a window's result is then bit-identical
     // wherever and with whatever else it runs, at some cost in load balance.
-    int r_ = build_work_table(c, n_windows, n_tiles, c->num_sms, cfg->slices, &c->tab_seg_ptr, &c->tab_segs,
+    const double cost = tf32 ? TF32_SEG_COST : FP32_SEG_COST;
+    int r_ = build_work_table(c, n_windows, n_tiles, c->num_sms, cfg->slices, cost, &c->tab_seg_ptr, &c->tab_segs,
                               &c->tab_nslot, &c->tab_ctas, &c->slices);
     if (r_ == MCMC_B200_OK)
-      r_ = build_work_table(c, 1, n_tiles, c->num_sms, cfg->slices, &c->xtab_seg_ptr, &c->xtab_segs,
+      r_ = build_work_table(c, 1, n_tiles, c->num_sms, cfg->slices, cost, &c->xtab_seg_ptr, &c->xtab_segs,
                             &c->xtab_nslot, &c->xtab_ctas, &c->slices_x);
     if (r_ != MCMC_B200_OK) { mcmc_b200_destroy(c); return r_; }
   } else {
     const long long capacity = (long long)c->num_sms * c->ctas_per_sm;
-    // the fewest CTAs per window that keep the longest CTA as short as `cap` CTAs would: fewer partial
-    // vectors to sum and fewer per-CTA prologues for the same critical path
-    auto balanced = [&](long long cap) {
-      if (cap < 1) cap = 1;
-      if (cap > n_tiles) cap = n_tiles;
-      if (cap > MAX_SLICES) cap = MAX_SLICES;
-      const long long tiles_per_cta = (n_tiles + cap - 1) / cap;
-      return (n_tiles + tiles_per_cta - 1) / tiles_per_cta;
+    // CTAs per window.  All CTAs of a launch take the same time: what counts is how many rounds of the GPU they make, and how
+    // many tiles the longest CTA of a round has; a CTA's start and end cost FP32_START tiles.  The fewest that come to the
+    // least: partial vectors have to be summed.
+    auto balanced = [&](int windows) {
+      long long best = 0, at = 1;
+      for (long long k = 1; k <= std::min<long long>(n_tiles, MAX_SLICES) && (k == 1 || k * windows <= 4 * capacity); ++k) {
+        const long long cost = (k * windows + capacity - 1) / capacity * ((n_tiles + k - 1) / k + FP32_START);
+        if (k == 1 || cost < best) {
+          best = cost;
+          at = k;
+        }
+      }
+      return at;
     };
-    long long s = cfg->slices > 0 ? cfg->slices : balanced(capacity / n_windows);
-    if (s < 1) s = 1;
+    long long s = cfg->slices > 0 ? cfg->slices : balanced(n_windows);
     if (s > n_tiles) s = n_tiles;
     if (s > MAX_SLICES) s = MAX_SLICES;
     c->slices = (int)s;
-    long long sx = cfg->slices > 0 ? cfg->slices : balanced(capacity);
+    long long sx = cfg->slices > 0 ? cfg->slices : balanced(1);
     if (sx > n_tiles) sx = n_tiles;
     if (sx > MAX_SLICES) sx = MAX_SLICES;
-    if (sx < 1) sx = 1;
     c->slices_x = (int)sx;
   }
 
@@ -646,7 +665,7 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
 
 // Host-only planner of the persistent kernels' work table: which (window, tile range, slot) segments each
 // CTA owns.  Pure arithmetic (no CUDA): also exported for inspection and CPU tests.
-static void plan_work_table(int windows, long long tiles_per_window, int max_ctas, int chunks_per_window,
+static void plan_work_table(int windows, long long tiles_per_window, int max_ctas, int chunks_per_window, double seg_cost,
                             std::vector<int>& seg_ptr, std::vector<int4>& segs, std::vector<int>& nslot) {
   const long long T = (long long)windows * tiles_per_window;
   seg_ptr.clear();
@@ -673,9 +692,6 @@ static void plan_work_table(int windows, long long tiles_per_window, int max_cta
     // read-out, worth about `seg_cost` tiles.  A CTA whose range crosses a window boundary therefore
     // gets fewer tiles than one that stays inside a window.  The smallest per-CTA budget that covers
     // all tiles with at most max_ctas CTAs is found by bisection over a greedy walk.
-    // measured with the current kernel (a tile is 0.53 us): 25-window step 0.5135 (8) -> 0.5063 (11) -> 0.5035 ms
-    // (14), flat up to 24; 13 windows 0.284 -> 0.282; 50, 100 and 200 windows unchanged within 0.5 %
-    const double seg_cost = 14.0;
     const long long tpw = tiles_per_window;
     const long long Gmax = std::max<long long>(1, std::min<long long>(max_ctas, T));
     auto walk = [&](double budget_per_cta, bool emit) -> long long {
@@ -715,11 +731,11 @@ static void plan_work_table(int windows, long long tiles_per_window, int max_cta
 }
 
 static int build_work_table(mcmc_b200_ctx* c, int windows, long long tiles_per_window, int max_ctas,
-                            int chunks_per_window, int** d_seg_ptr, int4** d_segs, int** d_nslot,
+                            int chunks_per_window, double seg_cost, int** d_seg_ptr, int4** d_segs, int** d_nslot,
                             int* n_ctas, int* max_slots) {
   std::vector<int> seg_ptr, nslot;
   std::vector<int4> segs;
-  plan_work_table(windows, tiles_per_window, max_ctas, chunks_per_window, seg_ptr, segs, nslot);
+  plan_work_table(windows, tiles_per_window, max_ctas, chunks_per_window, seg_cost, seg_ptr, segs, nslot);
   const long long G = (long long)seg_ptr.size() - 1;
   int ms = 1;
   for (int w = 0; w < windows; ++w) ms = std::max(ms, nslot[w]);
@@ -742,7 +758,7 @@ API int mcmc_b200_plan_work_table(int windows, int64_t tiles_per_window, int max
     return fail(MCMC_B200_ERR_INVALID, "bad arguments");
   std::vector<int> seg_ptr, nslot;
   std::vector<int4> segs;
-  plan_work_table(windows, tiles_per_window, max_ctas, slices, seg_ptr, segs, nslot);
+  plan_work_table(windows, tiles_per_window, max_ctas, slices, TF32_SEG_COST, seg_ptr, segs, nslot);
   *n_ctas = (int32_t)seg_ptr.size() - 1;
   *n_segs = (int32_t)segs.size();
   if (seg_ptr_out) {
@@ -892,11 +908,13 @@ static int launch_grad(mcmc_b200_ctx* c, GradParams g, bool single, cudaStream_t
   const int slots = single ? c->slices_x : c->slices;
   g.slices_in = slots;
   g.slices_out = slots;
-  if (c->cfg.precision == MCMC_B200_PREC_TF32) {
+  if (c->table) {
     g.nslot_in = single ? c->xtab_nslot : c->tab_nslot;
     g.seg_ptr = single ? c->xtab_seg_ptr : c->tab_seg_ptr;
     g.segs = single ? c->xtab_segs : c->tab_segs;
-    e = launch_grad_tf32(c->cfg.H, c->tmaps, g, single ? c->xtab_ctas : c->tab_ctas, st);
+    const int ctas = single ? c->xtab_ctas : c->tab_ctas;
+    e = c->cfg.precision == MCMC_B200_PREC_TF32 ? launch_grad_tf32(c->cfg.H, c->tmaps, g, ctas, st)
+                                                : launch_grad_fp32_split(g, ctas, st);
   } else {
     e = launch_grad_fp32(c->cfg.H, g, slots, single ? 1 : c->W, st);
   }

@@ -171,6 +171,11 @@ cudaError_t launch_resident_eval_fp32(const void* tmap, const ResidentEvalParams
 // gradient kernels
 cudaError_t launch_grad_fp32(int H, const GradParams& g, int slices, int windows, cudaStream_t st);
 int fp32_max_ctas_per_sm(int H);
+// FP32, 40 units, the forward product on the tensor core: persistent, over the work table in `g`, or one window in `ctas` slices
+cudaError_t launch_grad_fp32_split(const GradParams& g, int ctas, cudaStream_t st);
+// Launches of so few tiles are one latency after the other, of which that kernel has more: us an evaluation of 1000 rows (8 tiles)
+// 15.0 without the tensor core and 16.5 with it, 5000 rows (40) 20.5 and 20.7, 20000 rows 39.3 and 38.9, 58368 rows 65.6 and 45.1
+inline bool fp32_few_tiles(long long tiles) { return tiles <= 32; }
 int fp32_tile_rows(int H);
 
 // TF32 (tcgen05) path: persistent, one CTA per SM; `tmaps` are CUtensorMaps over the repacked dataset: one that stages a

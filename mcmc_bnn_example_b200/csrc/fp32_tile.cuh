@@ -1,7 +1,6 @@
 // FP32 (FFMA) arithmetic of a block of rows, by one warp on its own: forward, output layer, loss, dL/dz through the
-// warp's own shared memory, backward.  The streaming kernel (grad_fp32.cu) and the resident one (resident_fp32.cu) both
-// run it, so that a warp never waits for another: the warps of a scheduler drift apart, and one's tanh pass (MUFU) runs
-// beside another's multiplications.
+// warp's own shared memory, backward.  A warp never waits for another: the warps of a scheduler drift apart, and one's tanh pass
+// (MUFU) runs beside another's multiplications.  For 128 units, and for 40 in large batches of small windows (grad_fp32.cu).
 //
 // Layouts.  What bounds the multiplications is feeding them: a 16-byte load of a whole warp takes four passes over
 // shared memory, but two when lanes i and i ^ 1 (or i and i ^ 2) read the same address, measured; the same address in

@@ -12,7 +12,7 @@
 //
 // The scratch (the repacked copy of the dataset and the per-CTA partial
 // gradient vectors the FP32 gradient kernel writes before they are summed) lives
-// in `g_static_scratch` below: about 7.7 MB that every GPU which loads this
+// in `g_static_scratch` below: about 6.9 MB that every GPU which loads this
 // library holds until the process exits.  Limits that follow from its size:
 // rows <= 65536, D = 22, H = 40, FP32 mode.  Larger requests are refused.
 //
@@ -40,7 +40,7 @@ using namespace mcmc_b200;
 namespace {
 
 constexpr long long STATIC_MAX_ROWS = 65536;
-constexpr int STATIC_MAX_SLOTS = 296;  // 2 CTAs on each of 148 SMs
+constexpr int STATIC_MAX_SLOTS = 148;  // one CTA on each of 148 SMs (fewer tiles than that: one on each of as many)
 constexpr int STATIC_P = 961, STATIC_PP = 964;
 constexpr size_t XAUG_BYTES = (size_t)STATIC_MAX_ROWS * KP * sizeof(float);
 constexpr size_t PARTIAL_BYTES = (size_t)STATIC_MAX_SLOTS * STATIC_PP * sizeof(float);
@@ -109,7 +109,7 @@ extern "C" __attribute__((visibility("default"))) int mcmc_b200_potential_and_gr
   const int tile = fp32_tile_rows(cfg->H);
   const long long rows_pad = (rows + TF32_TILE - 1) / TF32_TILE * TF32_TILE;
   const long long n_tiles = rows_pad / tile;
-  long long slots = 2LL * g_num_sms[dev];
+  long long slots = g_num_sms[dev];  // (one CTA per SM)
   if (slots > STATIC_MAX_SLOTS) slots = STATIC_MAX_SLOTS;
   if (slots > n_tiles) slots = n_tiles;
 
@@ -152,7 +152,7 @@ extern "C" __attribute__((visibility("default"))) int mcmc_b200_potential_and_gr
   g.prior.neg_inv_s2 = (float)(-1.0 / (cfg->prior_scale * cfg->prior_scale));
   g.prior.inv_s = (float)(1.0 / cfg->prior_scale);
   g.prior.norm = (float)(0.5 * log(2.0 * pi) + log(cfg->prior_scale));
-  e = launch_grad_fp32(cfg->H, g, (int)slots, 1, st);
+  e = fp32_few_tiles(n_tiles) ? launch_grad_fp32(cfg->H, g, (int)slots, 1, st) : launch_grad_fp32_split(g, (int)slots, st);
   if (e != cudaSuccess) return fail_static(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
 
   AcceptParams a;

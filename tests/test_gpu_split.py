@@ -127,3 +127,26 @@ def test_prediction_tiles_and_their_ranges(built, rows, count):
     want = sum(_forward(p, x) for p in s) / count
     # a tanh of ex2 / rcp approximations (a few 1e-7) in each unit
     assert np.abs(got - want).max() <= 1e-6 * max(1.0, np.abs(s[:, D * H + H:-1]).sum(axis=1).max())
+
+
+@pytest.mark.parametrize("rows,W", [(128, 150), (385, 151), (513, 300), (1000, 200), (4097, 31)])
+def test_windows_that_share_ctas_are_what_they_are_alone(built, rows, W):
+    """More windows than CTAs (several segments each), windows cut between CTAs, segments of fewer tiles than warpgroups."""
+    m, _ = built
+    data = [m.synth_window(5, g, rows)[:2] for g in range(3)]
+    cfg = m.reference_config(precision=m.PREC_FP32, leapfrog_steps=3, burn_in=0, adapt_steps=0, sample_capacity=2, eps0=1e-3)
+
+    def run(first, last):
+        ctx = m.Context(cfg, last - first, rows)
+        for g in range(first, last):
+            ctx.set_window_data(g - first, *data[g % 3], global_window=g)
+        ctx.run_chain(2)
+        out = {g: ctx.get_samples(g - first) for g in {first, (first + last) // 2, last - 1}}
+        ctx.close()
+        return out
+
+    batch = run(0, W)
+    for g in batch:
+        alone = run(g, g + 1)[g]
+        # six gradients of the same rows with sums in another order, times a step of 1e-3
+        assert np.abs(batch[g] - alone).max() <= 1e-5 * np.abs(alone).max()
