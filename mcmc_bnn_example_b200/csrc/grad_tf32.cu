@@ -131,8 +131,7 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
   constexpr int NCOMPUTE = NWG * 128;
 
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* base =
-      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* base = smem_align1024(smem_raw);
   unsigned char* xb = base;                   // [NWG][NST][128 rows][128 B], TMA-written, 32-byte-chunk swizzle
   unsigned char* es = xb + G::XB_BYTES;       // [NWG][4 atoms][H lines][128 B], E operand, K-major, 16-byte-chunk swizzle
   unsigned char* w0s = es + G::ES_BYTES;      // [NF][128 B] weights, K-major, 16-byte-chunk swizzle
@@ -190,6 +189,7 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TF32_CTRL_REGS));
     // the warpgroup this warp issues for, in a form the compiler can see is the same in every lane
     const int wg = __shfl_sync(0xffffffffu, warp - NWG * 4, 0);
+    const uint32_t on = elect_one();
     uint32_t c_issued = 0;  // tiles of this warpgroup whose MMAs have been issued (mbarrier phases follow it)
     for (int sg = seg0; sg < seg1; ++sg) {
       const int4 seg = g.segs[sg];
@@ -211,13 +211,11 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
         uint32_t stage = 0;  // row stage of tile i of the segment: i % NST, kept as a running counter
         auto issue_fwd = [&]() {
           named_sync(BAR_ROWS0 + wg, 160);
-          if (lane == 0) {
-            tc_fence_after();
+          tc_fence_after();
 #pragma unroll
-            for (int kb = 0; kb < 3; ++kb)
-              tc_mma_tf32_ts(z_t, a_t + kb * 8, umma_desc_advance(wdesc0, kb * 2), IDESC_FWD, kb > 0);
-            tc_commit(&bar_fwd[wg]);
-          }
+          for (int kb = 0; kb < 3; ++kb)
+            tc_mma_tf32_ts_if(z_t, a_t + kb * 8, umma_desc_advance(wdesc0, kb * 2), IDESC_FWD, kb > 0, on);
+          tc_commit_if(&bar_fwd[wg], on);
           __syncwarp();
         };
         if (cnt > 0) issue_fwd();
@@ -394,6 +392,11 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
         float4 sp, sq;
         if (HAS_NEXT) stage_load(sb, 0, sp, sq);
         tc_wait_ld();
+        // The warpgroups take turns at the tanh pass: at it together they were all done after 1,085 cycles instead of one after every
+        // 368, and MUFU then had nothing to do until the next tile.  25 windows of 58368 rows 45.7 us a step without turns,
+        // 44.2 with them, 200 windows 275 and 266; handed over in the middle of the pass the same
+        const int tile = wg + i * NWG;
+        if (tile > 0) named_sync(BAR_TURN0 + (wg + NWG - 1) % NWG, 256);
         // hidden activations, kept as register pairs from here on (packed f32x2 arithmetic).  The tanh pass
         // is bound by the MUFU pipe (one warp instruction per 8 cycles): the staging of the next tile's row
         // (3 x {two loads, eight selects, one tensor-memory store}) is spread over it.
@@ -407,6 +410,7 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
           hp[(j >> 1) + 1] = pack2(tanh_fast(z[j + 2]), tanh_fast(z[j + 3]));
           pred2 = fma2(pack2(wv.x, wv.y), hp[j >> 1], pred2);
           pred2 = fma2(pack2(wv.z, wv.w), hp[(j >> 1) + 1], pred2);
+          if (j == H - 4 && tile + 1 < nt) named_arrive(BAR_TURN0 + wg, 256);
           if (HAS_NEXT) {
             constexpr int STEP = 12;  // hidden units between two staging steps
             if (j % STEP == 4) {

@@ -283,6 +283,10 @@ grad_tf32_wide_kernel(const __grid_constant__ CUtensorMap tmap_mn, const __grid_
         asm volatile("ld.shared.f32 %0, [%1];" : "=f"(y0) : "r"(y_off + st * G::STAGE_BYTES));
         asm volatile("ld.shared.f32 %0, [%1];" : "=f"(y1) : "r"((y_off ^ 32u) + 128u + st * G::STAGE_BYTES));
         tc_wait_ld();
+        // The pipelines take turns at the tanh, which MUFU bounds (512 cycles a tile): 8 windows of 1,048,576 rows 455 us a step without
+        // turns, 428 with them, 25 of 58368 rows 97.1 and 91.4; handed over after half of them the same
+        const int tile = wg + i * NWG;
+        if (tile > 0) named_sync(BAR_TURN0 + (wg + NWG - 1) % NWG, 256);
         // ---- h = tanh(Z), the units' share of the predictions ----
         uint64_t h[4][8], p[8];
 #pragma unroll
@@ -294,6 +298,7 @@ grad_tf32_wide_kernel(const __grid_constant__ CUtensorMap tmap_mn, const __grid_
             p[k] = u == 0 ? mul2(w1d[0], h[0][k]) : fma2(w1d[u], h[u][k], p[k]);
           }
         }
+        if (tile + 1 < nt) named_arrive(BAR_TURN0 + wg, 256);
         halve_pairs<8>(p, (lane & 16) != 0, 16);
         halve_pairs<4>(p, (lane & 8) != 0, 8);
         halve_pairs<2>(p, (lane & 4) != 0, 4);

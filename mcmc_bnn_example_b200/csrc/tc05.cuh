@@ -214,6 +214,7 @@ __device__ __forceinline__ void mbar_wait_q(uint64_t* bar, uint32_t parity, int*
 // (32 waiting threads): a few tens of cycles, no polling.  Ids 1..NWG are the warpgroups' own barriers.
 constexpr int BAR_ROWS0 = 4;   // + wg: rows of a tile are in tensor memory
 constexpr int BAR_E0 = 8;      // + wg: E of a tile is in shared memory
+constexpr int BAR_TURN0 = 12;  // + wg: this warpgroup's turn at the tanh is over
 __device__ __forceinline__ void named_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
