@@ -1070,10 +1070,11 @@ static void fill_chain_accept(mcmc_b200_ctx* c, AcceptParams& a, int mode, int L
   a.tr_eps = c->tr_eps;
 }
 
-// queue one gradient evaluation for all windows (+ the allreduce when sharded)
+// queue one gradient evaluation for all windows (+ the allreduce when sharded); s: step of the trajectory
 static int chain_grad(mcmc_b200_ctx* c, int mode, int s, cudaStream_t st) {
   GradParams g = base_grad_params(c);
   g.mode = mode;
+  g.no_loss = mode != MODE_EVAL && s < c->cfg.leapfrog_steps - 1;
   g.w_in = c->wbuf[s & 1];
   g.m_in = c->mbuf[s & 1];
   g.w_out = c->wbuf[(s + 1) & 1];
@@ -1513,6 +1514,7 @@ static int explicit_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, c
     g.ll_out = c->xllp[s & 1];
     g.eps = nullptr;
     g.eps_scalar = eps;
+    g.no_loss = !last;
     g.row_loss = last ? row_loss : nullptr;
     g.row_loss_stride = 0;
     int r = launch_grad(c, g, true, st);

@@ -66,6 +66,7 @@ struct GradParams {
   const float* eps;         // [windows] or null
   float eps_scalar;
   int mode;
+  int no_loss;              // 1: a step inside a trajectory, whose losses nobody reads (ll_out may be zero, row_loss is null)
   float* row_loss;          // optional [windows][rows_pad]
   long long row_loss_stride;
   LikParams lik;

@@ -30,7 +30,8 @@ struct Fp32Geom {
   static constexpr size_t SMEM = sizeof(float) * (BIG + Warp::WP + 2 * H + 4);
 };
 
-template <int H, int MINB>
+// LOSS: the rows' log-likelihood is wanted (the last step of a trajectory, evaluations)
+template <int H, int MINB, bool LOSS>
 __global__ void __launch_bounds__(Fp32Geom<H>::NT, MINB) grad_fp32_kernel(const GradParams g) {
   using G = Fp32Geom<H>;
   using Warp = Fp32Warp<H>;
@@ -108,8 +109,8 @@ __global__ void __launch_bounds__(Fp32Geom<H>::NT, MINB) grad_fp32_kernel(const 
     const float* xb = xs + (it & 1) * G::XS;
     const int r0 = t * FP32_TILE + warp * Warp::ROWS;
     float loss;
-    lanes.template block<true>(xb, wp, b0, w1, w1[H], g.lik, g.n_rows - r0, dys, es, dw1, db1, loss);
-    if (lanes.loss_first()) {
+    lanes.template block<LOSS>(xb, wp, b0, w1, w1[H], g.lik, g.n_rows - r0, dys, es, dw1, db1, loss);
+    if (LOSS && lanes.loss_first()) {
       llacc += (double)loss;
       const int row = r0 + lanes.loss_row();
       if (g.row_loss && row < g.n_rows) g.row_loss[(long long)win * g.row_loss_stride + row] = loss;
@@ -213,6 +214,7 @@ struct FspGeom {
   static_assert(Z_COL0 + FSP_NWG * SPLIT_Z_COLS <= TMEM_COLS, "tensor memory budget");
 };
 
+template <bool LOSS>
 __global__ void __launch_bounds__(FSP_THREADS, 1) grad_fp32_split_kernel(const GradParams g) {
   using G = FspGeom;
   using Warp = SplitWarp;
@@ -378,9 +380,11 @@ __global__ void __launch_bounds__(FSP_THREADS, 1) grad_fp32_split_kernel(const G
         const float y = xb[own * KP + COL_Y];
         float dy, pred;
         lanes.block(h, w1, g.lik, y, valid, es, dw1, dy, pred, [](int) {});
-        const float loss = valid ? lik_loss(g.lik, y, pred) : 0.f;
-        llacc += (double)loss;
-        store_row_loss(g.row_loss, (long long)win * g.row_loss_stride + row, loss, valid);
+        if (LOSS) {
+          const float loss = valid ? lik_loss(g.lik, y, pred) : 0.f;
+          llacc += (double)loss;
+          store_row_loss(g.row_loss, (long long)win * g.row_loss_stride + row, loss, valid);
+        }
         db1 += dy;
         lanes.backward<16>(xb, es, acc);
         __syncwarp();  // rows and dL/dz have been read: the next copy and the next tile may overwrite them
@@ -442,50 +446,56 @@ __global__ void __launch_bounds__(FSP_THREADS, 1) grad_fp32_split_kernel(const G
 }
 
 // ---- host side -----------------------------------------------------------
-template <int H, int MINB>
+template <int H, int MINB, bool LOSS>
 static cudaError_t fp32_attr() {
-  return cudaFuncSetAttribute(grad_fp32_kernel<H, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(grad_fp32_kernel<H, MINB, LOSS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)Fp32Geom<H>::SMEM);
 }
-template <int H, int MINB>
+template <int H, int MINB, bool LOSS>
 static cudaError_t launch_fp32_t(const GradParams& g, int slices, int windows, cudaStream_t st) {
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !attr_done[dev]) {
-    cudaError_t e = fp32_attr<H, MINB>();
+    cudaError_t e = fp32_attr<H, MINB, LOSS>();
     if (e != cudaSuccess) return e;
     attr_done[dev] = true;
   }
-  return launch_chain_kernel(grad_fp32_kernel<H, MINB>, dim3(slices, windows), dim3(Fp32Geom<H>::NT),
+  return launch_chain_kernel(grad_fp32_kernel<H, MINB, LOSS>, dim3(slices, windows), dim3(Fp32Geom<H>::NT),
                              Fp32Geom<H>::SMEM, st, g);
 }
 
 int fp32_tile_rows(int H) { (void)H; return FP32_TILE; }
 
 cudaError_t launch_grad_fp32(int H, const GradParams& g, int slices, int windows, cudaStream_t st) {
-  if (H == 40) return launch_fp32_t<40, 3>(g, slices, windows, st);
-  if (H == 128) return launch_fp32_t<128, 1>(g, slices, windows, st);
+  if (H == 40) return g.no_loss ? launch_fp32_t<40, 3, false>(g, slices, windows, st) : launch_fp32_t<40, 3, true>(g, slices, windows, st);
+  // (128 units with the losses always: without them 8 windows of 40013 rows took 108 us a step instead of 106.5)
+  if (H == 128) return launch_fp32_t<128, 1, true>(g, slices, windows, st);
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_grad_fp32_split(const GradParams& g, int ctas, cudaStream_t st) {
+template <bool LOSS>
+static cudaError_t launch_split_t(const GradParams& g, int ctas, cudaStream_t st) {
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !attr_done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(grad_fp32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FspGeom::SMEM);
+    cudaError_t e =
+        cudaFuncSetAttribute(grad_fp32_split_kernel<LOSS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FspGeom::SMEM);
     if (e != cudaSuccess) return e;
     if (dev < 64) attr_done[dev] = true;
   }
-  return launch_chain_kernel(grad_fp32_split_kernel, dim3(ctas), dim3(FSP_THREADS), FspGeom::SMEM, st, g);
+  return launch_chain_kernel(grad_fp32_split_kernel<LOSS>, dim3(ctas), dim3(FSP_THREADS), FspGeom::SMEM, st, g);
+}
+cudaError_t launch_grad_fp32_split(const GradParams& g, int ctas, cudaStream_t st) {
+  return g.no_loss ? launch_split_t<false>(g, ctas, st) : launch_split_t<true>(g, ctas, st);
 }
 
 template <int H, int MINB>
 static int fp32_ctas_per_sm() {
   int n = 0;
-  fp32_attr<H, MINB>();
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, grad_fp32_kernel<H, MINB>, Fp32Geom<H>::NT, Fp32Geom<H>::SMEM);
+  fp32_attr<H, MINB, true>();
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, grad_fp32_kernel<H, MINB, true>, Fp32Geom<H>::NT, Fp32Geom<H>::SMEM);
   return n;
 }
 int fp32_max_ctas_per_sm(int H) { return H == 40 ? fp32_ctas_per_sm<40, 3>() : H == 128 ? fp32_ctas_per_sm<128, 1>() : 0; }

@@ -121,7 +121,9 @@ __device__ __forceinline__ void store_e_pairs(const uint32_t* e_ptr, const uint6
   (store_e_pair<Js>(e_ptr, hp, dy2, ndy2, dw1p), ...);
 }
 
-template <int H>
+// LOSS: the rows' log-likelihood is wanted (the last step of a trajectory, evaluations).  In every step the losses cost 25 windows of 58368
+// rows 2.2 us of 41.6, 200 windows 18 of 258
+template <int H, bool LOSS>
 __global__ void __launch_bounds__(TF32_THREADS, 1)
 grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g) {
   using G = Tf32Geom<H>;
@@ -428,11 +430,7 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
         const bool b_done = n > 0 ? mbar_try_wait(&bar_bwd[wg], (n - 1) & 1) : true;
         const int grow = t * TF32_TILE + row_in_tile;
         const bool valid = grow < g.n_rows;
-        float loss, dy;
-        lik_terms(g.lik, y, pred, loss, dy);
-        if (!valid) { loss = 0.f; dy = 0.f; }
-        llacc += (double)loss;
-        store_row_loss(g.row_loss, (long long)win * g.row_loss_stride + grow, loss, valid);
+        const float dy = valid ? lik_grad(g.lik, y, pred) : 0.f;
         db1 += dy;
         if (!b_done) ok = mbar_wait_slow(&bar_bwd[wg], (n - 1) & 1, g.status, 203, ok);
         {
@@ -440,7 +438,13 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
           // applied once per segment at read-out): three packed operations per pair of hidden units, each
           // pair stored as soon as it is ready so that the stores spread over the arithmetic
           const uint64_t dy2 = pack2(dy, dy), ndy2 = pack2(-dy, -dy);
+          // (the loss beside them: before them it was a chain of its own, 25 windows of 58368 rows 42.4 us a step instead of 41.6)
+          const float loss = LOSS && valid ? lik_loss(g.lik, y, pred) : 0.f;
           store_e_pairs(e_ptr, hp, dy2, ndy2, dw1p, std::make_integer_sequence<int, H / 2>{});
+          if (LOSS) {
+            llacc += (double)loss;
+            store_row_loss(g.row_loss, (long long)win * g.row_loss_stride + grow, loss, valid);
+          }
         }
         fence_proxy_async_smem();
         named_arrive(BAR_E0 + wg, 160);
@@ -568,24 +572,24 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
 // ---- host side -----------------------------------------------------------
 int tf32_supported(int H) { return H == 40 || H == 128; }
 
-template <int H>
+template <int H, bool LOSS>
 static cudaError_t launch_tf32_t(const void* tmap_mn, const GradParams& g, int ctas, cudaStream_t st) {
   using G = Tf32Geom<H>;
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !attr_done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(grad_tf32_kernel<H>,
+    cudaError_t e = cudaFuncSetAttribute(grad_tf32_kernel<H, LOSS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM);
     if (e != cudaSuccess) return e;
     attr_done[dev] = true;
   }
-  return launch_chain_kernel(grad_tf32_kernel<H>, dim3(ctas), dim3(TF32_THREADS), G::SMEM, st,
+  return launch_chain_kernel(grad_tf32_kernel<H, LOSS>, dim3(ctas), dim3(TF32_THREADS), G::SMEM, st,
                              *reinterpret_cast<const CUtensorMap*>(tmap_mn), g);
 }
 
 cudaError_t launch_grad_tf32(int H, const void* tmaps, const GradParams& g, int ctas, cudaStream_t st) {
-  if (H == 40) return launch_tf32_t<40>(tmaps, g, ctas, st);
+  if (H == 40) return g.no_loss ? launch_tf32_t<40, false>(tmaps, g, ctas, st) : launch_tf32_t<40, true>(tmaps, g, ctas, st);
   if (H == 128) return launch_grad_tf32_wide(tmaps, g, ctas, st);  // grad_tf32_wide.cu
   return cudaErrorInvalidValue;
 }
