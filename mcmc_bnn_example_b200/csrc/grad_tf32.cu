@@ -302,18 +302,24 @@ grad_tf32_kernel(const __grid_constant__ CUtensorMap tmap_mn, const GradParams g
         }
       }
       // element (n = hidden unit, k) of the K-major B operand at n*128 + ((k/4) ^ (n%8))*16 + (k%4)*4
-      // (one after the other: all three of a thread's at once cost a register spilled in the tile loop.  20 iterations of 200
-      // windows of 58368 rows 67.3 ms, all at once 68.2; of 2000 rows, where the prologue counts for more, 5.1 and 4.6)
-      for (int p = tid; p < G::P; p += NCOMPUTE) {
-        float w[1];
-        leapfrog_params(g, win, p, NCOMPUTE, G::P, slot == 0, w);
-        if (p < D * H + H) {
-          const int k = p / H, n = p - k * H;
-          *reinterpret_cast<float*>(w0s + n * 128 + (((k >> 2) ^ (n & 7)) << 4) + ((k & 3) << 2)) = w[0];
-        } else if (p < D * H + 2 * H) {
-          w1s[p - (D * H + H)] = w[0];
-        } else {
-          b1s = w[0];
+      // (two of a thread's three at a time, so that their loads are under way together: 200 windows of 2000 rows, where the prologue
+      // counts for most, 21.5 us a step one by one and 19.2 so, 100 of 10000 33.5 and 31.4, 25 of 58368 39.3 and 39.0.  All three
+      // at once spill a register in the tile loop, and the loop unrolled takes 20.2 and 32.3)
+#pragma unroll 1
+      for (int p0 = tid; p0 < G::P; p0 += 2 * NCOMPUTE) {
+        float w[2];
+        leapfrog_params(g, win, p0, NCOMPUTE, G::P, slot == 0, w);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int p = p0 + i * NCOMPUTE;
+          if (p < D * H + H) {
+            const int k = p / H, n = p - k * H;
+            *reinterpret_cast<float*>(w0s + n * 128 + (((k >> 2) ^ (n & 7)) << 4) + ((k & 3) << 2)) = w[i];
+          } else if (p < D * H + 2 * H) {
+            w1s[p - (D * H + H)] = w[i];
+          } else if (p < G::P) {
+            b1s = w[i];
+          }
         }
       }
       fence_proxy_async_smem();
