@@ -1718,7 +1718,7 @@ API int mcmc_b200_predict_mean(mcmc_b200_ctx* c, int window, const float* xs, in
       !c->samples || first + count > c->cfg.sample_capacity)
     return fail(MCMC_B200_ERR_INVALID, "bad arguments or no sample storage");
   CK(cudaSetDevice(c->device));
-  const bool split = c->cfg.H == SPLIT_H;
+  const int H = c->cfg.H;
   const size_t D = c->cfg.D;
   ForwardParams a;
   memset(&a, 0, sizeof a);
@@ -1734,27 +1734,24 @@ API int mcmc_b200_predict_mean(mcmc_b200_ctx* c, int window, const float* xs, in
   // The rows come from pageable memory, through the driver's buffers, at 17 GB/s while the caller waits: 0.3 ms for 58368 of them,
   // as long as the pass over 230 samples.  So a block is copied beside the pass over the one before it; a first short one,
   // since nothing runs beside its copy.  800 samples 1.14 ms a call, in one block 1.37; 20 samples 0.36 either way.
-  const bool blocks = split && n >= 16 * FWS_ROWS && count >= 16;
+  const int64_t tile = forward_rows(H);
+  const bool blocks = n >= 16 * tile && count >= 16;
   int64_t cut[4] = {0, n, n, n};
   if (blocks) {
-    cut[1] = n / 8 / FWS_ROWS * FWS_ROWS;
-    cut[2] = n / 2 / FWS_ROWS * FWS_ROWS;
+    cut[1] = n / 8 / tile * tile;
+    cut[2] = n / 2 / tile * tile;
     r = copy_stream(c);
     if (r) return r;
   }
   auto rows = [&](int k) { return cut[k + 1] - cut[k]; };
-  // 128 units: a chunk's sums are 8 bytes a row beside the row's own 92: at most five chunks or 64 MB (5,000 samples of 10 M
-  // rows would take eight for less than one per cent), and one where there is no memory for more
-  const int most = (int)std::max<int64_t>(5, std::min<int64_t>(FWD_MAX_CHUNKS, (64 << 20) / (8 * n)));
-  int chunks = split ? 0 : forward_chunks(c->num_sms, n, count, most);
-  size_t sums = (size_t)chunks * n;
-  for (int k = 0; split && k < 3 && rows(k) > 0; ++k) {
+  size_t sums = 0;  // a row's sums from several CTAs, or one where there is no memory for more
+  for (int k = 0; k < 3 && rows(k) > 0; ++k) {
     a.n = rows(k);
-    sums = std::max<size_t>(sums, (size_t)forward_split_slots(c->num_sms, a) * a.n);
+    sums = std::max<size_t>(sums, (size_t)forward_slots(H, c->num_sms, a) * a.n);
   }
   r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, sums);
   if (r == MCMC_B200_ERR_NOMEM && sums > (size_t)n) {
-    chunks = a.whole = 1;
+    a.whole = 1;
     r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)n);
   }
   if (r) return r;
@@ -1769,11 +1766,8 @@ API int mcmc_b200_predict_mean(mcmc_b200_ctx* c, int window, const float* xs, in
       CK(cudaEventRecord(c->copy_events[k], copies));
       CK(cudaStreamWaitEvent(c->stream, c->copy_events[k], 0));
     }
-    cudaError_t e = split ? launch_forward_split(a, c->num_sms, false, c->stream)
-                          : launch_forward_samples(c->cfg.H, a, chunks, false, c->stream);
-    if (e == cudaSuccess)
-      e = split ? launch_forward_split_finish(a, c->num_sms, sum, c->stream)
-                : launch_forward_finish_predict(c->fwd_partial, chunks, n, count, sum, c->stream);
+    cudaError_t e = launch_forward(H, a, c->num_sms, false, c->stream);
+    if (e == cudaSuccess) e = launch_forward_finish_predict(H, a, c->num_sms, sum, c->stream);
     c->launches += 2;
     if (e == cudaSuccess && blocks) e = cudaEventRecord(c->copy_events[k], c->stream);
     if (e != cudaSuccess) return fail(MCMC_B200_ERR_CUDA, cudaGetErrorString(e));
@@ -1794,8 +1788,7 @@ API int mcmc_b200_final_loss(mcmc_b200_ctx* c, int window, int first, int count,
   if (!c->window_set[window]) return fail(MCMC_B200_ERR_INVALID, "window has no data yet");
   CK(cudaSetDevice(c->device));
   // all samples against the window's rows in one launch (FP32 forward pass, no gradient)
-  const int tiles = forward_row_tiles(c->cfg.H, c->rows);
-  const int chunks = forward_chunks(c->num_sms, c->rows, count, FWD_MAX_CHUNKS);
+  const int tiles = (int)forward_tiles(c->cfg.H, c->rows);
   int r = fwd_reserve(c, &c->fwd_partial, &c->fwd_partial_cap, (size_t)tiles * count + 2 * (size_t)count);
   if (r) return r;
   const float* xw = c->xaug + (size_t)window * c->rows_pad * KP;
@@ -1814,8 +1807,7 @@ API int mcmc_b200_final_loss(mcmc_b200_ctx* c, int window, int first, int count,
   double* d_ll = c->fwd_partial + (size_t)tiles * count;
   double* d_lp = d_ll + count;
   a.status = &c->hb->fwd_status;
-  cudaError_t e = c->cfg.H == SPLIT_H ? launch_forward_split(a, c->num_sms, true, c->stream)
-                                      : launch_forward_samples(c->cfg.H, a, chunks, true, c->stream);
+  cudaError_t e = launch_forward(c->cfg.H, a, c->num_sms, true, c->stream);
   if (e == cudaSuccess)
     e = launch_forward_finish_loss(c->fwd_partial, tiles, count, smp, c->P, make_prior(c->cfg), d_ll, d_lp, c->stream);
   c->launches += 2;

@@ -95,23 +95,17 @@ struct ForwardParams {
   const float* samples;    // [count][P]
   int count;
   LikParams lik;
-  double* partial;         // PREDICT: [chunks][n]   LOSS: [row tiles][count]
-  int whole;               // 40 units: every CTA takes whole row tiles, so that a row has one sum
-  int* status;             // 40 units: where a bounded wait that runs out leaves its code
+  double* partial;         // PREDICT: [forward_slots][n]   LOSS: [row tiles][count]
+  int whole;               // every CTA takes whole row tiles, so that a row has one sum
+  int* status;             // where a bounded wait that runs out leaves its code
 };
-// 40 units (SPLIT_H): four 128-row tiles to a CTA (forward_split_kernel)
-constexpr int SPLIT_H = 40;
-constexpr int FWS_ROWS = 512;
-__host__ __device__ inline long long forward_split_tiles(long long n) { return (n + FWS_ROWS - 1) / FWS_ROWS; }
-int forward_split_slots(int num_sms, const ForwardParams& a);
-cudaError_t launch_forward_split(const ForwardParams& a, int num_sms, bool loss, cudaStream_t st);
-cudaError_t launch_forward_split_finish(const ForwardParams& a, int num_sms, float* out, cudaStream_t st);
-int forward_row_tiles(int H, long long n);
-constexpr int FWD_MAX_CHUNKS = 64;
-int forward_chunks(int num_sms, long long n, int count, int most);
-cudaError_t launch_forward_samples(int H, const ForwardParams& a, int chunks, bool loss, cudaStream_t st);
-cudaError_t launch_forward_finish_predict(const double* partial, int chunks, long long n, int count, float* out,
-                                          cudaStream_t st);
+constexpr int SPLIT_H = 40;  // units of the gradient kernels with split_mma.cuh
+// rows of a CTA's tile: four or three 128-row tiles (forward.cu)
+__host__ __device__ constexpr int forward_rows(int H) { return H == 40 ? 512 : 384; }
+__host__ __device__ inline long long forward_tiles(int H, long long n) { return (n + forward_rows(H) - 1) / forward_rows(H); }
+int forward_slots(int H, int num_sms, const ForwardParams& a);
+cudaError_t launch_forward(int H, const ForwardParams& a, int num_sms, bool loss, cudaStream_t st);
+cudaError_t launch_forward_finish_predict(int H, const ForwardParams& a, int num_sms, float* out, cudaStream_t st);
 cudaError_t launch_forward_finish_loss(const double* partial, int tiles, int count, const float* samples, int P,
                                        const PriorParams& prior, double* out_ll, double* out_lp, cudaStream_t st);
 cudaError_t launch_philox_probe(const uint32_t ctr[4], const uint32_t key[2], int n, uint32_t* raw, float* normals,

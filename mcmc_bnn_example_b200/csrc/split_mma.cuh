@@ -80,18 +80,22 @@ __device__ __forceinline__ void split_store_row(uint32_t a_t, int j, const float
            make_float4(p[q][4], p[q][5], p[q][6], p[q][7]));
 }
 
-// The 18 MMAs of a 128-row tile, by a converged warp (`on` in one lane): smallest products first.
-__device__ __forceinline__ void split_issue(uint32_t z_t, uint32_t a_t, uint32_t b_smem, uint32_t on) {
-  constexpr uint32_t IDESC = umma_idesc_tf32(128, 48, 0, 0);
+// The 18 MMAs of a 128-row tile, by a converged warp (`on` in one lane): smallest products first.  N units' lines of every part,
+// PART bytes apart; S1 at column 0, S0 at column S0
+template <int N, int S0, int PART>
+__device__ __forceinline__ void split_issue_n(uint32_t z_t, uint32_t a_t, uint32_t b_smem, uint32_t on) {
+  constexpr uint32_t IDESC = umma_idesc_tf32(128, N, 0, 0);
   const uint64_t b0 = umma_desc_k128(b_smem);
   constexpr int XP[6] = {2, 0, 1, 1, 0, 0}, WP[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
   for (int q = 0; q < 6; ++q)
 #pragma unroll
     for (int kb = 0; kb < 3; ++kb)
-      tc_mma_tf32_ts_if(z_t + (q == 5 ? SPLIT_S0 : 0), a_t + XP[q] * SPLIT_K + kb * 8,
-                        umma_desc_advance(b0, WP[q] * (SPLIT_B_PART >> 4) + kb * 2), IDESC,
-                        (q % 5 > 0 || kb > 0) ? 1u : 0u, on);
+      tc_mma_tf32_ts_if(z_t + (q == 5 ? S0 : 0), a_t + XP[q] * SPLIT_K + kb * 8,
+                        umma_desc_advance(b0, WP[q] * (PART >> 4) + kb * 2), IDESC, (q % 5 > 0 || kb > 0) ? 1u : 0u, on);
+}
+__device__ __forceinline__ void split_issue(uint32_t z_t, uint32_t a_t, uint32_t b_smem, uint32_t on) {
+  split_issue_n<48, SPLIT_S0, SPLIT_B_PART>(z_t, a_t, b_smem, on);
 }
 
 }  // namespace mcmc_b200

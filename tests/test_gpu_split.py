@@ -17,14 +17,14 @@ def _with_samples(ctx, samples):
     ctx.restore(bytes(blob))
 
 
-def _sampler(m, count):
-    ctx = m.Context(m.baseline_config(precision=m.PREC_FP32, leapfrog_steps=3, sample_capacity=count), 1, 128)
-    ctx.set_window_data(0, *m.synth_window(1, 0, 128)[:2])
+def _sampler(m, count, H=H):
+    ctx = m.Context(m.baseline_config(H=H, precision=m.PREC_FP32, leapfrog_steps=3, sample_capacity=count), 1, 128)
+    ctx.set_window_data(0, *m.synth_window(1, 0, 128, H=H)[:2])
     ctx.run_chain(count)
     return ctx
 
 
-def _forward(p, x):
+def _forward(p, x, H=H):
     w0, b0, w1, b1 = np.split(np.asarray(p, np.float64), [D * H, D * H + H, D * H + 2 * H])
     return np.tanh(x.astype(np.float64) @ w0.reshape(D, H) + b0) @ w1 + b1[0]
 
@@ -60,10 +60,11 @@ def test_product_has_the_error_of_an_fp32_sum(built, unit, scaled):
 HARD = [np.inf, -np.inf, np.nan, 3e38, 2.0 ** 60, 2.0 ** 59, -1e-40]
 
 
+@pytest.mark.parametrize("H", [40, 128])
 @pytest.mark.parametrize("value", HARD)
-def test_predictions_of_values_that_cannot_be_split(built, value):
+def test_predictions_of_values_that_cannot_be_split(built, value, H):
     m, _ = built
-    ctx = _sampler(m, 3)
+    ctx = _sampler(m, 3, H)
     rng = np.random.default_rng(3)
     s = (0.2 * rng.standard_normal((3, ctx.P))).astype(np.float32)
     x = rng.standard_normal((700, D)).astype(np.float32)
@@ -71,7 +72,7 @@ def test_predictions_of_values_that_cannot_be_split(built, value):
     xe[5, 3], xe[-1, 0] = value, -value
     se[1, 7], se[2, D * H + 3] = value, -value
     with np.errstate(all="ignore"):
-        want = [np.mean([_forward(p, xx) for p in ss], axis=0) for ss, xx in ((s, xe), (se, x))]
+        want = [np.mean([_forward(p, xx, H) for p in ss], axis=0) for ss, xx in ((s, xe), (se, x))]
     for ss, xx, ref in zip((s, se), (xe, x), want):
         _with_samples(ctx, ss)
         got = ctx.predict_mean(0, xx)
@@ -114,17 +115,18 @@ def test_gradients_of_values_that_cannot_be_split(built, monkeypatch, value, str
     ctx.close()
 
 
-@pytest.mark.parametrize("rows,count", [(1, 149), (512, 1), (513, 3), (1537, 97), (76289, 2), (300000, 1)])
-def test_prediction_tiles_and_their_ranges(built, rows, count):
-    """Row tiles of 512 with a row more or less, one tile shared by every CTA, more tiles than CTAs."""
+@pytest.mark.parametrize("H,rows,count", [(40, 1, 149), (40, 512, 1), (40, 513, 3), (40, 1537, 97), (40, 76289, 2), (40, 300000, 1),
+                                          (128, 1, 149), (128, 384, 1), (128, 385, 4), (128, 1153, 97), (128, 57217, 2), (128, 200000, 1)])
+def test_prediction_tiles_and_their_ranges(built, H, rows, count):
+    """Row tiles of 512 (128 units: 384) with a row more or less, one tile shared by every CTA, more tiles than CTAs."""
     m, _ = built
-    ctx = _sampler(m, count)
+    ctx = _sampler(m, count, H)
     s = (0.2 * np.random.default_rng(rows).standard_normal((count, ctx.P))).astype(np.float32)
     _with_samples(ctx, s)
     x = np.random.default_rng(count).standard_normal((rows, D)).astype(np.float32)
     got = ctx.predict_mean(0, x)
     ctx.close()
-    want = sum(_forward(p, x) for p in s) / count
+    want = sum(_forward(p, x, H) for p in s) / count
     # a tanh of ex2 / rcp approximations (a few 1e-7) in each unit
     assert np.abs(got - want).max() <= 1e-6 * max(1.0, np.abs(s[:, D * H + H:-1]).sum(axis=1).max())
 
