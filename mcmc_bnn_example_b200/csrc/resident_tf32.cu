@@ -8,7 +8,9 @@
 //     last, the backward MMAs by one of the first warpgroup, which is done first (or by a warp without rows);
 //   * the warpgroups take turns at the tanh pass (MUFU bound, about 330 cycles for a warpgroup alone): in step with one
 //     another all of them would finish it at the end of its 1,300 cycles, and the E stores and backward MMAs of the
-//     first ones, 640 and 1,150 cycles for four tiles, would start only then;
+//     first ones, 640 and 1,150 cycles for four tiles, would start only then.  A turn is handed over half way, where the
+//     CTA has four tiles at its end (us a step, half way and at the end: 4096 rows 3.84 and 3.77, 58368 5.69 and 5.64; always
+//     at the three-quarter mark, fewer tiles: 2000 rows 2.95 and 3.02, 30011 4.79 and 4.85);
 //   * Z is read in the 16-lane quad shape: a thread holds 10 hidden units of 4 rows.  A row's output sum then takes
 //     two shuffle levels inside the quad, but dW1 is 10 sums of 4 rows in registers instead of 40 sums of one: 10
 //     shuffles instead of 45 per step (the shuffles were 1,800 of the step's cycles, the longest single item).
@@ -45,7 +47,7 @@ struct ResTf32 {
   bool tile_active, warp_active, next_active, valid;
   uint32_t tmem, par;
   float y;
-  uint32_t e_off[4], s_dst[3], s_neg[3];
+  uint32_t e_off, s_dst[3], s_neg[3];
   int row0;
 
   __device__ __forceinline__ uint64_t* bar(int w, int k) const {
@@ -74,9 +76,10 @@ struct ResTf32 {
     // E element (hidden j, row r): atom r / 32 (this warp), line j, 16-byte chunk (r % 32) / 4 ^ (j % 8).  This thread
     // stores rows q + 8 i and units 8 n + 2 c + e: chunk (q / 4 + 2 i) ^ (2 c + e), all 32 banks once per store
     const int q = lane >> 2, cc = lane & 3;
-    for (int i = 0; i < 4; ++i)
-      e_off[i] = smem_u32(base + ES + wg * ES_WG_BYTES + (warp & 3) * ES_ATOM_BYTES) + 2 * cc * 128 +
-                 ((((q >> 2) + 2 * i) ^ (2 * cc)) << 4) + ((q & 3) << 2);
+    // = (q / 4 ^ 2 c + e) ^ 2 i.  (One register instead of four: without it shared memory in its own address space made steps of 5000
+    // to 30011 rows 1 % slower than through generic addresses; 7219 rows x 3 4.10 us generic, 4.16, 4.08 now)
+    e_off = smem_u32(base + ES + wg * ES_WG_BYTES + (warp & 3) * ES_ATOM_BYTES) + 2 * cc * 128 + (((q >> 2) ^ (2 * cc)) << 4) +
+            ((q & 3) << 2);
     stage_setup();
   }
 
@@ -218,7 +221,7 @@ struct ResTf32 {
           unpack2(acc, lo, hi);
           pr[i] = lo + hi;
         }
-        if (hf == 0 && next_active) named_arrive(RES_BAR_T + wg + 1, 256);
+        if (next_active && hf == (nt == RES_NWG ? 1 : 0)) named_arrive(RES_BAR_T + wg + 1, 256);
       }
       // the quad's four lanes add up; lane c keeps row q + 8c
       const bool b1 = (lane & 2) != 0, b0 = (lane & 1) != 0;
@@ -253,11 +256,12 @@ struct ResTf32 {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const uint64_t dy2 = pack2(dy[i], dy[i]), ndy2 = pack2(-dy[i], -dy[i]);
-        store_e<0>(e_off[i], hp[i], dy2, ndy2, dw);
-        store_e<1>(e_off[i], hp[i], dy2, ndy2, dw);
-        store_e<2>(e_off[i], hp[i], dy2, ndy2, dw);
-        store_e<3>(e_off[i], hp[i], dy2, ndy2, dw);
-        store_e<4>(e_off[i], hp[i], dy2, ndy2, dw);
+        const uint32_t off = e_off ^ (i << 5);
+        store_e<0>(off, hp[i], dy2, ndy2, dw);
+        store_e<1>(off, hp[i], dy2, ndy2, dw);
+        store_e<2>(off, hp[i], dy2, ndy2, dw);
+        store_e<3>(off, hp[i], dy2, ndy2, dw);
+        store_e<4>(off, hp[i], dy2, ndy2, dw);
       }
       fence_proxy_async_smem();
       tc_fence_before();
