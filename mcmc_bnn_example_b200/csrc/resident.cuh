@@ -108,13 +108,19 @@ static __device__ __noinline__ void res_timeout(const ResidentParams& g, int cod
   if (g.status_host) *reinterpret_cast<volatile int*>(g.status_host) = code;
 }
 __device__ __forceinline__ uint32_t res_ticks() { return (uint32_t)(clock64() >> 16); }  // of 33 us at 1.965 GHz
-// mbarrier wait of the resident kernel: a bounded spin in line (each try_wait sleeps in hardware for a moment)
-__device__ __forceinline__ void res_wait(uint64_t* bar, uint32_t parity, const ResidentParams& g, uint32_t limit, int code,
+// mbarrier wait of the resident kernel: a bounded spin in line (each try_wait sleeps in hardware for a moment).  What ran out is noted
+// and reported at the kernel's end: calls in line would lengthen a step's code, which should stay in the instruction cache (32 KB: straight
+// code of 48 KB takes 2.7 cycles an instruction, of 32 KB 1.2).  The loop out of line is no way: the call costs registers, 0.3 to 0.6 us a step
+static __shared__ int res_code;
+__device__ __forceinline__ void res_wait(uint64_t* bar, uint32_t parity, const ResidentParams&, uint32_t limit, int code,
                                          bool& ok) {
   if (mbar_try_wait(bar, parity)) return;
   const uint32_t t0 = res_ticks();
   while (ok && !mbar_try_wait(bar, parity))
-    if (res_ticks() - t0 > limit) { ok = false; res_timeout(g, code); }
+    if (res_ticks() - t0 > limit) {
+      ok = false;
+      res_code = code;
+    }
 }
 // for a copy or MMAs that a wait has run out on already, before their memory is given back
 __device__ __forceinline__ void res_drain(uint64_t* bar, uint32_t parity, const ResidentParams& g) {
@@ -174,7 +180,9 @@ struct ResWords {
 __device__ __forceinline__ float res_w0(const ResidentParams& g, int p) { return __ldcg(g.w0 + p); }
 __device__ __forceinline__ float res_w0(const ResidentEvalParams& g, int p) { return g.w_val[p]; }
 
-template <class Tile, int C, class Params>
+// MULTI: windows of several clusters, which are clusters of eight.  (Windows of one do without the exchange through L2, its code and its
+// registers: 1000 rows TF32 2.94 -> 2.75 us a step)
+template <class Tile, int C, bool MULTI, class Params>
 __global__ void __launch_bounds__(RES_THREADS, 1)
 resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ Params g) {
   using Words = ResWords<Tile::H>;
@@ -183,7 +191,6 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   constexpr int XWARPS = (WPM * C + 31) / 32;          // warps that own words
   static_assert(WPM * C <= RES_THREADS && NWORDS <= RES_THREADS, "one thread per lane of a word");
   constexpr int XT = XWARPS * 32;
-  constexpr bool MULTI = C == 8;                       // windows of several clusters use clusters of eight
   constexpr int STR = (WPM + 7) / 8 * 8;               // a cluster's words start on a line
   constexpr int NR = MULTI ? (WPM * RES_MAX_CLUSTERS + XT - 1) / XT : 1;
   extern __shared__ unsigned char smem_raw[];
@@ -193,12 +200,18 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   __shared__ __align__(16) uint4 h_in[2][C * XWARPS + 1];   // {kinetic, log-prior} shares; log-likelihood
   __shared__ __align__(16) uint4 x_in[MULTI ? RES_MAX_CLUSTERS * WPM : 1];  // words of all clusters
   __shared__ __align__(8) uint64_t bar_part, bar_w, bar_h;
+  // A word's parameters: where they stand at the start of a trajectory (position, gradient, momentum) and now (position, momentum).
+  // A step needs their 15 registers for other things, and what it spills comes back from L2, next to all of L1 being shared memory.
+  // With these, the chain's state below and a kernel of its own for windows of one cluster, us a step (10-step trajectories): TF32 1000
+  // rows 2.88 -> 2.75, 4096 3.97 -> 3.86, 58368 5.76 -> 5.41; FP32 4.76 -> 4.50, 8.17 -> 8.07, 9.87 -> 9.56
+  __shared__ float kept[15][XT];
+  __shared__ struct { double ll, lp; int iter, n_acc; uint32_t gwin; } at_[XWARPS];  // the chain, as every warp that owns parameters follows it
   __shared__ int dead_;  // a wait has run out, here or in another CTA of the cluster
   volatile int& dead = dead_;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = C == 1 ? 0 : (int)cluster_rank();
-  const int K = g.clusters;
+  const int K = MULTI ? g.clusters : 1;
   const int cl = (int)blockIdx.x / C;
   const int win = cl / K, k = cl - win * K;
   const int cta = k * C + rank, n_cta = K * C;
@@ -222,32 +235,51 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   // ---- state of the word's parameters, the same in each of its lanes: read first, so that it arrives beside the rows ----
   const size_t so = (size_t)win * g.Pp;
   float eps = chain ? __ldcg(a.eps + win) : g.eps_scalar;
-  int iter = chain ? a.iter[win] : 0;
-  const uint32_t gwin = chain ? (uint32_t)a.gwin[win] : 0u;
-  double ll_cur = chain ? a.ll_cur[win] : 0.0, lp_cur = chain ? a.lp_cur[win] : 0.0;
-  int n_acc = 0;
-  float w_s[3] = {}, g_s[3] = {}, m_s[3] = {}, w[3] = {}, m[3] = {};
+  auto& at = at_[min(warp, XWARPS - 1)];
+  if (warp < XWARPS) {  // (all lanes the same)
+    at.ll = chain ? a.ll_cur[win] : 0.0;
+    at.lp = chain ? a.lp_cur[win] : 0.0;
+    at.iter = chain ? a.iter[win] : 0;
+    at.n_acc = 0;
+    at.gwin = chain ? (uint32_t)a.gwin[win] : 0u;
+  }
   bool has[3];
+  float* const kp = &kept[0][min(tid, XT - 1)];
+  auto w_s = [&](int q) -> float& { return kp[q * XT]; };
+  auto g_s = [&](int q) -> float& { return kp[(3 + q) * XT]; };
+  auto m_s = [&](int q) -> float& { return kp[(6 + q) * XT]; };
+  auto w_at = [&](int q) -> float& { return kp[(9 + q) * XT]; };
+  auto m_at = [&](int q) -> float& { return kp[(12 + q) * XT]; };
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     const int p = Words::param(word, q);
     has[q] = mine && Words::valid(word, q);
+    float w0 = 0.f, g0 = 0.f, m0 = 0.f;
     if (has[q]) {
-      w_s[q] = chain ? __ldcg(a.w_cur + so + p) : res_w0(g, p);
-      w[q] = w_s[q];
+      w0 = chain ? __ldcg(a.w_cur + so + p) : res_w0(g, p);
       if (g.mode != RES_EVAL) {
-        g_s[q] = __ldcg((chain ? a.g_cur + so : g.g0) + p);
-        m_s[q] = __ldcg((chain ? a.m_start + so : g.m0) + p);
-        m[q] = fmaf(eps * 0.5f, g_s[q], m_s[q]);  // half kick, drift (mcmc_step_ffma.h:106-120)
-        w[q] = fmaf(eps, m[q], w[q]);
+        g0 = __ldcg((chain ? a.g_cur + so : g.g0) + p);
+        m0 = __ldcg((chain ? a.m_start + so : g.m0) + p);
       }
+    }
+    if (tid < XT) {
+      w_s(q) = w0;
+      g_s(q) = g0;
+      m_s(q) = m0;
+      // half kick, drift (mcmc_step_ffma.h:106-120)
+      const bool drift = has[q] && g.mode != RES_EVAL;
+      const float m1 = drift ? fmaf(eps * 0.5f, g0, m0) : 0.f;
+      m_at(q) = m1;
+      w_at(q) = drift ? fmaf(eps, m1, w0) : w0;
     }
   }
   // (a status that is set already: see above)
   const int pending = __ldcg(g.status);
   if (pending != 0 && g.status_host && blockIdx.x == 0 && tid == 0)
     *reinterpret_cast<volatile int*>(g.status_host) = pending;
-  if (!c.setup(&tmap, g, win) || pending != 0) dead = 1;  // (setup holds a CTA barrier)
+  const bool loaded = c.setup(&tmap, g, win);  // (holds a CTA barrier)
+  if (!loaded) res_timeout(g, res_code);
+  if (!loaded || pending != 0) dead = 1;
   bool ok = true;     // no wait of this thread inside the cluster has run out
   bool lost = false;  // the launch has given up
   const int my_words = min(WPM, NWORDS - rank * WPM);
@@ -280,12 +312,15 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   // limits of the waits that may last until the last CTA of the launch has started, and of the others
   auto limit = [&](uint32_t n) { return g.wait_ticks << (n < 2 ? 8 : 2); };
 
-  auto send_weights = [&](bool bad) {
+  auto send_weights = [&](const float (&w)[3], bool bad) {
     if (mine) st_async16(w_dst, w_bar, __float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), bad);
   };
   uint32_t n = 0;        // steps done in this launch: the mbarrier phases follow it
   uint32_t n_traj = 0;
-  send_weights(dead != 0);
+  {
+    const float w[3] = {w_at(0), w_at(1), w_at(2)};
+    send_weights(w, dead != 0);
+  }
 
   const int L = g.n_steps;
   for (int it = 0; it < g.n_iter; ++it) {
@@ -313,13 +348,20 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       // ---- the CTA's sums to their owners ----
       {
         uint4 v;
-        if (c.collect(last, v)) st_async16(part_dst, part_bar, v.x, v.y, v.z, 0u);
+        if (c.collect(last, v)) {
+          st_async16(part_dst, part_bar, v.x, v.y, v.z, 0u);
+        }
       }
       if (warp >= XWARPS) continue;
-      float m_nx[3];
+      float w[3], m[3], m_nx[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        w[q] = w_at(q);
+        m[q] = m_at(q);
+      }
       if (last && chain) {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) m_nx[q] = has[q] ? res_momentum(a, gwin, iter + 1, Words::param(word, q)) : 0.f;
+        for (int q = 0; q < 3; ++q) m_nx[q] = has[q] ? res_momentum(a, at.gwin, at.iter + 1, Words::param(word, q)) : 0.f;
       }
       // ---- owners: the cluster's sum, then the window's ----
       // (the log-likelihood is wanted at the end of a trajectory only)
@@ -332,7 +374,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       double ll = 0.0;
       bool bad = !ok;
       if (ll_warp) ll = word_sum<C>(ll_word ? u2d(x.x, x.y) : 0.0);
-      if (MULTI && K > 1) {
+      if (MULTI) {
         uint4* const mb = msg + (seq & 1) * msg_buf;
         if (mine && l == 0) {
           const uint2 d = d2u(ll);
@@ -342,21 +384,28 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         uint4 y[NR];
 #pragma unroll
         for (int i = 0; i < NR; ++i) y[i] = x_has[i] ? ld_word16(mb + x_src[i]) : make_uint4(0u, 0u, 0u, seq);
+        auto missing = [&]() {
+          bool r = false;
+#pragma unroll
+          for (int i = 0; i < NR; ++i) r |= y[i].w != seq;
+          return r;
+        };
+        // (one loop over all words, not one a word: steps of 16384 rows and more 2 to 5 % shorter)
         const uint32_t t0 = res_ticks();
+#pragma unroll 1
+        while (missing()) {
 #pragma unroll
-        for (int i = 0; i < NR; ++i) {
-          while (y[i].w != seq) {
-#pragma unroll
-            for (int j = i; j < NR; ++j)  // (a word that has arrived is read once more: its value stays)
-              if (x_has[j]) y[j] = ld_word16(mb + x_src[j]);
-            if (res_ticks() - t0 > g.wait_ticks << (n == 0 ? 6 : 0)) {
-              dead = 1;
-              res_timeout(g, 603);
-              break;
-            }
+          for (int i = 0; i < NR; ++i)  // (a word that has arrived is read once more: its value stays)
+            if (x_has[i]) y[i] = ld_word16(mb + x_src[i]);
+          if (__builtin_expect(res_ticks() - t0 > g.wait_ticks << (n == 0 ? 6 : 0), 0)) {
+            dead = 1;
+            res_timeout(g, 603);
+            break;
           }
-          if (x_has[i]) x_in[tid + i * XT] = y[i];
         }
+#pragma unroll
+        for (int i = 0; i < NR; ++i)
+          if (x_has[i]) x_in[tid + i * XT] = y[i];
         if (!ok) dead = 1;
         named_sync(RES_BAR_X, XT);
         bad = dead != 0;
@@ -380,7 +429,12 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
           m[q] = fmaf(eps, gf[q], m[q]);
           w[q] = fmaf(eps, m[q], w[q]);
         }
-        send_weights(bad);
+        send_weights(w, bad);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          w_at(q) = w[q];
+          m_at(q) = m[q];
+        }
         continue;
       }
       // ---- end of the trajectory: this warp's share of the log-prior and of the kinetic difference ----
@@ -393,7 +447,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
           lp += (double)pl;
           if (chain) {  // closing half kick (kernel_helpers.h:163-175)
             const float mf = fmaf(eps * 0.5f, gf[q], m[q]);
-            dk += 0.5 * ((double)m_s[q] * (double)m_s[q] - (double)mf * (double)mf);
+            dk += 0.5 * ((double)m_s(q) * (double)m_s(q) - (double)mf * (double)mf);
           } else if (k == 0 && !bad) {
             const int p = Words::param(word, q);
             g.g_out[p] = gf[q];
@@ -438,7 +492,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
       }
       const double ll_new = u2d(h_in[hb][C * XWARPS].x, h_in[hb][C * XWARPS].y);
       if (lost) {
-        if (it + 1 < g.n_iter) send_weights(true);
+        if (it + 1 < g.n_iter) send_weights(w, true);
         continue;
       }
       if (!chain) {
@@ -448,10 +502,11 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         }
         continue;
       }
-      const double la = (ll_new - ll_cur) + (lp - lp_cur) + dk;
+      const int iter = at.iter;
+      const double la = (ll_new - at.ll) + (lp - at.lp) + dk;
       const float la_f = (float)la;
       const float log_u = a.ref_streams ? a.ref_log_u[iter % a.ref_cap]
-                                        : logf(philox_accept_uniform(a.seed, gwin, (uint32_t)iter));
+                                        : logf(philox_accept_uniform(a.seed, at.gwin, (uint32_t)iter));
       const bool acc = log_u < la_f;  // main.h:242; a NaN ratio rejects
       float eps_next = eps;
       if (iter < a.adapt_steps) {  // main.h:266-276
@@ -465,34 +520,43 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         a.tr_accept[ti] = acc;
         a.tr_eps[ti] = eps;
       }
+      __syncwarp();  // (every lane has read what follows)
       if (acc) {
-        ll_cur = ll_new;
-        lp_cur = lp;
-        ++n_acc;
+        at.ll = ll_new;
+        at.lp = lp;
       }
+      const int n_acc = at.n_acc;
+      __syncwarp();
+      at.n_acc = n_acc + (acc ? 1 : 0);
+      at.iter = iter + 1;
+      __syncwarp();
       eps = eps_next;
       const int store = iter - a.burn_in;
-      ++iter;
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         if (acc) {
-          w_s[q] = w[q];
-          g_s[q] = gf[q];
+          w_s(q) = w[q];
+          g_s(q) = gf[q];
         }
-        m_s[q] = m_nx[q];
+        m_s(q) = m_nx[q];
         // start of the next trajectory (main.h:207-218)
-        m[q] = fmaf(eps * 0.5f, g_s[q], m_s[q]);
-        w[q] = fmaf(eps, m[q], w_s[q]);
+        m[q] = fmaf(eps * 0.5f, g_s(q), m_nx[q]);
+        w[q] = fmaf(eps, m[q], w_s(q));
       }
-      if (it + 1 < g.n_iter) send_weights(false);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        w_at(q) = w[q];
+        m_at(q) = m[q];
+      }
+      if (it + 1 < g.n_iter) send_weights(w, false);
       if (k == 0 && l == 0) {
 #pragma unroll
         for (int q = 0; q < 3; ++q)
           if (has[q]) {
             const int p = Words::param(word, q);
             if (store >= 0 && store < a.sample_capacity)
-              a.samples[((size_t)win * a.sample_capacity + store) * P + p] = w_s[q];
-            if (iter < a.trace_iters) a.tr_mom[((size_t)win * a.trace_iters + iter) * P + p] = m_s[q];
+              a.samples[((size_t)win * a.sample_capacity + store) * P + p] = w_s(q);
+            if (iter + 1 < a.trace_iters) a.tr_mom[((size_t)win * a.trace_iters + iter + 1) * P + p] = m_s(q);
           }
       }
     }
@@ -503,25 +567,28 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     for (int q = 0; q < 3; ++q)
       if (has[q]) {
         const size_t p = so + Words::param(word, q);
-        a.w_cur[p] = w_s[q];
-        a.g_cur[p] = g_s[q];
-        a.w_start[p] = w_s[q];
-        a.m_start[p] = m_s[q];
-        a.m0[p] = m_s[q];
+        a.w_cur[p] = w_s(q);
+        a.g_cur[p] = g_s(q);
+        a.w_start[p] = w_s(q);
+        a.m_start[p] = m_s(q);
+        a.m0[p] = m_s(q);
       }
   }
   if (k == 0 && rank == 0 && tid == 0) {
     if (chain && !lost) {
-      a.ll_cur[win] = ll_cur;
-      a.lp_cur[win] = lp_cur;
+      a.ll_cur[win] = at.ll;
+      a.lp_cur[win] = at.lp;
       a.eps[win] = eps;
-      a.iter[win] = iter;
-      a.n_accept[win] += n_acc;
+      a.iter[win] = at.iter;
+      a.n_accept[win] += at.n_acc;
     }
     // (every cluster of the window has read the counter: this one has used words that carry later values)
     g.seq[win] = seq;
   }
-  if (!ok) dead = 1;
+  if (!ok) {
+    dead = 1;
+    res_timeout(g, res_code);
+  }
   c.teardown(g, dead);
   if (C > 1) cluster_sync_all();  // no rank leaves while another may still write to it
   if (dead) __nanosleep(100000);
@@ -554,10 +621,33 @@ static cudaError_t resident_launch(K kernel, int cluster, size_t smem, const voi
   return cudaLaunchKernelEx(&cfg, kernel, *reinterpret_cast<const CUtensorMap*>(tmap), g);
 }
 
+template <class Tile, int C>
+static cudaError_t resident_launch_c(const void* tmap, const ResidentParams& g, cudaStream_t st, int* max_clusters) {
+  if (C == 8 && (max_clusters || g.clusters > 1)) {
+    cudaError_t e = resident_launch(resident_kernel<Tile, C, C == 8, ResidentParams>, C, Tile::SMEM, tmap, g, st, max_clusters);
+    if (e != cudaSuccess || !max_clusters) return e;
+    int single = 0;  // (the kernel for windows of one cluster each takes no more of anything; its attribute is set here)
+    e = resident_launch(resident_kernel<Tile, C, false, ResidentParams>, C, Tile::SMEM, tmap, g, st, &single);
+    if (e == cudaSuccess && single < *max_clusters) *max_clusters = single;
+    return e;
+  }
+  return resident_launch(resident_kernel<Tile, C, false, ResidentParams>, C, Tile::SMEM, tmap, g, st, max_clusters);
+}
 template <class Tile>
-static cudaError_t resident_launch_eval(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
+static cudaError_t resident_launch_any(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st, int* max_clusters) {
+  switch (cluster) {
+    case 1: return resident_launch_c<Tile, 1>(tmap, g, st, max_clusters);
+    case 2: return resident_launch_c<Tile, 2>(tmap, g, st, max_clusters);
+    case 4: return resident_launch_c<Tile, 4>(tmap, g, st, max_clusters);
+    case 8: return resident_launch_c<Tile, 8>(tmap, g, st, max_clusters);
+  }
+  return cudaErrorInvalidValue;
+}
+
+template <class Tile, bool MULTI>
+static cudaError_t resident_launch_eval_m(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
   static bool attr_done[64] = {};
-  auto kernel = resident_kernel<Tile, 8, ResidentEvalParams>;
+  auto kernel = resident_kernel<Tile, 8, MULTI, ResidentEvalParams>;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !attr_done[dev]) {
@@ -566,6 +656,10 @@ static cudaError_t resident_launch_eval(const void* tmap, const ResidentEvalPara
     if (dev < 64) attr_done[dev] = true;
   }
   return resident_launch(kernel, 8, Tile::SMEM, tmap, g, st, nullptr);
+}
+template <class Tile>
+static cudaError_t resident_launch_eval(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
+  return g.clusters > 1 ? resident_launch_eval_m<Tile, true>(tmap, g, st) : resident_launch_eval_m<Tile, false>(tmap, g, st);
 }
 
 }  // namespace mcmc_b200

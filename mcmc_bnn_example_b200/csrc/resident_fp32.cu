@@ -272,13 +272,7 @@ struct ResFp32 {
 
 cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters) {
-  switch (cluster) {
-    case 1: return resident_launch(resident_kernel<ResFp32, 1, ResidentParams>, 1, ResFp32::SMEM, tmap, g, st, max_clusters);
-    case 2: return resident_launch(resident_kernel<ResFp32, 2, ResidentParams>, 2, ResFp32::SMEM, tmap, g, st, max_clusters);
-    case 4: return resident_launch(resident_kernel<ResFp32, 4, ResidentParams>, 4, ResFp32::SMEM, tmap, g, st, max_clusters);
-    case 8: return resident_launch(resident_kernel<ResFp32, 8, ResidentParams>, 8, ResFp32::SMEM, tmap, g, st, max_clusters);
-  }
-  return cudaErrorInvalidValue;
+  return resident_launch_any<ResFp32>(cluster, tmap, g, st, max_clusters);
 }
 
 cudaError_t launch_resident_eval_fp32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {

@@ -436,13 +436,7 @@ struct ResTf32 {
 
 cudaError_t launch_resident_tf32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters) {
-  switch (cluster) {
-    case 1: return resident_launch(resident_kernel<ResTf32, 1, ResidentParams>, 1, ResTf32::SMEM, tmap, g, st, max_clusters);
-    case 2: return resident_launch(resident_kernel<ResTf32, 2, ResidentParams>, 2, ResTf32::SMEM, tmap, g, st, max_clusters);
-    case 4: return resident_launch(resident_kernel<ResTf32, 4, ResidentParams>, 4, ResTf32::SMEM, tmap, g, st, max_clusters);
-    case 8: return resident_launch(resident_kernel<ResTf32, 8, ResidentParams>, 8, ResTf32::SMEM, tmap, g, st, max_clusters);
-  }
-  return cudaErrorInvalidValue;
+  return resident_launch_any<ResTf32>(cluster, tmap, g, st, max_clusters);
 }
 
 cudaError_t launch_resident_eval_tf32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
