@@ -1,5 +1,5 @@
 // FP32 arithmetic of a warp's 32 rows for 40 hidden units, behind the forward product on the tensor core (split_mma.cuh):
-// z out of tensor memory, output layer, loss, dL/dz through the warp's own shared memory, backward by FFMA.  No warp waits
+// z out of tensor memory, output layer, loss, dL/dz; and the backward pass by FFMA, or integers for it (int_mma.cuh).  No warp waits
 // for another inside it.
 //
 // Layouts.  z is read in the 16-lane quad shape: quad q = lane / 4 holds rows q, q + 8, q + 16, q + 24, its lane c units
@@ -11,7 +11,7 @@
 // packed FMAs (their common factor, dL/dz, is one value for both: 2.3 cycles a packed FMA instead of 2.8).
 // W1's factor of dL/dz is left to whoever reads the sums out.
 #pragma once
-#include "split_mma.cuh"
+#include "int_mma.cuh"
 
 namespace mcmc_b200 {
 
@@ -39,38 +39,49 @@ struct SplitWarp {
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
       const uint32_t t = z_t + ((uint32_t)(hf * 16) << 16);
-      float s1[20], s0[20];
+      float s1[16], s0[16];
       tc_ld_quad32(t, s1);
-      tc_ld_quad8(t + 32, s1 + 16);
       tc_ld_quad32(t + SPLIT_S0, s0);
-      tc_ld_quad8(t + SPLIT_S0 + 32, s0 + 16);
       tc_wait_ld();
 #pragma unroll
-      for (int n = 0; n < 5; ++n)
+      for (int n = 0; n < 4; ++n)
 #pragma unroll
         for (int i = 0; i < 2; ++i)
           z[2 * hf + i][n] = add2(pack2(s0[4 * n + 2 * i], s0[4 * n + 2 * i + 1]), pack2(s1[4 * n + 2 * i], s1[4 * n + 2 * i + 1]));
     }
+    float s1[2][4], s0[2][4];
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const uint32_t t = z_t + ((uint32_t)(hf * 16) << 16) + 32;
+      tc_ld_quad8(t, s1[hf]);
+      tc_ld_quad8(t + SPLIT_S0, s0[hf]);
+    }
+    tc_wait_ld();
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        z[2 * hf + i][4] = add2(pack2(s0[hf][2 * i], s0[hf][2 * i + 1]), pack2(s1[hf][2 * i], s1[hf][2 * i + 1]));
   }
   // the same by FFMA, for values that split_wide finds: the lane's row, through es.  A weight is
   // the sum of its parts (split_store_weight).  Even and odd features apart, added at the end
+  static __device__ __forceinline__ float plain_z(const float* x, const unsigned char* b, int j) {
+    float even = 0.f, odd = 0.f;
+#pragma unroll 1
+    for (int i = 0; i <= D; ++i) {
+      const int k = i == 0 ? D : i - 1;  // the bias first
+      const float* p = reinterpret_cast<const float*>(b + split_b_off(j, k & ~3)) + (k & 3);
+      const float w = p[0] + (p[SPLIT_B_PART / 4] + p[2 * (SPLIT_B_PART / 4)]);
+      if (i == 0) even = w;
+      else if (k & 1) odd = fmaf(x[k], w, odd);
+      else even = fmaf(x[k], w, even);
+    }
+    return even + odd;
+  }
   static __device__ __noinline__ void plain(const float* xb, const unsigned char* b, float* es) {
     const int lane = threadIdx.x & 31;
-    const float* x = xb + lane * KP;
 #pragma unroll 1
-    for (int j = 0; j < H; ++j) {
-      float even = 0.f, odd = 0.f;
-#pragma unroll 1
-      for (int i = 0; i <= D; ++i) {
-        const int k = i == 0 ? D : i - 1;  // the bias first
-        const float* p = reinterpret_cast<const float*>(b + split_b_off(j, k & ~3)) + (k & 3);
-        const float w = p[0] + (p[SPLIT_B_PART / 4] + p[2 * (SPLIT_B_PART / 4)]);
-        if (i == 0) even = w;
-        else if (k & 1) odd = fmaf(x[k], w, odd);
-        else even = fmaf(x[k], w, even);
-      }
-      es[lane * H + j] = even + odd;
-    }
+    for (int j = 0; j < H; ++j) es[lane * H + j] = plain_z(xb + lane * KP, b, j);
     __syncwarp();
   }
   __device__ __forceinline__ void load_plain(const float* es, uint64_t (&z)[4][5]) const {
@@ -80,12 +91,11 @@ struct SplitWarp {
       for (int n = 0; n < 5; ++n) z[i][n] = lds64(es + (q + 8 * i) * H + 8 * n + 2 * c);
   }
 
-  // Everything up to dL/dz: h in place of z, dL/dz without W1's factor to es, the lane's rows added to dw (units 8 n + 2 c, + 1).
-  // `valid`, y, dy and pred are those of the lane's own row.
-  // turn(i): called when the tanh of the i-th of a quad's four rows are under way, turn(4) at the end
+  // Output layer and loss: h in place of z, d[i] = dL/dpred of row q + 8 i.  `valid`, y, dy and pred are those of the lane's own row.
+  // turn(i): called when the tanh of the i-th of a quad's four rows are under way
   template <class Turn>
-  __device__ __forceinline__ void block(uint64_t (&h)[4][5], const float* w1, const LikParams& lik, float y, bool valid,
-                                        float* es, uint64_t (&dw)[5], float& dy, float& pred, Turn turn) const {
+  __device__ __forceinline__ void front(uint64_t (&h)[4][5], const float* w1, const LikParams& lik, float y, bool valid,
+                                        float (&d)[4], float& dy, float& pred, Turn turn) const {
     float pr[4];
     {
       uint64_t w1p[5];
@@ -114,7 +124,6 @@ struct SplitWarp {
     pred = (b0 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, s, 1) + w1[H];
     dy = valid ? lik_grad(lik, y, pred) : 0.f;
     // every lane of the quad needs the four dL/dpred
-    float d[4];
     {
       const float o1 = __shfl_xor_sync(0xffffffffu, dy, 1);
       const float a0 = b0 ? o1 : dy, a1 = b0 ? dy : o1;
@@ -124,6 +133,9 @@ struct SplitWarp {
       d[2] = b1 ? a0 : c0;
       d[3] = b1 ? a1 : c1;
     }
+  }
+  // dL/dz without W1's factor to es, the lane's rows added to dw (units 8 n + 2 c, + 1)
+  __device__ __forceinline__ void store_es(const uint64_t (&h)[4][5], const float (&d)[4], float* es, uint64_t (&dw)[5]) const {
     const uint64_t minus1 = pack2(-1.f, -1.f);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -135,37 +147,42 @@ struct SplitWarp {
         *reinterpret_cast<uint64_t*>(p + 8 * n) = mul2(fma2(h[i][n], h[i][n], minus1), nd2);  // tanh_t::bwd
       }
     }
-    turn(4);
     __syncwarp();
   }
+  // the same as integers, d times `scale`, to the warp's INT_E_WARP bytes (int_mma.cuh)
+  __device__ __forceinline__ void store_ei(const uint64_t (&h)[4][5], const float (&d)[4], float scale, float* ei,
+                                           uint64_t (&dw)[5]) const {
+    const uint64_t minus1 = pack2(-1.f, -1.f);
+    uint32_t* const dst = reinterpret_cast<uint32_t*>(ei) + (c >> 1) * 32 + q * 4 + (c & 1) * 2;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float nd = -d[i] * scale;
+      const uint64_t d2 = pack2(d[i], d[i]), nd2 = pack2(nd, nd);
+#pragma unroll
+      for (int n = 0; n < 5; ++n) {
+        dw[n] = fma2(d2, h[i][n], dw[n]);
+        *reinterpret_cast<uint2*>(dst + i * (2 * INT_E_ROW) + n * 64) = int_digits2(fma2(h[i][n], h[i][n], minus1), nd2);
+      }
+    }
+  }
+  template <class Turn>
+  __device__ __forceinline__ void block(uint64_t (&h)[4][5], const float* w1, const LikParams& lik, float y, bool valid,
+                                        float* es, uint64_t (&dw)[5], float& dy, float& pred, Turn turn) const {
+    float d[4];
+    front(h, w1, lik, y, valid, d, dy, pred, turn);
+    store_es(h, d, es, dw);
+  }
 
-  // Sums of dw over the eight quads to out[unit]
-  __device__ __forceinline__ void store_dw1(const uint64_t (&dw)[5], float* out) const {
-    float v[10];
+  // Sums of dw over the eight quads to out[unit], on an 8-byte boundary.  (All lanes make all sums: halving what a lane keeps takes fewer shuffles, but
+  // three times the code)
+  __device__ __forceinline__ void store_dw1(uint64_t (&dw)[5], float* out) const {
 #pragma unroll
-    for (int n = 0; n < 5; ++n) unpack2(dw[n], v[2 * n], v[2 * n + 1]);
-    const bool q2 = (lane & 16) != 0, q1 = (lane & 8) != 0;
+    for (int o = 16; o > 2; o >>= 1)
 #pragma unroll
-    for (int n = 0; n < 5; ++n) {  // lanes with bit 4 keep the odd units, the others the even ones
-      const float send = q2 ? v[2 * n] : v[2 * n + 1];
-      v[n] = (q2 ? v[2 * n + 1] : v[2 * n]) + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-    {  // bit 3: n = 3, 4 or n = 0, 1, 2
-      const float s0 = q1 ? v[0] : v[3], s1 = q1 ? v[1] : v[4], s2 = v[2];
-      const float r0 = __shfl_xor_sync(0xffffffffu, s0, 8), r1 = __shfl_xor_sync(0xffffffffu, s1, 8);
-      const float r2 = __shfl_xor_sync(0xffffffffu, s2, 8);
-      v[0] = (q1 ? v[3] : v[0]) + r0;
-      v[1] = (q1 ? v[4] : v[1]) + r1;
-      v[2] = v[2] + r2;
-    }
+      for (int n = 0; n < 5; ++n) dw[n] = add2(dw[n], __shfl_xor_sync(0xffffffffu, dw[n], o));
+    if (q == 0)
 #pragma unroll
-    for (int n = 0; n < 3; ++n) v[n] += __shfl_xor_sync(0xffffffffu, v[n], 4);
-    float* o = out + 2 * c + (q2 ? 1 : 0);
-    if ((lane & 4) == 0) {
-      o[q1 ? 24 : 0] = v[0];
-      o[q1 ? 32 : 8] = v[1];
-      if (!q1) o[16] = v[2];
-    }
+      for (int n = 0; n < 5; ++n) *reinterpret_cast<uint64_t*>(out + 8 * n + 2 * c) = dw[n];
   }
 
   // Sums of acc over the two row subsets, lanes 16 apart: the lower lane keeps features 0 - 5 of its twelve, the upper one 6 - 11.

@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(FSP_THREADS, 1) grad_fp32_split_kernel(const G
   float* const w1 = base + G::W1;       // W1, b1
   __shared__ __align__(8) uint64_t bar_rows[NW][2], bar_fwd[NWG];
   __shared__ uint32_t tmem_slot;
-  __shared__ float red_w1[NW][H];
+  __shared__ __align__(8) float red_w1[NW][H];
   __shared__ float red_db1[NW];
   __shared__ double red_ll[NW];
 

@@ -165,6 +165,7 @@ __device__ __forceinline__ double word_sum(double v) {
 //   collects()                       the word whose sum this thread makes, or -1
 //   collect(last, v)                 after the CTA barrier that follows step: the CTA's sums for that word
 //   teardown(g, dead)                gives memory back; dead: after one more wait for MMAs
+//   X_PLACE, x_at(u)                 whether it has room for the words of all clusters, once the CTA's sums are sent; word u
 // The parameters of a word, in an order of their own: words 0 .. 306 are W0 and b0 (the last one two of them), the next
 // fourteen W1 and b1, the last word is the log-likelihood.
 template <int H>
@@ -173,6 +174,7 @@ struct ResWords {
   static constexpr int W0 = (23 * H + 2) / 3;           // words of W0 and b0
   static constexpr int N = W0 + (H + 1 + 2) / 3 + 1;    // all words
   static constexpr int PAD = 3 * W0 - 23 * H;           // empty places of word W0 - 1
+  static constexpr int PER_RANK8 = (N + 7) / 8;         // words of a rank of eight
   __device__ static int param(int t, int q) { return t < W0 ? 3 * t + q : 3 * t + q - PAD; }
   __device__ static bool valid(int t, int q) { return t < W0 ? 3 * t + q < 23 * H : 3 * t + q - PAD < P; }
 };
@@ -198,7 +200,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   __shared__ __align__(16) uint4 part_in[C][WPM];           // sums of every rank for the words owned here
   __shared__ __align__(16) uint4 w_in[NWORDS];              // weights
   __shared__ __align__(16) uint4 h_in[2][C * XWARPS + 1];   // {kinetic, log-prior} shares; log-likelihood
-  __shared__ __align__(16) uint4 x_in[MULTI ? RES_MAX_CLUSTERS * WPM : 1];  // words of all clusters
+  __shared__ __align__(16) uint4 x_in_[MULTI && !Tile::X_PLACE ? RES_MAX_CLUSTERS * WPM : 1];  // words of all clusters
   __shared__ __align__(8) uint64_t bar_part, bar_w, bar_h;
   // A word's parameters: where they stand at the start of a trajectory (position, gradient, momentum) and now (position, momentum).
   // A step needs their 15 registers for other things, and what it spills comes back from L2, next to all of L1 being shared memory.
@@ -217,12 +219,17 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   const int cta = k * C + rank, n_cta = K * C;
   const int units = (g.n_rows + 31) / 32;
   Tile c(base, g, win, (int)((long long)cta * units / n_cta), (int)((long long)(cta + 1) * units / n_cta));
+  auto x_in = [&](int u) -> uint4& {
+    if constexpr (Tile::X_PLACE) return c.x_at(u);
+    else return x_in_[u];
+  };
   if (tid == 0) {
     mbar_init(&bar_part, 1);
     mbar_init(&bar_w, 1);
     mbar_init(&bar_h, 1);
     mbar_fence_init();
     dead = 0;
+    res_code = 0;
   }
   // ---- what this thread owns ----
   const int wl = tid / C, l = tid % C;       // word of this rank, lane of the word
@@ -278,7 +285,6 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
   if (pending != 0 && g.status_host && blockIdx.x == 0 && tid == 0)
     *reinterpret_cast<volatile int*>(g.status_host) = pending;
   const bool loaded = c.setup(&tmap, g, win);  // (holds a CTA barrier)
-  if (!loaded) res_timeout(g, res_code);
   if (!loaded || pending != 0) dead = 1;
   bool ok = true;     // no wait of this thread inside the cluster has run out
   bool lost = false;  // the launch has given up
@@ -399,19 +405,19 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
             if (x_has[i]) y[i] = ld_word16(mb + x_src[i]);
           if (__builtin_expect(res_ticks() - t0 > g.wait_ticks << (n == 0 ? 6 : 0), 0)) {
             dead = 1;
-            res_timeout(g, 603);
+            res_code = 603;
             break;
           }
         }
 #pragma unroll
         for (int i = 0; i < NR; ++i)
-          if (x_has[i]) x_in[tid + i * XT] = y[i];
+          if (x_has[i]) x_in(tid + i * XT) = y[i];
         if (!ok) dead = 1;
         named_sync(RES_BAR_X, XT);
         bad = dead != 0;
         // lane l adds clusters l and l + 8
         const int wi = min(wl, my_words - 1);
-        const uint4 y0 = x_in[min(l, K - 1) * my_words + wi], y1 = x_in[min(l + C, K - 1) * my_words + wi];
+        const uint4 y0 = x_in(min(l, K - 1) * my_words + wi), y1 = x_in(min(l + C, K - 1) * my_words + wi);
         const bool one = l < K, two = l + C < K;
         v[0] = (one ? __uint_as_float(y0.x) : 0.f) + (two ? __uint_as_float(y1.x) : 0.f);
         v[1] = (one ? __uint_as_float(y0.y) : 0.f) + (two ? __uint_as_float(y1.y) : 0.f);
@@ -585,11 +591,9 @@ resident_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     // (every cluster of the window has read the counter: this one has used words that carry later values)
     g.seq[win] = seq;
   }
-  if (!ok) {
-    dead = 1;
-    res_timeout(g, res_code);
-  }
-  c.teardown(g, dead);
+  if (!ok) dead = 1;
+  c.teardown(g, dead);  // (begins with a CTA barrier)
+  if (tid == 0 && *reinterpret_cast<volatile int*>(&res_code) != 0) res_timeout(g, res_code);
   if (C > 1) cluster_sync_all();  // no rank leaves while another may still write to it
   if (dead) __nanosleep(100000);
 }

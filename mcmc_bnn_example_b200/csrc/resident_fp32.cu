@@ -1,18 +1,15 @@
 // Tile arithmetic of the resident kernel in FP32 mode (resident.cuh has the launch structure, split_mma.cuh the forward product on
-// the tensor core, fp32_split.cuh what a warp does with its 32 rows behind it): every warp owns one 32-row unit for the
-// whole launch, its rows in three parts in tensor memory and once more, whole, in shared memory for the backward pass.
-// One launch per step took 29.5 us a step for a 58368-row window, this took 12.25 with the forward product on the FMA pipe and
-// takes 9.7 now (one B200); 4096 rows 10.45 and 7.9, 1000 rows 5.2 and 4.5.  What changed, us a step of 58368 rows: the product on
-// the tensor core 9.84, shared memory through its own address space and packed tanh 9.5 to 10.2, sums collected four warps a
-// turn 9.55 to 9.65, the schedulers' warps taking turns at the tanh 9.45 to 9.55, all products of parts 9.7.
-// What bounds a step (clock reads, 58368 rows, 18,600 cycles): weights arrive and are cut up 0 - 650; first z 1,450 (18 MMAs; 24 now, 200 more);
-// tanh and dL/dz of a scheduler's four warps one after the other, backward passes beside them, until about 11,500; sums
-// to their owners 13,000; then the exchange (resident.cuh), 5,500, of which 3,000 are the trip between clusters.  In the tile
-// the FMA pipe is busy for about half of the time: 480 packed FMAs a warp that issue every third cycle with three
-// different operand pairs, and 160 moves that make pairs of one value.
-// Tried and slower: sums of a scheduler's four warps passed on from one to the next (the chain is serial: 10.1); every feature
-// twice in shared memory, which spares the moves (bank conflicts: 10.3); single FMAs in the backward pass (10.0); the turn at the
-// tanh handed over after the stores of dL/dz (9.66).
+// the tensor core, fp32_split.cuh what a warp does with its 32 rows behind it, int_mma.cuh the sums over rows on the integer tensor core): every
+// warp owns one 32-row unit for the whole launch, its rows in three parts in tensor memory and once more, as integers, in shared memory.
+// A CTA's sums come out of one accumulator, where the backward pass by FFMA left every warp 960 products of 32 rows (2,250 cycles)
+// and sixteen partial sums.  us a step, one B200, by FFMA and now: 4096 rows 8.1 and 6.75, 16384 7.1 and 6.3, 58368 9.6 and 8.2, 70 windows of
+// 800 rows 7.9 and 5.9.  CTAs of one tile stay with FFMA (resident_fp32_ffma.cu).
+// What bounds a step (clock reads, 58368 rows, 16,500 cycles): weights arrive and are cut up 0 - 350, first z 1,300, tanh and dL/dz of a
+// scheduler's four warps one after the other, 1,030 cycles each (MUFU 640), until 7,000; the last tile's sums 7,850, read out and
+// sent 9,500; then the exchange (resident.cuh), 7,000.
+// What cost more than it gave: conversions of float to integer (the tanh's pipe: 440 cycles a warp), polls by warps that have
+// nothing to do, a scale from the step itself, sums issued by every tile's last warp, one accumulator pair for the product (tiles wait for
+// one another, 9.1 us), everything that made a step spill more than L1 holds (up to 2 us).
 #include <cuda.h>
 #include "fp32_split.cuh"
 #include "resident.cuh"
@@ -25,21 +22,29 @@ struct ResFp32 {
   using Warp = SplitWarp;
   static constexpr int NWARPS = RES_NWG * 4;
   static_assert(Warp::ROWS == 32 && NWARPS == RES_UNITS, "a warp owns one 32-row unit");
-  // a warp's sums of dW0 and db0, after the shuffle over its two row subsets a lane's 6 features x 5 units: eight
-  // floats between the feature groups make the stores free of bank conflicts.  They take the place of its dL/dz.
+  // the sums of dW0 and db0 of a warp whose values no integers hold, after the shuffle over its two row subsets a lane's 6 features x 5
+  // units; they take the place of its dL/dz
   static constexpr int GROUP = 6 * H, GSTR = GROUP + 8;
   static_assert(4 * GSTR <= Warp::ES, "sums fit where dL/dz was");
+  static_assert(Warp::ES * 4 == INT_E_WARP && RES_UNITS * 32 * KP <= NWARPS * Warp::ES, "rows land where dL/dz will be");
   static constexpr int RS = H + 4;   // dW1 and db1 of a warp's rows
-  // float offsets
-  static constexpr int WB = 0, XB = WB + SPLIT_B_BYTES / 4, ES = XB + RES_UNITS * 32 * KP, W1 = ES + NWARPS * Warp::ES,
-                       RW1 = W1 + RS, RLL = RW1 + NWARPS * RS, BAR = RLL + NWARPS * 2;
-  // barriers: rows landed; per tile, forward done; per accumulator buffer, read
-  static constexpr int NBARS = 1 + RES_NWG + 2;
+  // float offsets.  XI: features as integers; OWN: a thread's constants (target, factor of its line of sums, where its word's weights go),
+  // registers that the step needs for other things; XS: the features' scales.  The sums over rows take the weights' place once the product is done; words of other
+  // clusters take that of dL/dz.  (Up to 195 KB in all leave 60 KB of L1, for what a step spills; beyond that it is 28 KB, and half of it
+  // comes back from L2: 1000 rows 4.5 us a step, and 5.7)
+  static constexpr int WB = 0, S = WB, XI = WB + SPLIT_B_BYTES / 4, ES = XI + RES_UNITS * INT_X_WARP / 4, OWN = ES + NWARPS * Warp::ES,
+                       XS = OWN + 4 * RES_THREADS, W1 = XS + KP, RW1 = W1 + RS, RLL = RW1 + NWARPS * RS, MISC = RLL + NWARPS * 2,
+                       BAR = MISC + NWARPS + 4;
+  static_assert(INT_S_FLOATS * 4 <= SPLIT_B_BYTES && 4 * GSTR + 4 * 64 <= Warp::ES && RES_MAX_CLUSTERS * Words::PER_RANK8 <= NWARPS * 64,
+                "shared places");
+  // barriers: rows landed; per tile, forward done, accumulators read, dL/dz written; sums over rows done; the scale is known
+  static constexpr int NBARS = 3 + 3 * RES_NWG;
   static constexpr size_t SMEM = 1024 + (BAR + 2 * NBARS) * 4;
-  static_assert(XB % 4 == 0 && W1 % 4 == 0 && RW1 % 4 == 0 && RLL % 2 == 0 && BAR % 2 == 0, "vector alignment");
-  // tensor memory: the rows' parts for the whole launch; two accumulator buffers that the four tiles take in turn
-  static constexpr int ZBUF = 2, Z_COL0 = RES_NWG * SPLIT_A_COLS, TMEM_COLS = 512;
-  static_assert(Z_COL0 + ZBUF * SPLIT_Z_COLS <= TMEM_COLS, "tensor memory budget");
+  static_assert(XI % 64 == 0 && ES % 4 == 0 && XS % 4 == 0 && W1 % 4 == 0 && RW1 % 4 == 0 && RLL % 2 == 0 && BAR % 2 == 0, "alignment");
+  // Tensor memory: two accumulator pairs for the product, which the tiles take in turn and whose place, when all have been read, becomes
+  // the sums over rows; and the rows' parts for the whole launch
+  static constexpr int A_COL0 = 2 * SPLIT_Z_COLS, TMEM_COLS = 512;
+  static_assert(INT_ACC_COLS <= A_COL0 && A_COL0 + RES_NWG * SPLIT_A_COLS <= TMEM_COLS, "tensor memory budget");
 
   // named barriers: a warp's turn is over (those of the last four are not needed)
   static constexpr int BAR_LO = 1, BAR_HI = 10;
@@ -48,37 +53,71 @@ struct ResFp32 {
 
   Warp lanes;
   float* base;
-  int warp, wg, n_units;
+  int warp, wg, n_units, nt;
   int row0;          // this warp's first row in the window
-  bool active, plain_x, plain;
-  uint32_t s_dst[3], tmem, par;
+  bool active, plain_x, plain, fresh;   // fresh: a trajectory begins
+  int rows_are;
+  uint32_t tmem, par, first_par;
+  // What is in XI of this warp's rows.  FLOATS: a feature is beyond its range in one of them; FLOATS_NOW: a dL/dpred was, earlier in this
+  // trajectory
+  enum { INTS, FLOATS, FLOATS_NOW };
+  __device__ __forceinline__ float& own(int i) const { return base[OWN + i * RES_THREADS + threadIdx.x]; }
 
   __device__ __forceinline__ uint64_t* bar_rows() const { return reinterpret_cast<uint64_t*>(base + BAR); }
   __device__ __forceinline__ uint64_t* bar_fwd(int w) const { return bar_rows() + 1 + w; }
-  __device__ __forceinline__ uint64_t* bar_read(int b) const { return bar_rows() + 1 + RES_NWG + b; }
+  __device__ __forceinline__ uint64_t* bar_read(int w) const { return bar_rows() + 1 + RES_NWG + w; }
+  __device__ __forceinline__ uint64_t* bar_e(int w) const { return bar_rows() + 1 + 2 * RES_NWG + w; }
+  __device__ __forceinline__ uint64_t* bar_sum() const { return bar_rows() + 1 + 3 * RES_NWG; }
+  __device__ __forceinline__ uint64_t* bar_scale() const { return bar_rows() + 2 + 3 * RES_NWG; }
+  // statistics of dL/dpred per parity of the step; the sums' factor; whether a warp has taken FFMA
+  __device__ __forceinline__ uint32_t* stat(int ph) const { return reinterpret_cast<uint32_t*>(base + MISC) + ph; }
+  __device__ __forceinline__ float& sum_f() const { return base[MISC + 2]; }
+  __device__ __forceinline__ volatile uint32_t* far() const { return reinterpret_cast<volatile uint32_t*>(base + MISC + 4); }
+  __device__ __forceinline__ uint32_t far_warps() const {
+    return __ballot_sync(0xffffffffu, lanes.lane < NWARPS && far()[lanes.lane & (NWARPS - 1)] != 0u);
+  }
+  // words of clusters: 64 behind each warp's sums
+  static constexpr bool X_PLACE = true;
+  __device__ __forceinline__ uint4& x_at(int u) const {
+    return reinterpret_cast<uint4*>(base + ES + 4 * GSTR)[(u >> 6) * (Warp::ES / 4) + (u & 63)];
+  }
+  static __device__ __forceinline__ uint32_t a_col(int w) { return A_COL0 + w * SPLIT_A_COLS; }
+  static __device__ __forceinline__ uint32_t z_col(int w) { return (w & 1) * SPLIT_Z_COLS; }
 
-  __device__ __forceinline__ ResFp32(unsigned char* b, const ResidentParams& g, int, int u0, int u1)
+  __device__ __forceinline__ ResFp32(unsigned char* b, const ResidentParams& g, int win, int u0, int u1)
       : base(reinterpret_cast<float*>(b)) {
     warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     wg = warp >> 2;
     n_units = u1 - u0;
+    nt = (n_units + 3) / 4;
     active = warp < n_units;
     row0 = (u0 + warp) * 32;
-    par = 0;
+    par = first_par = 0;
     plain_x = plain = false;
+    rows_are = INTS;
+    fresh = true;
     const int t = threadIdx.x;
+    uint32_t off[3];
     for (int q = 0; q < 3; ++q) {
       const int p = Words::param(t, q);
       // (threads and places of a word without a parameter write where feature 28 of unit 0 would be: nobody reads there)
-      s_dst[q] = smem_u32(b) + split_b_off(0, 28);
-      if (t >= Words::N - 1 || !Words::valid(t, q)) continue;
-      if (p < D * H + H) s_dst[q] = smem_u32(b) + split_b_off(p % H, p / H & ~3) + (p / H & 3) * 4;
-      else s_dst[q] = smem_u32(base + W1 + p - (D * H + H));
+      uint32_t dst = smem_u32(b) + split_b_off(0, 28);
+      if (t < Words::N - 1 && Words::valid(t, q)) {
+        if (p < D * H + H) dst = smem_u32(b) + split_b_off(p % H, p / H & ~3) + (p / H & 3) * 4;
+        else dst = smem_u32(base + W1 + p - (D * H + H));
+      }
+      // (feature 23 is no weight, but the product reads it: sums have been there.  Threads behind the last word bring its zeros)
+      if (t >= Words::N && t < Words::N + H) dst = smem_u32(b) + q * SPLIT_B_PART + split_b_off(t - Words::N, 20) + 12;
+      off[q] = (dst - smem_u32(b)) >> 2;
     }
+    own(0) = own(1) = 0.f;
+    own(2) = __uint_as_float(off[0] | off[1] << 16);
+    own(3) = __uint_as_float(off[2]);
   }
 
   __device__ __forceinline__ bool setup(const CUtensorMap*, const ResidentParams& g, int win) {
-    __shared__ uint32_t tmem_slot;
+    __shared__ uint32_t tmem_slot, x_stat[KP], x_max[KP];
+    float* const x_scale = base + XS;
     bool ok = true;
     const int tid = threadIdx.x;
     if (warp == 0) {
@@ -88,17 +127,24 @@ struct ResFp32 {
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
+      auto warps_of = [&](int w) { return min(max(n_units - 4 * w, 1), 4); };
       mbar_init(bar_rows(), 1);
-      for (int w = 0; w < RES_NWG; ++w) mbar_init(bar_fwd(w), 1);
-      for (int b = 0; b < ZBUF; ++b) mbar_init(bar_read(b), 4);
+      for (int w = 0; w < RES_NWG; ++w) {
+        mbar_init(bar_fwd(w), 1);
+        mbar_init(bar_read(w), warps_of(w));
+        mbar_init(bar_e(w), warps_of(w));
+      }
+      mbar_init(bar_sum(), 1);
+      mbar_init(bar_scale(), warps_of(0));
       mbar_fence_init();
     }
-    // sums that nothing writes stay zero: those of warps without rows; and what the last MMAs read behind the weights
-    for (int i = tid; i < (W1 - ES) / 4; i += RES_THREADS)
-      reinterpret_cast<float4*>(base + ES)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int i = tid; i < (XB - WB) / 4; i += RES_THREADS)
+    if (tid < KP) x_stat[tid] = x_max[tid] = 0u;
+    if (tid < BAR - MISC) base[MISC + tid] = 0.f;
+    // what an MMA may read before it is written
+    for (int i = tid; i < (ES - WB) / 4; i += RES_THREADS)
       reinterpret_cast<float4*>(base + WB)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int i = tid; i < BAR - RW1; i += RES_THREADS) base[RW1 + i] = 0.f;
+    // sums that nothing writes stay zero
+    for (int i = tid; i < MISC - RW1; i += RES_THREADS) base[RW1 + i] = 0.f;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -108,14 +154,31 @@ struct ResFp32 {
       const uint32_t bytes = (uint32_t)n_units * 32 * KP * 4;
       if (tid == 0) {
         mbar_expect_tx(bar_rows(), bytes);
-        bulk_g2s(base + XB, g.xaug + ((size_t)(g.data_window0 + win) * g.rows_pad + row0) * KP, bytes, bar_rows());
+        bulk_g2s(base + ES, g.xaug + ((size_t)(g.data_window0 + win) * g.rows_pad + row0) * KP, bytes, bar_rows());
       }
       res_wait(bar_rows(), 0, g, g.wait_ticks << 2, 611, ok);
       if (!ok) res_drain(bar_rows(), 0, g);
       if (g.test_code == 611) res_wait(bar_rows(), 1, g, g.wait_ticks << 2, 611, ok);  // (nothing ends this phase)
+      const float* x = base + ES + tid * KP;
+      if (active) {
+        own(0) = base[ES + (warp * 32 + lanes.own()) * KP + COL_Y];
+        uint32_t st = 0u, mx = 0u;  // lane k: feature k
+#pragma unroll
+        for (int k = 0; k <= D; ++k) {
+          const uint32_t s = __reduce_add_sync(0xffffffffu, int_stat(x[k]));
+          const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(x[k]) & 0x7fffffffu);
+          if (lanes.lane == k) {
+            st = s;
+            mx = m;
+          }
+        }
+        if (lanes.lane <= D) {
+          atomicAdd(&x_stat[lanes.lane], st);
+          atomicMax(&x_max[lanes.lane], mx);
+        }
+      }
       if (4 * wg < n_units) {  // the tile's rows to tensor memory, zeros for warps without rows
-        const float* x = base + XB + tid * KP;
-        const uint32_t a_t = tmem + wg * SPLIT_A_COLS + ((uint32_t)((warp & 3) * 32) << 16);
+        const uint32_t a_t = tmem + a_col(wg) + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           float v[8];
@@ -129,6 +192,33 @@ struct ResFp32 {
         tc_wait_st();
         tc_fence_before();
       }
+      __syncthreads();
+      // features as integers: a scale each, from the CTA's rows
+      auto x_exp = [&](int k) {
+        return x_stat[k] ? min(int_scale_exp(x_stat[k], INT_ROOM_X), int_max_exp(x_max[k])) : 127;
+      };
+      bool in = true;
+#pragma unroll 1
+      for (int k = 0; k <= D; ++k) {
+        const int e = x_exp(k);
+        if (lanes.lane == 0 && warp == 0) x_scale[k] = int_scale_ok(e) ? int_scale(e) : 0.f;
+        in &= int_scale_ok(e) && (!active || fabsf(x[k]) * int_scale(e) < INT_TOP);
+      }
+      if (tid == 0) x_scale[D + 1] = 0.f;   // the target
+      if (!__all_sync(0xffffffffu, in)) rows_are = FLOATS;
+      __syncthreads();
+      float4* const xi = reinterpret_cast<float4*>(base + XI + warp * 32 * KP);
+      if (rows_are != INTS) {
+        for (int ch = 0; ch < KP / 4; ++ch) xi[lanes.lane * (KP / 4) + ch] = reinterpret_cast<const float4*>(x)[ch];
+      } else {
+        for (int ch = 0; ch < KP / 4; ++ch)
+          int_store_x4(smem_u32(xi) + int_x_off(lanes.lane, ch), active ? reinterpret_cast<const float4*>(x)[ch] : make_float4(0.f, 0.f, 0.f, 0.f),
+                       reinterpret_cast<const float4*>(x_scale)[ch]);
+      }
+      const int k = (warp & 3) * 8 + (lanes.lane >> 2);  // the line whose sums this lane reads
+      const int e = k <= D ? x_exp(k) : 127;
+      own(1) = int_scale_ok(e) ? int_unscale(e + 8 * (lanes.lane & 3)) : 0.f;
+      fence_proxy_async_smem();
     }
     plain_x = __syncthreads_or(wide) != 0;
     return ok;
@@ -136,7 +226,10 @@ struct ResFp32 {
 
   // word `threadIdx.x` of the weights
   __device__ __forceinline__ void stage(const uint4& v) {
-    const uint32_t x[3] = {v.x, v.y, v.z};
+    const bool word = (int)threadIdx.x < Words::N - 1;
+    const uint32_t x[3] = {word ? v.x : 0u, word ? v.y : 0u, word ? v.z : 0u};
+    const uint32_t off = __float_as_uint(own(2)), b = smem_u32(base);
+    const uint32_t s_dst[3] = {b + (off & 0xffffu) * 4, b + (off >> 16) * 4, b + __float_as_uint(own(3)) * 4};
     bool wide = plain_x;
     if ((int)threadIdx.x < Words::W0) {
 #pragma unroll
@@ -149,68 +242,182 @@ struct ResFp32 {
     plain = __syncthreads_or(wide) != 0;
   }
 
-  __device__ __forceinline__ void step(const ResidentParams& g, float* row_loss, bool last, bool& ok) {
-    const int nt = (n_units + 3) / 4;
-    const uint32_t ph = par;
-    par ^= 1;
-    if (warp == NWARPS - 1) {
-      // the MMAs of all tiles, by the warp whose own rows come last; a buffer's second tile when its first has been read
-      const uint32_t on = elect_one(), tm = __shfl_sync(0xffffffffu, tmem, 0);
-      for (int w = 0; w < nt; ++w) {
-        if (w >= ZBUF) res_wait(bar_read(w % ZBUF), ph, g, g.wait_ticks << 2, 613, ok);
-        tc_fence_after();
-        split_issue(tm + Z_COL0 + w % ZBUF * SPLIT_Z_COLS, tm + w * SPLIT_A_COLS, smem_u32(base + WB), on);
-        tc_commit_if(bar_fwd(w), on);
-      }
-      if (g.test_code == 613) res_wait(bar_read(0), nt > ZBUF ? ph ^ 1 : ph, g, g.wait_ticks << 2, 613, ok);  // (nothing ends this phase)
+  // The backward pass of a warp with a value beyond the range, which no integer holds, by FFMA.  A dL/dpred that is likely stays there, so
+  // the warp's rows remain floats until the trajectory's end.  (Functions of their own, so that the step does without the registers; a
+  // list of such rows instead, added to the sums one by one, cost every step 0.4 us)
+  static __device__ __noinline__ void ints_to_floats(float* xi, uint32_t a_t) {
+    float4* const row = reinterpret_cast<float4*>(xi) + (threadIdx.x & 31) * (KP / 4);
+#pragma unroll 1
+    for (int j = 0; j < 3; ++j) {
+      float hi[8], r[8];
+      tc_ld8(a_t + 8 * j, hi);
+      tc_ld8(a_t + SPLIT_K + 8 * j, r);   // (a row's middle part is all that is left of it)
+      tc_wait_ld();
+      row[2 * j] = make_float4(hi[0] + r[0], hi[1] + r[1], hi[2] + r[2], hi[3] + r[3]);
+      row[2 * j + 1] = make_float4(hi[4] + r[4], hi[5] + r[5], hi[6] + r[6], hi[7] + r[7]);
     }
-    if (!active) return;
-    const float* xb = base + XB + warp * 32 * KP;
-    float* es = base + ES + warp * Warp::ES;
-    const int left = g.n_rows - row0;
-    uint64_t h[4][5];
-    res_wait(bar_fwd(wg), ph, g, g.wait_ticks << 2, 612, ok);
-    tc_fence_after();
-    lanes.load(tmem + Z_COL0 + wg % ZBUF * SPLIT_Z_COLS + ((uint32_t)((warp & 3) * 32) << 16), h);
-    tc_fence_before();
-    if (wg + ZBUF < nt) {  // another tile takes the buffer (so this one is full: all its warps come here)
-      __syncwarp();
-      if (lanes.lane == 0) mbar_arrive(bar_read(wg % ZBUF));
-    }
-    if (plain) {
-      Warp::plain(xb, reinterpret_cast<const unsigned char*>(base + WB), es);
-      lanes.load_plain(es, h);
-    }
-    uint64_t dw1[5] = {};
-    float dy, pred;
-    const int own = lanes.own();
-    const bool valid = own < left;
-    const float y = xb[own * KP + COL_Y];
-    // The four warps of a scheduler take turns at the tanh, which MUFU bounds: side by side they would all end it late, and only
-    // then begin to multiply.  4096 rows 8.63 us a step without turns, 7.8 with them; 58368 rows 10.2 and 9.45
-    if (warp >= 4) named_sync(bar_turn(warp - 4), 64);
-    lanes.block(h, base + W1, g.lik, y, valid, es, dw1, dy, pred, [&](int i) {
-      if (i == 3 && warp + 4 < n_units) named_arrive(bar_turn(warp), 64);
-    });
-    if (last) {
-      if (g.test_code == 612) res_wait(bar_fwd(wg), ph ^ 1, g, g.wait_ticks << 2, 612, ok);  // (nothing ends this phase)
-      const float loss = valid ? lik_loss(g.lik, y, pred) : 0.f;
-      store_row_loss(row_loss, row0 + own, loss, valid);
-      double ld = (double)loss;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) ld += __shfl_xor_sync(0xffffffffu, ld, o);
-      if (lanes.lane == 0) reinterpret_cast<double*>(base + RLL)[warp] = ld;
-    }
-    float* rw1 = base + RW1 + warp * RS;
-    lanes.store_dw1(dw1, rw1);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dy += __shfl_xor_sync(0xffffffffu, dy, o);
-    if (lanes.lane == 0) rw1[H] = dy;
+    __syncwarp();
+  }
+  static __device__ __noinline__ void far_backward(const float* xi, float* es) {
+    const Warp lanes;
     uint64_t acc[Warp::KPT / 2][Warp::UPT] = {};
-    lanes.backward<2>(xb, es, acc);
-    // dW0: lanes 16 apart have the two row subsets; the lower one keeps features 0 - 5 of the twelve, the upper 6 - 11
+    lanes.backward<2>(xi, es, acc);
     __syncwarp();  // dL/dz has been read by every lane
     lanes.store_dw0(acc, es + (2 * lanes.kh + lanes.rsub) * GSTR);
+  }
+  static __device__ __noinline__ void floats_to_ints(float* xi, const float* x_scale) {
+    const int lane = threadIdx.x & 31;
+    float4 x[KP / 4];
+#pragma unroll
+    for (int ch = 0; ch < KP / 4; ++ch) x[ch] = reinterpret_cast<const float4*>(xi)[lane * (KP / 4) + ch];
+    __syncwarp();
+#pragma unroll
+    for (int ch = 0; ch < KP / 4; ++ch)
+      int_store_x4(smem_u32(xi) + int_x_off(lane, ch), x[ch], reinterpret_cast<const float4*>(x_scale)[ch]);
+    fence_proxy_async_smem();
+  }
+
+  __device__ __forceinline__ void rows_to_floats() {
+    if (rows_are != INTS) return;
+    ints_to_floats(base + XI + warp * 32 * KP, tmem + a_col(wg) + ((uint32_t)((warp & 3) * 32) << 16));
+    rows_are = FLOATS_NOW;
+  }
+
+  __device__ __forceinline__ void step(const ResidentParams& g, float* row_loss, bool last, bool& ok) {
+    const uint32_t ph = par;
+    par ^= 1;
+    if (n_units == 0) return;
+    const bool first = fresh;
+    fresh = last;
+    const uint32_t fph = first_par;
+    first_par ^= first ? 1u : 0u;
+    const uint32_t limit = g.wait_ticks << 2;
+    if (warp == NWARPS - 1) {
+      // the product's MMAs of all tiles, by the warp whose own rows come last; accumulators' next tile when they have been read
+      const uint32_t on = elect_one(), tm = __shfl_sync(0xffffffffu, tmem, 0), wb = smem_u32(base + WB);
+      for (int w = 0; w < nt; ++w) {
+        if (w >= 2) res_wait(bar_read(w - 2), ph, g, limit, 613, ok);
+        tc_fence_after();
+        split_issue(tm + z_col(w), tm + a_col(w), wb, on);
+        tc_commit_if(bar_fwd(w), on);
+      }
+    }
+    float* es = base + ES + warp * Warp::ES;
+    uint64_t dw1[5] = {};
+    float dy = 0.f, pred = 0.f;
+    bool near = true;
+    const bool valid = lanes.own() < g.n_rows - row0;
+    auto give_scale = [&]() {
+      const uint32_t st = __reduce_add_sync(0xffffffffu, int_stat(dy));
+      if (lanes.lane == 0 && st) atomicMax(stat(ph), int_stat_word(int_scale_exp(st, INT_ROOM_E)));
+    };
+    if (active) {
+      uint64_t h[4][5];
+      res_wait(bar_fwd(wg), ph, g, limit, 612, ok);
+      tc_fence_after();
+      if (__builtin_expect(plain, 0)) {
+        rows_to_floats();
+        Warp::plain(base + XI + warp * 32 * KP, reinterpret_cast<const unsigned char*>(base + WB), es);
+        lanes.load_plain(es, h);
+      } else {
+        lanes.load(tmem + z_col(wg) + ((uint32_t)((warp & 3) * 32) << 16), h);
+      }
+      tc_fence_before();
+      // (another tile or the sums take the accumulators' place)
+      __syncwarp();
+      if (lanes.lane == 0) mbar_arrive(bar_read(wg));
+      float d[4];
+      // The four warps of a scheduler take turns at the tanh, which MUFU bounds: side by side they would all end it late, and only
+      // then go on.  4096 rows 8.63 us a step without turns, 7.8 with them; 58368 rows 10.2 and 9.45
+      if (warp >= 4) named_sync(bar_turn(warp - 4), 64);
+      lanes.front(h, base + W1, g.lik, own(0), valid, d, dy, pred, [&](int i) {
+        if (i == 3 && warp + 4 < n_units) named_arrive(bar_turn(warp), 64);
+      });
+      // The first tile's rows give the scale, to all of them, in a trajectory's first step, and to the next step: a step that had to
+      // wait for its own would be 0.2 us longer.  It is the smallest that one of the tile's warps asks for, since an outlier may well
+      // move the mean of 32 exponents, but nothing outside its warp should depend on it
+      if (__builtin_expect(first, 0)) {
+        if (rows_are == FLOATS_NOW) {
+          floats_to_ints(base + XI + warp * 32 * KP, base + XS);
+          rows_are = INTS;
+        }
+        if (wg == 0) {
+          give_scale();
+          __syncwarp();
+          if (lanes.lane == 0) mbar_arrive(bar_scale());
+        }
+        res_wait(bar_scale(), fph, g, limit, 614, ok);
+      }
+      const int se = int_stat_exp(*reinterpret_cast<volatile uint32_t*>(stat(first ? ph : ph ^ 1)));
+      const bool s_ok = int_scale_ok(se);
+      const float scale = s_ok ? int_scale(se) : 0.f;
+      near = s_ok && rows_are == INTS && __all_sync(0xffffffffu, fabsf(dy) * scale < INT_TOP);
+      if (__builtin_expect(near, 1)) {
+        lanes.store_ei(h, d, scale, es, dw1);
+        fence_proxy_async_smem();
+      } else {
+        lanes.store_es(h, d, es, dw1);
+      }
+      if (threadIdx.x == 0) sum_f() = s_ok ? int_unscale(se) : 1.f;
+      if (lanes.lane == 0) far()[warp] = near ? 0u : 1u;
+      __syncwarp();
+      if (lanes.lane == 0) mbar_arrive(bar_e(wg));
+      if (__builtin_expect(!near, 0)) {
+        rows_to_floats();
+        far_backward(base + XI + warp * 32 * KP, es);
+      }
+      if (wg == 0 && !first) give_scale();
+      if (__builtin_expect(last, 0)) {
+        if (g.test_code == 612) res_wait(bar_fwd(wg), ph ^ 1, g, limit, 612, ok);  // (nothing ends this phase)
+        const float loss = valid ? lik_loss(g.lik, own(0), pred) : 0.f;
+        store_row_loss(row_loss, row0 + lanes.own(), loss, valid);
+        double ld = (double)loss;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ld += __shfl_xor_sync(0xffffffffu, ld, o);
+        if (lanes.lane == 0) reinterpret_cast<double*>(base + RLL)[warp] = ld;
+      }
+      float* rw1 = base + RW1 + warp * RS;
+      lanes.store_dw1(dw1, rw1);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) dy += __shfl_xor_sync(0xffffffffu, dy, o);
+      if (lanes.lane == 0) rw1[H] = dy;
+    }
+    // Sums over rows, by a warp that has no rows, or is done with them first
+    if (warp == (n_units < RES_UNITS ? NWARPS - 1 : 0)) {
+      const uint32_t on = elect_one(), tm = __shfl_sync(0xffffffffu, tmem, 0);
+      if (nt > 2) res_wait(bar_read(nt - 2), ph, g, limit, 614, ok);  // (their place must have been read)
+      if (nt > 1) res_wait(bar_read(nt - 1), ph, g, limit, 614, ok);
+      uint32_t more = 0u;
+#pragma unroll 1
+      for (int w = 0; w < nt; ++w) {
+        res_wait(bar_e(w), ph, g, limit, 614, ok);
+        tc_fence_after();
+        const uint32_t far = far_warps() >> 4 * w;
+        const uint64_t xd = int_x_desc(smem_u32(base + XI) + w * 4 * INT_X_WARP);
+        const uint64_t ed = int_e_desc(smem_u32(base + ES) + w * 4 * INT_E_WARP);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (4 * w + i < n_units && !(far >> i & 1)) {
+            int_mma_if(tm, umma_desc_advance(xd, i * (INT_X_WARP >> 4)), umma_desc_advance(ed, i * (INT_E_WARP >> 4)), more, on);
+            more = 1u;
+          }
+      }
+      tc_commit_if(bar_sum(), on);
+      res_wait(bar_sum(), ph, g, limit, 614, ok);
+    }
+    // the CTA's sums, ten units a warp
+    __syncthreads();
+    tc_fence_after();
+    if ((warp & 3) < INT_LINES / 32) {
+      float v[10];
+      int_read_out<10>(tmem + wg * 40 + ((uint32_t)((warp & 3) * 32) << 16), own(1), v);
+      const bool none = __popc(far_warps()) == n_units;  // (no MMA has been issued)
+#pragma unroll
+      for (int j = 0; j < 10; ++j) base[S + (wg * 10 + j) * INT_S_STR + (warp & 3) * 32 + lanes.lane] = none ? 0.f : v[j];
+    }
+    tc_fence_before();
+    if (g.test_code == 613 && warp == NWARPS - 1)  // (nothing ends this phase)
+      res_wait(bar_read(0), ph ^ 1, g, limit, 613, ok);
   }
 
   // Words of W0 and b0 go to the threads of the same number; those of W1 and b1 and the log-likelihood to the last warp
@@ -224,7 +431,7 @@ struct ResFp32 {
     float s[3] = {};
     if (warp == LAST) {
       const float* r = base + RW1 + 3 * min(lanes.lane, NW1 - 1);
-#pragma unroll 4
+#pragma unroll 2
       for (int w = 0; w < NWARPS; ++w)
 #pragma unroll
         for (int q = 0; q < 3; ++q) s[q] += r[w * RS + q];
@@ -232,7 +439,7 @@ struct ResFp32 {
       if (last && lanes.lane == NW1) {
         const double* d = reinterpret_cast<const double*>(base + RLL);
         double t[2] = {};
-#pragma unroll
+#pragma unroll 2
         for (int w = 0; w < NWARPS; ++w) t[w & 1] += d[w];
         const uint2 u = d2u(t[0] + t[1]);
         v.x = u.x;
@@ -240,20 +447,35 @@ struct ResFp32 {
       }
       return lanes.lane <= NW1;
     }
+    if (threadIdx.x == 0) *stat(par) = 0u;  // the step's, whose scale has been read
     const int t = min((int)threadIdx.x, Words::W0 - 1);
-    const float* gp = base + ES + 3 * t + 8 * (3 * t / GROUP);
-    // (four warps to a turn, and no turn for tiles without rows: fetching the straight code for sixteen took 1,100 of a step's cycles)
+    const float inv = sum_f();
+    // parameter 3 t + q: feature k, unit j
+    const int k0 = 3 * t / H, j0 = 3 * t - k0 * H;
+    float w1[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const bool next = j0 + q >= H;
+      const int j = next ? j0 + q - H : j0 + q;
+      s[q] = n_units > 0 ? int_sum4(base + S, next ? k0 + 1 : k0, j) * inv : 0.f;
+      w1[q] = base[W1 + j];
+    }
+    const uint32_t fb = far_warps();
+    if (__builtin_expect(fb != 0u, 0)) {  // what went by FFMA
+      const float* gp = base + ES + 3 * t + 8 * (3 * t / GROUP);
 #pragma unroll 1
-    for (int w0 = 0; w0 < n_units; w0 += 4) {
+      for (int w0 = 0; w0 < n_units; w0 += 4, gp += 4 * Warp::ES)
 #pragma unroll
-      for (int w = 0; w < 4; ++w)
+        for (int w = 0; w < 4; ++w)
 #pragma unroll
-        for (int q = 0; q < 3; ++q) s[q] += gp[w * Warp::ES + q];
-      gp += 4 * Warp::ES;
+          for (int q = 0; q < 3; ++q) {
+            const float v = gp[w * Warp::ES + q];
+            s[q] += fb >> (w0 + w) & 1 ? v : 0.f;
+          }
     }
     float o[3];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) o[q] = base[W1 + (3 * t + q) % H] * s[q];
+    for (int q = 0; q < 3; ++q) o[q] = w1[q] * s[q];
     // (a place without a parameter would get the sum of target x dL/dz, and its value a vote on the path in `stage`)
     if (t == Words::W0 - 1 && Words::PAD == 1) o[2] = 0.f;
     v = make_uint4(__float_as_uint(o[0]), __float_as_uint(o[1]), __float_as_uint(o[2]), 0u);
@@ -263,20 +485,34 @@ struct ResFp32 {
     tc_fence_before();
     __syncthreads();
     if (warp == 0 && dead)
-      for (int w = 0; 4 * w < n_units; ++w) res_drain(bar_fwd(w), par ^ 1, g);
+      for (int w = 0; w <= nt; ++w) res_drain(w < nt ? bar_fwd(w) : bar_sum(), par ^ 1, g);
     if (warp == 0)
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS)
                    : "memory");
   }
 };
 
+// Windows whose CTAs have one tile at most take the tile arithmetic without integers (resident_fp32_ffma.cu): as fast there, and an outlier
+// costs it nothing.  us a step, integers and FFMA: 148 windows of 128 rows 4.43, 4.21; 1000 rows 4.54, 4.50; 4097 5.87, 5.87; with
+// targets that are outliers 1000 rows 6.0, 4.50.  More tiles: 4096 rows 6.8, 8.1; 16384 6.3, 7.1; 58368 8.2, 9.6; with outliers 9.3 to 10.0, 9.6
+static bool one_tile(int rows, int clusters, int cluster) {
+  const int units = (rows + 31) / 32, ctas = clusters * cluster;
+  return (units + ctas - 1) / ctas <= 4;
+}
 cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters) {
-  return resident_launch_any<ResFp32>(cluster, tmap, g, st, max_clusters);
+  if (!max_clusters)
+    return one_tile(g.n_rows, g.clusters, cluster) ? launch_resident_fp32_ffma(cluster, tmap, g, st, nullptr)
+                                                   : resident_launch_any<ResFp32>(cluster, tmap, g, st, nullptr);
+  int n = 0;
+  cudaError_t e = resident_launch_any<ResFp32>(cluster, tmap, g, st, max_clusters);
+  if (e == cudaSuccess) e = launch_resident_fp32_ffma(cluster, tmap, g, st, &n);
+  if (e == cudaSuccess && n < *max_clusters) *max_clusters = n;
+  return e;
 }
 
 cudaError_t launch_resident_eval_fp32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
-  return resident_launch_eval<ResFp32>(tmap, g, st);
+  return one_tile(g.n_rows, g.clusters, 8) ? launch_resident_eval_fp32_ffma(tmap, g, st) : resident_launch_eval<ResFp32>(tmap, g, st);
 }
 
 }  // namespace mcmc_b200

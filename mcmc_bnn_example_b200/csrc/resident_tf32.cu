@@ -42,6 +42,7 @@ struct ResTf32 {
   static constexpr int TMEM_COLS = 512;
   static_assert(G_COL0 + GN <= TMEM_COLS, "tensor memory budget");
 
+  static constexpr bool X_PLACE = false;
   unsigned char* base;
   int wg, wtid, warp, lane, row, n_units;
   bool tile_active, warp_active, next_active, valid;

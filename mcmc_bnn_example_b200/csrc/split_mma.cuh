@@ -88,7 +88,9 @@ __device__ __forceinline__ void split_store_row(uint32_t a_t, int j, const float
            make_float4(p[q][4], p[q][5], p[q][6], p[q][7]));
 }
 
-// The 24 MMAs of a 128-row tile, by a converged warp (`on` in one lane): all products but rest x rest, smallest first
+// The 24 MMAs of a 128-row tile, by a converged warp (`on` in one lane): all products but rest x rest, smallest first.
+// (As a loop they take 150 cycles each, for want of operands that are constants apart; a predicate that keeps one from being issued
+// costs as much as the MMA)
 __device__ __forceinline__ void split_issue(uint32_t z_t, uint32_t a_t, uint32_t b_smem, uint32_t on) {
   constexpr uint32_t IDESC = umma_idesc_tf32(128, 48, 0, 0);
   const uint64_t b0 = umma_desc_k128(b_smem);
