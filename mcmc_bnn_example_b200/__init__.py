@@ -21,10 +21,11 @@ import numpy as np
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _ROOT = os.path.dirname(_HERE)
 LIB_PATH = os.path.join(_HERE, "libmcmc_b200.so")
-_SOURCES = ["api.cu", "chain.cu", "grad_fp32.cu", "grad_tf32.cu", "grad_tf32_wide.cu", "synth.cu", "noalloc.cu", "io.cu",
+_SOURCES = ["api.cu", "chain.cu", "grad_fp32.cu", "grad_fp32_int.cu", "grad_tf32.cu", "grad_tf32_wide.cu", "synth.cu", "noalloc.cu", "io.cu",
             "microbench.cu", "forward.cu", "resident_tf32.cu", "resident_fp32.cu",
             "resident_fp32_ffma.cu"]
-_HEADERS = ["common.cuh", "chain.cuh", "philox.h", "tc05.cuh", "resident.cuh", "refstream.cuh", "fp32_tile.cuh", "split_mma.cuh", "fp32_split.cuh"]
+_HEADERS = ["common.cuh", "chain.cuh", "philox.h", "tc05.cuh", "resident.cuh", "refstream.cuh", "fp32_tile.cuh", "split_mma.cuh", "fp32_split.cuh",
+            "int_mma.cuh"]
 
 OK = 0
 LIK_STUDENT_T, LIK_GAUSSIAN = 0, 1

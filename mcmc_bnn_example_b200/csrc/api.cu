@@ -154,6 +154,7 @@ struct mcmc_b200_ctx {
   int *tab_seg_ptr = nullptr, *tab_nslot = nullptr, *xtab_seg_ptr = nullptr, *xtab_nslot = nullptr;
   int4 *tab_segs = nullptr, *xtab_segs = nullptr;
   int tab_ctas = 0, xtab_ctas = 0;
+  bool tab_ints = false, xtab_ints = false;   // FP32: its segments are for grad_fp32_int.cu
   // chain state
   float *wbuf[2] = {}, *mbuf[2] = {}, *w_cur = nullptr, *g_cur = nullptr, *m0 = nullptr;
   float* partial[2] = {};
@@ -562,6 +563,16 @@ static bool plan_gradient(bool tf32, int H, int windows, long long tiles, int nu
   return tf32 || slices > 0 || !fp32_plain_faster(windows, tiles, num_sms, plan);
 }
 
+// FP32, 40 units: whether the sums over rows go by integers (grad_fp32_int.cu): a tile takes 1.1 us then instead of 1.39, a segment
+// 5 us instead of 3.  us a step, integers and FFMA, by tiles of a segment in the mean: 1 x 100000 rows (5) 18.5, 17.4; 200 x 2000 (9) 44.7, 43.4;
+// 4 x 58368 (12) 28.1, 26.9; 200 x 3000 (14) 57.6, 58.4; 60 x 8000 (18) 42.9, 44.1; 200 x 4000 (18) 69.5, 74.0; 6 x 58368 (18) 30.6, 34.8;
+// 149 x 5000 (20) 61.1, 68.2; 1 x 400000 (21) 34.9, 39.8; 16 x 40013 (31) 47.1, 57.1; 30 x 62000 (82) 122, 145
+static bool plan_ints(const mcmc_b200_config& cfg, const WorkPlan& plan) {
+  long long tiles = 0;
+  for (const int4& s : plan.segs) tiles += s.z - s.y;
+  return cfg.precision == MCMC_B200_PREC_FP32 && cfg.H == SPLIT_H && tiles >= 16 * (long long)plan.segs.size();
+}
+
 API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows, int64_t rows,
                          mcmc_b200_ctx** out) {
   if (!cfg || !out || n_windows < 1 || rows < 1) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
@@ -617,10 +628,12 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
     // window into that many fixed chunks (whole chunks per CTA): a window's result is then bit-identical
     // wherever and with whatever else it runs, at some cost in load balance.
     int r_ = upload_work_table(c, plan, &c->tab_seg_ptr, &c->tab_segs, &c->tab_nslot, &c->tab_ctas, &c->slices);
+    c->tab_ints = plan_ints(*cfg, plan);
     if (r_ == MCMC_B200_OK) {
       WorkPlan one;
       plan_work_table(1, n_tiles, c->num_sms, cfg->slices, tf32 ? TF32_SEG_COST : FP32_SEG_COST, one);
       r_ = upload_work_table(c, one, &c->xtab_seg_ptr, &c->xtab_segs, &c->xtab_nslot, &c->xtab_ctas, &c->slices_x);
+      c->xtab_ints = plan_ints(*cfg, one);
     }
     if (r_ != MCMC_B200_OK) { mcmc_b200_destroy(c); return r_; }
   } else {
@@ -971,7 +984,8 @@ static int launch_grad(mcmc_b200_ctx* c, GradParams g, bool single, cudaStream_t
     g.segs = single ? c->xtab_segs : c->tab_segs;
     const int ctas = single ? c->xtab_ctas : c->tab_ctas;
     e = c->cfg.precision == MCMC_B200_PREC_TF32 ? launch_grad_tf32(c->cfg.H, c->tmaps, g, ctas, st)
-                                                : launch_grad_fp32_split(g, ctas, st);
+                                                : (single ? c->xtab_ints : c->tab_ints) ? launch_grad_fp32_int(g, ctas, st)
+                                                                                        : launch_grad_fp32_split(g, ctas, st);
   } else {
     e = launch_grad_fp32(c->cfg.H, g, slots, single ? 1 : c->W, st);
   }

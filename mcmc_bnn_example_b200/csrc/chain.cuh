@@ -172,6 +172,8 @@ cudaError_t launch_grad_fp32(int H, const GradParams& g, int slices, int windows
 int fp32_max_ctas_per_sm(int H);
 // FP32, 40 units, the forward product on the tensor core: persistent, over the work table in `g`, or one window in `ctas` slices
 cudaError_t launch_grad_fp32_split(const GradParams& g, int ctas, cudaStream_t st);
+// ... the sums over rows there too
+cudaError_t launch_grad_fp32_int(const GradParams& g, int ctas, cudaStream_t st);
 // Launches of so few tiles are one latency after the other, of which that kernel has more: us a step of one window, without the tensor
 // core and with it, 4 tiles 7.8 and 9.0, 24 9.1 and 9.2, 32 9.3 and 9.4, 40 10.2 and 9.7, 148 11.7 and 10.6
 inline bool fp32_few_tiles(long long tiles) { return tiles <= 32; }

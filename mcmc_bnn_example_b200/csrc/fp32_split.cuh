@@ -63,27 +63,47 @@ struct SplitWarp {
       for (int i = 0; i < 2; ++i)
         z[2 * hf + i][4] = add2(pack2(s0[hf][2 * i], s0[hf][2 * i + 1]), pack2(s1[hf][2 * i], s1[hf][2 * i + 1]));
   }
-  // the same by FFMA, for values that split_wide finds: the lane's row, through es.  A weight is
-  // the sum of its parts (split_store_weight).  Even and odd features apart, added at the end
-  static __device__ __forceinline__ float plain_z(const float* x, const unsigned char* b, int j) {
-    float even = 0.f, odd = 0.f;
-#pragma unroll 1
-    for (int i = 0; i <= D; ++i) {
-      const int k = i == 0 ? D : i - 1;  // the bias first
-      const float* p = reinterpret_cast<const float*>(b + split_b_off(j, k & ~3)) + (k & 3);
-      const float w = p[0] + (p[SPLIT_B_PART / 4] + p[2 * (SPLIT_B_PART / 4)]);
-      if (i == 0) even = w;
-      else if (k & 1) odd = fmaf(x[k], w, odd);
-      else even = fmaf(x[k], w, even);
-    }
-    return even + odd;
-  }
+  // the same by FFMA, for values that split_wide finds: the lane's row, through es.  A weight is the sum of its parts
+  // (split_store_weight).  Even and odd features apart, added at the end.  UNITS side by side, four features' weights a load (58368 rows on the
+  // chip, Cauchy features: 31.5 us a step, 151 with a weight at a time); what registers more would need, a caller's loop loses
+  template <int UNITS>
   static __device__ __noinline__ void plain(const float* xb, const unsigned char* b, float* es) {
+    static_assert(D == 22 && KP == 24, "the bias is the third of the last four");
     const int lane = threadIdx.x & 31;
+    const float4* x = reinterpret_cast<const float4*>(xb + lane * KP);
+    auto weights = [&](int j, int c) {
+      const float4* p = reinterpret_cast<const float4*>(b + split_b_off(j, 4 * c));
+      const float4 hi = p[0], mid = p[SPLIT_B_PART / 16], lo = p[2 * (SPLIT_B_PART / 16)];
+      return make_float4(hi.x + (mid.x + lo.x), hi.y + (mid.y + lo.y), hi.z + (mid.z + lo.z), hi.w + (mid.w + lo.w));
+    };
 #pragma unroll 1
-    for (int j = 0; j < H; ++j) es[lane * H + j] = plain_z(xb + lane * KP, b, j);
+    for (int j = 0; j < H; j += UNITS) {
+      float even[UNITS], odd[UNITS];
+#pragma unroll
+      for (int u = 0; u < UNITS; ++u) {
+        even[u] = weights(j + u, KP / 4 - 1).z;  // the bias first
+        odd[u] = 0.f;
+      }
+#pragma unroll
+      for (int c = 0; c < KP / 4; ++c) {
+        const float4 v = x[c];
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+          const float4 w = weights(j + u, c);
+          even[u] = fmaf(v.x, w.x, even[u]);
+          odd[u] = fmaf(v.y, w.y, odd[u]);
+          if (c < KP / 4 - 1) {
+            even[u] = fmaf(v.z, w.z, even[u]);
+            odd[u] = fmaf(v.w, w.w, odd[u]);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < UNITS; ++u) es[lane * H + j + u] = even[u] + odd[u];
+    }
     __syncwarp();
   }
+
   __device__ __forceinline__ void load_plain(const float* es, uint64_t (&z)[4][5]) const {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -228,6 +248,50 @@ struct SplitWarp {
         for (int k = 0; k < KPT / 2; ++k) acc[k][u] = fma2(x[k], e2, acc[k][u]);
       }
     }
+  }
+
+  // backward and store_dw0 out of line, PAIRS pairs of features after others and acc in memory: what registers a call needs are lost to its
+  // caller's loop (streaming, 16 windows of 40013 rows: 49.0 us a step with all six pairs at once, 47.3 with one)
+  static constexpr int LEAN = KPT / 2 * UPT;
+  template <int PAIRS>
+  static __device__ __noinline__ void backward_lean(const float* xb, const float* es, uint64_t* acc) {
+    const SplitWarp lanes;
+#pragma unroll 1
+    for (int k = 0; k < KPT / 2; k += PAIRS) {
+      uint64_t a[PAIRS][UPT];
+#pragma unroll
+      for (int i = 0; i < PAIRS * UPT; ++i) a[i / UPT][i % UPT] = acc[k * UPT + i];
+#pragma unroll 2
+      for (int s = 0; s < ROWS / 2; ++s) {
+        const int row = 2 * s + lanes.rsub;
+        uint64_t x[PAIRS];
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) x[i] = lds64(xb + row * KP + lanes.kh * KPT + 2 * (k + i));
+        const float4 e4 = *reinterpret_cast<const float4*>(es + row * H + 4 * lanes.bcg);
+        const float e[UPT] = {e4.x, e4.y, e4.z, e4.w, es[row * H + 32 + lanes.bcg]};
+#pragma unroll
+        for (int u = 0; u < UPT; ++u)
+#pragma unroll
+          for (int i = 0; i < PAIRS; ++i) a[i][u] = fma2(x[i], pack2(e[u], e[u]), a[i][u]);
+      }
+#pragma unroll
+      for (int i = 0; i < PAIRS * UPT; ++i) acc[k * UPT + i] = a[i / UPT][i % UPT];
+    }
+    __syncwarp();
+  }
+  static __device__ __noinline__ void store_dw0_lean(const uint64_t* acc, float* out) {
+    const SplitWarp lanes;
+#pragma unroll 1
+    for (int k = 0; k < 3; ++k)
+#pragma unroll 1
+      for (int u = 0; u < UPT; ++u) {
+        const uint64_t lo = acc[k * UPT + u], hi = acc[(k + 3) * UPT + u];
+        float a, b;
+        unpack2(add2(lanes.rsub ? hi : lo, __shfl_xor_sync(0xffffffffu, lanes.rsub ? lo : hi, 16)), a, b);
+        const int unit = u < 4 ? 4 * lanes.bcg + u : 32 + lanes.bcg;
+        out[2 * k * H + unit] = a;
+        out[(2 * k + 1) * H + unit] = b;
+      }
   }
 };
 

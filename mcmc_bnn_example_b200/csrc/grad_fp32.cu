@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(FSP_THREADS, 1) grad_fp32_split_kernel(const G
         lanes.load(z_t, h);
         tc_fence_before();
         if (plain || plain_w) {
-          Warp::plain(xb, wb, es);
+          Warp::plain<1>(xb, wb, es);
           lanes.load_plain(es, h);
         }
         if (i + 1 < my_nt) plain = stage_rows(i + 1);

@@ -1,0 +1,507 @@
+// FP32 gradients of 40 units, rows streamed: forward product and sums over rows both on the tensor core (split_mma.cuh, int_mma.cuh,
+// fp32_split.cuh).  grad_fp32.cu has the kernel whose backward pass goes by FFMA, which stays for segments of few tiles (plan_ints in
+// api.cu draws the line).
+//
+// Persistent, one CTA per SM (a kernel with tensor memory gets no more), over the segments of the host's work table as in
+// grad_tf32.cu.  Four compute warpgroups take tiles of 128 rows in turn (a row per thread where rows are cut into parts and made
+// integers, 32 rows per warp everywhere else); one control warp issues the product's MMAs, another those of the sums.  Tensor memory: the
+// sums, 160 columns for the whole CTA (integers: their order is of no consequence), and two places for a tile's rows and accumulators,
+// which the tiles take in turn: z is in a warpgroup's registers soon after it is there.
+// Features' scales come from the segment's first tiles, that of dL/dpred from its very first one, with room for what the other rows
+// may have: 2^6 above the largest feature, 2^11 above the mean exponent.  A warp whose 32 rows have a value beyond that, or infinities or NaN, leaves
+// its part of the tile for the segment's end, where it goes by FFMA.  Gradients' error against 64 bits, here / there, segments of 23 to 228
+// tiles: N(0,1) features 0.75 to 0.99, feature by feature 0.5 to 0.9; ten other distributions 0.83 in the mean (FFMA adds up to 1,600 rows
+// in a chain; the room takes most of what bits are to spare for short ones).
+// A tile takes 2,200 cycles of an SM (FFMA 2,700) and 1,400 instructions a warp, issue slots half busy, MUFU 24 %, tensor pipe 32 %.  What an
+// instruction less gave was little; what a spill less gave was much, for shared memory leaves 28 KB of L1: hence the code for what is left over
+// in calls of few registers (47.3 us a step for 16 windows of 40013 rows; 49.0 with calls of many, 57 with their code in line).
+// Such a tile takes 9 us at its segment's end, side by side on 16 warps.
+// us a step, FFMA and here: 16 x 40013 rows 57.9, 48.0; 25 x 58368 118, 101; 100 x 10000 87.0, 75.6; 6 x 58368 35.5, 31.0; with 22 lognormal
+// features (sigma 1.5) 57.8, 58.2 and 35.5, 40.3 for the first and last, with Cauchy ones 112 and 159 here; targets with outliers of 300
+// sigma: the same as without.
+#include "fp32_split.cuh"
+
+namespace mcmc_b200 {
+
+constexpr int FIN_TILE = 128;
+
+constexpr int FIN_NWG = 4, FIN_THREADS = FIN_NWG * 128 + 128;
+// registers: 640 threads start with 96 each (4 * 128 * 112 + 128 * 32 = 61,440)
+constexpr int FIN_COMPUTE_REGS = 112, FIN_CTRL_REGS = 32;
+constexpr int FIN_SUB = 1000;                      // tiles of a segment between two read-outs: 2^17 rows' integers fit
+constexpr int FIN_ROOM_X = 6, FIN_ROOM_E = 11;      // above the first tiles' largest feature; above the mean exponent of dL/dpred
+struct FinGeom {
+  using Warp = SplitWarp;
+  static constexpr int NW = FIN_NWG * 4;
+  static constexpr int XS = Warp::ROWS * KP;           // floats of a warp's rows, and words of their integers
+  static constexpr int WARP = 2 * XS + Warp::ES;       // two stages of rows, dL/dz
+  static_assert(XS * 4 == INT_X_WARP && Warp::ES * 4 == INT_E_WARP && Warp::ES >= KP * SPLIT_H, "shared places");
+  static constexpr int WB = 0, ROWS0 = WB + SPLIT_B_BYTES / 4, S = ROWS0 + NW * WARP, W1 = S + INT_S_FLOATS, SCALE = W1 + SPLIT_H + 4;
+  static constexpr size_t SMEM = 1024 + (SCALE + KP) * 4;
+  static_assert(S % 4 == 0 && W1 % 4 == 0 && SCALE % 4 == 0, "vector alignment");
+  static constexpr int PLACE = SPLIT_A_COLS + SPLIT_Z_COLS, PLACE0 = INT_ACC_COLS, TMEM_COLS = 512;
+  static_assert(PLACE0 + 2 * PLACE <= TMEM_COLS, "tensor memory budget");
+};
+
+template <bool LOSS>
+__global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const GradParams g) {
+  using G = FinGeom;
+  using Warp = SplitWarp;
+  constexpr int D = SPLIT_D, H = SPLIT_H, P = Warp::P, NWG = FIN_NWG, NW = G::NW, NCOMPUTE = NWG * 128;
+  constexpr uint32_t WARP_BYTES = G::XS * sizeof(float);
+
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* const wb = smem_align1024(smem_raw);
+  float* const base = reinterpret_cast<float*>(wb);
+  float* const w1 = base + G::W1;       // W1, b1
+  float* const x_scale = base + G::SCALE;
+  // rows of a warp landed; per place, product done and read; per warpgroup, sums done; the scale is known
+  __shared__ __align__(8) uint64_t bar_rows[NW][2], bar_fwd[2], bar_read[2], bar_sum[NWG], bar_scale;
+  __shared__ uint32_t tmem_slot, x_stat[KP], x_max[KP], e_stat, none;
+  __shared__ uint32_t far[NW];                  // the warp's rows of its tile are not among the integers
+  constexpr int FAR_WORDS = (FIN_SUB / NWG + 31) / 32;
+  __shared__ uint32_t far_tiles[NW][FAR_WORDS], far_any[NW];   // ... earlier: which tiles of the part
+  __shared__ __align__(8) float red_w1[NW][H];
+  __shared__ float red_db1[NW];
+  __shared__ double red_ll[NW];
+
+  const Warp lanes;
+  const int tid = threadIdx.x, lane = lanes.lane;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const bool is_ctrl = warp >= NW;
+  const int wg = warp >> 2;
+  const int seg0 = g.segs ? g.seg_ptr[blockIdx.x] : 0, seg1 = g.segs ? g.seg_ptr[blockIdx.x + 1] : 1;
+  auto segment = [&](int sg) {  // window, first tile, end tile, slot
+    if (g.segs) return g.segs[sg];
+    const int S = gridDim.x, s = blockIdx.x;
+    return make_int4(0, (int)((long long)s * g.n_tiles / S), (int)((long long)(s + 1) * g.n_tiles / S), s);
+  };
+  // Tiles are numbered through a CTA's segments: tile n is warpgroup n % 4's, takes place n % 2 and the warp's stage n / 4 % 2
+  float* const xs = base + G::ROWS0 + warp * G::WARP;
+  float* const es = xs + 2 * G::XS;
+  auto rows_at = [&](const int4& seg, int i) {  // rows of this warp in tile i of a segment
+    return g.xaug + (long long)(g.data_window0 + seg.x) * g.window_stride + ((size_t)(seg.y + i) * FIN_TILE + (warp & 3) * Warp::ROWS) * KP;
+  };
+  auto fetch = [&](int n, int sg, int n0) {  // tile n, in segment sg, whose first one is n0, or a later one
+    int4 seg = segment(sg);
+    while (n - n0 >= seg.z - seg.y) {
+      n0 += seg.z - seg.y;
+      if (++sg == seg1) return;
+      seg = segment(sg);
+    }
+    uint64_t* const bar = &bar_rows[warp][n >> 2 & 1];
+    mbar_expect_tx(bar, WARP_BYTES);
+    bulk_g2s(xs + (n >> 2 & 1) * G::XS, rows_at(seg, n - n0), WARP_BYTES, bar);
+  };
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                 "r"((uint32_t)G::TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (!is_ctrl && lane == 0) {
+    mbar_init(&bar_rows[warp][0], 1);
+    mbar_init(&bar_rows[warp][1], 1);
+    if ((warp & 3) == 0) mbar_init(&bar_sum[wg], 1);
+    if (warp < 2) {
+      mbar_init(&bar_fwd[warp], 1);
+      mbar_init(&bar_read[warp], 4);
+    }
+    if (warp == 0) mbar_init(&bar_scale, 4);
+    mbar_fence_init();
+  }
+  __syncwarp();
+  // The first rows may be fetched ahead of the dependency wait only when no kernel directly before
+  // this one in the stream wrote the dataset (inside a chain none does; right after a repack one did).
+  const bool early_rows = g.data_fresh == 0, fetches = !is_ctrl && lane == 0 && seg0 < seg1;
+  if (early_rows && fetches) fetch(wg, seg0, 0);
+  // what the MMAs read besides weights: feature 23, and the lines behind the last part
+  for (int i = tid; i < SPLIT_B_BYTES / 16; i += FIN_THREADS)
+    reinterpret_cast<float4*>(wb)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (tid < KP) x_stat[tid] = x_max[tid] = 0u;
+  if (tid == 0) e_stat = 0u;
+  if (tid < NW * FAR_WORDS) far_tiles[tid / FAR_WORDS][tid % FAR_WORDS] = 0u;
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  pdl_trigger();
+  pdl_wait();
+  if (!early_rows && fetches) fetch(wg, seg0, 0);
+
+  bool ok = true;
+  int code = 0;
+  auto wait = [&](uint64_t* bar, uint32_t parity, int c) {  // (in line: a call would cost the tile loop registers)
+    if (mbar_try_wait(bar, parity)) return;
+    for (uint32_t i = 0; ok && !mbar_try_wait_hint(bar, parity, 20000u); ++i)
+      if (i >= MBAR_WAIT_SLICES) {
+        ok = false;
+        code = c;
+      }
+  };
+  auto hand_over = [&](int id) {  // to a control warp; a warp whose waits hold it no longer does not get ahead of that one either
+    if (__all_sync(0xffffffffu, ok)) named_arrive(id, 160);
+    else named_sync(id, 160);
+  };
+  auto place = [&](int n) { return G::PLACE0 + (n & 1) * G::PLACE; };
+
+  // Every segment begins with a CTA-wide barrier and has three for each of its parts (of FIN_SUB tiles), executed by both roles:
+  //   S1 parameters staged   S2 all tiles of the part done   S3 sums read out   S4 and stored
+  int n0 = 0;  // number of the segment's first tile
+  if (is_ctrl) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FIN_CTRL_REGS));
+    const uint32_t on = elect_one(), tm = __shfl_sync(0xffffffffu, tmem, 0);
+    for (int sg = seg0; sg < seg1; ++sg) {
+      const int4 seg = segment(sg);
+      const int end = n0 + seg.z - seg.y;
+      __syncthreads_or(0);  // S1
+      int p0 = n0, n = n0, rows = n0;  // tiles whose product has been issued, whose rows have come
+      do {
+        const int p1 = min(p0 + FIN_SUB, end);
+        if (warp == NW) {
+          // A warpgroup brings the next part's first tile before this part's end, the third and fourth behind the products of the first two
+          for (; n < min(p1 + 2, end); ++n) {
+            if (n == rows) named_sync(BAR_ROWS0 + (rows++ & 3), 160);
+            if (n >= 2) wait(&bar_read[n & 1], (n - 2) >> 1 & 1, 103);
+            tc_fence_after();
+            split_issue(tm + place(n) + SPLIT_A_COLS, tm + place(n), smem_u32(wb), on);
+            tc_commit_if(&bar_fwd[n & 1], on);
+          }
+          for (; rows < min(p1 + NWG, end); ++rows) named_sync(BAR_ROWS0 + (rows & 3), 160);
+        } else if (warp == NW + 1) {
+          uint32_t more = 0u;
+          for (int n = p0; n < p1; ++n) {
+            named_sync(BAR_E0 + (n & 3), 160);
+            tc_fence_after();
+            const uint32_t skip = __ballot_sync(0xffffffffu, lane < 4 && reinterpret_cast<volatile uint32_t*>(far)[(n & 3) * 4 + (lane & 3)] != 0u);
+            const uint32_t w0 = smem_u32(base + G::ROWS0 + (n & 3) * 4 * G::WARP);
+            const uint64_t xd = int_x_desc(w0 + (n >> 2 & 1) * WARP_BYTES), ed = int_e_desc(w0 + 2 * WARP_BYTES);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (!(skip >> i & 1)) {
+                int_mma_if(tm, umma_desc_advance(xd, i * (G::WARP * 4 >> 4)), umma_desc_advance(ed, i * (G::WARP * 4 >> 4)), more, on);
+                more = 1u;
+              }
+            tc_commit_if(&bar_sum[n & 3], on);
+          }
+          if (p1 > p0) wait(&bar_sum[(p1 - 1) & 3], (p1 - 1) >> 2 & 1, 104);
+          if (lane == 0) none = more ^ 1u;
+        }
+        __syncthreads();  // S2
+        __syncthreads();  // S3
+        __syncthreads();  // S4
+        p0 += FIN_SUB;
+      } while (p0 < end);
+      n0 = end;
+    }
+    if (!ok) atomicExch(g.status, code);
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FIN_COMPUTE_REGS));
+    const uint32_t sub = (uint32_t)((warp & 3) * 32) << 16;
+    const int own = lanes.own();
+    for (int sg = seg0; sg < seg1; ++sg) {
+      const int4 seg = segment(sg);
+      const int win = seg.x, end = n0 + seg.z - seg.y;
+      const int first = n0 + ((wg - n0) & 3);  // this warpgroup's first tile
+      bool wide = false;
+      {
+        // fused leapfrog update; parameters land where the MMAs read them
+        constexpr int N = (P + NCOMPUTE - 1) / NCOMPUTE;
+        float w[N];
+        leapfrog_params(g, win, tid, NCOMPUTE, P, seg.w == 0, w);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          const int p = tid + i * NCOMPUTE;
+          if (p < D * H + H) {
+            const int k = p / H, n = p - k * H;
+            wide |= split_store_weight(smem_u32(wb) + split_b_off(n, k & ~3) + (k & 3) * 4, w[i]);
+          } else if (p < P) {
+            w1[p - (D * H + H)] = w[i];
+          }
+        }
+        fence_proxy_async_smem();
+      }
+      if (first < end) {  // features' statistics
+        wait(&bar_rows[warp][first >> 2 & 1], first >> 3 & 1, 101);
+        if (lane <= D) {  // (a lane a feature: reductions over the warp took 2,700 cycles)
+          const float* x = xs + (first >> 2 & 1) * G::XS + lane;
+          uint32_t st = 0u, mx = 0u;
+#pragma unroll 16
+          for (int r = 0; r < Warp::ROWS; ++r) {
+            const float v = x[r * KP];
+            st += int_stat(v);
+            mx = max(mx, __float_as_uint(v) & 0x7fffffffu);
+          }
+          atomicAdd(&x_stat[lane], st);
+          atomicMax(&x_max[lane], mx);
+        }
+      }
+      const bool plain_w = __syncthreads_or(wide) != 0;  // S1
+      if (lane < KP) {  // (every warp writes the same)
+        const uint32_t st = *reinterpret_cast<volatile uint32_t*>(&x_stat[lane]), mx = *reinterpret_cast<volatile uint32_t*>(&x_max[lane]);
+        const int e = lane <= D && st ? min(int_scale_exp(st, 2 * FIN_ROOM_X), int_max_exp(mx) + FIN_ROOM_X) : 127;
+        x_scale[lane] = lane <= D ? int_scale_ok(e) ? int_scale(e) : __int_as_float(0x7f800000) : 0.f;  // (infinite: beyond any range)
+      }
+      __syncwarp();
+
+      bool plain = false, x_far = false;   // of the tile that comes next: rows for plain FFMA, a feature beyond its range
+      float y = 0.f;
+      // a tile's rows, once they have landed: to tensor memory, and integers in their own place
+      auto stage_rows = [&](int n) {
+        float* const xb = xs + (n >> 2 & 1) * G::XS;
+        wait(&bar_rows[warp][n >> 2 & 1], n >> 3 & 1, 101);
+        if (n >= 2) wait(&bar_fwd[n & 1], (n - 2) >> 1 & 1, 102);
+        tc_fence_after();
+        y = xb[own * KP + COL_Y];
+        float v[KP];
+#pragma unroll
+        for (int ch = 0; ch < KP / 4; ++ch) {
+          const float4 v4 = *reinterpret_cast<const float4*>(xb + lane * KP + 4 * ch);
+          v[4 * ch] = v4.x;
+          v[4 * ch + 1] = v4.y;
+          v[4 * ch + 2] = v4.z;
+          v[4 * ch + 3] = ch == KP / 4 - 1 ? 0.f : v4.w;
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const float p[8] = {v[8 * j], v[8 * j + 1], v[8 * j + 2], v[8 * j + 3], v[8 * j + 4], v[8 * j + 5], v[8 * j + 6], v[8 * j + 7]};
+          split_store_row(tmem + place(n) + sub, j, p);
+        }
+        tc_wait_st();
+        tc_fence_before();
+        hand_over(BAR_ROWS0 + wg);
+        __syncwarp();  // every lane has read its row
+        float top = 0.f;
+#pragma unroll
+        for (int ch = 0; ch < KP / 4; ++ch) {
+          const float4 s = *reinterpret_cast<const float4*>(x_scale + 4 * ch);
+          const uint64_t a = pack2(v[4 * ch], v[4 * ch + 1]), b = pack2(v[4 * ch + 2], v[4 * ch + 3]);
+          const uint64_t sa = pack2(s.x, s.y), sb = pack2(s.z, s.w);
+          float t0, t1;
+          unpack2(mul2(a, sa), t0, t1);
+          top = split_max(top, t0, t1);
+          unpack2(mul2(b, sb), t0, t1);
+          top = split_max(top, t0, t1);
+          const uint2 da = int_digits2(a, sa), db = int_digits2(b, sb);
+          *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(xb) + int_x_off(lane, ch)) = make_uint4(da.x, da.y, db.x, db.y);
+        }
+        x_far = !__all_sync(0xffffffffu, top < INT_TOP);
+        plain = false;
+        if (__builtin_expect(x_far, 0)) {  // (a value from 2^60 on is beyond any range)
+          top = 0.f;
+#pragma unroll
+          for (int k = 0; k < KP; k += 2) top = split_max(top, v[k], v[k + 1]);
+          plain = __any_sync(0xffffffffu, split_wide(top)) != 0;
+        }
+      };
+      uint64_t dw1[5] = {};
+      float db1 = 0.f, scale = 0.f;
+      double llacc = 0.0;
+      bool scaled = false;
+      if (first < end) stage_rows(first);
+
+      int p0 = n0;
+      do {
+        const int p1 = min(p0 + FIN_SUB, end), pf = p0 + ((wg - p0) & 3);
+        bool any_far = false;
+#pragma unroll 1
+        for (int n = pf; n < p1; n += NWG) {
+          wait(&bar_fwd[n & 1], n >> 1 & 1, 102);
+          tc_fence_after();
+          uint64_t h[4][5];
+          lanes.load(tmem + place(n) + SPLIT_A_COLS + sub, h);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar_read[n & 1]);
+          if (n >= NWG) wait(&bar_sum[wg], (n - NWG) >> 2 & 1, 104);  // the last tile's integers have been read
+          if (lane == 0) {
+            if (n + NWG < end) {
+              uint64_t* const bar = &bar_rows[warp][(n + NWG) >> 2 & 1];
+              mbar_expect_tx(bar, WARP_BYTES);
+              bulk_g2s(xs + ((n + NWG) >> 2 & 1) * G::XS, rows_at(seg, n + NWG - n0), WARP_BYTES, bar);
+            } else {
+              fetch(n + NWG, sg, n0);
+            }
+          }
+          const int row = (seg.y + n - n0) * FIN_TILE + (warp & 3) * Warp::ROWS + own;
+          const bool valid = row < g.n_rows;
+          float d[4], dy, pred;
+          lanes.front(h, w1, g.lik, y, valid, d, dy, pred, [](int) {});
+          if (!scaled) {
+            if (n == n0) {
+              const uint32_t st = __reduce_add_sync(0xffffffffu, int_stat(dy));
+              if (lane == 0) {
+                if (st && !plain && !plain_w) atomicMax(&e_stat, int_stat_word(int_scale_exp(st, FIN_ROOM_E)));
+                mbar_arrive(&bar_scale);
+              }
+            }
+            wait(&bar_scale, (sg - seg0) & 1, 105);
+            const int e = int_stat_exp(*reinterpret_cast<volatile uint32_t*>(&e_stat));
+            scale = int_scale_ok(e) ? int_scale(e) : 0.f;
+            scaled = true;
+          }
+          const bool near = scale > 0.f && !x_far && !plain_w && __all_sync(0xffffffffu, fabsf(dy) * scale < INT_TOP);
+          if (__builtin_expect(near, 1)) {
+            lanes.store_ei(h, d, scale, es, dw1);
+            fence_proxy_async_smem();
+          } else {
+            const int b = (n - pf) >> 2;  // (all of the tile is for later)
+            if (lane == 0) far_tiles[warp][b >> 5] |= 1u << (b & 31);
+            any_far = true;
+          }
+          if (lane == 0) far[warp] = near ? 0u : 1u;
+          hand_over(BAR_E0 + wg);
+          if (near) {
+            if (LOSS) {
+              const float loss = valid ? lik_loss(g.lik, y, pred) : 0.f;
+              llacc += (double)loss;
+              store_row_loss(g.row_loss, (long long)win * g.row_loss_stride + row, loss, valid);
+            }
+            db1 += dy;
+          }
+          if (n + NWG < end) stage_rows(n + NWG);
+        }
+        // ---- rows that are not among the integers: by FFMA, their sums where dL/dz was ----
+        if (__builtin_expect(any_far, 0)) {
+          const int last = pf + (p1 - 1 - pf) / NWG * NWG;
+          wait(&bar_sum[wg], last >> 2 & 1, 104);
+          float* const xb = xs + (last >> 2 & 1) * G::XS;
+          uint64_t acc[Warp::LEAN];
+          for (int i = 0; i < Warp::LEAN; ++i) acc[i] = 0ull;
+#pragma unroll 1
+          for (int n = pf; n < p1; n += NWG) {
+            const int b = (n - pf) >> 2;
+            if (!(reinterpret_cast<volatile uint32_t*>(far_tiles[warp])[b >> 5] >> (b & 31) & 1u)) continue;
+            const float4* src = reinterpret_cast<const float4*>(rows_at(seg, n - n0));
+            __syncwarp();
+            for (int i = lane; i < G::XS / 4; i += 32) reinterpret_cast<float4*>(xb)[i] = src[i];
+            __syncwarp();
+            uint64_t h[4][5];
+            float d[4], dy, pred;
+            Warp::plain<2>(xb, wb, es);
+            lanes.load_plain(es, h);
+            __syncwarp();
+            const int row = (seg.y + n - n0) * FIN_TILE + (warp & 3) * Warp::ROWS + own;
+            const bool valid = row < g.n_rows;
+            const float yf = xb[own * KP + COL_Y];
+            lanes.front(h, w1, g.lik, yf, valid, d, dy, pred, [](int) {});
+            lanes.store_es(h, d, es, dw1);
+            if (LOSS) {
+              const float loss = valid ? lik_loss(g.lik, yf, pred) : 0.f;
+              llacc += (double)loss;
+              store_row_loss(g.row_loss, (long long)win * g.row_loss_stride + row, loss, valid);
+            }
+            db1 += dy;
+            Warp::backward_lean<2>(xb, es, acc);
+          }
+          Warp::store_dw0_lean(acc, es + (lanes.kh * Warp::KPT + lanes.rsub * 6) * H);
+          for (int i = lane; i < FAR_WORDS; i += 32) far_tiles[warp][i] = 0u;
+          fence_proxy_async_smem();
+        }
+        if (lane == 0) far_any[warp] = any_far ? 1u : 0u;
+        // ---- lanes -> warp ----
+        if (p1 == end) {
+          lanes.store_dw1(dw1, red_w1[warp]);
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            db1 += __shfl_xor_sync(0xffffffffu, db1, o);
+            llacc += __shfl_xor_sync(0xffffffffu, llacc, o);
+          }
+          if (lane == 0) {
+            red_db1[warp] = db1;
+            red_ll[warp] = llacc;
+          }
+        }
+        __syncthreads();  // S2
+        tc_fence_after();
+        if ((warp & 3) < INT_LINES / 32) {
+          const float xsc = x_scale[(warp & 3) * 8 + (lane >> 2)];
+          const int e = int_stat_exp(e_stat);
+          float v[10];
+          int_read_out_long<10>(tmem + wg * 40 + sub, v);
+          const float f = xsc > 0.f ? (float)(1 << 8 * (lane & 3)) / xsc : 0.f, inv = int_scale_ok(e) ? int_unscale(e) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 10; ++j)
+            base[G::S + (wg * 10 + j) * INT_S_STR + (warp & 3) * 32 + lane] = none ? 0.f : v[j] * f * inv;
+        }
+        tc_fence_before();
+        __syncthreads();  // S3
+        // ---- one partial vector for (window, slot) ----
+        const size_t slot = (size_t)win * g.slices_out + seg.w;
+        float* po = g.partial_out + slot * g.Pp;
+        // warps in the order of the segment's tiles, whichever warpgroup took its first one: bits depend on the segment alone
+        auto nth = [&](int i) __attribute__((always_inline)) { return ((n0 + (i >> 2)) & 3) << 2 | (i & 3); };
+        const uint32_t far_w = __ballot_sync(0xffffffffu, lane < NW && far_any[nth(lane & (NW - 1))] != 0u);
+        for (int p = tid; p < P; p += NCOMPUTE) {
+          float s;
+          if (p < D * H + H) {
+            s = int_sum4(base + G::S, p / H, p % H);
+            for (uint32_t r = far_w; r; r &= r - 1) s += base[G::ROWS0 + nth(__ffs(r) - 1) * G::WARP + 2 * G::XS + p];
+            s *= w1[p % H];   // dL/dz was left without it
+            if (p0 > n0) s += po[p];
+          } else if (p1 < end) {
+            continue;
+          } else if (p < D * H + 2 * H) {
+            const int u = p - (D * H + H);
+            s = red_w1[nth(0)][u];
+#pragma unroll
+            for (int w = 1; w < NW; ++w) s += red_w1[nth(w)][u];
+          } else {
+            s = red_db1[nth(0)];
+#pragma unroll
+            for (int w = 1; w < NW; ++w) s += red_db1[nth(w)];
+          }
+          po[p] = s;
+        }
+        if (tid == 0 && p1 == end) {
+          double s = red_ll[nth(0)];
+#pragma unroll
+          for (int w = 1; w < NW; ++w) s += red_ll[nth(w)];
+          g.ll_out[slot] = s;
+        }
+        if (p1 == end) {
+          if (tid < KP) x_stat[tid] = x_max[tid] = 0u;
+          if (tid == 0) e_stat = 0u;
+        }
+        __syncthreads();  // S4: the next segment's parameters may take the place of this one's
+        p0 += FIN_SUB;
+      } while (p0 < end);
+      n0 = end;
+    }
+    if (g.test_code == 102) wait(&bar_fwd[0], (n0 + 1) >> 1 & 1, 102);  // (nothing ends this phase)
+    if (!ok) {  // copies and MMAs that did not arrive in time
+      atomicExch(g.status, code);
+      for (int n = max(n0 - 2 * NWG, 0); n < n0; ++n) {
+        if ((n & 3) != wg) continue;
+        mbar_drain(&bar_rows[warp][n >> 2 & 1], n >> 3 & 1);
+        if (n >= n0 - 2) mbar_drain(&bar_fwd[n & 1], n >> 1 & 1);
+        if (n >= n0 - NWG) mbar_drain(&bar_sum[wg], n >> 2 & 1);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)G::TMEM_COLS)
+                 : "memory");
+}
+
+template <bool LOSS>
+static cudaError_t launch_int_t(const GradParams& g, int ctas, cudaStream_t st) {
+  static bool attr_done[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !attr_done[dev]) {
+    cudaError_t e =
+        cudaFuncSetAttribute(grad_fp32_int_kernel<LOSS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FinGeom::SMEM);
+    if (e != cudaSuccess) return e;
+    if (dev < 64) attr_done[dev] = true;
+  }
+  return launch_chain_kernel(grad_fp32_int_kernel<LOSS>, dim3(ctas), dim3(FIN_THREADS), FinGeom::SMEM, st, g);
+}
+cudaError_t launch_grad_fp32_int(const GradParams& g, int ctas, cudaStream_t st) {
+  return g.no_loss ? launch_int_t<false>(g, ctas, st) : launch_int_t<true>(g, ctas, st);
+}
+
+}  // namespace mcmc_b200

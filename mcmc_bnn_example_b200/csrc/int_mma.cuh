@@ -101,6 +101,19 @@ __device__ __forceinline__ void int_read_out(uint32_t t, float f, float (&out)[N
     out[j] = fmaf((float)(v3 * 256 + v2), 65536.f, (float)(v1 + (v0 >> 8)) * 256.f) * f;
   }
 }
+// ... of any number of rows, without the factor
+template <int NU>
+__device__ __forceinline__ void int_read_out_long(uint32_t t, float (&out)[NU]) {
+  float a[4 * NU];
+#pragma unroll
+  for (int i = 0; i < NU / 2; ++i) tc_ld8(t + 8 * i, a + 8 * i);
+  tc_wait_ld();
+#pragma unroll
+  for (int j = 0; j < NU; ++j) {
+    const float s = fmaf((float)__float_as_int(a[4 * j + 1]), 256.f, (float)__float_as_int(a[4 * j]));
+    out[j] = fmaf((float)__float_as_int(a[4 * j + 3]), 16777216.f, fmaf((float)__float_as_int(a[4 * j + 2]), 65536.f, s));
+  }
+}
 // the sum over a feature's four lines
 __device__ __forceinline__ float int_sum4(const float* s, int k, int unit) {
   const float4 v = *reinterpret_cast<const float4*>(s + unit * INT_S_STR + 4 * k);

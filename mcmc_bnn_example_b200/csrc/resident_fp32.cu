@@ -317,7 +317,7 @@ struct ResFp32 {
       tc_fence_after();
       if (__builtin_expect(plain, 0)) {
         rows_to_floats();
-        Warp::plain(base + XI + warp * 32 * KP, reinterpret_cast<const unsigned char*>(base + WB), es);
+        Warp::plain<2>(base + XI + warp * 32 * KP, reinterpret_cast<const unsigned char*>(base + WB), es);
         lanes.load_plain(es, h);
       } else {
         lanes.load(tmem + z_col(wg) + ((uint32_t)((warp & 3) * 32) << 16), h);

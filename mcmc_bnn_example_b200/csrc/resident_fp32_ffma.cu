@@ -150,7 +150,7 @@ struct ResFp32Ffma {
     lanes.load(tmem + ((uint32_t)(warp * 32) << 16), h);
     tc_fence_before();
     if (plain) {
-      Warp::plain(xb, reinterpret_cast<const unsigned char*>(base + WB), es);
+      Warp::plain<2>(xb, reinterpret_cast<const unsigned char*>(base + WB), es);
       lanes.load_plain(es, h);
     }
     uint64_t dw1[5] = {};

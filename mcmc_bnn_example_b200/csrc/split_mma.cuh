@@ -79,9 +79,20 @@ __device__ __forceinline__ bool split_store_weight(uint32_t dst, float v) {
 // features 8 j .. 8 j + 7 of this thread's row (v[7] of j = 2 must be zero: column 23 is the target) to tensor memory
 template <int BITS = SPLIT_X_BITS>
 __device__ __forceinline__ void split_store_row(uint32_t a_t, int j, const float (&v)[8]) {
+  // (split_parts of two values at a time)
+  constexpr uint32_t HALF = 1u << (23 - BITS), KEEP = ~((1u << (24 - BITS)) - 1u);
+  const uint64_t minus1 = pack2(-1.f, -1.f);
   float p[3][8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) split_parts<BITS, false>(v[i], p[0][i], p[1][i], p[2][i]);
+  for (int i = 0; i < 8; i += 2) {
+    p[0][i] = __uint_as_float((__float_as_uint(v[i]) + HALF) & KEEP);
+    p[0][i + 1] = __uint_as_float((__float_as_uint(v[i + 1]) + HALF) & KEEP);
+    const uint64_t r = fma2(pack2(p[0][i], p[0][i + 1]), minus1, pack2(v[i], v[i + 1]));
+    unpack2(r, p[1][i], p[1][i + 1]);
+    const uint64_t cut = pack2(__uint_as_float(__float_as_uint(p[1][i]) & 0xffffe000u),
+                               __uint_as_float(__float_as_uint(p[1][i + 1]) & 0xffffe000u));
+    unpack2(fma2(cut, minus1, r), p[2][i], p[2][i + 1]);
+  }
 #pragma unroll
   for (int q = 0; q < 3; ++q)
     tc_st8(a_t + q * SPLIT_K + 8 * j, make_float4(p[q][0], p[q][1], p[q][2], p[q][3]),
