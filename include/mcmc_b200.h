@@ -397,7 +397,9 @@ int mcmc_b200_resident_plan(mcmc_b200_ctx* ctx, int explicit_calls, int* ctas_pe
  * at once.  What a B200 holds beyond 148, 74, 33 and 15 is not used: the order of
  * the sums, and with it every bit of a chain, then follows from precision, windows
  * and rows alone.  (An FP32 window of more than 4096 rows takes one cluster more
- * than a TF32 one where that leaves no CTA a fifth 32-row unit.) */
+ * than a TF32 one where that leaves no CTA a fifth 32-row unit.  From 2561 rows on
+ * an FP32 chain's window takes several clusters where that is faster; this is the
+ * chain's plan, explicit calls keep one cluster up to 4096 rows.) */
 int mcmc_b200_plan_resident_for(int precision, int windows, int64_t rows, int num_sms, const int32_t available[4],
                                 int32_t* ctas_per_cluster, int32_t* clusters);
 /* mcmc_b200_plan_resident_for(MCMC_B200_PREC_TF32, ...) */

@@ -393,21 +393,24 @@ constexpr int RES_CLUSTERS[4] = {148, 74, 33, 15};
 //   * rows that one cluster of 8 cannot hold: as many clusters of 8 as every window can have (up to 16) while each
 //     CTA still has at least four 32-row units (below that the step is all exchange and more CTAs only add to it).  FP32:
 //     as many as leave it at most four, since a fifth unit costs its scheduler a second round.
+//   * FP32 chains of more than RES_SPREAD units on one cluster: on several, if that leaves a CTA four units or one had 15 or 16
+//     (explicit calls keep one cluster: a call is as long as its launch and copies).
 // us a step by clusters, TF32: 4096 rows 4.2 (1), 4.2 (8); 4097 rows 3.9 (4, taken), 4.0 (5); 6000 rows 4.2 (3), 4.1 (5, taken),
-// 4.1 (6), 4.6 (15); 16384 rows 5.4 (4), 4.5 (8), 4.8 (15, taken).  FP32, tiles by FFMA as they were when the line was drawn: 4097 rows
-// 7.65 (4), 6.6 (5, taken); 6000 rows 8.1 (5), 6.7 (6, taken), 6.9 (8); 10000 rows 8.2 (9), 6.9 (10, taken); 13000 rows 8.3 (12), 7.1
-// (13, taken); three windows of 5000 rows 8.1 (4), 6.8 (5, taken); 16384 rows 8.4 (15, taken); 4096 rows 10.8 (1, taken), 6.9 (4).
-// What is taken, with the product on the tensor core: 4096 rows 7.9, 4097 5.8, 6000 5.9, 10000 6.1, 13000 6.1, three of 5000 5.9,
-// 16384 7.1.  So the rule is not the best one for a TF32 window of 16384 rows (8 and 15 clusters both give a CTA two 128-row
-// tiles) nor for an FP32 one of 4096.
+// 4.1 (6), 4.6 (15); 16384 rows 5.4 (4), 4.5 (8), 4.8 (15, taken): the rule is not the best one there (8 and 15 clusters both give a CTA two
+// 128-row tiles).  FP32, one cluster and several: 2048 rows 5.1, 5.2 (2); 2560 5.56, 5.46 (3); 3000 5.77, 5.49; 4096 6.81, 5.51 (4); four
+// windows of 4096 6.83, 6.23 (3 each, six units a CTA); seven of 2100, 3000 and 4096 5.55, 5.80, 6.83 and 6.09, 6.21, 6.39 (2 each).  Several:
+// 4097 rows 5.55 (5), 16384 6.3, 30000 6.6, 58368 8.3 (15); four units against five when tiles took twice as long: 6000 rows 6.7 (6), 8.1 (5).
 // Against one launch per step (one B200, 1 to 148 windows of 100 to 61440 rows that fit, 10-step iterations): 1.13 (FP32, one window of
-// 4096 rows: 8.2 and 9.2 us a step; 58368 rows 9.9 and 14.6) to 3.2 times as fast, so every window that fits goes this way.
+// 4096 rows when it took 8.2 us a step; 58368 rows 9.9 and 14.6) to 3.2 times as fast, so every window that fits goes this way.
+constexpr int RES_SPREAD = 80;
 template <typename F>
-static bool resident_plan(long long rows, int windows, int num_sms, bool fp32, F available, int* cluster, int* clusters) {
+static bool resident_plan(long long rows, int windows, int num_sms, bool fp32, bool chain, F available, int* cluster, int* clusters) {
   const long long units = (rows + 31) / 32;
   auto count = [&](int i) { return std::min(RES_CLUSTERS[i], available(i)); };
   if ((long long)windows * ((units + RES_UNITS - 1) / RES_UNITS) > num_sms) return false;
-  for (int i = 3; i >= 0; --i)
+  const long long share = windows <= RES_CLUSTERS[3] / 2 ? std::min<long long>(count(3) / windows, RES_MAX_CLUSTERS) : 1;
+  const bool spread = fp32 && chain && units > RES_SPREAD && share > 1 && (share >= (units + 31) / 32 || units > 112);
+  for (int i = 3; i >= 0 && !spread; --i)
     if (units <= (long long)RES_UNITS << i && windows <= RES_CLUSTERS[i] && windows <= count(i)) {
       *cluster = 1 << i;
       *clusters = 1;
@@ -431,7 +434,7 @@ static size_t resident_words_stride(int P, int cluster) {
 // enough for any plan of the context: only windows of several clusters of eight send such words
 static size_t resident_msg_bytes(const mcmc_b200_ctx* c, int windows) {
   const int clusters = std::min(RES_CLUSTERS[3] / windows, RES_MAX_CLUSTERS);
-  if (clusters < 2 || c->rows <= 8 * RES_UNITS * 32) return 0;
+  if (clusters < 2 || c->rows <= (c->cfg.precision == MCMC_B200_PREC_FP32 ? RES_SPREAD : 8 * RES_UNITS) * 32) return 0;
   return (size_t)2 * windows * clusters * 8 * resident_words_stride(c->P, 8) * 16;
 }
 
@@ -473,7 +476,7 @@ static bool use_resident(mcmc_b200_ctx* c, bool x, int L) {
   bool &asked = x ? c->res_x_asked : c->res_asked, &ok = x ? c->res_x_ok : c->res_ok;
   if (!asked) {
     ResidentParams& g = x ? c->res_x : c->res;
-    ok = resident_plan(c->rows, g.windows, c->num_sms, c->cfg.precision == MCMC_B200_PREC_FP32,
+    ok = resident_plan(c->rows, g.windows, c->num_sms, c->cfg.precision == MCMC_B200_PREC_FP32, !x,
                        [&](int i) { return resident_max_clusters(c, i); }, x ? &c->res_x_cluster : &c->res_cluster, &g.clusters);
     asked = true;
   }
@@ -495,7 +498,7 @@ API int mcmc_b200_plan_resident_for(int precision, int windows, int64_t rows, in
       !available || !ctas_per_cluster || !clusters)
     return fail(MCMC_B200_ERR_INVALID, "bad arguments");
   int C = 0, K = 0;
-  if (!resident_plan(rows, windows, num_sms, precision == MCMC_B200_PREC_FP32, [&](int i) { return available[i]; }, &C, &K))
+  if (!resident_plan(rows, windows, num_sms, precision == MCMC_B200_PREC_FP32, true, [&](int i) { return available[i]; }, &C, &K))
     C = K = 0;
   *ctas_per_cluster = C;
   *clusters = K;

@@ -66,6 +66,16 @@ def test_resident_launch_matches_oracle_and_per_step_launches(built, monkeypatch
         assert abs(g1["loglik"] - g2["loglik"]) <= 1e-6 * abs(g2["loglik"])
 
 
+@pytest.mark.parametrize("W,rows,clusters", [(1, 2560, 1), (1, 2561, 3), (4, 3584, 1), (4, 3585, 3), (7, 4096, 2), (8, 4096, 1)])
+def test_fp32_chains_on_several_clusters_below_one_clusters_rows(built, monkeypatch, W, rows, clusters):
+    """Where a chain's window is dealt to several clusters although one would hold it; explicit calls keep one.  Results as above."""
+    m, _ = built
+    ctx = m.Context(m.reference_config(precision=0, sample_capacity=0), n_windows=W, rows=rows)
+    assert ctx.resident_plan() == (8, clusters) and ctx.resident_plan(explicit_calls=True) == (8, 1)
+    ctx.close()
+    test_resident_launch_matches_oracle_and_per_step_launches(built, monkeypatch, 0, W, rows)
+
+
 @pytest.mark.parametrize("prec", [0, 1])
 def test_a_wait_that_runs_out_reports_and_leaves_the_chain_where_it_was(built, prec):
     """One cluster of the window is left out of a launch, so that the others' waits for its words run out: by themselves,
