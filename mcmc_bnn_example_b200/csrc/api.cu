@@ -342,6 +342,7 @@ static int make_tensor_map(mcmc_b200_ctx* c) {
 struct WorkPlan {
   std::vector<int> seg_ptr, nslot;
   std::vector<int4> segs;
+  bool ints = false;  // FP32: sums over rows by integers
 };
 static void plan_work_table(int windows, long long tiles_per_window, int max_ctas, int chunks_per_window, double seg_cost,
                             WorkPlan& plan);
@@ -514,7 +515,9 @@ API int mcmc_b200_plan_resident(int windows, int64_t rows, int num_sms, const in
 // 50, 100 and 200 windows unchanged within 0.5 %
 // FP32, 40 units (a tile is 1.4 us): 200 windows of 2000 rows 45.1 us a step (3), 46.6 (5, 8, 12); 100 of 10000 rows 89.5, 90.1,
 // 93.4, 97.7; 25 of 58368 rows 123.0 (3, 5), 125.1
-constexpr double TF32_SEG_COST = 14.0, FP32_SEG_COST = 3.0;
+// ... by integers (1.1 us): 200 of 4000 rows 71.3 (3), 69.5 (4.5), 69.3 (6), 60 of 8000 43.9, 41.8, 41.1, 40 of 20000 62.8, 60.9, 59.8 (9:
+// 60.0), 25 of 58368 101.6, 100.1, 99.5 (9: 99.3)
+constexpr double TF32_SEG_COST = 14.0, FP32_SEG_COST = 3.0, FP32_INT_SEG_COST = 6.0;
 constexpr int FP32_START = 3;  // FP32 without a table: a CTA
 
 // CTAs per window of the FP32 kernel without a table.  All CTAs of a launch take the same time: what counts is how many rounds
@@ -558,22 +561,25 @@ static bool fp32_plain_faster(int windows, long long tiles, int num_sms, const W
   return (6.0 + 5.4 * ((tiles + k - 1) / k)) * rounds + 0.2 * k <= 2.0 + 1.53 * longest;
 }
 
+// FP32, 40 units: whether the sums over rows go by integers (grad_fp32_int.cu): a tile takes 1.1 us then instead of 1.39, a segment
+// 5 us instead of 3.  us a step, integers and FFMA, by tiles of a segment in the mean: 1 x 100000 rows (5) 18.5, 17.4; 200 x 2000 (9) 44.7, 43.4;
+// 4 x 58368 (12) 28.1, 26.9; 200 x 3000 (14) 57.6, 58.4; 60 x 8000 (18) 42.9, 44.1; 200 x 4000 (18) 69.5, 74.0; 6 x 58368 (18) 30.6, 34.8;
+// 149 x 5000 (20) 61.1, 68.2; 1 x 400000 (21) 34.9, 39.8; 16 x 40013 (31) 47.1, 57.1; 30 x 62000 (82) 122, 145
+// The line was drawn with the FFMA kernel's table; the other one gets its own afterwards.
+static void plan_ints(int windows, long long tiles, int num_sms, int slices, WorkPlan& plan) {
+  plan.ints = windows * tiles >= 16 * (long long)plan.segs.size();
+  if (plan.ints) plan_work_table(windows, tiles, num_sms, slices, FP32_INT_SEG_COST, plan);
+}
+
 // The work table of a launch over `windows` windows; false: that of the FP32 kernel without one.  With fixed `slices` FP32 has a table
 // always (40 units): bits must not depend on the number of windows.
 static bool plan_gradient(bool tf32, int H, int windows, long long tiles, int num_sms, int slices, WorkPlan& plan) {
   if (!tf32 && (H != SPLIT_H || (slices == 0 && fp32_few_tiles(windows * tiles)))) return false;
   plan_work_table(windows, tiles, num_sms, slices, tf32 ? TF32_SEG_COST : FP32_SEG_COST, plan);
-  return tf32 || slices > 0 || !fp32_plain_faster(windows, tiles, num_sms, plan);
-}
-
-// FP32, 40 units: whether the sums over rows go by integers (grad_fp32_int.cu): a tile takes 1.1 us then instead of 1.39, a segment
-// 5 us instead of 3.  us a step, integers and FFMA, by tiles of a segment in the mean: 1 x 100000 rows (5) 18.5, 17.4; 200 x 2000 (9) 44.7, 43.4;
-// 4 x 58368 (12) 28.1, 26.9; 200 x 3000 (14) 57.6, 58.4; 60 x 8000 (18) 42.9, 44.1; 200 x 4000 (18) 69.5, 74.0; 6 x 58368 (18) 30.6, 34.8;
-// 149 x 5000 (20) 61.1, 68.2; 1 x 400000 (21) 34.9, 39.8; 16 x 40013 (31) 47.1, 57.1; 30 x 62000 (82) 122, 145
-static bool plan_ints(const mcmc_b200_config& cfg, const WorkPlan& plan) {
-  long long tiles = 0;
-  for (const int4& s : plan.segs) tiles += s.z - s.y;
-  return cfg.precision == MCMC_B200_PREC_FP32 && cfg.H == SPLIT_H && tiles >= 16 * (long long)plan.segs.size();
+  if (tf32) return true;
+  if (slices == 0 && fp32_plain_faster(windows, tiles, num_sms, plan)) return false;
+  plan_ints(windows, tiles, num_sms, slices, plan);
+  return true;
 }
 
 API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows, int64_t rows,
@@ -631,12 +637,13 @@ API int mcmc_b200_create(const mcmc_b200_config* cfg, int device, int n_windows,
     // window into that many fixed chunks (whole chunks per CTA): a window's result is then bit-identical
     // wherever and with whatever else it runs, at some cost in load balance.
     int r_ = upload_work_table(c, plan, &c->tab_seg_ptr, &c->tab_segs, &c->tab_nslot, &c->tab_ctas, &c->slices);
-    c->tab_ints = plan_ints(*cfg, plan);
+    c->tab_ints = plan.ints;
     if (r_ == MCMC_B200_OK) {
       WorkPlan one;
       plan_work_table(1, n_tiles, c->num_sms, cfg->slices, tf32 ? TF32_SEG_COST : FP32_SEG_COST, one);
+      if (!tf32) plan_ints(1, n_tiles, c->num_sms, cfg->slices, one);
       r_ = upload_work_table(c, one, &c->xtab_seg_ptr, &c->xtab_segs, &c->xtab_nslot, &c->xtab_ctas, &c->slices_x);
-      c->xtab_ints = plan_ints(*cfg, one);
+      c->xtab_ints = one.ints;
     }
     if (r_ != MCMC_B200_OK) { mcmc_b200_destroy(c); return r_; }
   } else {
