@@ -159,20 +159,28 @@ struct ResFp32 {
       res_wait(bar_rows(), 0, g, g.wait_ticks << 2, 611, ok);
       if (!ok) res_drain(bar_rows(), 0, g);
       if (g.test_code == 611) res_wait(bar_rows(), 1, g, g.wait_ticks << 2, 611, ok);  // (nothing ends this phase)
-      const float* x = base + ES + tid * KP;
+      // (four values a load, and the columns' statistics a lane each: a float at a time, with reductions over the warp and every thread working
+      // out all scales, an evaluation took 6 us longer)
+      float v[KP];
+#pragma unroll
+      for (int ch = 0; ch < KP / 4; ++ch) {
+        const float4 x = active ? reinterpret_cast<const float4*>(base + ES + tid * KP)[ch] : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[4 * ch] = x.x;
+        v[4 * ch + 1] = x.y;
+        v[4 * ch + 2] = x.z;
+        v[4 * ch + 3] = x.w;
+      }
       if (active) {
         own(0) = base[ES + (warp * 32 + lanes.own()) * KP + COL_Y];
-        uint32_t st = 0u, mx = 0u;  // lane k: feature k
-#pragma unroll
-        for (int k = 0; k <= D; ++k) {
-          const uint32_t s = __reduce_add_sync(0xffffffffu, int_stat(x[k]));
-          const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(x[k]) & 0x7fffffffu);
-          if (lanes.lane == k) {
-            st = s;
-            mx = m;
-          }
-        }
         if (lanes.lane <= D) {
+          const float* x = base + ES + warp * 32 * KP + lanes.lane;
+          uint32_t st = 0u, mx = 0u;
+#pragma unroll 16
+          for (int r = 0; r < 32; ++r) {
+            const float f = x[r * KP];
+            st += int_stat(f);
+            mx = max(mx, __float_as_uint(f) & 0x7fffffffu);
+          }
           atomicAdd(&x_stat[lanes.lane], st);
           atomicMax(&x_max[lanes.lane], mx);
         }
@@ -181,13 +189,10 @@ struct ResFp32 {
         const uint32_t a_t = tmem + a_col(wg) + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-          float v[8];
+          const float r[8] = {v[8 * j], v[8 * j + 1], v[8 * j + 2], v[8 * j + 3], v[8 * j + 4], v[8 * j + 5], v[8 * j + 6], j == 2 ? 0.f : v[8 * j + 7]};
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            v[k] = active && 8 * j + k <= D ? x[8 * j + k] : 0.f;
-            wide |= split_wide(v[k]);
-          }
-          split_store_row(a_t, j, v);
+          for (int k = 0; k < 8; ++k) wide |= split_wide(r[k]);
+          split_store_row(a_t, j, r);
         }
         tc_wait_st();
         tc_fence_before();
@@ -197,23 +202,25 @@ struct ResFp32 {
       auto x_exp = [&](int k) {
         return x_stat[k] ? min(int_scale_exp(x_stat[k], INT_ROOM_X), int_max_exp(x_max[k])) : 127;
       };
-      bool in = true;
-#pragma unroll 1
-      for (int k = 0; k <= D; ++k) {
-        const int e = x_exp(k);
-        if (lanes.lane == 0 && warp == 0) x_scale[k] = int_scale_ok(e) ? int_scale(e) : 0.f;
-        in &= int_scale_ok(e) && (!active || fabsf(x[k]) * int_scale(e) < INT_TOP);
+      if (tid < KP) {  // (infinite: beyond any range; the target has none)
+        const int e = tid <= D ? x_exp(tid) : 127;
+        x_scale[tid] = tid > D ? 0.f : int_scale_ok(e) ? int_scale(e) : __int_as_float(0x7f800000);
       }
-      if (tid == 0) x_scale[D + 1] = 0.f;   // the target
-      if (!__all_sync(0xffffffffu, in)) rows_are = FLOATS;
       __syncthreads();
+      bool in = true;
+#pragma unroll
+      for (int ch = 0; ch < KP / 4; ++ch) {
+        const float4 f = reinterpret_cast<const float4*>(x_scale)[ch];
+        in &= fabsf(v[4 * ch]) * f.x < INT_TOP && fabsf(v[4 * ch + 1]) * f.y < INT_TOP && fabsf(v[4 * ch + 2]) * f.z < INT_TOP &&
+              (ch == KP / 4 - 1 || fabsf(v[4 * ch + 3]) * f.w < INT_TOP);
+      }
+      if (!__all_sync(0xffffffffu, in)) rows_are = FLOATS;
       float4* const xi = reinterpret_cast<float4*>(base + XI + warp * 32 * KP);
-      if (rows_are != INTS) {
-        for (int ch = 0; ch < KP / 4; ++ch) xi[lanes.lane * (KP / 4) + ch] = reinterpret_cast<const float4*>(x)[ch];
-      } else {
-        for (int ch = 0; ch < KP / 4; ++ch)
-          int_store_x4(smem_u32(xi) + int_x_off(lanes.lane, ch), active ? reinterpret_cast<const float4*>(x)[ch] : make_float4(0.f, 0.f, 0.f, 0.f),
-                       reinterpret_cast<const float4*>(x_scale)[ch]);
+#pragma unroll
+      for (int ch = 0; ch < KP / 4; ++ch) {
+        const float4 x = make_float4(v[4 * ch], v[4 * ch + 1], v[4 * ch + 2], v[4 * ch + 3]);
+        if (rows_are != INTS) xi[lanes.lane * (KP / 4) + ch] = x;
+        else int_store_x4(smem_u32(xi) + int_x_off(lanes.lane, ch), x, reinterpret_cast<const float4*>(x_scale)[ch]);
       }
       const int k = (warp & 3) * 8 + (lanes.lane >> 2);  // the line whose sums this lane reads
       const int e = k <= D ? x_exp(k) : 127;
