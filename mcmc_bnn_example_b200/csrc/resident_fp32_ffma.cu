@@ -1,7 +1,8 @@
-// Tile arithmetic of the resident kernel in FP32 mode for CTAs of one tile (128 rows) at most: the forward product on the tensor core
-// (split_mma.cuh), the backward pass by FFMA, every warp for itself (fp32_split.cuh).  resident_fp32.cu has the rest, and the line
-// between the two.  The rows' three parts stay in tensor memory for the launch, the rows themselves in shared memory.
-// us a step on one B200: 1000 rows (one cluster of eight) 4.5, 148 windows of 128 rows 4.2, 4097 rows (five clusters) 5.9.  A chain of
+// Tile arithmetic of the resident kernel in FP32 mode for CTAs of one tile (128 rows) at most, for single evaluations and for calls of
+// one step: the forward product on the tensor core (split_mma.cuh), the backward pass by FFMA, every warp for itself (fp32_split.cuh).
+// resident_fp32.cu has the rest, and the line between the two.  The rows' three parts stay in tensor memory for the launch, the rows
+// themselves in shared memory.
+// us a step on one B200: 1000 rows (one cluster of eight) 4.3, 148 windows of 128 rows 4.0, 4097 rows (five clusters) 5.5.  A chain of
 // latencies: weights cut up, 24 MMAs, 40 tanh a row, 960 products of 32 rows a warp (2,250 cycles), exchange (resident.cuh).
 #include <cuda.h>
 #include "fp32_split.cuh"
@@ -9,11 +10,12 @@
 
 namespace mcmc_b200 {
 
+template <int TILES>
 struct ResFp32Ffma {
   static constexpr int H = SPLIT_H, D = SPLIT_D;
   using Words = ResWords<H>;
   using Warp = SplitWarp;
-  static constexpr int NWARPS = RES_NWG * 4, ROW_WARPS = 4;   // the first four have rows, a 32-row unit each
+  static constexpr int NWARPS = RES_NWG * 4, ROW_WARPS = 4 * TILES;   // those with rows, a 32-row unit each
   // a warp's sums of dW0 and db0, after the shuffle over its two row subsets a lane's 6 features x 5 units: eight
   // floats between the feature groups make the stores free of bank conflicts.  They take the place of its dL/dz.
   static constexpr int GROUP = 6 * H, GSTR = GROUP + 8;
@@ -22,25 +24,36 @@ struct ResFp32Ffma {
   // float offsets
   static constexpr int WB = 0, XB = WB + SPLIT_B_BYTES / 4, ES = XB + ROW_WARPS * 32 * KP, W1 = ES + ROW_WARPS * Warp::ES,
                        RW1 = W1 + RS, RLL = RW1 + ROW_WARPS * RS, BAR = RLL + ROW_WARPS * 2;
-  static constexpr int NBARS = 2;   // rows landed; forward done
+  static constexpr bool TURNS = TILES > 1;
+  // barriers: rows landed; per tile, forward done; per accumulator buffer that tiles share, read
+  static constexpr int NZ = TURNS ? 2 : 1, NBARS = 1 + TILES + (TURNS ? NZ : 0);
   static constexpr size_t SMEM = 1024 + (BAR + 2 * NBARS) * 4;
   static_assert(XB % 4 == 0 && W1 % 4 == 0 && RW1 % 4 == 0 && RLL % 2 == 0 && BAR % 2 == 0, "vector alignment");
-  static constexpr int A_COL0 = SPLIT_Z_COLS, TMEM_COLS = 256;   // accumulators; the rows' parts for the whole launch
-  static_assert(A_COL0 + SPLIT_A_COLS <= TMEM_COLS, "tensor memory budget");
+  // accumulators, which the tiles take in turn; the rows' parts for the whole launch
+  static constexpr int A_COL0 = NZ * SPLIT_Z_COLS, TMEM_COLS = TURNS ? 512 : 256;
+  static_assert(A_COL0 + TILES * SPLIT_A_COLS <= TMEM_COLS, "tensor memory budget");
+  static __device__ __forceinline__ uint32_t a_col(int w) { return A_COL0 + w * SPLIT_A_COLS; }
+  static __device__ __forceinline__ uint32_t z_col(int w) { return w % NZ * SPLIT_Z_COLS; }
+  // named barriers: a warp's turn is over (those of the last four are not needed)
+  static constexpr int BAR_LO = 1, BAR_HI = 10;
+  static_assert(BAR_LO + 8 <= RES_BAR_X && BAR_HI > RES_BAR_X && BAR_HI + 4 <= 16, "barrier numbers");
+  __device__ __forceinline__ static int bar_turn(int w) { return w < 8 ? BAR_LO + w : BAR_HI + w - 8; }
   static constexpr bool X_PLACE = false;
   Warp lanes;
   float* base;
-  int warp, n_units;
+  int warp, wg, n_units;
   int row0;          // this warp's first row in the window
   bool active, plain_x, plain;
   uint32_t s_dst[3], tmem, par;
 
   __device__ __forceinline__ uint64_t* bar_rows() const { return reinterpret_cast<uint64_t*>(base + BAR); }
-  __device__ __forceinline__ uint64_t* bar_fwd() const { return bar_rows() + 1; }
+  __device__ __forceinline__ uint64_t* bar_fwd(int w) const { return bar_rows() + 1 + w; }
+  __device__ __forceinline__ uint64_t* bar_read(int b) const { return bar_rows() + 1 + TILES + b; }
 
   __device__ __forceinline__ ResFp32Ffma(unsigned char* b, const ResidentParams& g, int, int u0, int u1)
       : base(reinterpret_cast<float*>(b)) {
     warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    wg = TURNS ? warp >> 2 : 0;
     n_units = u1 - u0;
     active = warp < n_units;
     row0 = (u0 + warp) * 32;
@@ -69,7 +82,8 @@ struct ResFp32Ffma {
     }
     if (tid == 0) {
       mbar_init(bar_rows(), 1);
-      mbar_init(bar_fwd(), 1);
+      for (int w = 0; w < TILES; ++w) mbar_init(bar_fwd(w), 1);
+      for (int b = 0; TURNS && b < NZ; ++b) mbar_init(bar_read(b), 4);
       mbar_fence_init();
     }
     // sums that nothing writes stay zero: those of warps without rows; and what the last MMAs read behind the weights
@@ -92,9 +106,9 @@ struct ResFp32Ffma {
       res_wait(bar_rows(), 0, g, g.wait_ticks << 2, 611, ok);
       if (!ok) res_drain(bar_rows(), 0, g);
       if (g.test_code == 611) res_wait(bar_rows(), 1, g, g.wait_ticks << 2, 611, ok);  // (nothing ends this phase)
-      if (warp < ROW_WARPS) {  // the tile's rows to tensor memory, zeros for warps without rows
+      if (TURNS ? 4 * wg < n_units : warp < ROW_WARPS) {  // the tile's rows to tensor memory, zeros for warps without rows
         const float* x = base + XB + tid * KP;
-        const uint32_t a_t = tmem + A_COL0 + ((uint32_t)(warp * 32) << 16);
+        const uint32_t a_t = tmem + a_col(wg) + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           float v[8];
@@ -132,23 +146,31 @@ struct ResFp32Ffma {
     if (n_units == 0) return;
     const uint32_t ph = par;
     par ^= 1;
-    if (warp == NWARPS - 1) {  // (it has no rows)
+    const int nt = TURNS ? (n_units + 3) / 4 : 1;
+    if (warp == NWARPS - 1) {  // (rows of its own, if any, come last)
       const uint32_t on = elect_one(), tm = __shfl_sync(0xffffffffu, tmem, 0);
-      tc_fence_after();
-      split_issue(tm, tm + A_COL0, smem_u32(base + WB), on);
-      tc_commit_if(bar_fwd(), on);
+      for (int w = 0; w < nt; ++w) {
+        if (w >= NZ) res_wait(bar_read(w % NZ), ph, g, g.wait_ticks << 2, 613, ok);  // a buffer's second tile when its first has been read
+        tc_fence_after();
+        split_issue(tm + z_col(w), tm + a_col(w), smem_u32(base + WB), on);
+        tc_commit_if(bar_fwd(w), on);
+      }
       if (g.test_code == 613)  // (nothing ends the second phase)
-        for (uint32_t p = 0; p < 2; ++p) res_wait(bar_fwd(), ph ^ p, g, g.wait_ticks << 2, 613, ok);
+        for (uint32_t p = 0; p < 2; ++p) res_wait(bar_fwd(0), ph ^ p, g, g.wait_ticks << 2, 613, ok);
     }
     if (!active) return;
     const float* xb = base + XB + warp * 32 * KP;
     float* es = base + ES + warp * Warp::ES;
     const int left = g.n_rows - row0;
     uint64_t h[4][5];
-    res_wait(bar_fwd(), ph, g, g.wait_ticks << 2, 612, ok);
+    res_wait(bar_fwd(wg), ph, g, g.wait_ticks << 2, 612, ok);
     tc_fence_after();
-    lanes.load(tmem + ((uint32_t)(warp * 32) << 16), h);
+    lanes.load(tmem + z_col(wg) + ((uint32_t)((warp & 3) * 32) << 16), h);
     tc_fence_before();
+    if (TURNS && wg + NZ < nt) {  // another tile takes the buffer (so this one is full: all its warps come here)
+      __syncwarp();
+      if (lanes.lane == 0) mbar_arrive(bar_read(wg % NZ));
+    }
     if (plain) {
       Warp::plain<2>(xb, reinterpret_cast<const unsigned char*>(base + WB), es);
       lanes.load_plain(es, h);
@@ -158,9 +180,13 @@ struct ResFp32Ffma {
     const int own = lanes.own();
     const bool valid = own < left;
     const float y = xb[own * KP + COL_Y];
-    lanes.block(h, base + W1, g.lik, y, valid, es, dw1, dy, pred, [](int) {});
+    // (a scheduler's four warps take turns at the tanh: resident_fp32.cu)
+    if (TURNS && warp >= 4) named_sync(bar_turn(warp - 4), 64);
+    lanes.block(h, base + W1, g.lik, y, valid, es, dw1, dy, pred, [&](int i) {
+      if (TURNS && i == 3 && warp + 4 < n_units) named_arrive(bar_turn(warp), 64);
+    });
     if (last) {
-      if (g.test_code == 612) res_wait(bar_fwd(), ph ^ 1, g, g.wait_ticks << 2, 612, ok);  // (nothing ends this phase)
+      if (g.test_code == 612) res_wait(bar_fwd(wg), ph ^ 1, g, g.wait_ticks << 2, 612, ok);  // (nothing ends this phase)
       const float loss = valid ? lik_loss(g.lik, y, pred) : 0.f;
       store_row_loss(row_loss, row0 + own, loss, valid);
       double ld = (double)loss;
@@ -191,7 +217,7 @@ struct ResFp32Ffma {
     float s[3] = {};
     if (warp == LAST) {
       const float* r = base + RW1 + 3 * min(lanes.lane, NW1 - 1);
-#pragma unroll
+#pragma unroll 4
       for (int w = 0; w < ROW_WARPS; ++w)
 #pragma unroll
         for (int q = 0; q < 3; ++q) s[q] += r[w * RS + q];
@@ -209,10 +235,13 @@ struct ResFp32Ffma {
     }
     const int t = min((int)threadIdx.x, Words::W0 - 1);
     const float* gp = base + ES + 3 * t + 8 * (3 * t / GROUP);
+    // (four warps to a turn: straight code for sixteen took 1,100 of a step's cycles to fetch)
+#pragma unroll 1
+    for (int w0 = 0; w0 < (TURNS ? n_units : 1); w0 += 4, gp += 4 * Warp::ES)
 #pragma unroll
-    for (int w = 0; w < ROW_WARPS; ++w)
+      for (int w = 0; w < 4; ++w)
 #pragma unroll
-      for (int q = 0; q < 3; ++q) s[q] += gp[w * Warp::ES + q];
+        for (int q = 0; q < 3; ++q) s[q] += gp[w * Warp::ES + q];
     float o[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) o[q] = base[W1 + (3 * t + q) % H] * s[q];
@@ -224,20 +253,23 @@ struct ResFp32Ffma {
   __device__ __forceinline__ void teardown(const ResidentParams& g, const volatile int& dead) {
     tc_fence_before();
     __syncthreads();
-    if (warp == 0 && dead && n_units > 0) res_drain(bar_fwd(), par ^ 1, g);
+    if (warp == 0 && dead)
+      for (int w = 0; 4 * w < n_units; ++w) res_drain(bar_fwd(w), par ^ 1, g);
     if (warp == 0)
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS)
                    : "memory");
   }
 };
 
-cudaError_t launch_resident_fp32_ffma(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
-                                 int* max_clusters) {
-  return resident_launch_any<ResFp32Ffma>(cluster, tmap, g, st, max_clusters);
+cudaError_t launch_resident_fp32_ffma(bool one_tile, int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
+                                      int* max_clusters) {
+  return one_tile ? resident_launch_any<ResFp32Ffma<1>>(cluster, tmap, g, st, max_clusters)
+                  : resident_launch_any<ResFp32Ffma<RES_NWG>>(cluster, tmap, g, st, max_clusters);
 }
 
-cudaError_t launch_resident_eval_fp32_ffma(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
-  return resident_launch_eval<ResFp32Ffma>(tmap, g, st);
+cudaError_t launch_resident_eval_fp32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
+  return (g.n_rows + 31) / 32 <= 4 * 8 * g.clusters ? resident_launch_eval<ResFp32Ffma<1>>(tmap, g, st)
+                                                    : resident_launch_eval<ResFp32Ffma<RES_NWG>>(tmap, g, st);
 }
 
 }  // namespace mcmc_b200
