@@ -159,8 +159,8 @@ cudaError_t launch_resident_tf32(int cluster, const void* tmap, const ResidentPa
                                  int* max_clusters);
 cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters);
-// ... in FP32 by FFMA; one_tile: CTAs have 128 rows at most
-cudaError_t launch_resident_fp32_ffma(bool one_tile, int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
+// ... in FP32 of windows whose CTAs have 128 rows at most
+cudaError_t launch_resident_fp32_ffma(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                       int* max_clusters);
 // ... of an evaluation with its parameters, for clusters of eight
 cudaError_t launch_resident_eval_tf32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st);

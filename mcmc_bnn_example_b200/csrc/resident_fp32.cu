@@ -502,23 +502,21 @@ struct ResFp32 {
 // Windows whose CTAs have one tile at most take the tile arithmetic without integers (resident_fp32_ffma.cu): as fast there, and an outlier
 // costs it nothing.  us a step, integers and FFMA: 148 windows of 128 rows 4.43, 4.21; 1000 rows 4.54, 4.50; 4097 5.87, 5.87; with
 // targets that are outliers 1000 rows 6.0, 4.50.  More tiles: 4096 rows 6.8, 8.1; 16384 6.3, 7.1; 58368 8.2, 9.6; with outliers 9.3 to 10.0, 9.6.
-// So do evaluations and calls of a single step, for which making integers of the rows and a scale in the first step, 1 to 2 us together,
-// does not pay.  us a call, integers and FFMA: evaluations of 2048, 20000 and 58368 rows 37.0, 39.5, 42.4 and 35.3, 37.3, 41.0; one step of 2048,
-// 4096 and 20000 rows 30.3, 33.0, 32.4 and 29.0, 29.0, 32.0.  Two steps 33.4, 37.7, 36.9 and 37.6, 37.7, 44.2
+// So do evaluations on host pointers, for which making integers of the rows and a scale, 1 to 2 us together, does not pay.  us a call, integers
+// and FFMA: 2048, 20000 and 58368 rows 37.0, 39.5, 42.4 and 35.3, 37.3, 41.0.  (Calls of one step: 30.3, 32.4, 35.4 and 29.0, 32.0, 35.5; of two
+// 33.4, 36.9, 41.7 and 37.6, 44.2, 49.8.)
 static bool one_tile(int rows, int clusters, int cluster) {
   const int units = (rows + 31) / 32, ctas = clusters * cluster;
   return (units + ctas - 1) / ctas <= 4;
 }
 cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters) {
-  if (!max_clusters) {
-    const bool one = one_tile(g.n_rows, g.clusters, cluster);
-    return one || g.mode == RES_EVAL || (g.mode == RES_STEPS && g.n_steps == 1) ? launch_resident_fp32_ffma(one, cluster, tmap, g, st, nullptr)
-                                                          : resident_launch_any<ResFp32>(cluster, tmap, g, st, nullptr);
-  }
+  if (!max_clusters)
+    return one_tile(g.n_rows, g.clusters, cluster) ? launch_resident_fp32_ffma(cluster, tmap, g, st, nullptr)
+                                                   : resident_launch_any<ResFp32>(cluster, tmap, g, st, nullptr);
   int n = 0;
   cudaError_t e = resident_launch_any<ResFp32>(cluster, tmap, g, st, max_clusters);
-  if (e == cudaSuccess) e = launch_resident_fp32_ffma(true, cluster, tmap, g, st, &n);
+  if (e == cudaSuccess) e = launch_resident_fp32_ffma(cluster, tmap, g, st, &n);
   if (e == cudaSuccess && n < *max_clusters) *max_clusters = n;
   return e;
 }

@@ -1,5 +1,5 @@
-// Tile arithmetic of the resident kernel in FP32 mode for CTAs of one tile (128 rows) at most, for single evaluations and for calls of
-// one step: the forward product on the tensor core (split_mma.cuh), the backward pass by FFMA, every warp for itself (fp32_split.cuh).
+// Tile arithmetic of the resident kernel in FP32 mode for CTAs of one tile (128 rows) at most and for evaluations on host
+// pointers: the forward product on the tensor core (split_mma.cuh), the backward pass by FFMA, every warp for itself (fp32_split.cuh).
 // resident_fp32.cu has the rest, and the line between the two.  The rows' three parts stay in tensor memory for the launch, the rows
 // themselves in shared memory.
 // us a step on one B200: 1000 rows (one cluster of eight) 4.3, 148 windows of 128 rows 4.0, 4097 rows (five clusters) 5.5.  A chain of
@@ -261,10 +261,9 @@ struct ResFp32Ffma {
   }
 };
 
-cudaError_t launch_resident_fp32_ffma(bool one_tile, int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
+cudaError_t launch_resident_fp32_ffma(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                       int* max_clusters) {
-  return one_tile ? resident_launch_any<ResFp32Ffma<1>>(cluster, tmap, g, st, max_clusters)
-                  : resident_launch_any<ResFp32Ffma<RES_NWG>>(cluster, tmap, g, st, max_clusters);
+  return resident_launch_any<ResFp32Ffma<1>>(cluster, tmap, g, st, max_clusters);
 }
 
 cudaError_t launch_resident_eval_fp32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {

@@ -76,6 +76,28 @@ def test_fp32_chains_on_several_clusters_below_one_clusters_rows(built, monkeypa
     test_resident_launch_matches_oracle_and_per_step_launches(built, monkeypatch, 0, W, rows)
 
 
+@pytest.mark.parametrize("rows", [1025, 2049, 4096, 16500, 30000, 61440])
+def test_fp32_steps_and_evaluations_agree(built, rows):
+    """Steps go by integers, evaluations on host pointers by FFMA: the gradient that a step ends with is the evaluation's at its end, and three
+    steps are three times one, but for FP32 rounding, 1e-5 of the largest as against the oracle."""
+    m, _ = built
+    x, y, _ = m.synth_window(7, 0, rows)
+    ctx = m.Context(m.reference_config(precision=0, sample_capacity=0), 1, rows)
+    ctx.set_window_data(0, x, y)
+    rng = np.random.default_rng(rows)
+    w, mom = (0.15 * rng.standard_normal(P)).astype(np.float32), rng.standard_normal(P).astype(np.float32)
+    start = ctx.potential_and_grad(0, w)["grad"]
+    whole = ctx.leapfrog(0, 3, 1e-4, w, mom, start)
+    g = start
+    for _ in range(3):
+        s = ctx.leapfrog(0, 1, 1e-4, w, mom, g)
+        w, mom, g = s["w_next"], s["mom_next"], s["grad_cur"]
+        assert np.abs(g - ctx.potential_and_grad(0, w)["grad"]).max() <= 1e-5 * np.abs(g).max()
+    for k, v in (("w_next", w), ("grad_cur", g)):
+        assert np.abs(whole[k] - v).max() <= 1e-5 * np.abs(v).max()
+    ctx.close()
+
+
 @pytest.mark.parametrize("prec", [0, 1])
 def test_a_wait_that_runs_out_reports_and_leaves_the_chain_where_it_was(built, prec):
     """One cluster of the window is left out of a launch, so that the others' waits for its words run out: by themselves,
