@@ -12,11 +12,11 @@
 // its part of the tile for the segment's end, where it goes by FFMA.  Gradients' error against 64 bits, here / there, segments of 23 to 228
 // tiles: N(0,1) features 0.75 to 0.99, feature by feature 0.5 to 0.9; ten other distributions 0.83 in the mean (FFMA adds up to 1,600 rows
 // in a chain; the room takes most of what bits are to spare for short ones).
-// A tile takes 2,200 cycles of an SM (FFMA 2,700) and 1,400 instructions a warp, issue slots half busy, MUFU 24 %, tensor pipe 32 %.  What an
+// A tile takes 2,240 cycles of an SM (FFMA 2,640) and 1,330 instructions a warp, issue slots 59 % busy, MUFU 29 %, tensor pipe 40 %.  What an
 // instruction less gave was little; what a spill less gave was much, for shared memory leaves 28 KB of L1: hence the code for what is left over
-// in calls of few registers (47.3 us a step for 16 windows of 40013 rows; 49.0 with calls of many, 57 with their code in line).
+// in calls of few registers (16 windows of 40013 rows: 47.3 us a step before left-over rows read four weights a load, 48.0 since; 49.0 with calls of many, 57 with their code in line).
 // Such a tile takes 9 us at its segment's end, side by side on 16 warps.
-// us a step, FFMA and here: 16 x 40013 rows 57.9, 48.0; 25 x 58368 118, 101; 100 x 10000 87.0, 75.6; 6 x 58368 35.5, 31.0; with 22 lognormal
+// us a step, FFMA and here: 16 x 40013 rows 57.9, 48.0; 25 x 58368 118, 98.5; 100 x 10000 87.0, 74.8; 6 x 58368 35.5, 31.0; with 22 lognormal
 // features (sigma 1.5) 57.8, 58.2 and 35.5, 40.3 for the first and last, with Cauchy ones 112 and 159 here; targets with outliers of 300
 // sigma: the same as without.
 #include "fp32_split.cuh"
