@@ -240,8 +240,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
       const bool plain_w = __syncthreads_or(wide) != 0;  // S1
       if (lane < KP) {  // (every warp writes the same)
         const uint32_t st = *reinterpret_cast<volatile uint32_t*>(&x_stat[lane]), mx = *reinterpret_cast<volatile uint32_t*>(&x_max[lane]);
-        const int e = lane <= D && st ? min(int_scale_exp(st, 2 * FIN_ROOM_X), int_max_exp(mx) + FIN_ROOM_X) : 127;
-        x_scale[lane] = lane <= D ? int_scale_ok(e) ? int_scale(e) : __int_as_float(0x7f800000) : 0.f;  // (infinite: beyond any range)
+        x_scale[lane] = lane <= D ? int_scale(int_range_exp(min(int_scale_exp(st, 2 * FIN_ROOM_X), int_max_exp(mx) + FIN_ROOM_X))) : 0.f;
       }
       __syncwarp();
 
@@ -337,11 +336,10 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
               }
             }
             wait(&bar_scale, (sg - seg0) & 1, 105);
-            const int e = int_stat_exp(*reinterpret_cast<volatile uint32_t*>(&e_stat));
-            scale = int_scale_ok(e) ? int_scale(e) : 0.f;
+            scale = int_scale(int_stat_exp(*reinterpret_cast<volatile uint32_t*>(&e_stat)));
             scaled = true;
           }
-          const bool near = scale > 0.f && !x_far && !plain_w && __all_sync(0xffffffffu, fabsf(dy) * scale < INT_TOP);
+          const bool near = !x_far && !plain_w && __all_sync(0xffffffffu, fabsf(dy) * scale < INT_TOP);
           if (__builtin_expect(near, 1)) {
             lanes.store_ei(h, d, scale, es, dw1);
             fence_proxy_async_smem();
@@ -417,10 +415,9 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
         tc_fence_after();
         if ((warp & 3) < INT_LINES / 32) {
           const float xsc = x_scale[(warp & 3) * 8 + (lane >> 2)];
-          const int e = int_stat_exp(e_stat);
           float v[10];
           int_read_out_long<10>(tmem + wg * 40 + sub, v);
-          const float f = xsc > 0.f ? (float)(1 << 8 * (lane & 3)) / xsc : 0.f, inv = int_scale_ok(e) ? int_unscale(e) : 0.f;
+          const float f = xsc > 0.f ? (float)(1 << 8 * (lane & 3)) / xsc : 0.f, inv = int_unscale(int_stat_exp(e_stat));
 #pragma unroll
           for (int j = 0; j < 10; ++j)
             base[G::S + (wg * 10 + j) * INT_S_STR + (warp & 3) * 32 + lane] = none ? 0.f : v[j] * f * inv;

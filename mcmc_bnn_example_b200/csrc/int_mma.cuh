@@ -63,18 +63,19 @@ __device__ __forceinline__ uint32_t int_stat(float v) {
   return e - 1u < 254u ? e | 1u << 20 : 0u;
 }
 constexpr int INT_ROOM_X = 8, INT_ROOM_E = 5;   // (see above)
-// Biased exponent of the power of two that bounds the range: 2^room over the mean of the exponents
+// Biased exponent of the power of two that bounds the range: 2^room over the mean of the exponents.  INT_NONE: nothing is known of the
+// values, or scales and their products might leave the range of a float: then only zeros are in range, all else is an outlier (2^126 as a scale)
+constexpr int INT_NONE = 32;
 __device__ __forceinline__ int int_scale_exp(uint32_t stat, int room) {
   const float n = (float)(stat >> 20);
-  return n > 0.f ? (int)__fdividef((float)(stat & 0xfffffu) + 0.5f * n, n) + room : 127;
+  return n > 0.f ? (int)__fdividef((float)(stat & 0xfffffu) + 0.5f * n, n) + room : INT_NONE;
 }
 // the same for the largest magnitude, whose bits these are
 __device__ __forceinline__ int int_max_exp(uint32_t bits) { return (int)((bits + 0x30000u) >> 23) + 1; }
-// the smallest of several, as the largest of these words; 127 where there is none (0)
+__device__ __forceinline__ int int_range_exp(int e) { return e >= 87 && e <= 187 ? e : INT_NONE; }
+// the smallest of several, as the largest of these words; 0 where there is none
 __device__ __forceinline__ uint32_t int_stat_word(int e) { return 1024u - (uint32_t)e; }
-__device__ __forceinline__ int int_stat_exp(uint32_t word) { return word ? (int)(1024u - word) : 127; }
-// ... outside of which numbers, scales or their products may leave the range of a float
-__device__ __forceinline__ bool int_scale_ok(int e) { return e >= 87 && e <= 187; }
+__device__ __forceinline__ int int_stat_exp(uint32_t word) { return word ? int_range_exp((int)(1024u - word)) : INT_NONE; }
 __device__ __forceinline__ float int_scale(int e) { return __int_as_float((127 + 31 + 127 - e) << 23); }    // 2^31 / 2^(e - 127)
 __device__ __forceinline__ float int_unscale(int e) { return __int_as_float((e - 31) << 23); }              // its inverse
 

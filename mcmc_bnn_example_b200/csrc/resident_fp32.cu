@@ -199,13 +199,8 @@ struct ResFp32 {
       }
       __syncthreads();
       // features as integers: a scale each, from the CTA's rows
-      auto x_exp = [&](int k) {
-        return x_stat[k] ? min(int_scale_exp(x_stat[k], INT_ROOM_X), int_max_exp(x_max[k])) : 127;
-      };
-      if (tid < KP) {  // (infinite: beyond any range; the target has none)
-        const int e = tid <= D ? x_exp(tid) : 127;
-        x_scale[tid] = tid > D ? 0.f : int_scale_ok(e) ? int_scale(e) : __int_as_float(0x7f800000);
-      }
+      auto x_exp = [&](int k) { return int_range_exp(min(int_scale_exp(x_stat[k], INT_ROOM_X), int_max_exp(x_max[k]))); };
+      if (tid < KP) x_scale[tid] = tid > D ? 0.f : int_scale(x_exp(tid));  // (the target has none)
       __syncthreads();
       bool in = true;
 #pragma unroll
@@ -223,8 +218,7 @@ struct ResFp32 {
         else int_store_x4(smem_u32(xi) + int_x_off(lanes.lane, ch), x, reinterpret_cast<const float4*>(x_scale)[ch]);
       }
       const int k = (warp & 3) * 8 + (lanes.lane >> 2);  // the line whose sums this lane reads
-      const int e = k <= D ? x_exp(k) : 127;
-      own(1) = int_scale_ok(e) ? int_unscale(e + 8 * (lanes.lane & 3)) : 0.f;
+      own(1) = k <= D ? int_unscale(x_exp(k) + 8 * (lanes.lane & 3)) : 0.f;
       fence_proxy_async_smem();
     }
     plain_x = __syncthreads_or(wide) != 0;
@@ -356,16 +350,15 @@ struct ResFp32 {
         res_wait(bar_scale(), fph, g, limit, 614, ok);
       }
       const int se = int_stat_exp(*reinterpret_cast<volatile uint32_t*>(stat(first ? ph : ph ^ 1)));
-      const bool s_ok = int_scale_ok(se);
-      const float scale = s_ok ? int_scale(se) : 0.f;
-      near = s_ok && rows_are == INTS && __all_sync(0xffffffffu, fabsf(dy) * scale < INT_TOP);
+      const float scale = int_scale(se);
+      near = rows_are == INTS && __all_sync(0xffffffffu, fabsf(dy) * scale < INT_TOP);
       if (__builtin_expect(near, 1)) {
         lanes.store_ei(h, d, scale, es, dw1);
         fence_proxy_async_smem();
       } else {
         lanes.store_es(h, d, es, dw1);
       }
-      if (threadIdx.x == 0) sum_f() = s_ok ? int_unscale(se) : 1.f;
+      if (threadIdx.x == 0) sum_f() = int_unscale(se);
       if (lanes.lane == 0) far()[warp] = near ? 0u : 1u;
       __syncwarp();
       if (lanes.lane == 0) mbar_arrive(bar_e(wg));
