@@ -342,12 +342,12 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
           const bool near = !x_far && !plain_w && __all_sync(0xffffffffu, fabsf(dy) * scale < INT_TOP);
           if (__builtin_expect(near, 1)) {
             lanes.store_ei(h, d, scale, es, dw1);
-            fence_proxy_async_smem();
           } else {
             const int b = (n - pf) >> 2;  // (all of the tile is for later)
             if (lane == 0) far_tiles[warp][b >> 5] |= 1u << (b & 31);
             any_far = true;
           }
+          fence_proxy_async_smem();  // (also without an MMA: the next copy goes to where the rows' integers are)
           if (lane == 0) far[warp] = near ? 0u : 1u;
           hand_over(BAR_E0 + wg);
           if (near) {
