@@ -31,6 +31,7 @@ struct SplitWarp {
     rsub = lane >> 4;
   }
   __device__ __forceinline__ int own() const { return q + 8 * c; }  // the row whose dL/dpred this lane computes
+  __device__ __forceinline__ int owner() const { return 4 * (lane & 7) + (lane >> 3); }  // the lane that has row `lane`'s
 
   static __device__ __forceinline__ uint64_t lds64(const float* p) { return *reinterpret_cast<const uint64_t*>(p); }
 
@@ -169,14 +170,15 @@ struct SplitWarp {
     }
     __syncwarp();
   }
-  // the same as integers, d times `scale`, to the warp's INT_E_WARP bytes (int_mma.cuh)
+  // the same as integers, d times `scale`, to the warp's INT_E_WARP bytes (int_mma.cuh).  WITH_D false: without d's factor
+  template <bool WITH_D = true>
   __device__ __forceinline__ void store_ei(const uint64_t (&h)[4][5], const float (&d)[4], float scale, float* ei,
                                            uint64_t (&dw)[5]) const {
     const uint64_t minus1 = pack2(-1.f, -1.f);
     uint32_t* const dst = reinterpret_cast<uint32_t*>(ei) + (c >> 1) * 32 + q * 4 + (c & 1) * 2;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float nd = -d[i] * scale;
+      const float nd = WITH_D ? -d[i] * scale : -scale;
       const uint64_t d2 = pack2(d[i], d[i]), nd2 = pack2(nd, nd);
 #pragma unroll
       for (int n = 0; n < 5; ++n) {

@@ -7,18 +7,25 @@
 // integers, 32 rows per warp everywhere else); one control warp issues the product's MMAs, another those of the sums.  Tensor memory: the
 // sums, 160 columns for the whole CTA (integers: their order is of no consequence), and two places for a tile's rows and accumulators,
 // which the tiles take in turn: z is in a warpgroup's registers soon after it is there.
-// Features' scales come from the segment's first tiles, that of dL/dpred from its very first one, with room for what the other rows
-// may have: 2^6 above the largest feature, 2^11 above the mean exponent.  A warp whose 32 rows have a value beyond that, or infinities or NaN, leaves
-// its part of the tile for the segment's end, where it goes by FFMA.  Gradients' error against 64 bits, here / there, segments of 23 to 228
-// tiles: N(0,1) features 0.75 to 0.99, feature by feature 0.5 to 0.9; ten other distributions 0.83 in the mean (FFMA adds up to 1,600 rows
-// in a chain; the room takes most of what bits are to spare for short ones).
+// The integers are those of x dL/dpred, feature by feature, and of 1 - h^2, which needs no range: its step is 2^-30, where h alone leaves an error of 2^-24.
+// A feature's range is 2^12 over the mean exponent of its x dL/dpred, 2^7 over the largest at most, in the first tiles' rows; those are 32 of every
+// sixteenth of the segment (row_at), 16 of which are looked at.  So a feature's error is measured against its own terms: its step is 2^-19 of
+// a mean that they have in those rows, and smaller terms elsewhere cost no more than in a chain of FFMAs that has begun with them.  (x and
+// dL/dpred as two integers, the latter with one range for all: a feature that is only there where dL/dpred is a hundredth of what it was in
+// the segment's first tile was 8e-6 off, 1e-4 with a thousandth; FFMA 5e-7, here 1.4e-7 and 2e-7.)  A warp whose 32 rows have a product beyond its range,
+// infinities or NaN leaves them for the segment's end, where they go by FFMA.  A feature that is zero in all the rows looked at has
+// no range; should it be there later, the warp sees whether it is what 1 would be (unit_again).
+// Gradients' error against 64 bits, here / by FFMA, segments of 24, 64, 118 and 938 tiles: N(0,1) features 0.81, 0.59, 0.65, 0.58, the worst feature of 23
+// 0.93, 0.88, 0.96, 0.93; 16 other distributions and orders of rows 0.71 and 0.80 in the mean, none above 1.0 and 1.07 but for a late indicator's 1.27 over
+// 24 tiles (FFMA adds up to 1,600 rows in a chain; the room takes most of what bits are to spare for short ones; 2^13: 1.14 over 24 tiles).
 // A tile takes 2,240 cycles of an SM (FFMA 2,640) and 1,330 instructions a warp, issue slots 59 % busy, MUFU 29 %, tensor pipe 40 %.  What an
 // instruction less gave was little; what a spill less gave was much, for shared memory leaves 28 KB of L1: hence the code for what is left over
 // in calls of few registers (16 windows of 40013 rows: 47.3 us a step before left-over rows read four weights a load, 48.0 since; 49.0 with calls of many, 57 with their code in line).
-// Such a tile takes 9 us at its segment's end, side by side on 16 warps.
-// us a step, FFMA and here: 16 x 40013 rows 57.9, 48.0; 25 x 58368 118, 98.5; 100 x 10000 87.0, 74.8; 6 x 58368 35.5, 31.0; with 22 lognormal
-// features (sigma 1.5) 57.8, 58.2 and 35.5, 40.3 for the first and last, with Cauchy ones 112 and 159 here; targets with outliers of 300
-// sigma: the same as without.
+// The next tile's rows go to tensor memory before this one's products are made integers: its forward product goes on beside them (16 windows of 40013 rows
+// 52.7 us without).  Left-over rows take 9 us at their segment's end, side by side on 16 warps.
+// us a step, FFMA and here: 16 x 40013 rows 58.0, 48.5; 25 x 58368 118, 98.3; 100 x 10000 87.3, 74.2; 6 x 58368 35.7, 31.4; with 17 features of zeros (16 x 40013 and
+// 6 x 58368) 58.0, 51.8 and 35.7, 33.4; an indicator that begins late 58.1, 49.0 and 35.7, 33.2; one in a thousand rows 58.0, 63.5 and 35.7, 43.8; 22 lognormal features (sigma
+// 1.5) 58.1, 59.3 and 35.7, 41.7; Cauchy ones 58.1, 129 and 35.8, 91; 0.2 % targets with outliers of 300 sigma 58.1, 74 and 35.7, 46.
 #include "fp32_split.cuh"
 
 namespace mcmc_b200 {
@@ -28,20 +35,60 @@ constexpr int FIN_TILE = 128;
 constexpr int FIN_NWG = 4, FIN_THREADS = FIN_NWG * 128 + 128;
 // registers: 640 threads start with 96 each (4 * 128 * 112 + 128 * 32 = 61,440)
 constexpr int FIN_COMPUTE_REGS = 112, FIN_CTRL_REGS = 32;
-constexpr int FIN_SUB = 1000;                      // tiles of a segment between two read-outs: 2^17 rows' integers fit
-constexpr int FIN_ROOM_X = 6, FIN_ROOM_E = 11;      // above the first tiles' largest feature; above the mean exponent of dL/dpred
+constexpr int FIN_SUB = 1000;                      // tiles of a segment between two read-outs: 128,000 rows' products of bytes fit 31 bits
+constexpr int FIN_ROOM = 12, FIN_ROOM_MAX = 7;      // above the mean exponent of a feature x dL/dpred, above their largest
+constexpr float FIN_ONE = 1073741824.f;            // 1 - h^2 = 1 as an integer
+// a feature that is zero in all rows that ranges come from: as if it were 1, and its largest value among 32 rows has 22 bits at least
+constexpr int FIN_ROOM_NEW = 5;
+constexpr float FIN_LOW_NEW = 4194304.f;
+constexpr int FIN_MOST = 97;                       // ranges up to 2^97 and from 2^-77 on: sums and their factors are floats
 struct FinGeom {
   using Warp = SplitWarp;
   static constexpr int NW = FIN_NWG * 4;
   static constexpr int XS = Warp::ROWS * KP;           // floats of a warp's rows, and words of their integers
   static constexpr int WARP = 2 * XS + Warp::ES;       // two stages of rows, dL/dz
   static_assert(XS * 4 == INT_X_WARP && Warp::ES * 4 == INT_E_WARP && Warp::ES >= KP * SPLIT_H, "shared places");
-  static constexpr int WB = 0, ROWS0 = WB + SPLIT_B_BYTES / 4, S = ROWS0 + NW * WARP, W1 = S + INT_S_FLOATS, SCALE = W1 + SPLIT_H + 4;
-  static constexpr size_t SMEM = 1024 + (SCALE + KP) * 4;
-  static_assert(S % 4 == 0 && W1 % 4 == 0 && SCALE % 4 == 0, "vector alignment");
+  static constexpr int WB = 0, ROWS0 = WB + SPLIT_B_BYTES / 4, S = ROWS0 + NW * WARP, W1 = S + INT_S_FLOATS, SCALE = W1 + SPLIT_H + 4, UNIT = SCALE + KP, NEW = UNIT + KP;
+  static constexpr size_t SMEM = 1024 + (NEW + KP) * 4;
+  static_assert(S % 4 == 0 && W1 % 4 == 0 && SCALE % 4 == 0 && KP % 4 == 0, "vector alignment");
   static constexpr int PLACE = SPLIT_A_COLS + SPLIT_Z_COLS, PLACE0 = INT_ACC_COLS, TMEM_COLS = 512;
   static_assert(PLACE0 + 2 * PLACE <= TMEM_COLS, "tensor memory budget");
 };
+
+// A warp's 32 rows of which a product is beyond the range: floats at xb, times `dy` (of row `lane`).  Where all that is wrong is a feature whose range was not
+// known (scale and unit differ), they become integers all the same, if it is as large as they were taken to be or zero.  Returns whether.
+static __device__ __noinline__ bool unit_again(float* xb, float dy, const float* scale, const float* unit) {
+  const int lane = threadIdx.x & 31;
+  float v[KP];
+#pragma unroll
+  for (int ch = 0; ch < KP / 4; ++ch) {
+    float4 x = *reinterpret_cast<const float4*>(xb + lane * KP + 4 * ch);
+    if (ch == KP / 4 - 1) x.w = 0.f;
+    v[4 * ch] = x.x * dy;
+    v[4 * ch + 1] = x.y * dy;
+    v[4 * ch + 2] = x.z * dy;
+    v[4 * ch + 3] = x.w * dy;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int ch = 0; ch < KP / 4; ++ch)
+    *reinterpret_cast<float4*>(xb + lane * KP + 4 * ch) = make_float4(v[4 * ch], v[4 * ch + 1], v[4 * ch + 2], v[4 * ch + 3]);
+  __syncwarp();
+  bool in = true;
+  if (lane < KP) {
+    float top = 0.f;
+#pragma unroll 8
+    for (int r = 0; r < SplitWarp::ROWS; r += 2) top = split_max(top, xb[r * KP + lane], xb[(r + 1) * KP + lane]);
+    const float t = top * unit[lane];
+    in = t < INT_TOP && (scale[lane] == unit[lane] || top == 0.f || t >= FIN_LOW_NEW);
+  }
+  if (!__all_sync(0xffffffffu, in)) return false;
+#pragma unroll
+  for (int ch = 0; ch < KP / 4; ++ch)
+    int_store_x4(smem_u32(xb) + int_x_off(lane, ch), make_float4(v[4 * ch], v[4 * ch + 1], v[4 * ch + 2], v[4 * ch + 3]),
+                 reinterpret_cast<const float4*>(unit)[ch]);
+  return true;
+}
 
 template <bool LOSS>
 __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const GradParams g) {
@@ -55,9 +102,13 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
   float* const base = reinterpret_cast<float*>(wb);
   float* const w1 = base + G::W1;       // W1, b1
   float* const x_scale = base + G::SCALE;
+  // Features that are zero in the segment's first rows have no scale, and their values, should there be any, another unit; 2^126 in
+  // x_new, in which others have 0
+  float* const x_unit = base + G::UNIT;
+  float* const x_new = base + G::NEW;
   // rows of a warp landed; per place, product done and read; per warpgroup, sums done; the scale is known
   __shared__ __align__(8) uint64_t bar_rows[NW][2], bar_fwd[2], bar_read[2], bar_sum[NWG], bar_scale;
-  __shared__ uint32_t tmem_slot, x_stat[KP], x_max[KP], e_stat, none;
+  __shared__ uint32_t tmem_slot, x_stat[KP], x_max[KP], none;
   __shared__ uint32_t far[NW];                  // the warp's rows of its tile are not among the integers
   constexpr int FAR_WORDS = (FIN_SUB / NWG + 31) / 32;
   __shared__ uint32_t far_tiles[NW][FAR_WORDS], far_any[NW];   // ... earlier: which tiles of the part
@@ -76,11 +127,17 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
     const int S = gridDim.x, s = blockIdx.x;
     return make_int4(0, (int)((long long)s * g.n_tiles / S), (int)((long long)(s + 1) * g.n_tiles / S), s);
   };
-  // Tiles are numbered through a CTA's segments: tile n is warpgroup n % 4's, takes place n % 2 and the warp's stage n / 4 % 2
+  // Tiles are numbered through a CTA's segments: tile n is warpgroup n % 4's, takes place n % 2 and the warp's stage n / 4 % 2.  Which rows
+  // those are: a warp's tiles are a stretch of the segment, one after the other, so that the first tiles' rows, from which ranges
+  // come, are of all its parts
   float* const xs = base + G::ROWS0 + warp * G::WARP;
   float* const es = xs + 2 * G::XS;
-  auto rows_at = [&](const int4& seg, int i) {  // rows of this warp in tile i of a segment
-    return g.xaug + (long long)(g.data_window0 + seg.x) * g.window_stride + ((size_t)(seg.y + i) * FIN_TILE + (warp & 3) * Warp::ROWS) * KP;
+  auto row_at = [&](const int4& seg, int i) {  // the first row of this warp in tile i of a segment
+    const int len = (seg.z - seg.y) >> 2, more = (seg.z - seg.y) & 3, j = i & 3;
+    return seg.y * FIN_TILE + (4 * (j * len + min(j, more)) + (warp & 3) * (len + (j < more ? 1 : 0)) + (i >> 2)) * Warp::ROWS;
+  };
+  auto rows_at = [&](const int4& seg, int i) {
+    return g.xaug + (long long)(g.data_window0 + seg.x) * g.window_stride + (size_t)row_at(seg, i) * KP;
   };
   auto fetch = [&](int n, int sg, int n0) {  // tile n, in segment sg, whose first one is n0, or a later one
     int4 seg = segment(sg);
@@ -108,7 +165,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
       mbar_init(&bar_fwd[warp], 1);
       mbar_init(&bar_read[warp], 4);
     }
-    if (warp == 0) mbar_init(&bar_scale, 4);
+    if (warp == 0) mbar_init(&bar_scale, NW);
     mbar_fence_init();
   }
   __syncwarp();
@@ -120,7 +177,6 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
   for (int i = tid; i < SPLIT_B_BYTES / 16; i += FIN_THREADS)
     reinterpret_cast<float4*>(wb)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (tid < KP) x_stat[tid] = x_max[tid] = 0u;
-  if (tid == 0) e_stat = 0u;
   if (tid < NW * FAR_WORDS) far_tiles[tid / FAR_WORDS][tid % FAR_WORDS] = 0u;
   tc_fence_before();
   __syncthreads();
@@ -204,6 +260,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
       const int4 seg = segment(sg);
       const int win = seg.x, end = n0 + seg.z - seg.y;
       const int first = n0 + ((wg - n0) & 3);  // this warpgroup's first tile
+      const int row0 = row_at(seg, first - n0) + own;
       bool wide = false;
       {
         // fused leapfrog update; parameters land where the MMAs read them
@@ -222,31 +279,11 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
         }
         fence_proxy_async_smem();
       }
-      if (first < end) {  // features' statistics
-        wait(&bar_rows[warp][first >> 2 & 1], first >> 3 & 1, 101);
-        if (lane <= D) {  // (a lane a feature: reductions over the warp took 2,700 cycles)
-          const float* x = xs + (first >> 2 & 1) * G::XS + lane;
-          uint32_t st = 0u, mx = 0u;
-#pragma unroll 16
-          for (int r = 0; r < Warp::ROWS; ++r) {
-            const float v = x[r * KP];
-            st += int_stat(v);
-            mx = max(mx, __float_as_uint(v) & 0x7fffffffu);
-          }
-          atomicAdd(&x_stat[lane], st);
-          atomicMax(&x_max[lane], mx);
-        }
-      }
       const bool plain_w = __syncthreads_or(wide) != 0;  // S1
-      if (lane < KP) {  // (every warp writes the same)
-        const uint32_t st = *reinterpret_cast<volatile uint32_t*>(&x_stat[lane]), mx = *reinterpret_cast<volatile uint32_t*>(&x_max[lane]);
-        x_scale[lane] = lane <= D ? int_scale(int_range_exp(min(int_scale_exp(st, 2 * FIN_ROOM_X), int_max_exp(mx) + FIN_ROOM_X))) : 0.f;
-      }
-      __syncwarp();
 
-      bool plain = false, x_far = false;   // of the tile that comes next: rows for plain FFMA, a feature beyond its range
+      bool plain = false, some_new = false;   // of the tile that comes next: rows for plain FFMA; of the segment: features without a scale
       float y = 0.f;
-      // a tile's rows, once they have landed: to tensor memory, and integers in their own place
+      // a tile's rows to tensor memory, once they have landed
       auto stage_rows = [&](int n) {
         float* const xb = xs + (n >> 2 & 1) * G::XS;
         wait(&bar_rows[warp][n >> 2 & 1], n >> 3 & 1, 101);
@@ -270,35 +307,89 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
         tc_wait_st();
         tc_fence_before();
         hand_over(BAR_ROWS0 + wg);
+        float top = 0.f;
+#pragma unroll
+        for (int k = 0; k < KP; k += 2) top = split_max(top, v[k], v[k + 1]);
+        plain = __any_sync(0xffffffffu, split_wide(top)) != 0;
+      };
+      // Integers of the tile's rows times dL/dpred (of row `lane`) in the rows' place; false: one is beyond its range
+      auto products = [&](float* xb, float dy, bool known, bool first) __attribute__((always_inline)) {
+        uint64_t t[KP / 2];
+        const uint64_t dy2 = pack2(dy, dy);
+#pragma unroll
+        for (int ch = 0; ch < KP / 4; ++ch) {
+          const float4 v = *reinterpret_cast<const float4*>(xb + lane * KP + 4 * ch);
+          t[2 * ch] = mul2(pack2(v.x, v.y), dy2);
+          t[2 * ch + 1] = mul2(pack2(v.z, ch == KP / 4 - 1 ? 0.f : v.w), dy2);
+        }
         __syncwarp();  // every lane has read its row
+        if (__builtin_expect(first, 0)) {
+          // their ranges: from every second of all warps' first 32 rows, 256 in all (a lane a feature; all 512 rows: 0.4 us more)
+#pragma unroll
+          for (int k = 0; k < KP / 2; ++k) *reinterpret_cast<uint64_t*>(xb + lane * KP + 2 * k) = t[k];
+          __syncwarp();
+          if (lane <= D && known) {
+            uint32_t st = 0u, mx = 0u;
+#pragma unroll 16
+            for (int r = 0; r < Warp::ROWS; r += 2) {
+              const float p = xb[r * KP + lane];
+              st += int_stat(p);
+              mx = max(mx, __float_as_uint(p) & 0x7fffffffu);
+            }
+            atomicAdd(&x_stat[lane], st);
+            atomicMax(&x_max[lane], mx);
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar_scale);
+          wait(&bar_scale, (sg - seg0) & 1, 105);
+          if (lane < KP) {  // (every warp writes the same)
+            const volatile uint32_t *st = x_stat, *mx = x_max;
+            const bool is_new = lane < D && st[lane] == 0u;
+            const int e = is_new ? int_scale_exp(st[D], FIN_ROOM_NEW) : min(int_scale_exp(st[lane], FIN_ROOM), int_max_exp(mx[lane]) + FIN_ROOM_MAX);
+            const float u = int_scale(int_range_exp<FIN_MOST>(e));
+            x_scale[lane] = lane > D || is_new ? 0.f : u;
+            x_unit[lane] = lane > D ? 0.f : u;
+            x_new[lane] = is_new ? int_scale(INT_NONE) : 0.f;
+          }
+          __syncwarp();
+          some_new = __any_sync(0xffffffffu, lane < D && x_new[lane] > 0.f) != 0;
+        }
         float top = 0.f;
 #pragma unroll
         for (int ch = 0; ch < KP / 4; ++ch) {
           const float4 s = *reinterpret_cast<const float4*>(x_scale + 4 * ch);
-          const uint64_t a = pack2(v[4 * ch], v[4 * ch + 1]), b = pack2(v[4 * ch + 2], v[4 * ch + 3]);
-          const uint64_t sa = pack2(s.x, s.y), sb = pack2(s.z, s.w);
           float t0, t1;
-          unpack2(mul2(a, sa), t0, t1);
+          t[2 * ch] = mul2(t[2 * ch], pack2(s.x, s.y));
+          unpack2(t[2 * ch], t0, t1);
           top = split_max(top, t0, t1);
-          unpack2(mul2(b, sb), t0, t1);
+          t[2 * ch + 1] = mul2(t[2 * ch + 1], pack2(s.z, s.w));
+          unpack2(t[2 * ch + 1], t0, t1);
           top = split_max(top, t0, t1);
-          const uint2 da = int_digits2(a, sa), db = int_digits2(b, sb);
-          *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(xb) + int_x_off(lane, ch)) = make_uint4(da.x, da.y, db.x, db.y);
         }
-        x_far = !__all_sync(0xffffffffu, top < INT_TOP);
-        plain = false;
-        if (__builtin_expect(x_far, 0)) {  // (a value from 2^60 on is beyond any range)
-          top = 0.f;
+        if (some_new) {
+          float x = 0.f;
 #pragma unroll
-          for (int k = 0; k < KP; k += 2) top = split_max(top, v[k], v[k + 1]);
-          plain = __any_sync(0xffffffffu, split_wide(top)) != 0;
+          for (int ch = 0; ch < KP / 4; ++ch) {
+            const float4 v = *reinterpret_cast<const float4*>(xb + lane * KP + 4 * ch), f = *reinterpret_cast<const float4*>(x_new + 4 * ch);
+            x = split_max(x, v.x * f.x, v.y * f.y);
+            x = split_max(x, v.z * f.z, v.w * f.w);
+          }
+          if (!(x < 1.f)) top = INT_TOP;
+          __syncwarp();
         }
+        if (__builtin_expect(!__all_sync(0xffffffffu, top < INT_TOP), 0)) return unit_again(xb, first ? 1.f : dy, x_scale, x_unit);
+#pragma unroll
+        for (int ch = 0; ch < KP / 4; ++ch) {
+          const uint2 a = int_digits2(t[2 * ch]), b = int_digits2(t[2 * ch + 1]);
+          *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(xb) + int_x_off(lane, ch)) = make_uint4(a.x, a.y, b.x, b.y);
+        }
+        return true;
       };
       uint64_t dw1[5] = {};
-      float db1 = 0.f, scale = 0.f;
+      float db1 = 0.f;
       double llacc = 0.0;
-      bool scaled = false;
       if (first < end) stage_rows(first);
+      else if (lane == 0) mbar_arrive(&bar_scale);
 
       int p0 = n0;
       do {
@@ -323,34 +414,13 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
               fetch(n + NWG, sg, n0);
             }
           }
-          const int row = (seg.y + n - n0) * FIN_TILE + (warp & 3) * Warp::ROWS + own;
+          const int row = row0 + (n - first) * (Warp::ROWS / NWG);
           const bool valid = row < g.n_rows;
           float d[4], dy, pred;
           lanes.front(h, w1, g.lik, y, valid, d, dy, pred, [](int) {});
-          if (!scaled) {
-            if (n == n0) {
-              const uint32_t st = __reduce_add_sync(0xffffffffu, int_stat(dy));
-              if (lane == 0) {
-                if (st && !plain && !plain_w) atomicMax(&e_stat, int_stat_word(int_scale_exp(st, FIN_ROOM_E)));
-                mbar_arrive(&bar_scale);
-              }
-            }
-            wait(&bar_scale, (sg - seg0) & 1, 105);
-            scale = int_scale(int_stat_exp(*reinterpret_cast<volatile uint32_t*>(&e_stat)));
-            scaled = true;
-          }
-          const bool near = !x_far && !plain_w && __all_sync(0xffffffffu, fabsf(dy) * scale < INT_TOP);
-          if (__builtin_expect(near, 1)) {
-            lanes.store_ei(h, d, scale, es, dw1);
-          } else {
-            const int b = (n - pf) >> 2;  // (all of the tile is for later)
-            if (lane == 0) far_tiles[warp][b >> 5] |= 1u << (b & 31);
-            any_far = true;
-          }
-          fence_proxy_async_smem();  // (also without an MMA: the next copy goes to where the rows' integers are)
-          if (lane == 0) far[warp] = near ? 0u : 1u;
-          hand_over(BAR_E0 + wg);
-          if (near) {
+          const bool known = !plain && !plain_w;  // what the tensor core made of these rows is their z
+          if (__builtin_expect(known, 1)) {
+            lanes.template store_ei<false>(h, d, FIN_ONE, es, dw1);
             if (LOSS) {
               const float loss = valid ? lik_loss(g.lik, y, pred) : 0.f;
               llacc += (double)loss;
@@ -358,9 +428,18 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
             }
             db1 += dy;
           }
-          if (n + NWG < end) stage_rows(n + NWG);
+          if (n + NWG < end) stage_rows(n + NWG);  // (its product goes on beside what follows)
+          const bool near = products(xs + (n >> 2 & 1) * G::XS, __shfl_sync(0xffffffffu, dy, lanes.owner()), known, n == first) && known;
+          if (__builtin_expect(!near, 0)) {
+            const int b = (n - pf) >> 2;
+            if (lane == 0) far_tiles[warp][b >> 5] |= 1u << (b & 31);
+            any_far = true;
+          }
+          fence_proxy_async_smem();  // (also without an MMA: the next copy goes to where the rows' integers are)
+          if (lane == 0) far[warp] = near ? 0u : 1u;
+          hand_over(BAR_E0 + wg);
         }
-        // ---- rows that are not among the integers: by FFMA, their sums where dL/dz was ----
+        // ---- rows that are not among the integers: by FFMA, their sums where dL/dz was (and all else of them, if their z was not known) ----
         if (__builtin_expect(any_far, 0)) {
           const int last = pf + (p1 - 1 - pf) / NWG * NWG;
           wait(&bar_sum[wg], last >> 2 & 1, 104);
@@ -377,20 +456,28 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
             __syncwarp();
             uint64_t h[4][5];
             float d[4], dy, pred;
+            bool known = !plain_w;
+            for (int k = 0; k <= D; ++k) known &= !split_wide(xb[lane * KP + k]);
+            known = __all_sync(0xffffffffu, known) != 0;
             Warp::plain<2>(xb, wb, es);
             lanes.load_plain(es, h);
             __syncwarp();
-            const int row = (seg.y + n - n0) * FIN_TILE + (warp & 3) * Warp::ROWS + own;
+            const int row = row_at(seg, n - n0) + own;
             const bool valid = row < g.n_rows;
             const float yf = xb[own * KP + COL_Y];
             lanes.front(h, w1, g.lik, yf, valid, d, dy, pred, [](int) {});
-            lanes.store_es(h, d, es, dw1);
-            if (LOSS) {
-              const float loss = valid ? lik_loss(g.lik, yf, pred) : 0.f;
-              llacc += (double)loss;
-              store_row_loss(g.row_loss, (long long)win * g.row_loss_stride + row, loss, valid);
+            uint64_t dw[5] = {};
+            lanes.store_es(h, d, es, dw);
+            if (!known) {
+#pragma unroll
+              for (int i = 0; i < 5; ++i) dw1[i] = add2(dw1[i], dw[i]);
+              if (LOSS) {
+                const float loss = valid ? lik_loss(g.lik, yf, pred) : 0.f;
+                llacc += (double)loss;
+                store_row_loss(g.row_loss, (long long)win * g.row_loss_stride + row, loss, valid);
+              }
+              db1 += dy;
             }
-            db1 += dy;
             Warp::backward_lean<2>(xb, es, acc);
           }
           Warp::store_dw0_lean(acc, es + (lanes.kh * Warp::KPT + lanes.rsub * 6) * H);
@@ -414,10 +501,10 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
         __syncthreads();  // S2
         tc_fence_after();
         if ((warp & 3) < INT_LINES / 32) {
-          const float xsc = x_scale[(warp & 3) * 8 + (lane >> 2)];
+          const float unit = x_unit[(warp & 3) * 8 + (lane >> 2)];
           float v[10];
           int_read_out_long<10>(tmem + wg * 40 + sub, v);
-          const float f = xsc > 0.f ? (float)(1 << 8 * (lane & 3)) / xsc : 0.f, inv = int_unscale(int_stat_exp(e_stat));
+          const float f = (float)(1 << 8 * (lane & 3)) / FIN_ONE, inv = unit > 0.f ? 1.f / unit : 0.f;
 #pragma unroll
           for (int j = 0; j < 10; ++j)
             base[G::S + (wg * 10 + j) * INT_S_STR + (warp & 3) * 32 + lane] = none ? 0.f : v[j] * f * inv;
@@ -459,7 +546,6 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
         }
         if (p1 == end) {
           if (tid < KP) x_stat[tid] = x_max[tid] = 0u;
-          if (tid == 0) e_stat = 0u;
         }
         __syncthreads();  // S4: the next segment's parameters may take the place of this one's
         p0 += FIN_SUB;

@@ -2,14 +2,15 @@
 //
 // By FFMA it was half of a tile's instructions.  TF32 or bf16 parts, as the forward product has them (split_mma.cuh), are no way for it: the
 // tensor core cuts off every addition in the same direction, and over thousands of rows that adds up.  Its integer form adds exactly.
-//   * A feature becomes an integer of 32 bits, round(x 2^31 / X), X a power of two per feature; a dL/dz likewise with a power of
-//     two B for all of them.  Either is four signed bytes (adding 0x808080 and flipping the lower bytes' top bits makes the digits), which
+//   * One factor becomes an integer of 32 bits, round(x 2^31 / X), X a power of two per feature; the other likewise with a power of
+//     two B for all of them.  On the chip (resident_fp32.cu) they are the feature and dL/dz, streaming (grad_fp32_int.cu) the feature x dL/dpred
+//     and 1 - h^2.  Either is four signed bytes (adding 0x808080 and flipping the lower bytes' top bits makes the digits), which
 //     is how memory holds it: no byte has to be moved.
 //   * One tcgen05.mma kind::i8 multiplies all 4 x 4 bytes of 32 rows, a warp's: M = 96 lines (byte a of feature k is line 4 k + a;
 //     the instruction's other 32 read whatever follows, and nobody reads their sums), N = 160 columns (byte b of unit j is column 4 j + b).
-//     Sums stay below 2^31 for 2^17 rows; their order is of no consequence.
+//     Sums stay below 2^31 for 128,000 rows (127 x 128 x 128,000); their order is of no consequence.
 //   * Whoever reads them weighs them by 2^(8 a + 8 b) in FP32: the first rounding after those of the integers.
-// X is bounded by the rows' largest value, where that is less than 2^8 over the mean binary exponent (int_scale_exp); B is 2^5 over the mean
+// On the chip X is bounded by the rows' largest value, where that is less than 2^8 over the mean binary exponent (int_scale_exp); B is 2^5 over the mean
 // exponent of dL/dpred: a normal distribution ends at half of that, and what lies beyond is an outlier.  A warp that has one takes
 // FFMA, as infinities and NaN do.  So an integer of dL/dz is off by 2^-29 of their rms.  Gradients' error against 64 bits, here / by
 // FFMA: N(0,1) features 0.95 to 1.00 of it over 1000 to 58368 rows, feature by feature 0.86 to 0.98; t-distributed, lognormal, constant,
@@ -46,15 +47,21 @@ __device__ __forceinline__ void int_mma_if(uint32_t d_tmem, uint64_t adesc, uint
 // done by additions: high = x scale + INT_HI is that number in units of 512, INT_HI + INT_LO - high the rest's offset, and the low bits of
 // both floats are integers.  Their offsets go, and 0x808080 comes (digits from -128 on), in one addition.
 constexpr float INT_HI = 6442450944.f, INT_LO = 12582912.f;   // 1.5 x 2^32, 1.5 x 2^23
-__device__ __forceinline__ uint2 int_digits2(uint64_t x, uint64_t scale) {
-  const uint64_t hi = fma2(x, scale, pack2(INT_HI, INT_HI));
-  const uint64_t lo = fma2(x, scale, fma2(hi, pack2(-1.f, -1.f), pack2(INT_HI + INT_LO, INT_HI + INT_LO)));
+__device__ __forceinline__ uint2 int_digits2_of(uint64_t hi, uint64_t lo) {
   float h0, h1, l0, l1;
   unpack2(hi, h0, h1);
   unpack2(lo, l0, l1);
   constexpr uint32_t OFF = 0x808080u - (0x80000000u + 0x4b400000u);
   return make_uint2(((__float_as_uint(h0) << 9) + __float_as_uint(l0) + OFF) ^ 0x808080u,
                     ((__float_as_uint(h1) << 9) + __float_as_uint(l1) + OFF) ^ 0x808080u);
+}
+__device__ __forceinline__ uint2 int_digits2(uint64_t x, uint64_t scale) {
+  const uint64_t hi = fma2(x, scale, pack2(INT_HI, INT_HI));
+  return int_digits2_of(hi, fma2(x, scale, fma2(hi, pack2(-1.f, -1.f), pack2(INT_HI + INT_LO, INT_HI + INT_LO))));
+}
+__device__ __forceinline__ uint2 int_digits2(uint64_t x) {  // of values that have been scaled
+  const uint64_t hi = add2(x, pack2(INT_HI, INT_HI));
+  return int_digits2_of(hi, add2(x, fma2(hi, pack2(-1.f, -1.f), pack2(INT_HI + INT_LO, INT_HI + INT_LO))));
 }
 
 // Statistics behind a scale: a value's contribution; sums of them over at most 2^12 - 1 values
@@ -72,7 +79,8 @@ __device__ __forceinline__ int int_scale_exp(uint32_t stat, int room) {
 }
 // the same for the largest magnitude, whose bits these are
 __device__ __forceinline__ int int_max_exp(uint32_t bits) { return (int)((bits + 0x30000u) >> 23) + 1; }
-__device__ __forceinline__ int int_range_exp(int e) { return e >= 87 && e <= 187 ? e : INT_NONE; }
+template <int MOST = 60>
+__device__ __forceinline__ int int_range_exp(int e) { return e >= 147 - MOST && e <= 127 + MOST ? e : INT_NONE; }
 // the smallest of several, as the largest of these words; 0 where there is none
 __device__ __forceinline__ uint32_t int_stat_word(int e) { return 1024u - (uint32_t)e; }
 __device__ __forceinline__ int int_stat_exp(uint32_t word) { return word ? int_range_exp((int)(1024u - word)) : INT_NONE; }
