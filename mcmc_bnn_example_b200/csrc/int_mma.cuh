@@ -95,8 +95,9 @@ __device__ __forceinline__ void int_store_x4(uint32_t dst, float4 x, float4 scal
 }
 
 // Sums of NU units (columns 4 j, ... + 3 at `t`), line 32 q + lane of the accumulator with q the warp's quarter, times `f`.  Of at most 2^9
-// rows, so that the two upper bytes' fit an integer; what of the lowest one's is below the next one's unit is left out: 2^-38 of the largest
-// product
+// rows, so that the two upper bytes' fit an integer.  Of the two lower ones' 2 bits are cut off, 2^-36 of the largest product X B.  (Cut off at the
+// upper one's unit, 2^-30 of it and always downwards, they were as much as all other roundings of the integers, and more where a CTA has few rows
+// with a feature)
 template <int NU>
 __device__ __forceinline__ void int_read_out(uint32_t t, float f, float (&out)[NU]) {
   float a[4 * NU];
@@ -107,7 +108,7 @@ __device__ __forceinline__ void int_read_out(uint32_t t, float f, float (&out)[N
   for (int j = 0; j < NU; ++j) {
     const int v0 = __float_as_int(a[4 * j]), v1 = __float_as_int(a[4 * j + 1]), v2 = __float_as_int(a[4 * j + 2]),
               v3 = __float_as_int(a[4 * j + 3]);
-    out[j] = fmaf((float)(v3 * 256 + v2), 65536.f, (float)(v1 + (v0 >> 8)) * 256.f) * f;
+    out[j] = fmaf((float)(v3 * 256 + v2), 65536.f, (float)(v1 * 64 + (v0 >> 2)) * 4.f) * f;
   }
 }
 // ... of any number of rows, without the factor
