@@ -27,6 +27,8 @@ constexpr int INT_X_ROW = SPLIT_K * 4, INT_E_ROW = SPLIT_H * 4;          // byte
 constexpr int INT_X_WARP = 32 * INT_X_ROW, INT_E_WARP = 32 * INT_E_ROW;  // ... and of 32
 constexpr int INT_ACC_COLS = INT_E_ROW, INT_LINES = INT_X_ROW;
 constexpr float INT_TOP = 2126008811.f;      // 0.99 x 2^31: the bound of scaled values
+constexpr float INT_LOW = 1048576.f;         // 2^-6 of their mean exponent, which 0.5 % of normal ones are below: of 32 rows five once in a million
+constexpr int INT_FEW = 5;
 // sums of a unit's 96 lines side by side; four floats more keep readers of neighbouring units apart
 constexpr int INT_S_STR = INT_LINES + 4, INT_S_FLOATS = SPLIT_H * INT_S_STR;
 

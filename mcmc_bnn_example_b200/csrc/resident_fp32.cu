@@ -351,7 +351,9 @@ struct ResFp32 {
       }
       const int se = int_stat_exp(*reinterpret_cast<volatile uint32_t*>(stat(first ? ph : ph ^ 1)));
       const float scale = int_scale(se);
-      near = rows_are == INTS && __all_sync(0xffffffffu, fabsf(dy) * scale < INT_TOP);
+      // (A few rows whose dL/dpred is much smaller than the first tile's are no accident: FFMA has all their bits)
+      const float m = fabsf(dy) * scale;
+      near = rows_are == INTS && __all_sync(0xffffffffu, m < INT_TOP) && __popc(__ballot_sync(0xffffffffu, m < INT_LOW && m > 0.f)) < INT_FEW;
       if (__builtin_expect(near, 1)) {
         lanes.store_ei(h, d, scale, es, dw1);
         fence_proxy_async_smem();
