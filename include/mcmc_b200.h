@@ -436,7 +436,13 @@ int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* ctx, int code, int limit_us)
 /* The same for kernels whose limits are fixed (1.3 s): a launch in which one
  * wait more, for MMAs, runs out in every CTA.
  *   102  an evaluation by the FP32 kernel of 40 units that streams its rows
- *        with the product on the tensor core (mcmc_b200_plan_work_table_for)
+ *        with the product on the tensor core (mcmc_b200_plan_work_table_for),
+ *        behind its last tile
+ *   103, 104, 105  the same inside a segment, where its sums over rows go by
+ *        integers: in the warp that issues the product's MMAs, in the one that
+ *        issues the sums', in one that has rows.  The others' waits then run
+ *        out too, and any of their codes (101 to 107) may be the one reported.
+ *        Needs a window in chunks of 16 tiles and more.
  *   402  a prediction; needs sample storage
  */
 int mcmc_b200_selftest_kernel_wait(mcmc_b200_ctx* ctx, int code);

@@ -425,7 +425,7 @@ class Context:
         return code, lib().mcmc_b200_last_error().decode()
 
     def selftest_kernel_wait(self, code):
-        """Runs one wait more of a prediction (402) or a streaming FP32 evaluation (102) into its limit of 1.3 s."""
+        """Runs one wait more of a prediction (402) or a streaming FP32 evaluation (102 to 105) into its limit of 1.3 s."""
         code = lib().mcmc_b200_selftest_kernel_wait(self._h, int(code))
         return code, lib().mcmc_b200_last_error().decode()
 

@@ -1564,7 +1564,7 @@ static int explicit_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, c
                           float* w_last, float* m_last, float* g_out, float* row_loss, float* prior_loss, cudaStream_t st,
                           bool eval_only, bool data_fresh = false);
 API int mcmc_b200_selftest_kernel_wait(mcmc_b200_ctx* c, int code) {
-  if (!c || (code != 102 && code != 402)) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
+  if (!c || ((code < 102 || code > 105) && code != 402)) return fail(MCMC_B200_ERR_INVALID, "bad arguments");
   CK(cudaSetDevice(c->device));
   int r;
   if (code == 402) {
@@ -1576,6 +1576,7 @@ API int mcmc_b200_selftest_kernel_wait(mcmc_b200_ctx* c, int code) {
   } else {
     if (c->cfg.precision != MCMC_B200_PREC_FP32 || !c->table || !c->window_set[0])
       return fail(MCMC_B200_ERR_INVALID, "needs an FP32 context of 40 units with a work table, and data");
+    if (code != 102 && !c->xtab_ints) return fail(MCMC_B200_ERR_INVALID, "needs segments of 16 tiles in the mean");
     CK(cudaMemsetAsync(c->xw[0], 0, (size_t)c->P * 4, c->stream));
     c->test_code = code;
     r = explicit_steps(c, 0, 1, 0.f, c->xw[0], c->xm[0], c->xg, nullptr, nullptr, c->g_out, nullptr, nullptr, c->stream, true);

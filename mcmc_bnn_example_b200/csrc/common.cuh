@@ -74,7 +74,8 @@ struct GradParams {
   int* status;              // device error word (bounded waits that ran out)
   int data_fresh;           // 1: xaug was written by the launch directly before this one in the stream, so
                             // no row may be fetched ahead of the programmatic-dependency wait
-  int test_code;            // self-test: 102 adds a wait for MMAs that nothing ends (streaming FP32 kernels with the tensor core)
+  // self-test: 102 adds a wait for MMAs that nothing ends (streaming FP32 kernels with the tensor core), 103 to 105 one inside a segment (grad_fp32_int.cu)
+  int test_code;
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

@@ -55,6 +55,43 @@ struct FinGeom {
   static_assert(PLACE0 + 2 * PLACE <= TMEM_COLS, "tensor memory budget");
 };
 
+// A warp's first 32 rows (floats at xb), times `dy` (of row `lane`) in their place; their features' statistics, a lane a feature, if z was `known`
+static __device__ __noinline__ void unit_statistics(float* xb, float dy, bool known, uint32_t* x_stat, uint32_t* x_max) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int ch = 0; ch < KP / 4; ++ch) {
+    float4* const x = reinterpret_cast<float4*>(xb + lane * KP + 4 * ch);
+    *x = make_float4(x->x * dy, x->y * dy, x->z * dy, ch == KP / 4 - 1 ? 0.f : x->w * dy);
+  }
+  __syncwarp();
+  if (lane <= SPLIT_D && known) {
+    uint32_t st = 0u, mx = 0u;
+#pragma unroll 16
+    for (int r = 0; r < SplitWarp::ROWS; r += 2) {
+      const float p = xb[r * KP + lane];
+      st += int_stat(p);
+      mx = max(mx, __float_as_uint(p) & 0x7fffffffu);
+    }
+    atomicAdd(&x_stat[lane], st);
+    atomicMax(&x_max[lane], mx);
+  }
+  __syncwarp();
+}
+// ... of all warps: the ranges (every warp writes the same): three arrays of KP, scale, unit and new (FinGeom)
+static __device__ __noinline__ void unit_ranges(const volatile uint32_t* st, const volatile uint32_t* mx, float* scale) {
+  constexpr int D = SPLIT_D;
+  const int lane = threadIdx.x & 31;
+  if (lane < KP) {
+    const bool is_new = lane < D && st[lane] == 0u;
+    const int e = is_new ? int_scale_exp(st[D], FIN_ROOM_NEW) : min(int_scale_exp(st[lane], FIN_ROOM), int_max_exp(mx[lane]) + FIN_ROOM_MAX);
+    const float u = int_scale(int_range_exp<FIN_MOST>(e));
+    scale[lane] = lane > D || is_new ? 0.f : u;
+    scale[KP + lane] = lane > D ? 0.f : u;
+    scale[2 * KP + lane] = is_new ? int_scale(INT_NONE) : 0.f;
+  }
+  __syncwarp();
+}
+
 // A warp's 32 rows of which a product is beyond the range: floats at xb, times `dy` (of row `lane`).  Where all that is wrong is a feature whose range was not
 // known (scale and unit differ), they become integers all the same, if it is as large as they were taken to be or zero.  Returns whether.
 static __device__ __noinline__ bool unit_again(float* xb, float dy, const float* scale, const float* unit) {
@@ -106,9 +143,12 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
   // x_new, in which others have 0
   float* const x_unit = base + G::UNIT;
   float* const x_new = base + G::NEW;
-  // rows of a warp landed; per place, product done and read; per warpgroup, sums done; the scale is known
-  __shared__ __align__(8) uint64_t bar_rows[NW][2], bar_fwd[2], bar_read[2], bar_sum[NWG], bar_scale;
+  // rows of a warp landed; per place, product done and read; per warpgroup, rows in tensor memory, integers written, sums done; the scale is known.
+  // (No named barriers between the roles: they have no limit, and a warp that goes on behind a wait that ran out would arrive at one for its next
+  // tile before the control warp has come for this one; their counts lose step then, and somebody waits for good.  All waits here end.)
+  __shared__ __align__(8) uint64_t bar_rows[NW][2], bar_fwd[2], bar_read[2], bar_in[NWG], bar_e[NWG], bar_sum[NWG], bar_scale;
   __shared__ uint32_t tmem_slot, x_stat[KP], x_max[KP], none;
+  __shared__ int late;                          // code of a wait that ran out
   __shared__ uint32_t far[NW];                  // the warp's rows of its tile are not among the integers
   constexpr int FAR_WORDS = (FIN_SUB / NWG + 31) / 32;
   __shared__ uint32_t far_tiles[NW][FAR_WORDS], far_any[NW];   // ... earlier: which tiles of the part
@@ -160,7 +200,11 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
   if (!is_ctrl && lane == 0) {
     mbar_init(&bar_rows[warp][0], 1);
     mbar_init(&bar_rows[warp][1], 1);
-    if ((warp & 3) == 0) mbar_init(&bar_sum[wg], 1);
+    if ((warp & 3) == 0) {
+      mbar_init(&bar_in[wg], 4);
+      mbar_init(&bar_e[wg], 4);
+      mbar_init(&bar_sum[wg], 1);
+    }
     if (warp < 2) {
       mbar_init(&bar_fwd[warp], 1);
       mbar_init(&bar_read[warp], 4);
@@ -187,18 +231,28 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
   if (!early_rows && fetches) fetch(wg, seg0, 0);
 
   bool ok = true;
-  int code = 0;
   auto wait = [&](uint64_t* bar, uint32_t parity, int c) {  // (in line: a call would cost the tile loop registers)
     if (mbar_try_wait(bar, parity)) return;
     for (uint32_t i = 0; ok && !mbar_try_wait_hint(bar, parity, 20000u); ++i)
       if (i >= MBAR_WAIT_SLICES) {
         ok = false;
-        code = c;
+        late = c;
       }
   };
-  auto hand_over = [&](int id) {  // to a control warp; a warp whose waits hold it no longer does not get ahead of that one either
-    if (__all_sync(0xffffffffu, ok)) named_arrive(id, 160);
-    else named_sync(id, 160);
+  // ... of the control warps: tries without a time to sleep (with one, as above, they woke up late behind a segment's start: 200 windows of 4000 rows 71.1
+  // us a step, 66.8 so), for 1.3 s at 1.965 GHz
+  auto wait_c = [&](uint64_t* bar, uint32_t parity, int c) {
+    if (mbar_try_wait(bar, parity)) return;
+    const uint32_t t0 = (uint32_t)(clock64() >> 16);
+    while (ok && !mbar_try_wait(bar, parity))
+      if ((uint32_t)(clock64() >> 16) - t0 > 40000u) {
+        ok = false;
+        late = c;
+      }
+  };
+  auto hand_over = [&](uint64_t* bar) {  // to a control warp
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
   };
   auto place = [&](int n) { return G::PLACE0 + (n & 1) * G::PLACE; };
 
@@ -218,17 +272,21 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
         if (warp == NW) {
           // A warpgroup brings the next part's first tile before this part's end, the third and fourth behind the products of the first two
           for (; n < min(p1 + 2, end); ++n) {
-            if (n == rows) named_sync(BAR_ROWS0 + (rows++ & 3), 160);
-            if (n >= 2) wait(&bar_read[n & 1], (n - 2) >> 1 & 1, 103);
+            if (n == rows) {
+              wait_c(&bar_in[n & 3], n >> 2 & 1, 106);
+              ++rows;
+            }
+            if (n >= 2) wait_c(&bar_read[n & 1], (n - 2) >> 1 & 1, 103);
+            if (g.test_code == 103 && n == n0 + 2) wait_c(&bar_read[n & 1], n >> 1 & 1, 103);  // (nothing ends this phase before what follows)
             tc_fence_after();
             split_issue(tm + place(n) + SPLIT_A_COLS, tm + place(n), smem_u32(wb), on);
             tc_commit_if(&bar_fwd[n & 1], on);
           }
-          for (; rows < min(p1 + NWG, end); ++rows) named_sync(BAR_ROWS0 + (rows & 3), 160);
+          for (; rows < min(p1 + NWG, end); ++rows) wait_c(&bar_in[rows & 3], rows >> 2 & 1, 106);
         } else if (warp == NW + 1) {
           uint32_t more = 0u;
           for (int n = p0; n < p1; ++n) {
-            named_sync(BAR_E0 + (n & 3), 160);
+            wait_c(&bar_e[n & 3], n >> 2 & 1, 107);
             tc_fence_after();
             const uint32_t skip = __ballot_sync(0xffffffffu, lane < 4 && reinterpret_cast<volatile uint32_t*>(far)[(n & 3) * 4 + (lane & 3)] != 0u);
             const uint32_t w0 = smem_u32(base + G::ROWS0 + (n & 3) * 4 * G::WARP);
@@ -239,9 +297,10 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
                 int_mma_if(tm, umma_desc_advance(xd, i * (G::WARP * 4 >> 4)), umma_desc_advance(ed, i * (G::WARP * 4 >> 4)), more, on);
                 more = 1u;
               }
+            if (g.test_code == 104 && n == n0 + 1) wait_c(&bar_sum[n & 3], n >> 2 & 1, 104);  // (as above)
             tc_commit_if(&bar_sum[n & 3], on);
           }
-          if (p1 > p0) wait(&bar_sum[(p1 - 1) & 3], (p1 - 1) >> 2 & 1, 104);
+          if (p1 > p0) wait_c(&bar_sum[(p1 - 1) & 3], (p1 - 1) >> 2 & 1, 104);
           if (lane == 0) none = more ^ 1u;
         }
         __syncthreads();  // S2
@@ -251,7 +310,11 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
       } while (p0 < end);
       n0 = end;
     }
-    if (!ok) atomicExch(g.status, code);
+    if (!ok) {
+      atomicExch(g.status, late);
+      if (warp == NW + 1)  // (in line: no room for a call in so few registers)
+        for (uint32_t i = 0; i < MBAR_WAIT_SLICES && !mbar_try_wait_hint(&bar_sum[(n0 - 1) & 3], (n0 - 1) >> 2 & 1, 20000u); ++i) {}
+    }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FIN_COMPUTE_REGS));
     const uint32_t sub = (uint32_t)((warp & 3) * 32) << 16;
@@ -306,14 +369,14 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
         }
         tc_wait_st();
         tc_fence_before();
-        hand_over(BAR_ROWS0 + wg);
+        hand_over(&bar_in[wg]);
         float top = 0.f;
 #pragma unroll
         for (int k = 0; k < KP; k += 2) top = split_max(top, v[k], v[k + 1]);
         plain = __any_sync(0xffffffffu, split_wide(top)) != 0;
       };
       // Integers of the tile's rows times dL/dpred (of row `lane`) in the rows' place; false: one is beyond its range
-      auto products = [&](float* xb, float dy, bool known, bool first) __attribute__((always_inline)) {
+      auto products = [&](float* xb, float dy) __attribute__((always_inline)) {
         uint64_t t[KP / 2];
         const uint64_t dy2 = pack2(dy, dy);
 #pragma unroll
@@ -323,37 +386,6 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
           t[2 * ch + 1] = mul2(pack2(v.z, ch == KP / 4 - 1 ? 0.f : v.w), dy2);
         }
         __syncwarp();  // every lane has read its row
-        if (__builtin_expect(first, 0)) {
-          // their ranges: from every second of all warps' first 32 rows, 256 in all (a lane a feature; all 512 rows: 0.4 us more)
-#pragma unroll
-          for (int k = 0; k < KP / 2; ++k) *reinterpret_cast<uint64_t*>(xb + lane * KP + 2 * k) = t[k];
-          __syncwarp();
-          if (lane <= D && known) {
-            uint32_t st = 0u, mx = 0u;
-#pragma unroll 16
-            for (int r = 0; r < Warp::ROWS; r += 2) {
-              const float p = xb[r * KP + lane];
-              st += int_stat(p);
-              mx = max(mx, __float_as_uint(p) & 0x7fffffffu);
-            }
-            atomicAdd(&x_stat[lane], st);
-            atomicMax(&x_max[lane], mx);
-          }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bar_scale);
-          wait(&bar_scale, (sg - seg0) & 1, 105);
-          if (lane < KP) {  // (every warp writes the same)
-            const volatile uint32_t *st = x_stat, *mx = x_max;
-            const bool is_new = lane < D && st[lane] == 0u;
-            const int e = is_new ? int_scale_exp(st[D], FIN_ROOM_NEW) : min(int_scale_exp(st[lane], FIN_ROOM), int_max_exp(mx[lane]) + FIN_ROOM_MAX);
-            const float u = int_scale(int_range_exp<FIN_MOST>(e));
-            x_scale[lane] = lane > D || is_new ? 0.f : u;
-            x_unit[lane] = lane > D ? 0.f : u;
-            x_new[lane] = is_new ? int_scale(INT_NONE) : 0.f;
-          }
-          __syncwarp();
-          some_new = __any_sync(0xffffffffu, lane < D && x_new[lane] > 0.f) != 0;
-        }
         float top = 0.f;
 #pragma unroll
         for (int ch = 0; ch < KP / 4; ++ch) {
@@ -377,7 +409,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
           if (!(x < 1.f)) top = INT_TOP;
           __syncwarp();
         }
-        if (__builtin_expect(!__all_sync(0xffffffffu, top < INT_TOP), 0)) return unit_again(xb, first ? 1.f : dy, x_scale, x_unit);
+        if (__builtin_expect(!__all_sync(0xffffffffu, top < INT_TOP), 0)) return unit_again(xb, dy, x_scale, x_unit);
 #pragma unroll
         for (int ch = 0; ch < KP / 4; ++ch) {
           const uint2 a = int_digits2(t[2 * ch]), b = int_digits2(t[2 * ch + 1]);
@@ -429,7 +461,17 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
             db1 += dy;
           }
           if (n + NWG < end) stage_rows(n + NWG);  // (its product goes on beside what follows)
-          const bool near = products(xs + (n >> 2 & 1) * G::XS, __shfl_sync(0xffffffffu, dy, lanes.owner()), known, n == first) && known;
+          float dx = __shfl_sync(0xffffffffu, dy, lanes.owner());
+          if (__builtin_expect(n == first, 0)) {  // ranges: from every second of all warps' first 32 rows, 256 in all (all 512: 0.4 us more)
+            unit_statistics(xs + (n >> 2 & 1) * G::XS, dx, known, x_stat, x_max);
+            dx = 1.f;
+            if (lane == 0) mbar_arrive(&bar_scale);
+            wait(&bar_scale, (sg - seg0) & 1, 105);
+            if (g.test_code == 105 && warp == 5) wait(&bar_scale, (sg - seg0 + 1) & 1, 105);  // (the next segment's)
+            unit_ranges(x_stat, x_max, x_scale);
+            some_new = __any_sync(0xffffffffu, lane < D && x_new[lane] > 0.f) != 0;
+          }
+          const bool near = products(xs + (n >> 2 & 1) * G::XS, dx) && known;
           if (__builtin_expect(!near, 0)) {
             const int b = (n - pf) >> 2;
             if (lane == 0) far_tiles[warp][b >> 5] |= 1u << (b & 31);
@@ -437,7 +479,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
           }
           fence_proxy_async_smem();  // (also without an MMA: the next copy goes to where the rows' integers are)
           if (lane == 0) far[warp] = near ? 0u : 1u;
-          hand_over(BAR_E0 + wg);
+          hand_over(&bar_e[wg]);
         }
         // ---- rows that are not among the integers: by FFMA, their sums where dL/dz was (and all else of them, if their z was not known) ----
         if (__builtin_expect(any_far, 0)) {
@@ -554,7 +596,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
     }
     if (g.test_code == 102) wait(&bar_fwd[0], (n0 + 1) >> 1 & 1, 102);  // (nothing ends this phase)
     if (!ok) {  // copies and MMAs that did not arrive in time
-      atomicExch(g.status, code);
+      atomicExch(g.status, late);
       for (int n = max(n0 - 2 * NWG, 0); n < n0; ++n) {
         if ((n & 3) != wg) continue;
         mbar_drain(&bar_rows[warp][n >> 2 & 1], n >> 3 & 1);
