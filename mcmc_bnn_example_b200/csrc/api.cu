@@ -1525,12 +1525,16 @@ static bool resident_steps(mcmc_b200_ctx* c, int data_window, int L, float eps, 
 }
 
 API int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* c, int code, int limit_us) {
+  const bool steps = code >= 621 && code <= 624;
   if (!c || limit_us < 40 || limit_us > 10000 ||
-      (code != 603 && code != 611 && code != 901 && (c->cfg.precision != MCMC_B200_PREC_FP32 || (code != 612 && code != 613))))
+      (code != 603 && code != 611 && code != 901 &&
+       (c->cfg.precision != MCMC_B200_PREC_FP32 || (!steps && code != 612 && code != 613))))
     return fail(MCMC_B200_ERR_INVALID, "bad arguments");
   CK(cudaSetDevice(c->device));
   if (c->W != 1 || !c->window_set[0] || !use_resident(c, true, 1) || (code == 603 && c->res_x.clusters < 2))
     return fail(MCMC_B200_ERR_INVALID, "needs one window with data whose rows (603: more than 4096) fit on the chip");
+  if (steps && resident_one_tile((int)c->rows, c->res_x.clusters, c->res_x_cluster))
+    return fail(MCMC_B200_ERR_INVALID, "needs more than a tile of rows in a CTA");
   if (code == 901) {
     cudaError_t e = launch_wait_probe(c->status, (unsigned int)(limit_us / 20), c->stream);
     c->launches++;
@@ -1538,9 +1542,10 @@ API int mcmc_b200_selftest_resident_wait(mcmc_b200_ctx* c, int code, int limit_u
   }
   const std::vector<float> w(c->P, 0.f);
   if (code != 603) {
-    c->res_x.test_code = code;
+    c->res_x.test_code = steps ? code - 10 : code;
     c->res_x.wait_ticks = (unsigned int)limit_us / 33;
-    const int r = mcmc_b200_potential_and_grad(c, 0, w.data(), nullptr, nullptr, nullptr, nullptr);
+    const int r = steps ? mcmc_b200_leapfrog(c, 0, 3, 0.f, w.data(), w.data(), w.data(), nullptr, nullptr, nullptr, nullptr, nullptr)
+                        : mcmc_b200_potential_and_grad(c, 0, w.data(), nullptr, nullptr, nullptr, nullptr);
     c->res_x.test_code = 0;
     c->res_x.wait_ticks = RES_WAIT_TICKS;
     return r;

@@ -140,7 +140,7 @@ struct ResidentParams {
   int* status_host;         // optional: the same code for the host to read without a copy; also one that was set before
   unsigned int wait_ticks;  // limit of the waits, in 2^16 cycles
   int missing;              // self-test: clusters of the last window that do not start
-  int test_code;            // self-test: 611 adds a wait for rows that nothing ends, 612 and 613 (FP32) one for MMAs and for an accumulator
+  int test_code;            // self-test: 611 adds a wait for rows that nothing ends, FP32: 612, 613, 614 one for MMAs, for an accumulator, for sums
   // RES_STEPS / RES_EVAL (one window); all outputs but g_out and scalars are optional
   const float *w0, *m0, *g0;
   float eps_scalar;
@@ -160,6 +160,7 @@ cudaError_t launch_resident_tf32(int cluster, const void* tmap, const ResidentPa
 cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters);
 // ... in FP32 of windows whose CTAs have 128 rows at most
+bool resident_one_tile(int rows, int clusters, int cluster);
 cudaError_t launch_resident_fp32_ffma(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                       int* max_clusters);
 // ... of an evaluation with its parameters, for clusters of eight

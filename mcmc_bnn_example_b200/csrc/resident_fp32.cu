@@ -406,6 +406,7 @@ struct ResFp32 {
       }
       tc_commit_if(bar_sum(), on);
       res_wait(bar_sum(), ph, g, limit, 614, ok);
+      if (g.test_code == 614) res_wait(bar_sum(), ph ^ 1, g, limit, 614, ok);  // (nothing ends this phase)
     }
     // the CTA's sums, ten units a warp
     __syncthreads();
@@ -500,14 +501,14 @@ struct ResFp32 {
 // So do evaluations on host pointers, for which making integers of the rows and a scale, 1 to 2 us together, does not pay.  us a call, integers
 // and FFMA: 2048, 20000 and 58368 rows 37.0, 39.5, 42.4 and 35.3, 37.3, 41.0.  (Calls of one step: 30.3, 32.4, 35.4 and 29.0, 32.0, 35.5; of two
 // 33.4, 36.9, 41.7 and 37.6, 44.2, 49.8.)
-static bool one_tile(int rows, int clusters, int cluster) {
+bool resident_one_tile(int rows, int clusters, int cluster) {
   const int units = (rows + 31) / 32, ctas = clusters * cluster;
   return (units + ctas - 1) / ctas <= 4;
 }
 cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters) {
   if (!max_clusters)
-    return one_tile(g.n_rows, g.clusters, cluster) ? launch_resident_fp32_ffma(cluster, tmap, g, st, nullptr)
+    return resident_one_tile(g.n_rows, g.clusters, cluster) ? launch_resident_fp32_ffma(cluster, tmap, g, st, nullptr)
                                                    : resident_launch_any<ResFp32>(cluster, tmap, g, st, nullptr);
   int n = 0;
   cudaError_t e = resident_launch_any<ResFp32>(cluster, tmap, g, st, max_clusters);

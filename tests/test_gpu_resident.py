@@ -361,3 +361,25 @@ def test_two_contexts_at_once(built, prec):
     for c in both:
         assert np.array_equal(c.get_samples(0), want)
         c.close()
+
+
+@pytest.mark.parametrize("rows", [1025, 4096, 16500, 58368])
+@pytest.mark.parametrize("code", [621, 622, 623, 624])
+def test_steps_by_integers_report_waits_that_run_out(built, code, rows):
+    """The tile arithmetic of FP32 steps (evaluations have another): 611 to 614 in it."""
+    m, _ = built
+    x, y, _ = m.synth_window(8, 0, rows)
+    w = (0.1 * np.random.default_rng(2).standard_normal(P)).astype(np.float32)
+    ctx = m.Context(m.baseline_config(precision=m.PREC_FP32), 1, rows)
+    ctx.set_window_data(0, x, y)
+    before = ctx.leapfrog(0, 3, 1e-4, w, w, w)
+    got, msg = ctx.selftest_resident_wait(code)
+    assert got == 4 and str(code - 10) in msg, (got, msg)
+    ctx.synchronize()  # (reported once)
+    after = ctx.leapfrog(0, 3, 1e-4, w, w, w)
+    assert all(np.array_equal(before[k], after[k]) for k in ("w_next", "mom_next", "grad_cur", "loglik"))
+    ctx.close()
+    small = m.Context(m.baseline_config(precision=m.PREC_FP32), 1, 1024)
+    small.set_window_data(0, x[:1024], y[:1024])
+    assert small.selftest_resident_wait(code)[0] == 1   # (CTAs of one tile have the evaluations' arithmetic)
+    small.close()
