@@ -383,3 +383,46 @@ def test_steps_by_integers_report_waits_that_run_out(built, code, rows):
     small.set_window_data(0, x[:1024], y[:1024])
     assert small.selftest_resident_wait(code)[0] == 1   # (CTAs of one tile have the evaluations' arithmetic)
     small.close()
+
+
+@pytest.mark.parametrize("rows", [2000, 4096, 16500, 58368])
+def test_rows_that_leave_the_integers_in_every_trajectory(built, monkeypatch, rows):
+    """FP32 on the chip, targets with outliers, in the CTAs' first rows too: their rows become floats within a trajectory and integers again at the next
+    one's start, in launches of several.  Against one launch per step, as in the test of all launches."""
+    m, _ = built
+    x, y, _ = m.synth_window(8, 0, rows)
+    rng = np.random.default_rng(rows)
+    y = y.copy()
+    y[rng.random(rows) < 2e-3] += 500
+    y[3] -= 2000
+
+    def run():
+        ctx = m.Context(m.baseline_config(precision=m.PREC_FP32, leapfrog_steps=3, burn_in=0, adapt_steps=0, sample_capacity=6, trace_iters=6,
+                                          eps0=1e-5), 1, rows)
+        ctx.set_window_data(0, x, y)
+        ctx.run_chain(1)
+        ctx.run_chain(5)
+        out = ctx.get_samples(0), ctx.get_trace(0), ctx.get_state(0)
+        ctx.close()
+        return out
+
+    s1, t1, g1 = run()
+    monkeypatch.setenv("MCMC_B200_NO_MULTISTEP", "1")
+    s2, t2, g2 = run()
+    assert t1["accepted"].any() and np.array_equal(t1["accepted"], t2["accepted"])
+    assert np.abs(s1 - s2).max() <= 1e-5 * np.abs(s2).max()
+    assert np.abs(g1["grad"] - g2["grad"]).max() <= 1e-5 * np.abs(g2["grad"]).max()
+
+
+@pytest.mark.parametrize("rows", [16500, 58368])
+@pytest.mark.parametrize("eps0", [1e19, 1e30])
+def test_a_diverging_trajectory_by_integers_rejects_and_the_chain_stays(built, eps0, rows):
+    """As test_a_diverging_trajectory_rejects_and_the_chain_stays, with more than a tile in a CTA."""
+    m, _ = built
+    x, y, _ = m.synth_window(8, 0, rows)
+    ctx = m.Context(m.baseline_config(precision=m.PREC_FP32, leapfrog_steps=8, sample_capacity=4, trace_iters=4, eps0=eps0), 1, rows)
+    ctx.set_window_data(0, x, y)
+    ctx.run_chain(4)
+    assert not ctx.get_trace(0)["accepted"].any() and not ctx.get_samples(0).any()   # the chain's start, w = 0
+    assert np.abs(ctx.leapfrog(0, 1, 0.0, *[np.zeros(P, np.float32)] * 3)["grad_cur"] - ctx.get_state(0)["grad"]).max() <= 1e-5 * np.abs(ctx.get_state(0)["grad"]).max()
+    ctx.close()
