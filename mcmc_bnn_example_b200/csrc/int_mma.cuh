@@ -83,9 +83,10 @@ __device__ __forceinline__ int int_scale_exp(uint32_t stat, int room) {
 __device__ __forceinline__ int int_max_exp(uint32_t bits) { return (int)((bits + 0x30000u) >> 23) + 1; }
 template <int MOST = 60>
 __device__ __forceinline__ int int_range_exp(int e) { return e >= 147 - MOST && e <= 127 + MOST ? e : INT_NONE; }
-// the smallest of several, as the largest of these words; 0 where there is none
-__device__ __forceinline__ uint32_t int_stat_word(int e) { return 1024u - (uint32_t)e; }
-__device__ __forceinline__ int int_stat_exp(uint32_t word) { return word ? int_range_exp((int)(1024u - word)) : INT_NONE; }
+// the smallest of several, as the largest of these words; 0 where there is none.  (Kept within what int_range_exp allows: values for which that is
+// no range are out of it)
+__device__ __forceinline__ uint32_t int_stat_word(int e) { return 1024u - (uint32_t)min(max(e, 87), 187); }
+__device__ __forceinline__ int int_stat_exp(uint32_t word) { return word ? (int)(1024u - word) : INT_NONE; }
 __device__ __forceinline__ float int_scale(int e) { return __int_as_float((127 + 31 + 127 - e) << 23); }    // 2^31 / 2^(e - 127)
 __device__ __forceinline__ float int_unscale(int e) { return __int_as_float((e - 31) << 23); }              // its inverse
 

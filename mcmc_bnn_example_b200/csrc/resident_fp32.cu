@@ -120,12 +120,6 @@ struct ResFp32 {
     float* const x_scale = base + XS;
     bool ok = true;
     const int tid = threadIdx.x;
-    if (warp == 0) {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                   "r"((uint32_t)TMEM_COLS)
-                   : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
     if (tid == 0) {
       auto warps_of = [&](int w) { return min(max(n_units - 4 * w, 1), 4); };
       mbar_init(bar_rows(), 1);
@@ -137,6 +131,19 @@ struct ResFp32 {
       mbar_init(bar_sum(), 1);
       mbar_init(bar_scale(), warps_of(0));
       mbar_fence_init();
+      // (the rows come beside all that follows; nothing else is written where they land)
+      if (n_units > 0) {
+        const uint32_t bytes = (uint32_t)n_units * 32 * KP * 4;
+        mbar_expect_tx(bar_rows(), bytes);
+        bulk_g2s(base + ES, g.xaug + ((size_t)(g.data_window0 + win) * g.rows_pad + row0) * KP, bytes, bar_rows());
+      }
+    }
+    __syncwarp();
+    if (warp == 0) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                   "r"((uint32_t)TMEM_COLS)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid < KP) x_stat[tid] = x_max[tid] = 0u;
     if (tid < BAR - MISC) base[MISC + tid] = 0.f;
@@ -151,11 +158,6 @@ struct ResFp32 {
     tmem = tmem_slot;
     bool wide = false;
     if (n_units > 0) {
-      const uint32_t bytes = (uint32_t)n_units * 32 * KP * 4;
-      if (tid == 0) {
-        mbar_expect_tx(bar_rows(), bytes);
-        bulk_g2s(base + ES, g.xaug + ((size_t)(g.data_window0 + win) * g.rows_pad + row0) * KP, bytes, bar_rows());
-      }
       res_wait(bar_rows(), 0, g, g.wait_ticks << 2, 611, ok);
       if (!ok) res_drain(bar_rows(), 0, g);
       if (g.test_code == 611) res_wait(bar_rows(), 1, g, g.wait_ticks << 2, 611, ok);  // (nothing ends this phase)
@@ -353,7 +355,8 @@ struct ResFp32 {
       const float scale = int_scale(se);
       // (A few rows whose dL/dpred is much smaller than the first tile's are no accident: FFMA has all their bits)
       const float m = fabsf(dy) * scale;
-      near = rows_are == INTS && __all_sync(0xffffffffu, m < INT_TOP) && __popc(__ballot_sync(0xffffffffu, m < INT_LOW && m > 0.f)) < INT_FEW;
+      const uint32_t out = __ballot_sync(0xffffffffu, m != 0.f && !(m >= INT_LOW && m < INT_TOP));
+      near = rows_are == INTS && (out == 0u || (__popc(out) < INT_FEW && __all_sync(0xffffffffu, m < INT_TOP)));
       if (__builtin_expect(near, 1)) {
         lanes.store_ei(h, d, scale, es, dw1);
         fence_proxy_async_smem();
