@@ -161,6 +161,8 @@ cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentPa
                                  int* max_clusters);
 // ... in FP32 of windows whose CTAs have 128 rows at most
 bool resident_one_tile(int rows, int clusters, int cluster);
+// ... of one leapfrog step of a window, for clusters of eight
+cudaError_t launch_resident_step_fp32(const void* tmap, const ResidentParams& g, cudaStream_t st);
 cudaError_t launch_resident_fp32_ffma(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                       int* max_clusters);
 // ... of an evaluation with its parameters, for clusters of eight

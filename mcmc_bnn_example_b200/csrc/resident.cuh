@@ -648,10 +648,10 @@ static cudaError_t resident_launch_any(int cluster, const void* tmap, const Resi
   return cudaErrorInvalidValue;
 }
 
-template <class Tile, bool MULTI>
-static cudaError_t resident_launch_eval_m(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
+template <class Tile, bool MULTI, class Params>
+static cudaError_t resident_launch_single_m(const void* tmap, const Params& g, cudaStream_t st) {
   static bool attr_done[64] = {};
-  auto kernel = resident_kernel<Tile, 8, MULTI, ResidentEvalParams>;
+  auto kernel = resident_kernel<Tile, 8, MULTI, Params>;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !attr_done[dev]) {
@@ -661,9 +661,10 @@ static cudaError_t resident_launch_eval_m(const void* tmap, const ResidentEvalPa
   }
   return resident_launch(kernel, 8, Tile::SMEM, tmap, g, st, nullptr);
 }
-template <class Tile>
-static cudaError_t resident_launch_eval(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
-  return g.clusters > 1 ? resident_launch_eval_m<Tile, true>(tmap, g, st) : resident_launch_eval_m<Tile, false>(tmap, g, st);
+// ... of explicit calls, in clusters of eight: nobody has asked how many there can be
+template <class Tile, class Params>
+static cudaError_t resident_launch_single(const void* tmap, const Params& g, cudaStream_t st) {
+  return g.clusters > 1 ? resident_launch_single_m<Tile, true>(tmap, g, st) : resident_launch_single_m<Tile, false>(tmap, g, st);
 }
 
 }  // namespace mcmc_b200

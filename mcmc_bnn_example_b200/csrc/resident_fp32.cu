@@ -501,15 +501,18 @@ struct ResFp32 {
 // Windows whose CTAs have one tile at most take the tile arithmetic without integers (resident_fp32_ffma.cu): as fast there, and an outlier
 // costs it nothing.  us a step, integers and FFMA: 148 windows of 128 rows 4.43, 4.21; 1000 rows 4.54, 4.50; 4097 5.87, 5.87; with
 // targets that are outliers 1000 rows 6.0, 4.50.  More tiles: 4096 rows 6.8, 8.1; 16384 6.3, 7.1; 58368 8.2, 9.6; with outliers 9.3 to 10.0, 9.6.
-// So do evaluations on host pointers, for which making integers of the rows and a scale, 1 to 2 us together, does not pay.  us a call, integers
-// and FFMA: 2048, 20000 and 58368 rows 37.0, 39.5, 42.4 and 35.3, 37.3, 41.0.  (Calls of one step: 30.3, 32.4, 35.4 and 29.0, 32.0, 35.5; of two
-// 33.4, 36.9, 41.7 and 37.6, 44.2, 49.8.)
+// So do evaluations on host pointers and calls of one step, for which making integers of the rows and a scale, 1 to 2 us together, does not pay.
+// us a call alone, integers and FFMA: evaluations of 2048, 20000 and 58368 rows 37.0, 39.5, 42.4 and 35.3, 37.3, 41.0; us a call among others: one step
+// of 1500, 2048, 4096, 20000 and 58368 rows 17.1, 18.1, 20.9, 19.8, 23.0 and 15.8, 16.1, 18.9, 16.9, 20.9 (with FFMA for all calls of several tiles 16.8, 16.8,
+// 20.3, 18.8, 22.5).  Two steps of 2048, 20000 and 58368 rows, alone: 33.4, 36.9, 41.7 and 37.6, 44.2, 49.8.
 bool resident_one_tile(int rows, int clusters, int cluster) {
   const int units = (rows + 31) / 32, ctas = clusters * cluster;
   return (units + ctas - 1) / ctas <= 4;
 }
 cudaError_t launch_resident_fp32(int cluster, const void* tmap, const ResidentParams& g, cudaStream_t st,
                                  int* max_clusters) {
+  if (!max_clusters && cluster == 8 && g.mode == RES_STEPS && g.n_steps == 1 && !resident_one_tile(g.n_rows, g.clusters, cluster))
+    return launch_resident_step_fp32(tmap, g, st);
   if (!max_clusters)
     return resident_one_tile(g.n_rows, g.clusters, cluster) ? launch_resident_fp32_ffma(cluster, tmap, g, st, nullptr)
                                                    : resident_launch_any<ResFp32>(cluster, tmap, g, st, nullptr);

@@ -1,5 +1,5 @@
-// Tile arithmetic of the resident kernel in FP32 mode for CTAs of one tile (128 rows) at most and for evaluations on host
-// pointers: the forward product on the tensor core (split_mma.cuh), the backward pass by FFMA, every warp for itself (fp32_split.cuh).
+// Tile arithmetic of the resident kernel in FP32 mode for CTAs of one tile (128 rows) at most, for evaluations on host
+// pointers and for calls of one step: the forward product on the tensor core (split_mma.cuh), the backward pass by FFMA, every warp for itself (fp32_split.cuh).
 // resident_fp32.cu has the rest, and the line between the two.  The rows' three parts stay in tensor memory for the launch, the rows
 // themselves in shared memory.
 // us a step on one B200: 1000 rows (one cluster of eight) 4.3, 148 windows of 128 rows 4.0, 4097 rows (five clusters) 5.5.  A chain of
@@ -267,8 +267,11 @@ cudaError_t launch_resident_fp32_ffma(int cluster, const void* tmap, const Resid
 }
 
 cudaError_t launch_resident_eval_fp32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
-  return (g.n_rows + 31) / 32 <= 4 * 8 * g.clusters ? resident_launch_eval<ResFp32Ffma<1>>(tmap, g, st)
-                                                    : resident_launch_eval<ResFp32Ffma<RES_NWG>>(tmap, g, st);
+  return (g.n_rows + 31) / 32 <= 4 * 8 * g.clusters ? resident_launch_single<ResFp32Ffma<1>>(tmap, g, st)
+                                                    : resident_launch_single<ResFp32Ffma<RES_NWG>>(tmap, g, st);
+}
+cudaError_t launch_resident_step_fp32(const void* tmap, const ResidentParams& g, cudaStream_t st) {
+  return resident_launch_single<ResFp32Ffma<RES_NWG>>(tmap, g, st);
 }
 
 }  // namespace mcmc_b200

@@ -441,7 +441,7 @@ cudaError_t launch_resident_tf32(int cluster, const void* tmap, const ResidentPa
 }
 
 cudaError_t launch_resident_eval_tf32(const void* tmap, const ResidentEvalParams& g, cudaStream_t st) {
-  return resident_launch_eval<ResTf32>(tmap, g, st);
+  return resident_launch_single<ResTf32>(tmap, g, st);
 }
 
 }  // namespace mcmc_b200

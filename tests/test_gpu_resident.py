@@ -426,3 +426,34 @@ def test_a_diverging_trajectory_by_integers_rejects_and_the_chain_stays(built, e
     assert not ctx.get_trace(0)["accepted"].any() and not ctx.get_samples(0).any()   # the chain's start, w = 0
     assert np.abs(ctx.leapfrog(0, 1, 0.0, *[np.zeros(P, np.float32)] * 3)["grad_cur"] - ctx.get_state(0)["grad"]).max() <= 1e-5 * np.abs(ctx.get_state(0)["grad"]).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("rows", [1000, 1025, 4096, 16500, 58368])
+def test_a_calls_only_step_ends_with_the_evaluations_gradient(built, rows):
+    """FP32, calls of one step: the tile arithmetic of evaluations, whose bits hang on nothing but the position; captured in a graph before anything
+    else has run it, with row losses, in place."""
+    import torch
+    m, _ = built
+    ctx = m.Context(m.reference_config(precision=0, sample_capacity=0), 1, rows)
+    x, y, _ = m.synth_window(8, 0, rows)
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    p, out, keep = _step_args(m, torch, ctx, xd, yd, False)
+    s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        ctx.mcmc_step(*p, 1, 1e-3, stream=s.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    got = [v.cpu().numpy() for v in out]
+    ctx.set_window_data(0, x, y)
+    at = ctx.potential_and_grad(0, got[0], want_row_loss=True)
+    assert np.array_equal(got[2], at["grad"]) and np.array_equal(got[4][:rows], at["row_loss"])
+    del graph
+    p, out, keep = _step_args(m, torch, ctx, xd, yd, True)
+    ctx.mcmc_step(*p, 1, 1e-3)
+    ctx.synchronize()
+    for a, b in zip(got, out):
+        assert np.array_equal(a, b.cpu().numpy())
+    h = [v.cpu().numpy() for v in _step_args(m, torch, ctx, xd, yd, False)[2][:3]]
+    one = ctx.leapfrog(0, 1, 1e-3, *h)
+    assert np.array_equal(one["w_next"], got[0]) and np.array_equal(one["grad_cur"], got[2])
+    ctx.close()
