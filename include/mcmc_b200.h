@@ -126,6 +126,14 @@ int mcmc_b200_potential_and_grad(mcmc_b200_ctx* ctx, int window, const float* w,
  * (mcmc_step_ffma.h:395-427 / mcmc_step_tc.h:679-696).  First kick is a half
  * kick with grad_prev, the closing half kick is NOT applied (it belongs to the
  * accept ratio, kernel_helpers.h:163-175).  All vectors [P] host.
+ *
+ * The gradient of one step, and that of mcmc_b200_potential_and_grad, hangs on
+ * the position alone, to the last bit.  In a call of several steps (and in a
+ * chain's trajectories) an FP32 window on the chip whose CTAs have more than
+ * 128 rows takes a step's fixed-point range of dL/dpred from the step before:
+ * the same position reached another way may differ there in the last bits,
+ * a few 1e-7 of the gradient, so that three steps in one call are not bit for
+ * bit three calls of one.  The same call always gives the same bits.
  */
 int mcmc_b200_leapfrog(mcmc_b200_ctx* ctx, int window, int L, float eps, const float* w_prev,
                        const float* mom_prev, const float* grad_prev, float* w_next,
@@ -278,6 +286,7 @@ int mcmc_b200_selftest_oneshot_timeout(mcmc_b200_ctx* ctx, int polls);
  * loss_values[0..N) per-row log-likelihood and [N..N+P) per-parameter
  * log-prior.  Unlike the reference the caller's buffer roles are NOT rotated:
  * outputs always land in the buffers named here.  Queued on `stream`.
+ * (Of the last bits of several steps in one call see mcmc_b200_leapfrog.)
  * The context must have been created with n_windows = 1 and rows = N.
  */
 int mcmc_b200_mcmc_step(mcmc_b200_ctx* ctx, const float* x, const float* y, const float* weights_prev,

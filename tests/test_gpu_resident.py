@@ -428,6 +428,28 @@ def test_a_diverging_trajectory_by_integers_rejects_and_the_chain_stays(built, e
     ctx.close()
 
 
+@pytest.mark.parametrize("rows", [1025, 4096, 16500, 61440])
+def test_steps_of_one_call_are_those_of_several_calls_but_for_rounding(built, rows):
+    """FP32: a step's range comes from the step before it or, first in a call, from its own rows, or it goes by FFMA; whole calls have the same bits again.
+    Gradients by either are off by 2^-21 of their terms' root sum of squares at most (test_gpu_split.py), which is below the largest of a gradient's values here:
+    1e-6 of it for two of them."""
+    m, _ = built
+    x, y, _ = m.synth_window(7, 0, rows)
+    ctx = m.Context(m.reference_config(precision=0, sample_capacity=0), 1, rows)
+    ctx.set_window_data(0, x, y)
+    rng = np.random.default_rng(rows)
+    w, mom = (0.15 * rng.standard_normal(P)).astype(np.float32), rng.standard_normal(P).astype(np.float32)
+    start = ctx.potential_and_grad(0, w)["grad"]
+    whole, again = (ctx.leapfrog(0, 6, 1e-5, w, mom, start) for _ in range(2))
+    assert np.array_equal(whole["grad_cur"], again["grad_cur"]) and np.array_equal(whole["w_next"], again["w_next"])
+    for L in (1, 2, 3):
+        s = {"w_next": w, "mom_next": mom, "grad_cur": start}
+        for _ in range(6 // L):
+            s = ctx.leapfrog(0, L, 1e-5, s["w_next"], s["mom_next"], s["grad_cur"])
+        assert np.abs(s["grad_cur"] - whole["grad_cur"]).max() <= 1e-6 * np.abs(whole["grad_cur"]).max()
+    ctx.close()
+
+
 @pytest.mark.parametrize("rows", [1000, 1025, 4096, 16500, 58368])
 def test_a_calls_only_step_ends_with_the_evaluations_gradient(built, rows):
     """FP32, calls of one step: the tile arithmetic of evaluations, whose bits hang on nothing but the position; captured in a graph before anything
