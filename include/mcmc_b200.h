@@ -439,7 +439,7 @@ int mcmc_b200_selftest_wait_timeout(mcmc_b200_ctx* ctx, int limit_us);
  *   611  the load of the rows.  An evaluation (mcmc_b200_potential_and_grad).
  *   612, 613  FP32: MMAs, and an accumulator of theirs.  An evaluation.
  *   621 to 624  FP32 steps whose sums over rows go by integers: the load, the
- *        product's MMAs, its accumulator, the sums' MMAs (reported as 611 to
+ *        product's MMAs, its accumulator, the scale of dL/dpred (reported as 611 to
  *        614).  Three leapfrog steps (mcmc_b200_leapfrog); needs more than 128
  *        rows in each of the launch's CTAs.
  *   901  a wait of an earlier launch that nobody has asked about yet, before

@@ -140,7 +140,7 @@ struct ResidentParams {
   int* status_host;         // optional: the same code for the host to read without a copy; also one that was set before
   unsigned int wait_ticks;  // limit of the waits, in 2^16 cycles
   int missing;              // self-test: clusters of the last window that do not start
-  int test_code;            // self-test: 611 adds a wait for rows that nothing ends, FP32: 612, 613, 614 one for MMAs, for an accumulator, for sums
+  int test_code;            // self-test: 611 adds a wait for rows that nothing ends, FP32: 612, 613, 614 one for MMAs, for an accumulator, for a scale
   // RES_STEPS / RES_EVAL (one window); all outputs but g_out and scalars are optional
   const float *w0, *m0, *g0;
   float eps_scalar;

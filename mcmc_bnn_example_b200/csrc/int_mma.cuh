@@ -97,10 +97,11 @@ __device__ __forceinline__ void int_store_x4(uint32_t dst, float4 x, float4 scal
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(a.x), "r"(a.y), "r"(b.x), "r"(b.y) : "memory");
 }
 
-// Sums of NU units (columns 4 j, ... + 3 at `t`), line 32 q + lane of the accumulator with q the warp's quarter, times `f`.  Of at most 2^9
+// Sums of NU units (columns 4 j, ... + 3 at `t`), line 32 q + lane of the accumulator with q the warp's quarter, times `f` over 2^INT_READ_SHIFT.  Of at most 2^9
 // rows, so that the two upper bytes' fit an integer.  Of the two lower ones' 2 bits are cut off, 2^-36 of the largest product X B.  (Cut off at the
 // upper one's unit, 2^-30 of it and always downwards, they were as much as all other roundings of the integers, and more where a CTA has few rows
 // with a feature)
+constexpr int INT_READ_SHIFT = 2;
 template <int NU>
 __device__ __forceinline__ void int_read_out(uint32_t t, float f, float (&out)[NU]) {
   float a[4 * NU];
@@ -111,7 +112,7 @@ __device__ __forceinline__ void int_read_out(uint32_t t, float f, float (&out)[N
   for (int j = 0; j < NU; ++j) {
     const int v0 = __float_as_int(a[4 * j]), v1 = __float_as_int(a[4 * j + 1]), v2 = __float_as_int(a[4 * j + 2]),
               v3 = __float_as_int(a[4 * j + 3]);
-    out[j] = fmaf((float)(v3 * 256 + v2), 65536.f, (float)(v1 * 64 + (v0 >> 2)) * 4.f) * f;
+    out[j] = fmaf((float)(v3 * 256 + v2), 16384.f, (float)(v1 * 64 + (v0 >> 2))) * f;
   }
 }
 // ... of any number of rows, without the factor

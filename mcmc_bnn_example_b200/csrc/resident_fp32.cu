@@ -220,7 +220,7 @@ struct ResFp32 {
         else int_store_x4(smem_u32(xi) + int_x_off(lanes.lane, ch), x, reinterpret_cast<const float4*>(x_scale)[ch]);
       }
       const int k = (warp & 3) * 8 + (lanes.lane >> 2);  // the line whose sums this lane reads
-      own(1) = k <= D ? int_unscale(x_exp(k) + 8 * (lanes.lane & 3)) : 0.f;
+      own(1) = k <= D ? int_unscale(x_exp(k) + 8 * (lanes.lane & 3) + INT_READ_SHIFT) : 0.f;
       fence_proxy_async_smem();
     }
     plain_x = __syncthreads_or(wide) != 0;
@@ -374,6 +374,8 @@ struct ResFp32 {
       if (wg == 0 && !first) give_scale();
       if (__builtin_expect(last, 0)) {
         if (g.test_code == 612) res_wait(bar_fwd(wg), ph ^ 1, g, limit, 612, ok);  // (nothing ends this phase)
+        // (nor this one before the next trajectory.  In every step, behind the wait for sums, the question took 0.1 us)
+        if (g.test_code == 614) res_wait(bar_scale(), first_par, g, limit, 614, ok);
         const float loss = valid ? lik_loss(g.lik, own(0), pred) : 0.f;
         store_row_loss(row_loss, row0 + lanes.own(), loss, valid);
         double ld = (double)loss;
@@ -409,7 +411,6 @@ struct ResFp32 {
       }
       tc_commit_if(bar_sum(), on);
       res_wait(bar_sum(), ph, g, limit, 614, ok);
-      if (g.test_code == 614) res_wait(bar_sum(), ph ^ 1, g, limit, 614, ok);  // (nothing ends this phase)
     }
     // the CTA's sums, ten units a warp
     __syncthreads();
