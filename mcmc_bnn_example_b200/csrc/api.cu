@@ -565,7 +565,8 @@ static bool fp32_plain_faster(int windows, long long tiles, int num_sms, const W
 // 5 us instead of 3.  us a step, integers and FFMA, by tiles of a segment in the mean: 1 x 100000 rows (5) 18.5, 17.4; 200 x 2000 (9) 44.7, 43.4;
 // 4 x 58368 (12) 28.1, 26.9; 200 x 3000 (14) 57.6, 58.4; 60 x 8000 (18) 42.9, 44.1; 200 x 4000 (18) 69.5, 74.0; 6 x 58368 (18) 30.6, 34.8;
 // 149 x 5000 (20) 61.1, 68.2; 1 x 400000 (21) 34.9, 39.8; 16 x 40013 (31) 47.1, 57.1; 30 x 62000 (82) 122, 145
-// These are both kernels' times with the FFMA kernel's table; the other one gets its own afterwards (FP32_INT_SEG_COST: 60 x 8000 41.1).
+// These are both kernels' times, when the line was drawn, with the FFMA kernel's table; the other one gets its own afterwards (FP32_INT_SEG_COST: 60 x 8000
+// 41.4, 200 x 4000 66.9, 6 x 58368 31.1, 16 x 40013 46.8).
 static void plan_ints(int windows, long long tiles, int num_sms, int slices, WorkPlan& plan) {
   plan.ints = windows * tiles >= 16 * (long long)plan.segs.size();
   if (plan.ints) plan_work_table(windows, tiles, num_sms, slices, FP32_INT_SEG_COST, plan);

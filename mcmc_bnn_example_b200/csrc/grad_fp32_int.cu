@@ -12,20 +12,22 @@
 // sixteenth of the segment (row_at), 16 of which are looked at.  So a feature's error is measured against its own terms: its step is 2^-19 of
 // a mean that they have in those rows, and smaller terms elsewhere cost no more than in a chain of FFMAs that has begun with them.  (x and
 // dL/dpred as two integers, the latter with one range for all: a feature that is only there where dL/dpred is a hundredth of what it was in
-// the segment's first tile was 8e-6 off, 1e-4 with a thousandth; FFMA 5e-7, here 1.4e-7 and 2e-7.)  A warp whose 32 rows have a product beyond its range,
-// infinities or NaN leaves them for the segment's end, where they go by FFMA.  A feature that is zero in all the rows looked at has
-// no range; should it be there later, the warp sees whether it is what 1 would be (unit_again).
+// the segment's first tile was 8e-6 off, 1e-4 with a thousandth; FFMA 5e-7, here 1.4e-7 and 2e-7.)  A warp whose 32 rows have a product beyond its range
+// adds them up by FFMA on the spot, from the products and the integers of 1 - h^2 (unit_far: 1.3 us; left for the segment's end, with their forward
+// product once more, they took 9 us, side by side on 16 warps); rows of infinities, NaN and values from 2^60 on, whose z the tensor core does not
+// know, are left for the segment's end.  A feature that is zero in all the rows looked at has no range; should it be there later, the warp sees whether it
+// is what 1 would be (unit_again).
 // Gradients' error against 64 bits, here / by FFMA, segments of 24, 64, 118 and 938 tiles: N(0,1) features 0.81, 0.59, 0.65, 0.58, the worst feature of 23
-// 0.93, 0.88, 0.96, 0.93; 16 other distributions and orders of rows 0.71 and 0.80 in the mean, none above 1.0 and 1.07 but for a late indicator's 1.27 over
+// 0.93, 0.88, 0.96, 0.93; 16 other distributions and orders of rows 0.71 and 0.80 in the mean, none above 1.01 and 1.07 but for a late indicator's 1.27 over
 // 24 tiles (FFMA adds up to 1,600 rows in a chain; the room takes most of what bits are to spare for short ones; 2^13: 1.14 over 24 tiles).
-// A tile takes 2,240 cycles of an SM (FFMA 2,640) and 1,330 instructions a warp, issue slots 59 % busy, MUFU 29 %, tensor pipe 40 %.  What an
-// instruction less gave was little; what a spill less gave was much, for shared memory leaves 28 KB of L1: hence the code for what is left over
-// in calls of few registers (16 windows of 40013 rows: 47.3 us a step before left-over rows read four weights a load, 48.0 since; 49.0 with calls of many, 57 with their code in line).
-// The next tile's rows go to tensor memory before this one's products are made integers: its forward product goes on beside them (16 windows of 40013 rows
-// 52.7 us without).  Left-over rows take 9 us at their segment's end, side by side on 16 warps.
-// us a step, FFMA and here: 16 x 40013 rows 58.0, 48.5; 25 x 58368 118, 98.3; 100 x 10000 87.3, 74.2; 6 x 58368 35.7, 31.4; with 17 features of zeros (16 x 40013 and
-// 6 x 58368) 58.0, 51.8 and 35.7, 33.4; an indicator that begins late 58.1, 49.0 and 35.7, 33.2; one in a thousand rows 58.0, 63.5 and 35.7, 43.8; 22 lognormal features (sigma
-// 1.5) 58.1, 59.3 and 35.7, 41.7; Cauchy ones 58.1, 129 and 35.8, 91; 0.2 % targets with outliers of 300 sigma 58.1, 74 and 35.7, 46.
+// A tile takes 2,140 cycles of an SM (FFMA 2,640) and 1,320 instructions a warp, issue slots 62 % busy, MUFU 30 %, tensor pipe 42 %.  What an
+// instruction less gave was little; what a spill less gave was much, for shared memory leaves 28 KB of L1: hence functions of few registers for all that is
+// rare (FFMA's code in line: 57 us a step for 16 windows of 40013 rows; the first tiles' statistics in line, with 28 bytes spilled: 50.3).
+// The next tile's rows go to tensor memory before this one's products are made integers: its forward product goes on beside them (the same windows:
+// 52.7 us without).
+// us a step, FFMA and here: 16 x 40013 rows 57.9, 46.8; 25 x 58368 118, 96; 100 x 10000 87.1, 72.5; 6 x 58368 35.7, 31.1; 200 x 4000 75.4, 67.0; with 17 features of
+// zeros (16 x 40013 and 6 x 58368) 57.9, 51.1 and 35.7, 33.2; an indicator that begins late 58.0, 46.7 and 35.7, 33.0; one in a thousand rows 57.9, 56.6 and 35.7, 37.7; 22
+// lognormal features (sigma 1.5) 57.9, 51.8 and 35.7, 36.0; Cauchy ones 57.9, 88 and 35.7, 57.5; 0.2 % targets with outliers of 300 sigma 58.0, 66.4 and 35.7, 41.9.
 #include "fp32_split.cuh"
 
 namespace mcmc_b200 {
@@ -125,6 +127,26 @@ static __device__ __noinline__ bool unit_again(float* xb, float dy, const float*
     int_store_x4(smem_u32(xb) + int_x_off(lane, ch), make_float4(v[4 * ch], v[4 * ch + 1], v[4 * ch + 2], v[4 * ch + 3]),
                  reinterpret_cast<const float4*>(unit)[ch]);
   return true;
+}
+
+// The sums of such rows by FFMA, added to acc: their products with dL/dpred are floats at xb (unit_again), 1 - h^2 integers at es, which become floats
+static __device__ __noinline__ void unit_far(const float* xb, float* es, uint64_t* acc) {
+  const SplitWarp lanes;
+  const uint32_t* const src = reinterpret_cast<const uint32_t*>(es) + (lanes.c >> 1) * 32 + lanes.q * 4 + (lanes.c & 1) * 2;  // (store_ei)
+  uint2 e[4][5];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int n = 0; n < 5; ++n) e[i][n] = *reinterpret_cast<const uint2*>(src + i * (2 * INT_E_ROW) + n * 64);
+  __syncwarp();
+  auto value = [](uint32_t w) { return (float)(int)((w ^ 0x808080u) - 0x808080u) * (1.f / FIN_ONE); };  // (int_digits2)
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int n = 0; n < 5; ++n)
+      *reinterpret_cast<float2*>(es + (lanes.q + 8 * i) * SPLIT_H + 2 * lanes.c + 8 * n) = make_float2(value(e[i][n].x), value(e[i][n].y));
+  __syncwarp();
+  SplitWarp::backward_lean<2>(xb, es, acc);
 }
 
 template <bool LOSS>
@@ -427,6 +449,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
       do {
         const int p1 = min(p0 + FIN_SUB, end), pf = p0 + ((wg - p0) & 3);
         bool any_far = false;
+        uint64_t acc[Warp::LEAN];  // sums by FFMA, once there are any
 #pragma unroll 1
         for (int n = pf; n < p1; n += NWG) {
           wait(&bar_fwd[n & 1], n >> 1 & 1, 102);
@@ -473,21 +496,22 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
           }
           const bool near = products(xs + (n >> 2 & 1) * G::XS, dx) && known;
           if (__builtin_expect(!near, 0)) {
-            const int b = (n - pf) >> 2;
-            if (lane == 0) far_tiles[warp][b >> 5] |= 1u << (b & 31);
+            if (!any_far)
+              for (int i = 0; i < Warp::LEAN; ++i) acc[i] = 0ull;
             any_far = true;
+            const int b = (n - pf) >> 2;
+            if (known) unit_far(xs + (n >> 2 & 1) * G::XS, es, acc);
+            else if (lane == 0) far_tiles[warp][b >> 5] |= 1u << (b & 31);
           }
           fence_proxy_async_smem();  // (also without an MMA: the next copy goes to where the rows' integers are)
           if (lane == 0) far[warp] = near ? 0u : 1u;
           hand_over(&bar_e[wg]);
         }
-        // ---- rows that are not among the integers: by FFMA, their sums where dL/dz was (and all else of them, if their z was not known) ----
+        // ---- rows whose z the tensor core does not know: all of them by FFMA; the sums of what has gone that way to where dL/dz was ----
         if (__builtin_expect(any_far, 0)) {
           const int last = pf + (p1 - 1 - pf) / NWG * NWG;
           wait(&bar_sum[wg], last >> 2 & 1, 104);
           float* const xb = xs + (last >> 2 & 1) * G::XS;
-          uint64_t acc[Warp::LEAN];
-          for (int i = 0; i < Warp::LEAN; ++i) acc[i] = 0ull;
 #pragma unroll 1
           for (int n = pf; n < p1; n += NWG) {
             const int b = (n - pf) >> 2;
@@ -498,9 +522,6 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
             __syncwarp();
             uint64_t h[4][5];
             float d[4], dy, pred;
-            bool known = !plain_w;
-            for (int k = 0; k <= D; ++k) known &= !split_wide(xb[lane * KP + k]);
-            known = __all_sync(0xffffffffu, known) != 0;
             Warp::plain<2>(xb, wb, es);
             lanes.load_plain(es, h);
             __syncwarp();
@@ -508,18 +529,13 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
             const bool valid = row < g.n_rows;
             const float yf = xb[own * KP + COL_Y];
             lanes.front(h, w1, g.lik, yf, valid, d, dy, pred, [](int) {});
-            uint64_t dw[5] = {};
-            lanes.store_es(h, d, es, dw);
-            if (!known) {
-#pragma unroll
-              for (int i = 0; i < 5; ++i) dw1[i] = add2(dw1[i], dw[i]);
-              if (LOSS) {
-                const float loss = valid ? lik_loss(g.lik, yf, pred) : 0.f;
-                llacc += (double)loss;
-                store_row_loss(g.row_loss, (long long)win * g.row_loss_stride + row, loss, valid);
-              }
-              db1 += dy;
+            lanes.store_es(h, d, es, dw1);
+            if (LOSS) {
+              const float loss = valid ? lik_loss(g.lik, yf, pred) : 0.f;
+              llacc += (double)loss;
+              store_row_loss(g.row_loss, (long long)win * g.row_loss_stride + row, loss, valid);
             }
+            db1 += dy;
             Warp::backward_lean<2>(xb, es, acc);
           }
           Warp::store_dw0_lean(acc, es + (lanes.kh * Warp::KPT + lanes.rsub * 6) * H);

@@ -12,9 +12,10 @@
 //   * Whoever reads them weighs them by 2^(8 a + 8 b) in FP32: the first rounding after those of the integers.
 // On the chip X is bounded by the rows' largest value, where that is less than 2^8 over the mean binary exponent (int_scale_exp); B is 2^5 over the mean
 // exponent of dL/dpred: a normal distribution ends at half of that, and what lies beyond is an outlier.  A warp that has one takes
-// FFMA, as infinities and NaN do.  So an integer of dL/dz is off by 2^-29 of their rms.  Gradients' error against 64 bits, here / by
-// FFMA: N(0,1) features 0.95 to 1.00 of it over 1000 to 58368 rows, feature by feature 0.86 to 0.98; t-distributed, lognormal, constant,
-// zero-one and differently scaled features, targets with outliers 0.92 to 1.03, in the mean 0.98.  With 2^8 in the place of 2^5, and
+// FFMA, as infinities and NaN do.  So does one with INT_FEW rows far below the mean, of which integers would have fewer bits than a float: behind a first tile with residuals a
+// thousand times theirs, gradients of a feature that is only there were 1e-5 off (FFMA and now 1e-7).  So an integer of dL/dz is off by 2^-29 of their rms.
+// Gradients' error against 64 bits, on the chip / by FFMA: N(0,1) features 0.95 to 1.00 of it over 1000 to 58368 rows, feature by feature 0.86 to 0.98; t-distributed, lognormal, constant,
+// zero-one and differently scaled features, targets with outliers, ordered rows 0.8 to 1.02, in the mean 0.96.  (Streaming: grad_fp32_int.cu.)  With 2^8 in the place of 2^5, and
 // 30 bits instead of 31, it was 1.1 to 1.7 times as large for 100 rows.
 // Operands lie in shared memory without a swizzle, rows as K: groups of 8 rows, in them 16 bytes of a row (four values), row after row.
 // An MMA of 128 x 160 x 32 takes 81 cycles (one B200).

@@ -2,8 +2,8 @@
 // the tensor core, fp32_split.cuh what a warp does with its 32 rows behind it, int_mma.cuh the sums over rows on the integer tensor core): every
 // warp owns one 32-row unit for the whole launch, its rows in three parts in tensor memory and once more, as integers, in shared memory.
 // A CTA's sums come out of one accumulator, where the backward pass by FFMA left every warp 960 products of 32 rows (2,250 cycles)
-// and sixteen partial sums.  us a step, one B200, by FFMA and now: 4096 rows 8.1 and 6.75, 16384 7.1 and 6.3, 58368 9.6 and 8.2, 70 windows of
-// 800 rows 7.9 and 5.9.  CTAs of one tile stay with FFMA (resident_fp32_ffma.cu).
+// and sixteen partial sums.  us a step, one B200, by FFMA and now (trajectories of ten steps; on one cluster 4096 rows, eight windows): 8 x 4096 rows 8.4 and 7.0, 16384 7.5 and
+// 6.55, 58368 10.1 and 8.5, 70 windows of 800 rows 8.1 and 6.1.  CTAs of one tile stay with FFMA (resident_fp32_ffma.cu).
 // What bounds a step (clock reads, 58368 rows, 16,500 cycles): weights arrive and are cut up 0 - 350, first z 1,300, tanh and dL/dz of a
 // scheduler's four warps one after the other, 1,030 cycles each (MUFU 640), until 7,000; the last tile's sums 7,850, read out and
 // sent 9,500; then the exchange (resident.cuh), 7,000.
@@ -500,8 +500,8 @@ struct ResFp32 {
 };
 
 // Windows whose CTAs have one tile at most take the tile arithmetic without integers (resident_fp32_ffma.cu): as fast there, and an outlier
-// costs it nothing.  us a step, integers and FFMA: 148 windows of 128 rows 4.43, 4.21; 1000 rows 4.54, 4.50; 4097 5.87, 5.87; with
-// targets that are outliers 1000 rows 6.0, 4.50.  More tiles: 4096 rows 6.8, 8.1; 16384 6.3, 7.1; 58368 8.2, 9.6; with outliers 9.3 to 10.0, 9.6.
+// costs it nothing.  us a step, integers and FFMA (ten a trajectory): 148 windows of 128 rows 4.88, 4.15; 1000 rows 5.00, 4.52; 4097 6.10, 5.76; with
+// targets that are outliers 1000 rows 6.2, 4.51.  More tiles: 8 x 4096 rows 7.0, 8.4; 16384 6.55, 7.5; 58368 8.5, 10.1; with outliers, a hundred a trajectory, 9.6, 9.65.
 // So do evaluations on host pointers and calls of one step, for which making integers of the rows and a scale, 1 to 2 us together, does not pay.
 // us a call alone, integers and FFMA: evaluations of 2048, 20000 and 58368 rows 37.0, 39.5, 42.4 and 35.3, 37.3, 41.0; us a call among others: one step
 // of 1500, 2048, 4096, 20000 and 58368 rows 17.1, 18.1, 20.9, 19.8, 23.0 and 15.8, 16.1, 18.9, 16.9, 20.9 (with FFMA for all calls of several tiles 16.8, 16.8,

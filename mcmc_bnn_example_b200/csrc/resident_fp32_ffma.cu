@@ -2,7 +2,7 @@
 // pointers and for calls of one step: the forward product on the tensor core (split_mma.cuh), the backward pass by FFMA, every warp for itself (fp32_split.cuh).
 // resident_fp32.cu has the rest, and the line between the two.  The rows' three parts stay in tensor memory for the launch, the rows
 // themselves in shared memory.
-// us a step on one B200: 1000 rows (one cluster of eight) 4.3, 148 windows of 128 rows 4.0, 4097 rows (five clusters) 5.5.  A chain of
+// us a step on one B200 (ten a trajectory): 1000 rows (one cluster of eight) 4.5, 148 windows of 128 rows 4.15, 4097 rows (five clusters) 5.8.  A chain of
 // latencies: weights cut up, 24 MMAs, 40 tanh a row, 960 products of 32 rows a warp (2,250 cycles), exchange (resident.cuh).
 #include <cuda.h>
 #include "fp32_split.cuh"
