@@ -129,9 +129,20 @@ static __device__ __noinline__ bool unit_again(float* xb, float dy, const float*
   return true;
 }
 
-// The sums of such rows by FFMA, added to acc: their products with dL/dpred are floats at xb (unit_again), 1 - h^2 integers at es, which become floats
-static __device__ __noinline__ void unit_far(const float* xb, float* es, uint64_t* acc) {
+// The sums of such rows by FFMA, added to acc: their products with dL/dpred are floats at xb (unit_again), 1 - h^2 integers at es, which become floats.  Where
+// a product is no float, the rows are read once more, and dL/dpred (`dy` of row `lane`) goes to 1 - h^2, which may well be zero
+static __device__ __noinline__ void unit_far(float* xb, float* es, uint64_t* acc, const float* rows, float dy) {
   const SplitWarp lanes;
+  float top = 0.f;
+#pragma unroll
+  for (int ch = 0; ch < KP / 4; ++ch) {
+    const float4 p = *reinterpret_cast<const float4*>(xb + lanes.lane * KP + 4 * ch);
+    top = split_max(split_max(top, p.x, p.y), p.z, p.w);
+  }
+  const bool floats = __all_sync(0xffffffffu, top < __int_as_float(0x7f800000)) != 0;
+  if (!floats)
+    for (int i = lanes.lane; i < SplitWarp::ROWS * KP / 4; i += 32)
+      reinterpret_cast<float4*>(xb)[i] = reinterpret_cast<const float4*>(rows)[i];
   const uint32_t* const src = reinterpret_cast<const uint32_t*>(es) + (lanes.c >> 1) * 32 + lanes.q * 4 + (lanes.c & 1) * 2;  // (store_ei)
   uint2 e[4][5];
 #pragma unroll
@@ -141,10 +152,12 @@ static __device__ __noinline__ void unit_far(const float* xb, float* es, uint64_
   __syncwarp();
   auto value = [](uint32_t w) { return (float)(int)((w ^ 0x808080u) - 0x808080u) * (1.f / FIN_ONE); };  // (int_digits2)
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 4; ++i) {
+    const float f = __shfl_sync(0xffffffffu, floats ? 1.f : dy, lanes.q + 8 * i);
 #pragma unroll
     for (int n = 0; n < 5; ++n)
-      *reinterpret_cast<float2*>(es + (lanes.q + 8 * i) * SPLIT_H + 2 * lanes.c + 8 * n) = make_float2(value(e[i][n].x), value(e[i][n].y));
+      *reinterpret_cast<float2*>(es + (lanes.q + 8 * i) * SPLIT_H + 2 * lanes.c + 8 * n) = make_float2(f * value(e[i][n].x), f * value(e[i][n].y));
+  }
   __syncwarp();
   SplitWarp::backward_lean<2>(xb, es, acc);
 }
@@ -484,7 +497,8 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
             db1 += dy;
           }
           if (n + NWG < end) stage_rows(n + NWG);  // (its product goes on beside what follows)
-          float dx = __shfl_sync(0xffffffffu, dy, lanes.owner());
+          const float dy_row = __shfl_sync(0xffffffffu, dy, lanes.owner());
+          float dx = dy_row;
           if (__builtin_expect(n == first, 0)) {  // ranges: from every second of all warps' first 32 rows, 256 in all (all 512: 0.4 us more)
             unit_statistics(xs + (n >> 2 & 1) * G::XS, dx, known, x_stat, x_max);
             dx = 1.f;
@@ -500,7 +514,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 1) grad_fp32_int_kernel(const Gra
               for (int i = 0; i < Warp::LEAN; ++i) acc[i] = 0ull;
             any_far = true;
             const int b = (n - pf) >> 2;
-            if (known) unit_far(xs + (n >> 2 & 1) * G::XS, es, acc);
+            if (known) unit_far(xs + (n >> 2 & 1) * G::XS, es, acc, rows_at(seg, n - n0), dy_row);
             else if (lane == 0) far_tiles[warp][b >> 5] |= 1u << (b & 31);
           }
           fence_proxy_async_smem();  // (also without an MMA: the next copy goes to where the rows' integers are)
